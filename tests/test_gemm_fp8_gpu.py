@@ -48,3 +48,22 @@ def test_fp8_unit_scales_equal_plain_product():
     ones_a, ones_b = torch.ones(256, 2), torch.ones(2, 2)
     c = matmul_fp8_blockscaled(a8.to(DEV), ones_a.to(DEV), b8.to(DEV), ones_b.to(DEV)).float().cpu()
     assert torch.equal(c, (a @ b).bfloat16().float())      # small integers: every partial sum is exact
+
+
+# One shape per choice of the dispatch (tile of one CTA or of a pair, K in 1, 2, 4, 8 parts), each with a remainder in M
+# and, for the pairs, an N that ends in the middle of a 256-column tile.  The sums of the parts of K are added in fp32,
+# so the bound is the same as for one part: the bf16 rounding of the result.
+@pytest.mark.parametrize("m,n,k", [(1, 128, 128), (7, 128, 256), (64, 1024, 7168), (130, 512, 2048), (60, 2048, 1024), (33, 3968, 4096),
+                                   (129, 8192, 256), (520, 4224, 640), (1025, 8064, 128), (2049, 4224, 384)])
+@pytest.mark.parametrize("nk", [False, True])
+def test_fp8_tile_shapes_and_parts_of_k(m, n, k, nk):
+    g = torch.Generator(device=DEV).manual_seed(m + n + k)
+    a8, a_s = W.quantize_block_e4m3(torch.randn(m, k, generator=g, device=DEV), 1, 128)
+    b8, b_s = W.quantize_block_e4m3(torch.randn(k, n, generator=g, device=DEV), 128, 128)
+    b = b8.t().contiguous().t() if nk else b8
+    c = matmul_fp8_blockscaled(a8, a_s, b, b_s).double()
+    deq_a = a8.view(torch.float8_e4m3fn).double().view(m, k // 128, 128) * a_s.double()[..., None]
+    deq_b = b8.view(torch.float8_e4m3fn).double().view(k // 128, 128, n // 128, 128) * b_s.double()[:, None, :, None]
+    ref = deq_a.view(m, k) @ deq_b.view(k, n)
+    # 2^-8 of the value for the bf16 result, 2^-17 of the largest value for sums in fp32 in any order
+    assert ((c - ref).abs() <= 2 ** -8 * ref.abs() + 2 ** -17 * ref.abs().max()).all()

@@ -11,7 +11,7 @@
 
 namespace ftb {
 
-constexpr long long kWaitLimitCycles = 2000000000LL;   // about one second at B200 clocks
+constexpr uint32_t kWaitLimitCycles = 2000000000u;      // about one second at B200 clocks; below 2^32, so a 32-bit clock difference shows it
 constexpr uint32_t kWaitSleepNs = 20000;                // longest sleep of one try_wait inside a bounded wait
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -58,16 +58,17 @@ __device__ __forceinline__ bool mbar_try_wait_sleep(uint32_t bar, uint32_t parit
 // Bounded wait.  `abort_flag` lives in shared memory; once set every later wait returns at once.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   if (mbar_try_wait(bar, parity)) return true;
-  if (*abort_flag) return false;
-  const long long t0 = clock64();
-  while (!mbar_try_wait_sleep(bar, parity, kWaitSleepNs)) {
+  const uint32_t t0 = static_cast<uint32_t>(clock());
+  // one short loop: a role-split kernel holds dozens of copies of this wait, and its roles share an instruction cache
+#pragma unroll 1
+  for (;;) {
     if (*abort_flag) return false;
-    if (clock64() - t0 > kWaitLimitCycles) {
+    if (mbar_try_wait_sleep(bar, parity, kWaitSleepNs)) return true;
+    if (static_cast<uint32_t>(clock()) - t0 > kWaitLimitCycles) {
       *abort_flag = 1;
       return false;
     }
   }
-  return true;
 }
 
 // ---------------------------------------------------------------- cp.async (16-byte rows gather)

@@ -1,32 +1,33 @@
 // Top-k sparse MLA forward, persistent role-split CTA pairs (bf16 KV), one ring for K and Q.
 //
 // One pair of CTAs (a cluster of 2) walks through query tokens pair, pair + pairs, ...  CTA 0 computes
-// S = Q.K^T (Q in tensor memory, K column blocks from a ring in shared memory filled by TMA gather4) and the
+// S = Q.K^T (Q in tensor memory, K column blocks from a ring in shared memory filled by cp.async row gathers) and the
 // softmax; P travels to CTA 1 by bulk copies over distributed shared memory; CTA 1 accumulates O += P.V in
 // tensor memory and writes the output.  Every barrier keeps counting across tokens.
 //
-// The ring of CTA 0.  Eleven slots of [128 rows x 128 B] hold a stream of entries that the MMA issuer
-// consumes strictly in order: per token nine Q entries (the 64-column blocks of the token's query rows,
-// fetched by a TMA tile load and moved on to tensor memory by the issuer itself with tcgen05.cp, which runs
-// in order with its MMAs) and then nine K entries per tile of 128 selected rows (one 64-column block
-// each, fetched by one warp with a 32-lane gather4, multiplied by four MMAs).  Entry n lives in slot n % 11.
-// A tile needs nine slots, so two entries of look-ahead remain: a slot is refilled from the moment its
-// MMAs (or its copy to tensor memory) have completed, and the time that takes, about 5000 cycles in the kernel
-// with a nine-slot ring against 2300 cycles of MMAs per tile, is what bounds the tile period; each further slot
-// takes 256 cycles off it.  The room for the two slots comes from a single staging buffer for P.  The next
-// token's Q needs no special case: its entries follow the last tile's in the ring, its loads go out while
-// the last tile is still being multiplied (and the token after it is asked into L2), and no warp has to
-// carry Q from shared to tensor memory.
+// The ring of CTA 0.  Ten slots of [128 rows x 128 B] hold a stream of entries that the MMA issuer consumes strictly in
+// order: per token eight Q entries (64-column blocks of the token's query rows, fetched by a TMA tile load and moved
+// on to tensor memory by the issuer itself with tcgen05.cp, which runs in order with its MMAs) and then nine K entries per
+// tile of 128 selected rows (one 64-column block each, multiplied by four MMAs).  Entry n lives in slot n % 10; the commit
+// behind an entry frees its slot.  The ninth (rope) block of Q stays in a buffer of its own in shared memory and is
+// multiplied from there: that leaves 256 columns of tensor memory for two score buffers, so that the issuer starts the next
+// tile while the softmax fetches this one (the hand-over of a single buffer cost 550 cycles per tile).  The next token's
+// Q needs no special case: its entries follow the last tile's in the ring, and the token after it is asked into L2.
 //
-// Gather warps.  A warp hands the TMA unit one gather4 every 65 to 70 cycles, lane after lane (a 32-lane
-// instruction keeps it busy for 2240 cycles, 16 lanes for 1260), and warps that share a scheduler share its
-// dispatch of such operations (about one per 20 cycles per scheduler).  So every K entry belongs to two warps, 16
-// lanes and 64 rows each, eighteen gather warps in all, and they sit on the three schedulers that the MMA
-// issuer is not on (warp ids 9-31 except those that are 0 modulo 4): with four gather warps beside it the
-// issuer needed 420 instead of 265 cycles per block.
-// The kernel runs 32 warps per CTA; registers move from the gather warps to the softmax / correction warps
-// (setmaxnreg), and every group of warps runs its own copy of the batch loop so that its budget applies to its
-// own code only.
+// Gather warps.  One warp per column block of K (nine) and per half slab of V (eight) copies rows with 16-byte cp.async:
+// the lanes keep the tile's row numbers and pass them round with shuffles.  148 SMs fetch random rows at 70 bytes
+// per clock and SM this way, as fast as TMA row gathers do (both are bound by L2), but a gather4 from divergent lanes
+// occupies its scheduler for about 20 cycles and slowed the softmax and the issuer beside it.  The K warps sit on the
+// three schedulers that the MMA issuer is not on.  cp.async writes through the generic proxy, so the issuers fence
+// (fence.proxy.async) between the barrier wait and their MMAs.
+//
+// What bounds it: instruction supply, not memory or the tensor pipe (32 % busy).  Seventeen warps run ten different
+// roles, and a warp that has a scheduler's instruction cache to share runs 5 or more cycles per instruction; fully unrolled
+// role loops with a private copy of the wait loop each (95 KB of code) kept a third of all warps stalled on
+// instruction fetch.  So every role has one rolled loop, the softmax has one path (masked entries become -inf once) with
+// two-wide fp32 instructions, role state is warp-uniform, and the issuer waits for three entries at once (a wait with its
+// fences costs it 350 cycles, twelve MMAs take 768).  740 tokens, 128 heads, topk 2048: 832 -> 1065 TFLOP/s (one launch
+// alone); prefill of 4096 causal tokens, back to back under the power limit: 2247 -> 2036 us; one token: 58.8 -> 50.3 us.
 //
 // Softmax: two threads per head row; the running maximum moves only when it grows by more than 2^8, so that
 // the accumulator in CTA 1 is rarely rescaled.  P (bf16) and the rescale factors go to a staging area and
@@ -36,13 +37,10 @@
 // The number of tiles of a token (last non-negative index, rounded up to 128 rows, at least one) is
 // found for 64 tokens at a time by all warps of a CTA, with a CTA barrier on either side.
 //
-// Warps (1024 threads per CTA): CTA 0: 0-7 softmax, 8 MMA issuer, eighteen ring producers (producer 2c + hf: rows
-// 64 hf .. 64 hf + 63 of block c of every tile; hf = 0 also loads block c of Q).  CTA 1: 0-3 correction, 4 relay,
-// 8 MMA issuer, 9-16 V producers, 0-7 and 9-16 epilogue.
+// Warps (640 threads per CTA): CTA 0: 0-7 softmax, 8 MMA issuer, nine ring producers (the warps 9-19 whose id is not 0
+// modulo 4).  CTA 1: 0-3 correction, 4 relay, 8 MMA issuer, 9-16 V producers, 0-7 and 9-16 epilogue.
 // Every wait is bounded; a wait that runs out sets the abort flag, after which every later wait returns at
 // once and the status word reports a timeout.
-#include <type_traits>
-
 #include "sm100.cuh"
 #include "tmap.cuh"
 
@@ -57,7 +55,8 @@ constexpr int kDqk = 576;
 constexpr int kNChunk = 9;
 constexpr int kNT = 128;                       // gathered rows per tile
 constexpr int kQBlock = 128 * 128;             // 16384: [128 heads x 128 B]
-constexpr int kNK = 11;                        // ring slots of CTA 0: entry n (a Q block or a K block of a tile) lives in slot n % 11
+constexpr int kNQ = 8;                         // 64-column blocks of Q that live in tensor memory; the ninth (rope) stays in shared memory
+constexpr int kNK = 10;                        // ring slots of CTA 0: entry n (a Q block or a K block of a tile) lives in slot n % 10
 constexpr int kKSlot = kNT * 128;              // 16384: [128 rows x 128 B]
 constexpr int kNV = 4;                         // V ring slots: one whole tile, slab s in slot s
 constexpr int kVSlabRows = 32;
@@ -65,20 +64,23 @@ constexpr int kVBlock = kVSlabRows * 128;      // 4096: one 64-column block of a
 constexpr int kVSlab = 8 * kVBlock;            // 32768
 constexpr int kPBuf = 2 * kQBlock;             // 32768: P [128 heads x 128 rows] bf16 as two 64-row blocks
 constexpr int kBatch = 64;                     // tokens whose tile counts are found in one go
-// CTA 0 layout: ring of 11 slots | P staging | misc.
+// CTA 0 layout: ring of 10 slots | rope block of Q | P staging | misc.
 // CTA 1 layout: V ring | P x 2 | misc; between tokens the P buffer of the last tile stages O.
 constexpr int kOff0K = 0;
-constexpr int kOff0P = kOff0K + kNK * kKSlot;              // 180224
+constexpr int kOff0Q8 = kOff0K + kNK * kKSlot;             // 163840
+constexpr int kOff0P = kOff0Q8 + kQBlock;                  // 180224
 constexpr int kOff0Misc = kOff0P + kPBuf;                  // 212992
 constexpr int kOff1P = kNV * kVSlab;                       // 131072
 constexpr int kOff1Misc = kOff1P + 2 * kPBuf;              // 196608
 constexpr int kSmemBytes = kOff0Misc + 4096 + 1024;        // the larger of the two + misc + alignment slack
-constexpr int kThreads = 1024;
+constexpr int kThreads = 640;                  // 20 warps
 constexpr int kWarps = kThreads / 32;
-constexpr uint32_t kColQ = 0;                  // TMEM columns of CTA 0: Q (288), then S
-constexpr uint32_t kColS = 320;
+constexpr uint32_t kColQ = 0;                  // TMEM columns of CTA 0: Q (256), then two score buffers of 128
+constexpr uint32_t kColS = 256;
 
 struct Params {
+  const __nv_bfloat16* kv;
+  long long kv_sr;
   const int32_t* indices;
   float* lse;
   int s_q, h, s_kv, topk;
@@ -89,10 +91,12 @@ struct Params {
 };
 
 struct Misc0 {   // CTA 0
-  unsigned long long k_full[kNK];   // two arrivals, one per gather warp of the entry, each announcing its bytes (8 KB of gathers; the tile load of a Q entry counts on the first)
+  unsigned long long k_full[kNK];   // one arrival per gather thread (when its copies have landed; the tile load of a Q entry counts on one of them)
   unsigned long long k_free[kNK];   // tcgen05.commit behind the entry's MMAs or its copy to tensor memory
-  unsigned long long s_full;        // tcgen05.commit
-  unsigned long long s_free;        // 8 softmax warps
+  unsigned long long s_full[2];     // tcgen05.commit
+  unsigned long long s_free[2];     // 8 softmax warps
+  unsigned long long q8_full;       // the token's rope block of Q has landed
+  unsigned long long q8_free;       // tcgen05.commit behind the token's last tile
   unsigned long long p_free[2];     // relay warp of CTA 1 (remote arrival)
   unsigned long long stage_free;    // correction warp 0 of CTA 1 (remote arrival): P and the factors of the tile have landed there
   unsigned long long epi_done[2];   // CTA 1 (remote arrival): the epilogue of token t (t % 2) is over
@@ -100,13 +104,13 @@ struct Misc0 {   // CTA 0
   int abort_flag;
   int bad_index;
   int pad;
-  uint32_t valid_mask[4][4];        // per tile (mod 4): 128 validity bits
+  alignas(16) uint32_t valid_mask[8][4];  // per tile (mod 8): 128 validity bits
   unsigned short nt[kBatch];        // tiles per token of the current batch
   float xchg[2][256];               // row maximum / row sum exchange between the two threads of a head row
   alignas(16) float alpha_stage[128]; // rescale factors of a tile on their way to CTA 1 (sent with P)
 };
 struct Misc1 {   // CTA 1
-  unsigned long long v_full[kNV];   // one arrival announcing 32 KB of gathers
+  unsigned long long v_full[kNV];   // one arrival per gather thread, when its copies have landed
   unsigned long long v_free[kNV];   // tcgen05.commit
   unsigned long long p_full[2];     // 8 softmax warps of CTA 0 (remote arrivals, each announcing its bulk copies: 4 KB of P, 128 B of factors)
   unsigned long long corr_done[2];  // 4 correction warps
@@ -127,15 +131,10 @@ static_assert(kOff1Misc + 4096 + 1024 <= kSmemBytes, "CTA 1 layout fits");
 static_assert(kNV == kNT / kVSlabRows, "V ring slot index = slab index");
 static_assert(kNK > kNChunk && kNK < 2 * kNChunk, "a ring position advances by one tile with a single wrap test");
 
+// the same value in every lane, made visible to the compiler: loop counts and role state then stay in uniform registers
+__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-// Four rows (indices r0..r3) x 64 columns starting at column `col` -> 512 contiguous bytes of shared memory.
-__device__ __forceinline__ void tma_gather4(uint32_t dst, const void* tmap, uint32_t bar, int col, int r0, int r1, int r2, int r3) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-      ::"r"(dst), "l"(tmap), "r"(bar), "r"(col), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
-      : "memory");
 }
 __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
@@ -160,6 +159,23 @@ __device__ __forceinline__ void tmem_cp_128x256b(uint32_t taddr, uint32_t desc_l
       ::"r"(taddr), "r"(desc_lo), "r"(desc_hi)
       : "memory");
 }
+// two fp32 lanes per instruction
+__device__ __forceinline__ float2 ffma2(float a0, float a1, float2 b, float2 c) {
+  float2 r;
+  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
+      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a0), "f"(a1), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+__device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
+      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+      "add.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
 // position of a role in the stream of ring entries: slot = n % kNK, use = n / kNK
 struct RingPos {
   uint32_t slot, use;
@@ -182,13 +198,14 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
-sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant__ CUtensorMap tm_q,
+sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
                          const __grid_constant__ CUtensorMap tm_o, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (base - raw_addr);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = warp_uniform(tid >> 5);
   const int cta = static_cast<int>(cluster_ctarank());
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   Misc0* m0 = reinterpret_cast<Misc0*>(sm + kOff0Misc);
@@ -202,13 +219,14 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
     *abort_flag = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
     if (cta == 0) {
       m0->bad_index = 0;
-      for (int i = 0; i < kNK; ++i) { mbar_init(smem_u32(&m0->k_full[i]), 2); mbar_init(smem_u32(&m0->k_free[i]), 1); }
-      mbar_init(smem_u32(&m0->s_full), 1);
-      mbar_init(smem_u32(&m0->s_free), 8);
+      for (int i = 0; i < kNK; ++i) { mbar_init(smem_u32(&m0->k_full[i]), 32); mbar_init(smem_u32(&m0->k_free[i]), 1); }
+      for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&m0->s_full[i]), 1); mbar_init(smem_u32(&m0->s_free[i]), 8); }
+      mbar_init(smem_u32(&m0->q8_full), 1);
+      mbar_init(smem_u32(&m0->q8_free), 1);
       for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&m0->p_free[i]), 1); mbar_init(smem_u32(&m0->epi_done[i]), 1); }
       mbar_init(smem_u32(&m0->stage_free), 1);
     } else {
-      for (int i = 0; i < kNV; ++i) { mbar_init(smem_u32(&m1->v_full[i]), 1); mbar_init(smem_u32(&m1->v_free[i]), 1); }
+      for (int i = 0; i < kNV; ++i) { mbar_init(smem_u32(&m1->v_full[i]), 64); mbar_init(smem_u32(&m1->v_free[i]), 1); }
       for (int i = 0; i < 2; ++i) {
         mbar_init(smem_u32(&m1->p_full[i]), 8);
         mbar_init(smem_u32(&m1->corr_done[i]), 4);
@@ -239,7 +257,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
   if (cta == 0 && p.h < 128) {
     // a Q entry only writes h rows of its slot; the rows below feed head rows that are never stored, but they
     // should hold numbers
-    for (int x = tid; x < kNK * kKSlot / 16; x += kThreads)
+    for (int x = tid; x < (kNK * kKSlot + kQBlock) / 16; x += kThreads)
       asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(base + x * 16), "r"(0) : "memory");
     fence_proxy_async_smem();
   }
@@ -255,18 +273,13 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
   // tokens of this pair: pair, pair + n_pairs, ...  (the host launches no more pairs than tokens)
   const int my_tokens = (p.s_q - pair + n_pairs - 1) / n_pairs;
   uint32_t gt = 0;   // tiles processed before the current token: every role counts the same way
-  // CTA 0: index of this warp among the eighteen ring producers (-1 = not one): the warps 9-31 whose id is not 0
-  // modulo 4, in order (they share no scheduler with the MMA issuer, warp 8).
+  // CTA 0: the nine gather warps, one per column block: the warps 9-19 whose id is not 0 modulo 4, in order (they share no
+  // scheduler with the MMA issuer, warp 8)
   const int prod = (warp >= 9 && (warp & 3) != 0) ? (warp - 9) - ((warp - 8) >> 2) : -1;
   RingPos pos;       // CTA 0, issuer and producers: position in the stream of ring entries
-  pos.slot = (cta == 0 && prod >= 0) ? static_cast<uint32_t>(prod >> 1) : 0u;
+  pos.slot = (cta == 0 && prod >= 0) ? static_cast<uint32_t>(prod) : 0u;
   pos.use = 0;
 
-  // The body of the kernel as a function of the warp group it is compiled for (0: warps 0-7, 1: warps 8-19,
-  // 2: warps 20-31): every group runs the same batch loop, but each copy only holds its own roles, so that the
-  // register budget set for the group applies to exactly the code that the group executes.
-  auto run = [&](auto group_tag) {
-  constexpr int GRP = decltype(group_tag)::value;
   for (int batch0 = 0; batch0 < my_tokens; batch0 += kBatch) {
     const int nb = min(kBatch, my_tokens - batch0);
     // ------------------------------------------------------------------ tiles per token of this batch
@@ -287,7 +300,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
     if (cta == 0) {
       // ===================================================================== CTA 0: scores
       const uint32_t k_s = base + kOff0K;
-      if constexpr (GRP == 0) {
+      if (warp < 8) {
         // -------------------------------------------------------------- softmax (two threads per head row)
         // thread tid: head row = tid % 128 (TMEM lane), columns 64*(tid/128) .. +63 of the tile
         const int rowi = tid & 127;
@@ -302,39 +315,40 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
         for (int t = 0; t < nb; ++t) {
           const int ti = batch0 + t;
           const int tok = pair + ti * n_pairs;
-          const int n_tiles = nt[t];
+          const int n_tiles = warp_uniform(nt[t]);
           // 1/l and the `fin` barrier of parity ti % 2 were last used by token ti - 2: its epilogue is over
           if (ti >= 2) mbar_wait(smem_u32(&m0->epi_done[ti & 1]), ((ti >> 1) - 1) & 1u, abort_flag);
           float m_run = -INFINITY, l_run = 0.0f;
           for (int i = 0; i < n_tiles; ++i) {
             const uint32_t G = gt + i;
             const int b = G & 1;
-            mbar_wait(smem_u32(&m0->s_full), G & 1u, abort_flag);
+            mbar_wait(smem_u32(&m0->s_full[b]), (G >> 1) & 1u, abort_flag);
             tc_fence_after();
-            const uint32_t vmA = m0->valid_mask[G & 3][2 * ch], vmB = m0->valid_mask[G & 3][2 * ch + 1];
-            const bool all_valid = (m0->valid_mask[G & 3][0] & m0->valid_mask[G & 3][1] & m0->valid_mask[G & 3][2] &
-                                    m0->valid_mask[G & 3][3]) == 0xffffffffu;      // uniform over the CTA
-            // copy this thread's 64 scores to registers and hand the single S buffer back at once
+            const uint4 vm4 = *reinterpret_cast<const uint4*>(&m0->valid_mask[G & 7][0]);
+            const uint32_t vmA = ch == 0 ? vm4.x : vm4.z, vmB = ch == 0 ? vm4.y : vm4.w;
+            const bool all_valid = (vm4.x & vm4.y & vm4.z & vm4.w) == 0xffffffffu;      // uniform over the CTA
+            // copy this thread's 64 scores to registers and hand the S buffer back at once
             uint32_t sr[2][32];
-            const uint32_t t_s = tmem_addr(tmem, lane_base, kColS + ch * 64);
+            const uint32_t t_s = tmem_addr(tmem, lane_base, kColS + b * kNT + ch * 64);
             tmem_ld32(t_s, sr[0]);
             tmem_ld32(t_s + 32, sr[1]);
             tmem_wait_ld();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&m0->s_free));
+            if (lane == 0) mbar_arrive(smem_u32(&m0->s_free[b]));
+            if (!all_valid) {
+              // masked entries of the tile: no weight (2^-inf = 0) and no say in the maximum
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
+                if (!((vmA >> j) & 1u)) sr[0][j] = 0xff800000u;
+                if (!((vmB >> j) & 1u)) sr[1][j] = 0xff800000u;
+              }
+            }
             float mx = -INFINITY;
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
-              if (all_valid) {
 #pragma unroll
-                for (int j = 0; j < 32; ++j) mx = fmaxf(mx, __uint_as_float(sr[q][j]));
-              } else {
-                const uint32_t vm = q == 0 ? vmA : vmB;
-#pragma unroll
-                for (int j = 0; j < 32; ++j)
-                  if ((vm >> j) & 1u) mx = fmaxf(mx, __uint_as_float(sr[q][j]));
-              }
+              for (int j = 0; j < 32; j += 2) mx = fmaxf(mx, fmaxf(__uint_as_float(sr[q][j]), __uint_as_float(sr[q][j + 1])));
             }
             m0->xchg[b][tid] = mx;
             named_bar_sync(2, 256);
@@ -352,23 +366,19 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
             if (G >= 2) mbar_wait(smem_u32(&m0->p_free[b]), ((G - 2) >> 1) & 1u, abort_flag);
             // the staging area is single: CTA 1 reports as soon as the copies of the tile before have landed
             if (G >= 1) mbar_wait(smem_u32(&m0->stage_free), (G - 1) & 1u, abort_flag);
-            float psum = 0.0f;
+            float2 psum2 = make_float2(0.0f, 0.0f);
+            const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), neg_m2 = make_float2(-m_use, -m_use);
             // this thread's 64 columns are block `ch` of the P buffer: row rowi, eight 16-byte chunks
             const uint32_t p_row = p_local + ch * kQBlock + rowi * 128;
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
-              const uint32_t vm = all_valid ? 0xffffffffu : (q == 0 ? vmA : vmB);
               uint32_t pk[16];
 #pragma unroll
               for (int j = 0; j < 32; j += 2) {
-                float a0 = fast_exp2(fmaf(__uint_as_float(sr[q][j]), p.scale_log2, -m_use));
-                float a1 = fast_exp2(fmaf(__uint_as_float(sr[q][j + 1]), p.scale_log2, -m_use));
-                if (!all_valid) {
-                  a0 = ((vm >> j) & 1u) ? a0 : 0.0f;
-                  a1 = ((vm >> (j + 1)) & 1u) ? a1 : 0.0f;
-                }
-                psum += a0 + a1;
-                pk[j >> 1] = pack_bf16x2(a0, a1);
+                const float2 x = ffma2(__uint_as_float(sr[q][j]), __uint_as_float(sr[q][j + 1]), scale2, neg_m2);
+                const float2 e = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+                psum2 = fadd2(psum2, e);
+                pk[j >> 1] = pack_bf16x2(e.x, e.y);
               }
 #pragma unroll
               for (int c = 0; c < 4; ++c) {
@@ -376,7 +386,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
                 st_shared_v4(p_row + ((chunk ^ (rowi & 7)) << 4), pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
               }
             }
-            l_run = l_run * alpha + psum;
+            l_run = l_run * alpha + (psum2.x + psum2.y);
             if (ch == 0) m0->alpha_stage[rowi] = alpha;
             fence_proxy_async_smem();   // the bulk copies read this warp's rows through the async proxy
             __syncwarp();
@@ -412,56 +422,79 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(fin_r[ti & 1]);
         }
-      } else if (GRP == 1 && warp == 8) {
+      } else if (warp == 8) {
         // -------------------------------------------------------------- ring consumer: Q copies and Q.K^T
         // The whole warp runs the loop and waits; an elected lane (always the same one, so that its commits
-        // cover its MMAs and copies) issues.  The descriptors differ in their low word only.  Per token: nine Q
-        // entries, each moved to its 32 columns of tensor memory by four tcgen05.cp (they run in order behind
-        // the MMAs issued before them, so the previous token's last tile has read the block by then), then nine K
-        // entries per tile with four MMAs each.  The commit behind an entry frees its slot.
+        // cover its MMAs and copies) issues.  Per token: eight Q entries, each moved to its 32 columns of tensor memory by
+        // four tcgen05.cp (they run in order behind the MMAs issued before them, so the previous token's last tile
+        // has read the block by then), then nine K entries per tile with four MMAs each.  The commit behind an entry
+        // frees its slot.  The tensor pipe takes four MMAs ahead of the one it executes (256 cycles), while a wait, its
+        // fences and the issue of four MMAs by a lone warp take about 340: so the warp waits for a group of entries
+        // at once, lane by lane, and issues twelve MMAs behind one wait.
         {
           constexpr uint32_t kIdesc = umma_idesc(kFmtBF16, 128, kNT, 0, 0);
           const uint64_t bd0 = smem_desc_sw128(k_s, 16, 1024);
+          const uint64_t qd0 = smem_desc_sw128(base + kOff0Q8, 16, 1024);
           const uint32_t bd_lo = static_cast<uint32_t>(bd0), bd_hi = static_cast<uint32_t>(bd0 >> 32);
-          const uint32_t t_s = tmem + kColS, t_q = tmem + kColQ;
+          const uint32_t t_q = tmem + kColQ;
           const uint32_t k_full0 = smem_u32(&m0->k_full[0]), k_free0 = smem_u32(&m0->k_free[0]);
-          const uint32_t s_full = smem_u32(&m0->s_full), s_free = smem_u32(&m0->s_free);
-          for (int t = 0; t < nb; ++t) {
-            const int n_tiles = nt[t];
+          auto wait_group = [&](uint32_t n) {                // entries pos .. pos + n - 1 (n <= 4): lane l waits for entry l % n
+            RingPos at = pos;
+            at.advance(static_cast<uint32_t>(lane) % n);
+            mbar_wait(k_full0 + at.slot * 8, at.use & 1u, abort_flag);
+            __syncwarp();
+            fence_proxy_async_smem();                        // the rows were written by cp.async (generic proxy)
+            tc_fence_after();
+          };
 #pragma unroll 1
-            for (int cc = 0; cc < kNChunk; ++cc) {
-              mbar_wait(k_full0 + pos.slot * 8, pos.use & 1u, abort_flag);
-              tc_fence_after();
-              if (elect_one()) {
-                const uint32_t lo = bd_lo + ((pos.slot * kKSlot) >> 4);
+          for (int t = 0; t < nb; ++t) {
+            const int n_tiles = warp_uniform(nt[t]);
+#pragma unroll 1
+            for (int c0 = 0; c0 < kNQ; c0 += 4) {
+              wait_group(4);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) tmem_cp_128x256b(t_q + cc * 32 + k * 8, lo + ((k * 32) >> 4), bd_hi);
-                umma_commit(k_free0 + pos.slot * 8);
-              }
-              __syncwarp();
-              pos.advance(1);
-            }
-            for (int i = 0; i < n_tiles; ++i) {
-              const uint32_t G = gt + i;
-              // the single S buffer: the softmax of tile G-1 has copied it to registers
-              if (G >= 1) mbar_wait(s_free, (G & 1u) ^ 1u, abort_flag);
-#pragma unroll
-              for (int cc = 0; cc < kNChunk; ++cc) {
-                mbar_wait(k_full0 + pos.slot * 8, pos.use & 1u, abort_flag);
-                tc_fence_after();
+              for (int j = 0; j < 4; ++j) {
                 if (elect_one()) {
                   const uint32_t lo = bd_lo + ((pos.slot * kKSlot) >> 4);
 #pragma unroll
-                  for (int k = 0; k < 4; ++k) {
-                    if (cc == 0 && k == 0) umma_f16_ts_lohi<false>(t_s, t_q + cc * 32 + k * 8, lo + ((k * 32) >> 4), bd_hi, kIdesc);
-                    else umma_f16_ts_lohi<true>(t_s, t_q + cc * 32 + k * 8, lo + ((k * 32) >> 4), bd_hi, kIdesc);
-                  }
+                  for (int k = 0; k < 4; ++k) tmem_cp_128x256b(t_q + (c0 + j) * 32 + k * 8, lo + ((k * 32) >> 4), bd_hi);
                   umma_commit(k_free0 + pos.slot * 8);
                 }
                 __syncwarp();
                 pos.advance(1);
               }
-              if (elect_one()) umma_commit(s_full);
+            }
+#pragma unroll 1
+            for (int i = 0; i < n_tiles; ++i) {
+              const uint32_t G = gt + i;
+              const uint32_t b = G & 1u;
+              const uint32_t t_s = tmem + kColS + b * kNT;
+              // score buffer b: the softmax of tile G-2 has copied it to registers
+              if (G >= 2) mbar_wait(smem_u32(&m0->s_free[b]), ((G >> 1) & 1u) ^ 1u, abort_flag);
+#pragma unroll 1
+              for (int c0 = 0; c0 < kNChunk; c0 += 3) {
+                if (c0 == 6 && i == 0) mbar_wait(smem_u32(&m0->q8_full), (batch0 + t) & 1u, abort_flag);
+                wait_group(3);
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                  if (elect_one()) {
+                    const uint32_t lo = bd_lo + ((pos.slot * kKSlot) >> 4);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                      const uint64_t bd = (static_cast<uint64_t>(bd_hi) << 32) | (lo + ((k * 32) >> 4));
+                      if (j == 2 && c0 == 6) umma_f16_ss(t_s, qd0 + ((k * 32) >> 4), bd, kIdesc, 1u);
+                      else umma_f16_ts(t_s, t_q + (c0 + j) * 32 + k * 8, bd, kIdesc, (j | k) == 0 ? static_cast<uint32_t>(c0) : 1u);
+                    }
+                    umma_commit(k_free0 + pos.slot * 8);
+                  }
+                  __syncwarp();
+                  pos.advance(1);
+                }
+              }
+              if (elect_one()) {
+                umma_commit(smem_u32(&m0->s_full[b]));
+                if (i == n_tiles - 1) umma_commit(smem_u32(&m0->q8_free));
+              }
               __syncwarp();
             }
             gt += n_tiles;
@@ -469,70 +502,78 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
         }
       } else if (prod >= 0) {
         // -------------------------------------------------------------- ring producers
-        // producer 2c + hf supplies rows 64 hf .. 64 hf + 63 of block c of every tile (lane l < 16 owns tile rows
-        // 64 hf + 4l .. + 3: one gather4) and, if hf = 0, block c of every token's Q (one TMA tile load), in the
-        // order of the ring: its entries are c, c + 9, c + 18, ...  A slot is free once the commit behind the
-        // entry that used it last has arrived (k_free); the parity wait is exact because the entry eleven places
-        // back is at most one phase away.  Each of the two warps of an entry arrives on its barrier with its own
-        // byte count.  Block c of the token after this one is asked into L2 when this token's is loaded.
-        const int c = prod >> 1, hf = prod & 1;
-        const bool glane = lane < 16;
-        const int r0 = 64 * hf + 4 * (lane & 15);
+        // Producer c supplies block c of every token's Q (a TMA tile load) and of every tile (32 copies of 16 bytes per lane:
+        // lane l copies piece l % 8 of rows 4 q + l / 8), in the order of the ring: its entries are c, c + 9, c + 18, ...
+        // A slot is free once the commit behind the entry that used it last has arrived (k_free); the parity wait is exact
+        // because the entry ten places back is at most one phase away.  Block c of the token after this one is asked
+        // into L2 when this token's is loaded.
+        const int c = prod;
+        const __nv_bfloat16* src0 = p.kv + c * 64 + (lane & 7) * 8;
+        uint32_t dst0[2];                                    // rows 8 m + 0..3 and 8 m + 4..7 (the 128-byte swizzle goes with row % 8)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int r = 4 * q + (lane >> 3);
+          dst0[q] = k_s + r * 128 + (((lane & 7) ^ r) << 4);
+        }
+#pragma unroll 1
         for (int t = 0; t < nb; ++t) {
           const int ti = batch0 + t;
           const int tok = pair + ti * n_pairs;
-          const int n_tiles = nt[t];
+          const int n_tiles = warp_uniform(nt[t]);
           const int32_t* idx_row = p.indices + static_cast<long long>(tok) * p.idx_st;
-          int nxt[4];
+          int nxt[4];                                        // rows lane, lane + 32, lane + 64, lane + 96 of the next tile
 #pragma unroll
-          for (int j = 0; j < 4; ++j) nxt[j] = (glane && r0 + j < p.topk) ? idx_row[r0 + j] : -1;
-          // ---- the Q entry
-          if (pos.use >= 1) mbar_wait(smem_u32(&m0->k_free[pos.slot]), (pos.use - 1) & 1u, abort_flag);
-          if (lane == 0) {
-            const uint32_t full = smem_u32(&m0->k_full[pos.slot]);
-            if (hf == 0) {
+          for (int j = 0; j < 4; ++j) nxt[j] = (32 * j + lane < p.topk) ? idx_row[32 * j + lane] : -1;
+          // ---- the Q entry (block 8 has a buffer of its own)
+          {
+            uint32_t full, dst;
+            if (c < kNQ) {
+              if (pos.use >= 1) mbar_wait(smem_u32(&m0->k_free[pos.slot]), (pos.use - 1) & 1u, abort_flag);
+              full = smem_u32(&m0->k_full[pos.slot]);
+              dst = k_s + pos.slot * kKSlot;
+            } else {
+              if (ti >= 1) mbar_wait(smem_u32(&m0->q8_free), (ti - 1) & 1u, abort_flag);
+              full = smem_u32(&m0->q8_full);
+              dst = base + kOff0Q8;
+            }
+            if (lane == 0) {
               mbar_arrive_expect_tx(full, static_cast<uint32_t>(p.h * 128));
-              tma_load_3d(k_s + pos.slot * kKSlot, &tm_q, full, c * 64, 0, tok);
+              tma_load_3d(dst, &tm_q, full, c * 64, 0, tok);
               if (tok + n_pairs < p.s_q)
                 asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
                              ::"l"(&tm_q), "r"(c * 64), "r"(0), "r"(tok + n_pairs) : "memory");
-            } else {
+            } else if (c < kNQ) {
               mbar_arrive(full);
             }
+            __syncwarp();
+            pos.advance(kNQ);
           }
-          __syncwarp();
-          pos.advance(kNChunk);
           // ---- the K entries
+#pragma unroll 1
           for (int i = 0; i < n_tiles; ++i) {
             const uint32_t G = gt + i;
             int row[4];
-            uint32_t nib = 0;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const bool ok = nxt[j] >= 0 && nxt[j] < p.s_kv;
-              if (c == 0 && (nxt[j] >= p.s_kv || nxt[j] < -1)) m0->bad_index = 1;
-              row[j] = ok ? nxt[j] : 0;
-              nib |= ok ? (1u << j) : 0u;
+              if (c == 0) {
+                if (nxt[j] >= p.s_kv || nxt[j] < -1) m0->bad_index = 1;
+                const uint32_t v = __ballot_sync(0xffffffffu, ok);
+                if (lane == 0) m0->valid_mask[G & 7][j] = v;
+              }
+              row[j] = ok ? nxt[j] : 0;                      // a masked entry fetches row 0 and is multiplied by zero
+              const int jn = (i + 1) * kNT + 32 * j + lane;
+              nxt[j] = (i + 1 < n_tiles && jn < p.topk) ? idx_row[jn] : -1;
             }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int jn = (i + 1) * kNT + r0 + j;
-              nxt[j] = (glane && i + 1 < n_tiles && jn < p.topk) ? idx_row[jn] : -1;
-            }
-            if (c == 0) {
-              // 64 validity bits of this half of the tile: word 2 hf + w = rows 64 hf + 32w .. + 31 = lanes 8w .. 8w + 7
-              uint32_t v = glane ? (nib << ((lane & 7) * 4)) : 0u;
-              v |= __shfl_xor_sync(0xffffffffu, v, 1);
-              v |= __shfl_xor_sync(0xffffffffu, v, 2);
-              v |= __shfl_xor_sync(0xffffffffu, v, 4);
-              if (glane && (lane & 7) == 0) m0->valid_mask[G & 3][2 * hf + (lane >> 3)] = v;
-            }
+            __syncwarp();
             if (pos.use >= 1) mbar_wait(smem_u32(&m0->k_free[pos.slot]), (pos.use - 1) & 1u, abort_flag);
-            const uint32_t full = smem_u32(&m0->k_full[pos.slot]);
-            __syncwarp();
-            if (lane == 0) mbar_arrive_expect_tx(full, kKSlot / 2);
-            __syncwarp();
-            if (glane) tma_gather4(k_s + pos.slot * kKSlot + r0 * 128, &tm_kv, full, c * 64, row[0], row[1], row[2], row[3]);
+            const uint32_t at = pos.slot * kKSlot;
+#pragma unroll
+            for (int q = 0; q < 32; ++q) {
+              const int r = __shfl_sync(0xffffffffu, row[q >> 3], (q & 7) * 4 + (lane >> 3));
+              cp_async16(dst0[q & 1] + at + (q >> 1) * 1024, src0 + static_cast<long long>(r) * p.kv_sr);
+            }
+            cp_async_mbar_arrive_noinc(smem_u32(&m0->k_full[pos.slot]));
             pos.advance(kNChunk);
           }
           gt += n_tiles;
@@ -601,13 +642,13 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
           mbar_arrive(smem_u32(&m1->epi_cnt));
         }
       };
-      if constexpr (GRP == 0) {
+      if (warp < 8) {
         const uint32_t p_free_r[2] = {mapa_shared(smem_u32(&m0->p_free[0]), 0), mapa_shared(smem_u32(&m0->p_free[1]), 0)};
         const uint32_t stage_free_r = mapa_shared(smem_u32(&m0->stage_free), 0);
         for (int t = 0; t < nb; ++t) {
           const int ti = batch0 + t;
           const int tok = pair + ti * n_pairs;
-          const int n_tiles = nt[t];
+          const int n_tiles = warp_uniform(nt[t]);
           if (warp < 4) {
             // ------------------------------------------------------------ correction (thread = head)
             for (int i = 0; i < n_tiles; ++i) {
@@ -655,7 +696,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
             mbar_arrive_cluster_relaxed(epi_done_r[ti & 1]);
           }
         }
-      } else if (GRP == 1 && warp == 8) {
+      } else if (warp == 8) {
         // -------------------------------------------------------------- P.V issuer (whole warp, an elected lane issues)
         {
           constexpr uint32_t kIdesc = umma_idesc(kFmtBF16, 128, 256, 0, 1);
@@ -666,7 +707,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
           const uint32_t v_full0 = smem_u32(&m1->v_full[0]), v_free0 = smem_u32(&m1->v_free[0]);
           for (int t = 0; t < nb; ++t) {
             const int ti = batch0 + t;
-            const int n_tiles = nt[t];
+            const int n_tiles = warp_uniform(nt[t]);
             // the epilogue of the previous token has read the accumulator
             if (ti >= 1) mbar_wait(smem_u32(&m1->o_free), (ti - 1) & 1u, abort_flag);
             for (int i = 0; i < n_tiles; ++i) {
@@ -676,25 +717,22 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
               mbar_wait(smem_u32(&m1->corr_done[b]), (G >> 1) & 1u, abort_flag);
               tc_fence_after();
               const uint32_t a_lo = ad_lo + ((b * kPBuf) >> 4);
-#pragma unroll
+#pragma unroll 1
               for (int sl = 0; sl < kNV; ++sl) {
                 mbar_wait(v_full0 + sl * 8, ph, abort_flag);
+                fence_proxy_async_smem();   // the rows were written by cp.async (generic proxy)
                 tc_fence_after();
                 if (elect_one()) {
+                  // slab sl = 16-row steps 2 sl and 2 sl + 1 of the tile
+                  const uint32_t alo = a_lo + (((sl >> 1) * kQBlock + (sl & 1) * 64) >> 4);
+                  const uint32_t blo = bd_lo + ((sl * kVSlab) >> 4);
 #pragma unroll
                   for (int kk = 0; kk < 2; ++kk) {
-                    const int j = sl * 2 + kk;   // 16-row step inside the tile
-                    const uint32_t alo = a_lo + (((j >> 2) * kQBlock + (j & 3) * 32) >> 4);
 #pragma unroll
-                    for (int hv = 0; hv < 2; ++hv) {
-                      const uint32_t blo = bd_lo + ((sl * kVSlab + hv * 4 * kVBlock + kk * 2048) >> 4);
-                      if (j == 0) {
-                        if (i == 0) umma_f16_ss_lohi<false>(tmem + hv * 256, alo, ad_hi, blo, bd_hi, kIdesc);
-                        else umma_f16_ss_lohi<true>(tmem + hv * 256, alo, ad_hi, blo, bd_hi, kIdesc);
-                      } else {
-                        umma_f16_ss_lohi<true>(tmem + hv * 256, alo, ad_hi, blo, bd_hi, kIdesc);
-                      }
-                    }
+                    for (int hv = 0; hv < 2; ++hv)
+                      umma_f16_ss(tmem + hv * 256, (static_cast<uint64_t>(ad_hi) << 32) | (alo + ((kk * 32) >> 4)),
+                                  (static_cast<uint64_t>(bd_hi) << 32) | (blo + ((hv * 4 * kVBlock + kk * 2048) >> 4)), kIdesc,
+                                  kk == 0 ? static_cast<uint32_t>(i | sl) : 1u);
                   }
                   umma_commit(v_free0 + sl * 8);
                 }
@@ -706,63 +744,56 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
             gt += n_tiles;
           }
         }
-      } else if (warp >= 9 && warp < 17) {
+      } else if (warp < 17) {
         // -------------------------------------------------------------- V producers (warps 9-16)
-        // warp 9+w fetches 64-column block w of the 512 value columns; lane l owns tile rows 4l..4l+3, which
-        // are rows 4(l%8).. of slab l/8.
+        // Producer w fetches four of the eight column blocks of slab w / 2 of every tile (lane l: piece l % 8 of rows
+        // 4 q + l / 8).
         const int w = warp - 9;
-        const int sl = lane >> 3;
-        for (int t = 0; t < nb; ++t) {
+        const int sl = w >> 1;
+        const __nv_bfloat16* src0 = p.kv + (w & 1) * 256 + (lane & 7) * 8;
+        const uint32_t v_full = smem_u32(&m1->v_full[sl]), v_free = smem_u32(&m1->v_free[sl]);
+        uint32_t dst0[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int r = 4 * q + (lane >> 3);
+          dst0[q] = v_s + sl * kVSlab + (w & 1) * 4 * kVBlock + r * 128 + (((lane & 7) ^ r) << 4);
+        }
+#pragma unroll 1
+        for (int t = 0; t <= nb; ++t) {                      // pass nb: nothing to fetch, the last token's epilogue is left
           const int ti = batch0 + t;
           const int tok = pair + ti * n_pairs;
-          const int n_tiles = nt[t];
-          const int32_t* idx_row = p.indices + static_cast<long long>(tok) * p.idx_st;
-          int nxt[4];
+          const int n_tiles = t < nb ? warp_uniform(nt[t]) : 1;
+          const int32_t* idx_row = p.indices + static_cast<long long>(t < nb ? tok : pair) * p.idx_st;
+          int nxt = sl * kVSlabRows + lane < p.topk ? idx_row[sl * kVSlabRows + lane] : -1;   // row `lane` of the slab
+#pragma unroll 1
+          for (int i = 0; i < n_tiles; ++i) {
+            if (t < nb) {
+              const uint32_t G = gt + i;
+              const int row = (nxt >= 0 && nxt < p.s_kv) ? nxt : 0;
+              const int jn = (i + 1) * kNT + sl * kVSlabRows + lane;
+              nxt = (i + 1 < n_tiles && jn < p.topk) ? idx_row[jn] : -1;
+              if (G >= 1) mbar_wait(v_free, (G - 1) & 1u, abort_flag);
+              __syncwarp();
 #pragma unroll
-          for (int j = 0; j < 4; ++j) nxt[j] = (4 * lane + j < p.topk) ? idx_row[4 * lane + j] : -1;
-          auto issue_tile = [&](int i) {
-            const uint32_t G = gt + i;
-            int row[4];
+              for (int q = 0; q < 8; ++q) {
+                const __nv_bfloat16* src = src0 + static_cast<long long>(__shfl_sync(0xffffffffu, row, 4 * q + (lane >> 3))) * p.kv_sr;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) row[j] = (nxt[j] >= 0 && nxt[j] < p.s_kv) ? nxt[j] : 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int jn = (i + 1) * kNT + 4 * lane + j;
-              nxt[j] = (i + 1 < n_tiles && jn < p.topk) ? idx_row[jn] : -1;
+                for (int cb = 0; cb < 4; ++cb) cp_async16(dst0[q & 1] + (q >> 1) * 1024 + cb * kVBlock, src + cb * 64);
+              }
+              cp_async_mbar_arrive_noinc(v_full);
             }
-            if (G >= 1) mbar_wait(smem_u32(&m1->v_free[sl]), (G - 1) & 1u, abort_flag);
-            const uint32_t full = smem_u32(&m1->v_full[sl]);
-            // one arrival per slab announces all 64 gathers of the eight warps (the byte count may run
-            // ahead of the announcement: the phase cannot complete before this arrival)
-            if (w == 0 && (lane & 7) == 0) mbar_arrive_expect_tx(full, kVSlab);
-            tma_gather4(v_s + sl * kVSlab + w * kVBlock + (lane & 7) * 512, &tm_kv, full, w * 64, row[0], row[1], row[2], row[3]);
-          };
-          // the first tile goes out before this warp helps with the previous token's epilogue, so that the
-          // gathers run underneath it
-          issue_tile(0);
-          __syncwarp();
-          if (t > 0) epilogue_duty(ti - 1, gt - 1, tok - n_pairs);
-          for (int i = 1; i < n_tiles; ++i) issue_tile(i);
-          gt += n_tiles;
+            // the first tile goes out before this warp helps with the previous token's epilogue, so that the
+            // gathers run underneath it
+            if (i == 0 && t > 0) {
+              __syncwarp();
+              epilogue_duty(ti - 1, gt - 1, tok - n_pairs);
+            }
+          }
+          if (t < nb) gt += n_tiles;
         }
-        // the last token of the batch: nothing of the next batch is known yet
-        __syncwarp();
-        epilogue_duty(batch0 + nb - 1, gt - 1, pair + (batch0 + nb - 1) * n_pairs);
       }
     }
     __syncthreads();   // nt[] is rewritten by the next batch
-  }
-  };
-  // Registers follow the work: the gather warps need few, the softmax and correction / epilogue warps many
-  // (64 scores per thread live at once).
-  if (warp < 8) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
-    run(std::integral_constant<int, 0>{});
-  } else if (warp < 20) {
-    run(std::integral_constant<int, 1>{});
-  } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-    run(std::integral_constant<int, 2>{});
   }
 
   tc_fence_before();
@@ -814,19 +845,14 @@ int launch_sparse_mla_ring(const ftb_sparse_mla_args* a, cudaStream_t st) {
   // through its tokens without a stop; a longer batch of query tokens is a sequence of such launches on the
   // stream (a launch boundary every pairs x kBatch tokens costs next to nothing).
   const long long cap = static_cast<long long>(pairs_dev) * mla_ring::kBatch;
-  // KV: box = 64 columns x 1 row (tile::gather4 fetches four such rows per instruction);
   // Q: boxes of [h rows x 64 columns] of one token; O: boxes of [32 rows x 64 columns] (a store that
   // reaches past row h is clipped)
   const uint32_t box_h = static_cast<uint32_t>(a->h < 128 ? a->h : 128);
-  CUtensorMap tm_kv;
-  if (!make_tmap_2d(&tm_kv, a->kv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, static_cast<uint64_t>(a->s_kv), mla_ring::kDqk,
-                    static_cast<uint64_t>(a->kv_stride_row), 1, 64)) {
-    set_last_error("sparse_mla_ring: cuTensorMapEncodeTiled failed");
-    return FTB_ERR_CUDA;
-  }
   for (long long t0 = 0; t0 < a->s_q; t0 += cap) {
     const int n_tok = static_cast<int>(a->s_q - t0 < cap ? a->s_q - t0 : cap);
     mla_ring::Params p;
+    p.kv = static_cast<const __nv_bfloat16*>(a->kv);
+    p.kv_sr = a->kv_stride_row;
     p.indices = a->indices + t0 * a->idx_stride_token;
     p.lse = a->lse + t0 * a->lse_stride_token;
     p.s_q = n_tok; p.h = a->h; p.s_kv = a->s_kv; p.topk = a->topk;
@@ -849,7 +875,7 @@ int launch_sparse_mla_ring(const ftb_sparse_mla_args* a, cudaStream_t st) {
     }
     const int pairs = pairs_dev < n_tok ? pairs_dev : n_tok;
     cfg.gridDim = dim3(static_cast<unsigned>(pairs) * 2u);
-    e = cudaLaunchKernelEx(&cfg, mla_ring::sparse_mla_ring_kernel, tm_kv, tm_q, tm_o, p);
+    e = cudaLaunchKernelEx(&cfg, mla_ring::sparse_mla_ring_kernel, tm_q, tm_o, p);
     if (e != cudaSuccess) return check_cuda(e, "sparse_mla_ring launch");
   }
   return FTB_OK;

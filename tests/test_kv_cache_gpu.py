@@ -98,3 +98,34 @@ def test_written_cache_feeds_the_paged_forward():
     from oracle.sparse_mla_ref import e4m3_decode
     deq = (e4m3_decode(cache.cpu()) * scale.cpu()[:, None, None]).view(-1, 576)[slots.long()]
     assert ((deq - rows.float()).abs() <= rows.float().abs() * 2 ** -3 + scale.cpu().max() * 2 ** -9).all()
+
+
+@pytest.mark.parametrize("n,page,order", [(1, 64, "runs"), (1024, 64, "runs"), (1024, 16, "shuffled"), (1025, 64, "runs"),
+                                          (1500, 64, "shuffled"), (1500, 64, "halves"), (1100, 1, "runs"), (1100, 3, "runs"),
+                                          (700, 512, "runs"), (1300, 512, "runs")])
+def test_write_paths_bit_exact(n, page, order):
+    """Every route of a row: one launch for small calls, runs of a page taken by a warp or a CTA, pages with several
+    runs, pages longer than a run may be; with zeros of both signs, rows of very different size (scales outside the range
+    that the reciprocal serves among them), and pages that held rows before."""
+    g = torch.Generator().manual_seed(n + page)
+    n_pages = -(-n // page) + 3
+    perm = torch.randperm(n_pages, generator=g)
+    at = torch.arange(n) + min(5, page - 1)                               # the first page is filled from its sixth row on
+    slots = perm[at // page] * page + at % page
+    if order == "shuffled":
+        slots = slots[torch.randperm(n, generator=g)]
+    elif order == "halves":                                               # a page comes in two runs
+        half = (torch.arange(n) % 64 < 32)
+        slots = torch.cat([slots[half], slots[~half]])
+    x = torch.randn(n, 576, generator=g)
+    x[:, ::7] = 0.0
+    x[:, 1::7] = -0.0
+    x[n // 2:n // 2 + page] *= 1e-35
+    x[n // 3:n // 3 + page] *= 1e33
+    slots = slots.int()
+    slots[n // 5] = -1
+    cache = torch.randint(0, 120, (n_pages, page, 576), generator=g, dtype=torch.uint8)
+    scale = torch.rand(n_pages, generator=g) * 0.01 * (torch.rand(n_pages, generator=g) < 0.5)
+    g_cache, g_scale, r_cache, r_scale = _write_both(x.bfloat16(), slots, cache, scale, page)
+    assert torch.equal(g_scale, r_scale)
+    assert torch.equal(g_cache, r_cache)

@@ -92,3 +92,24 @@ def test_causal_lengths_feed_the_forward():
     ref_out, ref_lse = sparse_mla_fwd_ref(q, kv, idx.cpu(), 0.05)
     assert (out.float().cpu() - ref_out).abs().max().item() <= 2e-2
     assert ((lse.cpu() - ref_lse).abs() / ref_lse.abs().clamp(min=1)).max().item() <= 1e-3
+
+
+@pytest.mark.parametrize("s_kv", [4095, 4097, 32767, 32768, 32769, 33791, 50001, 65535, 65536, 65537])
+def test_edges_of_the_row_kernels(s_kv):
+    """Lengths around what the registers and the shared memory hold, rows that are not 16-byte aligned (odd strides),
+    rows of two values (more ties than the candidate list holds), rows that rise or fall (the candidates of a row sit in
+    few warps), a sample unlike the rest, NaN patterns, and more rows than SMs for the ragged case."""
+    g = torch.Generator().manual_seed(s_kv)
+    odd = torch.randn(s_kv, generator=g)
+    odd[(torch.arange(256) * s_kv >> 8) + (torch.arange(256) & 15)] = -1e6
+    nan = torch.randn(s_kv, generator=g)
+    nan[3::1000] = float("nan")
+    nan[5::1000] = -float("nan")
+    rows = [torch.randn(s_kv, generator=g), torch.randint(0, 2, (s_kv,), generator=g).float(), torch.full((s_kv,), -0.0),
+            torch.arange(s_kv).float(), -torch.arange(s_kv).float(), odd, nan, torch.randn(s_kv, generator=g).bfloat16().float()]
+    sc = torch.stack(rows * (20 if s_kv == 32769 else 1))
+    lengths = torch.full((sc.shape[0],), s_kv, dtype=torch.int32)
+    lengths[-1] = max(1, s_kv - 777)
+    for k in (2048, 1, s_kv - 1):
+        got = topk_indices(sc.to(DEV), k, lengths.to(DEV)).cpu()
+        assert torch.equal(got, topk_indices_ref(sc, k, lengths)), k

@@ -462,45 +462,41 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_fwd_kernel(const MlaPa
 // Merge of the per-split partial results (the role of the reference's _fwd_kernel_stage2,
 // third_party/mthreads/python/test/wmma/test_accuracy_musa_vllm_mla.py:426-477): weights 2^(lse_k - max),
 // out = sum w_k out_k / sum w_k, and the merged LSE, which the reference does not store.
-// One warp per (token, head); lane i owns output columns [16 i, 16 i + 16).
-__global__ void __launch_bounds__(256) sparse_mla_merge_kernel(const float* __restrict__ part_out,
+// One CTA of 128 threads per (token, head), four columns each: a decode step merges few rows of many parts, so what counts is
+// that the loads of all parts are in flight at once (a warp per row that took one part after the other: 13 us for 3 tokens
+// of 128 heads and 16 parts).
+constexpr int kMergeBatch = 16;
+__global__ void __launch_bounds__(128) sparse_mla_merge_kernel(const float* __restrict__ part_out,
                                                                const float* __restrict__ part_lse, __nv_bfloat16* out,
-                                                               float* lse, int s_q, int h, int n_splits, long long out_st,
+                                                               float* lse, int h, int n_splits, long long out_st,
                                                                long long out_sh, long long lse_st, int lse_base2) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (w >= s_q * h) return;
-  const int token = w / h, head = w - token * h;
-  float mx = -INFINITY;
-  for (int k = 0; k < n_splits; ++k) mx = fmaxf(mx, part_lse[(static_cast<long long>(token) * n_splits + k) * h + head]);
-  float acc[16];
+  const int token = blockIdx.x / h, head = blockIdx.x - token * h;
+  const float* lrow = part_lse + static_cast<long long>(token) * n_splits * h + head;
+  const float4* src = reinterpret_cast<const float4*>(part_out + (static_cast<long long>(token) * n_splits * h + head) * 512) + threadIdx.x;
+  float mx = -INFINITY, wsum = 0.0f;
+  for (int k = 0; k < n_splits; ++k) mx = fmaxf(mx, lrow[static_cast<long long>(k) * h]);
+  float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  for (int k0 = 0; k0 < n_splits && mx != -INFINITY; k0 += kMergeBatch) {
+    float4 v[kMergeBatch];
+    float w[kMergeBatch];
 #pragma unroll
-  for (int j = 0; j < 16; ++j) acc[j] = 0.0f;
-  float wsum = 0.0f;
-  if (mx != -INFINITY) {
-    for (int k = 0; k < n_splits; ++k) {
-      const long long row = (static_cast<long long>(token) * n_splits + k) * h + head;
-      const float l2 = part_lse[row];
-      if (l2 == -INFINITY) continue;
-      const float wk = fast_exp2(l2 - mx);
+    for (int k = 0; k < kMergeBatch; ++k) {
+      const bool in = k0 + k < n_splits;
+      w[k] = in ? lrow[static_cast<long long>(k0 + k) * h] : -INFINITY;
+      v[k] = in ? __ldcs(src + static_cast<long long>(k0 + k) * h * 128) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+#pragma unroll
+    for (int k = 0; k < kMergeBatch; ++k) {
+      if (w[k] == -INFINITY) continue;
+      const float wk = fast_exp2(w[k] - mx);
       wsum += wk;
-      const float4* src = reinterpret_cast<const float4*>(part_out + row * 512 + lane * 16);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float4 v = src[j];
-        acc[4 * j] += wk * v.x; acc[4 * j + 1] += wk * v.y; acc[4 * j + 2] += wk * v.z; acc[4 * j + 3] += wk * v.w;
-      }
+      acc.x += wk * v[k].x; acc.y += wk * v[k].y; acc.z += wk * v[k].z; acc.w += wk * v[k].w;
     }
   }
   const float inv = wsum > 0.0f ? 1.0f / wsum : 0.0f;
-  uint4 o[2];
-  uint32_t* ow = reinterpret_cast<uint32_t*>(o);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) ow[j] = pack_bf16x2(acc[2 * j] * inv, acc[2 * j + 1] * inv);
-  uint4* dst = reinterpret_cast<uint4*>(out + token * out_st + head * out_sh + lane * 16);
-  dst[0] = o[0];
-  dst[1] = o[1];
-  if (lane == 0) {
+  *reinterpret_cast<uint2*>(out + token * out_st + head * out_sh + threadIdx.x * 4) =
+      make_uint2(pack_bf16x2(acc.x * inv, acc.y * inv), pack_bf16x2(acc.z * inv, acc.w * inv));
+  if (threadIdx.x == 0) {
     const float l2 = wsum > 0.0f ? mx + log2f(wsum) : -INFINITY;
     lse[token * lse_st + head] = (lse_base2 || l2 == -INFINITY) ? l2 : l2 * 0.6931471805599453f;
   }
@@ -580,7 +576,7 @@ __global__ void __launch_bounds__(256) sparse_mla_merge_parts_kernel(const T* __
 namespace ftb {
 void set_last_error(const char* fmt, ...);
 int check_cuda(cudaError_t e, const char* what);
-int launch_sparse_mla_ring(const ftb_sparse_mla_args* a, cudaStream_t st);
+int launch_sparse_mla_ring(const ftb_sparse_mla_args* a, int n_splits, float* part_out, float* part_lse, cudaStream_t st);
 int launch_sparse_mla_few(const ftb_sparse_mla_args* a, cudaStream_t st);
 }  // namespace ftb
 
@@ -636,8 +632,8 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
     return FTB_ERR_INVALID;
   }
   if (a->algo_id == 2) return launch_sparse_mla_few(a, reinterpret_cast<cudaStream_t>(stream));
-  if (!a->kv_is_fp8 && a->dbg_scores == nullptr && a->n_splits <= 1 && (a->algo_id == 0 || a->algo_id == 5))
-    return launch_sparse_mla_ring(a, reinterpret_cast<cudaStream_t>(stream));
+  if (plain && (a->algo_id == 0 || a->algo_id == 5))
+    return launch_sparse_mla_ring(a, 1, nullptr, nullptr, reinterpret_cast<cudaStream_t>(stream));
   MlaParams p;
   memset(&p, 0, sizeof(p));
   p.q = reinterpret_cast<const __nv_bfloat16*>(a->q);
@@ -662,7 +658,17 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
   // Paged FP8 form with a workspace for the dequantised rows (algo 0 or 6, no split): convert the selected
   // rows once, then run the persistent bf16 kernel on the compact table.  Without such a workspace the
   // one-pass kernel below converts while it gathers.
-  if (a->kv_is_fp8 && n_splits == 1 && a->dbg_scores == nullptr && (a->algo_id == 0 || a->algo_id == 6)) {
+  const int64_t split_bytes = ftb_sparse_mla_workspace_bytes(a->s_q, a->h, n_splits);
+  auto merge = [&]() {
+    sparse_mla_merge_kernel<<<static_cast<unsigned>(a->s_q * a->h), 128, 0, st>>>(p.part_out, p.part_lse, p.out, p.lse, a->h, n_splits,
+                                                                               p.out_st, p.out_sh, p.lse_st, p.lse_base2);
+    return check_cuda(cudaGetLastError(), "sparse_mla_merge launch");
+  };
+  // With a split, algo 6 wants room for both: the dequantised rows, then the partial results (from a 16-byte boundary).
+  const int64_t rows_bytes = (ftb_sparse_mla_dequant_workspace_bytes(a->s_q, a->topk) + 15) / 16 * 16;
+  if (a->kv_is_fp8 && a->dbg_scores == nullptr &&
+      (n_splits == 1 ? (a->algo_id == 0 || a->algo_id == 6)
+                     : (a->algo_id == 6 && a->workspace_bytes >= rows_bytes + split_bytes))) {
     const int64_t need = ftb_sparse_mla_dequant_workspace_bytes(a->s_q, a->topk);
     const bool have = a->workspace != nullptr && a->workspace_bytes >= need && need > 0 &&
                       (reinterpret_cast<uintptr_t>(a->workspace) & 15u) == 0 &&
@@ -691,7 +697,11 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
       b.idx_stride_token = a->topk;
       b.algo_id = 5;
       b.workspace = nullptr; b.workspace_bytes = 0; b.n_splits = 0;
-      return launch_sparse_mla_ring(&b, st);
+      if (n_splits == 1) return launch_sparse_mla_ring(&b, 1, nullptr, nullptr, st);
+      p.part_out = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(a->workspace) + rows_bytes);
+      p.part_lse = p.part_out + static_cast<size_t>(a->s_q) * n_splits * a->h * 512;
+      rc0 = launch_sparse_mla_ring(&b, n_splits, p.part_out, p.part_lse, st);
+      return rc0 != FTB_OK ? rc0 : merge();
     }
   }
   if (n_splits > 1) {
@@ -703,6 +713,12 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
     p.part_lse = p.part_out + static_cast<size_t>(a->s_q) * n_splits * a->h * 512;
   }
   p.n_splits = n_splits;
+  // bf16 rows: the persistent pairs take a part of a token as they take a token (up to as many parts as a pair has room for)
+  if (n_splits > 1 && n_splits <= 64 && !a->kv_is_fp8 && a->dbg_scores == nullptr && (a->algo_id == 0 || a->algo_id == 5) &&
+      (reinterpret_cast<uintptr_t>(a->workspace) & 15u) == 0) {
+    const int rc0 = launch_sparse_mla_ring(a, n_splits, p.part_out, p.part_lse, st);
+    return rc0 != FTB_OK ? rc0 : merge();
+  }
   const dim3 grid(static_cast<unsigned>(a->s_q) * 2u * static_cast<unsigned>(n_splits)), block(kThreads);
   cudaError_t e;
   if (a->kv_is_fp8) {
@@ -716,10 +732,7 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
   }
   int rc = check_cuda(cudaGetLastError(), "sparse_mla_fwd launch");
   if (rc != FTB_OK || n_splits == 1) return rc;
-  const int warps = a->s_q * a->h;
-  sparse_mla_merge_kernel<<<(warps * 32 + 255) / 256, 256, 0, st>>>(p.part_out, p.part_lse, p.out, p.lse, a->s_q, a->h, n_splits,
-                                                                    p.out_st, p.out_sh, p.lse_st, p.lse_base2);
-  return check_cuda(cudaGetLastError(), "sparse_mla_merge launch");
+  return merge();
 }
 
 extern "C" FTB_API int64_t ftb_sparse_mla_dequant_workspace_bytes(int32_t s_q, int32_t topk) {

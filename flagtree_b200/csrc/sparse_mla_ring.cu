@@ -29,13 +29,18 @@
 // fences costs it 350 cycles, twelve MMAs take 768).  740 tokens, 128 heads, topk 2048: 832 -> 1065 TFLOP/s (one launch
 // alone); prefill of 4096 causal tokens, back to back under the power limit: 2247 -> 2036 us; one token: 58.8 -> 50.3 us.
 //
+// Few tokens.  A launch may cut the top-k list of every token in parts; an item of work is then a part of a token, its result
+// leaves as fp32 (32 columns per TMA store instead of 64) with a base-2 LSE, and a second kernel merges the parts.  One token
+// of topk 2048: 49 us whole, 23 us in 16 parts.  (Stores straight from registers, 16 bytes per lane and row, took 6 us more:
+// half sectors.)
+//
 // Softmax: two threads per head row; the running maximum moves only when it grows by more than 2^8, so that
 // the accumulator in CTA 1 is rarely rescaled.  P (bf16) and the rescale factors go to a staging area and
 // from there to CTA 1 with bulk copies that complete on CTA 1's barrier; the arrival that announces them
 // carries no release (the data travels with the copies), which keeps the softmax warps from stalling.
 //
-// The number of tiles of a token (last non-negative index, rounded up to 128 rows, at least one) is
-// found for 64 tokens at a time by all warps of a CTA, with a CTA barrier on either side.
+// The number of tiles of an item (last non-negative index, rounded up to 128 rows, at least one) is
+// found for 64 items at a time by all warps of a CTA, with CTA barriers between.
 //
 // Warps (640 threads per CTA): CTA 0: 0-7 softmax, 8 MMA issuer, nine ring producers (the warps 9-19 whose id is not 0
 // modulo 4).  CTA 1: 0-3 correction, 4 relay, 8 MMA issuer, 9-16 V producers, 0-7 and 9-16 epilogue.
@@ -88,6 +93,9 @@ struct Params {
   float scale_log2;
   int lse_base2;
   int* status;
+  // the top-k list of a token in n_splits parts, an item of work each; their results go to fp32 partials that are merged later
+  int n_splits;
+  float* part_lse;     // [s_q, n_splits, h], base 2
 };
 
 struct Misc0 {   // CTA 0
@@ -105,7 +113,8 @@ struct Misc0 {   // CTA 0
   int bad_index;
   int pad;
   alignas(16) uint32_t valid_mask[8][4];  // per tile (mod 8): 128 validity bits
-  unsigned short nt[kBatch];        // tiles per token of the current batch
+  unsigned short nt[2 * kBatch];    // per item of the current batch: number of tiles, first tile
+  int last[kBatch];                 // entries of its list up to the last that is not negative
   float xchg[2][256];               // row maximum / row sum exchange between the two threads of a head row
   alignas(16) float alpha_stage[128]; // rescale factors of a tile on their way to CTA 1 (sent with P)
 };
@@ -122,7 +131,8 @@ struct Misc1 {   // CTA 1
   uint32_t tmem_base;
   int abort_flag;
   int pad[2];
-  unsigned short nt[kBatch];
+  unsigned short nt[2 * kBatch];
+  int last[kBatch];
   alignas(16) float alpha[2][128];  // rescale factor of the tile (two buffers), written by bulk copies from CTA 0
   float inv_l[2][128];              // final 1/l of token t (t % 2)
 };
@@ -214,6 +224,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
   volatile int* abort_flag = cta == 0 ? &m0->abort_flag : &m1->abort_flag;
   uint32_t* tmem_base_p = cta == 0 ? &m0->tmem_base : &m1->tmem_base;
   unsigned short* nt = cta == 0 ? m0->nt : m1->nt;
+  int* last = cta == 0 ? m0->last : m1->last;
 
   if (tid == 0) {
     *abort_flag = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
@@ -270,8 +281,9 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
   cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem = *tmem_base_p;
-  // tokens of this pair: pair, pair + n_pairs, ...  (the host launches no more pairs than tokens)
-  const int my_tokens = (p.s_q - pair + n_pairs - 1) / n_pairs;
+  // items (tokens, or parts of tokens) of this pair: pair, pair + n_pairs, ...  (the host launches no more pairs than items)
+  auto token_of = [&](int item) { return p.n_splits == 1 ? item : item / p.n_splits; };
+  const int my_tokens = (p.s_q * p.n_splits - pair + n_pairs - 1) / n_pairs;
   uint32_t gt = 0;   // tiles processed before the current token: every role counts the same way
   // CTA 0: the nine gather warps, one per column block: the warps 9-19 whose id is not 0 modulo 4, in order (they share no
   // scheduler with the MMA issuer, warp 8)
@@ -283,17 +295,36 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
   for (int batch0 = 0; batch0 < my_tokens; batch0 += kBatch) {
     const int nb = min(kBatch, my_tokens - batch0);
     // ------------------------------------------------------------------ tiles per token of this batch
-    for (int t = warp; t < nb; t += kWarps) {
-      const int tok = pair + (batch0 + t) * n_pairs;
-      const int32_t* idx_row = p.indices + static_cast<long long>(tok) * p.idx_st;
-      int local = 0;
-      for (int j = lane; j < p.topk; j += 32)
-        if (idx_row[j] >= 0) local = j + 1;
+    // the warps share the lists out in pieces of 512 entries, all loads of a piece in flight (one token's list of 2048 entries, read
+    // by one warp 32 at a time, took 10 us)
+    for (int t = tid; t < nb; t += kThreads) last[t] = 0;
+    __syncthreads();
+    const int pieces = (p.topk + 511) >> 9;
+#pragma unroll 1
+    for (int x = warp; x < nb * pieces; x += kWarps) {
+      const int t = x / pieces, j0 = (x - t * pieces) * 512 + lane;
+      const int32_t* idx_row = p.indices + static_cast<long long>(token_of(pair + (batch0 + t) * n_pairs)) * p.idx_st;
+      int v[16];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) local = max(local, __shfl_xor_sync(0xffffffffu, local, o));
-      // at least one tile (entirely masked if the token selects nothing): every stage of the pipeline
-      // then runs once per token and the hand-overs between tokens need no special case
-      if (lane == 0) nt[t] = static_cast<unsigned short>(min(65535, max(1, (local + kNT - 1) / kNT)));
+      for (int j = 0; j < 16; ++j) v[j] = j0 + 32 * j < p.topk ? idx_row[j0 + 32 * j] : -1;
+      int local = 0;
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (v[j] >= 0) local = j0 + 32 * j + 1;
+      local = __reduce_max_sync(0xffffffffu, local);
+      if (lane == 0 && local > 0) atomicMax(&last[t], local);
+    }
+    __syncthreads();
+    // at least one tile (entirely masked if the item selects nothing): every stage of the pipeline
+    // then runs once per item and the hand-overs between items need no special case
+    for (int t = tid; t < nb; t += kThreads) {
+      const int item = pair + (batch0 + t) * n_pairs;
+      const int tiles = min(65535, max(1, (last[t] + kNT - 1) / kNT));
+      const int part = (tiles + p.n_splits - 1) / p.n_splits;
+      int first = (item - token_of(item) * p.n_splits) * part;
+      if (first >= tiles) first = 65535;                     // nothing left for this part: a tile past the list
+      nt[t] = static_cast<unsigned short>(max(1, min(part, tiles - first)));
+      nt[kBatch + t] = static_cast<unsigned short>(first);
     }
     __syncthreads();
 
@@ -314,7 +345,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32);
         for (int t = 0; t < nb; ++t) {
           const int ti = batch0 + t;
-          const int tok = pair + ti * n_pairs;
+          const int item = pair + ti * n_pairs;
           const int n_tiles = warp_uniform(nt[t]);
           // 1/l and the `fin` barrier of parity ti % 2 were last used by token ti - 2: its epilogue is over
           if (ti >= 2) mbar_wait(smem_u32(&m0->epi_done[ti & 1]), ((ti >> 1) - 1) & 1u, abort_flag);
@@ -411,12 +442,9 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
             const float inv_l = (l_tot > 0.0f) ? 1.0f / l_tot : 0.0f;
             st_cluster_f32(invl_remote + ((ti & 1) * 128 + rowi) * 4, inv_l);
             if (rowi < p.h) {
-              float v = -INFINITY;
-              if (l_tot > 0.0f) {
-                const float l2 = m_run + log2f(l_tot);
-                v = p.lse_base2 ? l2 : l2 * 0.6931471805599453f;
-              }
-              p.lse[static_cast<long long>(tok) * p.lse_st + rowi] = v;
+              const float l2 = l_tot > 0.0f ? m_run + log2f(l_tot) : -INFINITY;
+              if (p.n_splits == 1) p.lse[static_cast<long long>(item) * p.lse_st + rowi] = (p.lse_base2 || l_tot <= 0.0f) ? l2 : l2 * 0.6931471805599453f;
+              else p.part_lse[static_cast<long long>(item) * p.h + rowi] = l2;
             }
           }
           __syncwarp();
@@ -518,12 +546,12 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
 #pragma unroll 1
         for (int t = 0; t < nb; ++t) {
           const int ti = batch0 + t;
-          const int tok = pair + ti * n_pairs;
-          const int n_tiles = warp_uniform(nt[t]);
-          const int32_t* idx_row = p.indices + static_cast<long long>(tok) * p.idx_st;
+          const int tok = token_of(pair + ti * n_pairs), tok_next = token_of(pair + (ti + 1) * n_pairs);
+          const int n_tiles = warp_uniform(nt[t]), row0 = warp_uniform(nt[kBatch + t]) * kNT, n_rows = p.topk - row0;
+          const int32_t* idx_row = p.indices + static_cast<long long>(tok) * p.idx_st + row0;
           int nxt[4];                                        // rows lane, lane + 32, lane + 64, lane + 96 of the next tile
 #pragma unroll
-          for (int j = 0; j < 4; ++j) nxt[j] = (32 * j + lane < p.topk) ? idx_row[32 * j + lane] : -1;
+          for (int j = 0; j < 4; ++j) nxt[j] = (32 * j + lane < n_rows) ? idx_row[32 * j + lane] : -1;
           // ---- the Q entry (block 8 has a buffer of its own)
           {
             uint32_t full, dst;
@@ -539,9 +567,9 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
             if (lane == 0) {
               mbar_arrive_expect_tx(full, static_cast<uint32_t>(p.h * 128));
               tma_load_3d(dst, &tm_q, full, c * 64, 0, tok);
-              if (tok + n_pairs < p.s_q)
+              if (tok_next < p.s_q)
                 asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
-                             ::"l"(&tm_q), "r"(c * 64), "r"(0), "r"(tok + n_pairs) : "memory");
+                             ::"l"(&tm_q), "r"(c * 64), "r"(0), "r"(tok_next) : "memory");
             } else if (c < kNQ) {
               mbar_arrive(full);
             }
@@ -563,7 +591,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
               }
               row[j] = ok ? nxt[j] : 0;                      // a masked entry fetches row 0 and is multiplied by zero
               const int jn = (i + 1) * kNT + 32 * j + lane;
-              nxt[j] = (i + 1 < n_tiles && jn < p.topk) ? idx_row[jn] : -1;
+              nxt[j] = (i + 1 < n_tiles && jn < n_rows) ? idx_row[jn] : -1;
             }
             __syncwarp();
             if (pos.use >= 1) mbar_wait(smem_u32(&m0->k_free[pos.slot]), (pos.use - 1) & 1u, abort_flag);
@@ -593,7 +621,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
       // p_free back until the last store has read it; the V ring is not touched, so the gathers of the
       // next token run underneath.  Warp w < 8 and warp 9 + w share piece w: the V producers come later
       // (they first send out the next token's first gathers) and wait for their partner (stg_free).
-      auto epilogue_duty = [&](int ti, uint32_t Gl, int tok) {
+      auto epilogue_duty = [&](int ti, uint32_t Gl, int item) {
         const int q4 = warp & 3;
         const int grp = warp < 8 ? (warp >> 2) : 2 + ((warp - 9) >> 2);
         const int piece = warp < 8 ? warp : warp - 9;
@@ -606,6 +634,16 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
         const int row = q4 * 32 + lane;
         const float inv_l = m1->inv_l[ti & 1][row];
         const uint32_t stg = p_s + (Gl & 1u) * kPBuf + piece * 4096 + lane * 128;
+        auto send = [&](int col) {
+          fence_proxy_async_smem();   // the tile store reads the piece through the async proxy
+          __syncwarp();
+          if (lane == 0) {
+            if (q4 * 32 < p.h) tma_store_3d(&tm_o, stg - lane * 128, col, q4 * 32, item);
+            bulk_commit();
+            bulk_wait_read_all();
+          }
+          __syncwarp();
+        };
 #pragma unroll 1
         for (int cb = 0; cb < 2; ++cb) {
 #pragma unroll
@@ -613,6 +651,16 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
             uint32_t acc[32];
             tmem_ld32(tmem_addr(tmem, q4 * 32, grp * 128 + cb * 64 + c2 * 32), acc);
             tmem_wait_ld();
+            if (p.n_splits > 1) {
+              // a partial result stays fp32: 32 columns fill the piece
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                st_shared_v4(stg + ((j ^ (lane & 7)) << 4), __float_as_uint(__uint_as_float(acc[4 * j]) * inv_l),
+                             __float_as_uint(__uint_as_float(acc[4 * j + 1]) * inv_l), __float_as_uint(__uint_as_float(acc[4 * j + 2]) * inv_l),
+                             __float_as_uint(__uint_as_float(acc[4 * j + 3]) * inv_l));
+              if (c2 == 0) send((grp * 4 + cb * 2) * 32);
+              continue;
+            }
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
               const int chunk = c2 * 4 + (j >> 3);
@@ -628,14 +676,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&m1->o_free));   // the next token's P.V may overwrite the accumulator
           }
-          fence_proxy_async_smem();   // the tile store reads the piece through the async proxy
-          __syncwarp();
-          if (lane == 0) {
-            if (q4 * 32 < p.h) tma_store_3d(&tm_o, stg - lane * 128, (grp * 2 + cb) * 64, q4 * 32, tok);
-            bulk_commit();
-            bulk_wait_read_all();
-          }
-          __syncwarp();
+          send(p.n_splits > 1 ? (grp * 4 + cb * 2 + 1) * 32 : (grp * 2 + cb) * 64);
         }
         if (lane == 0) {
           if (warp < 8) mbar_arrive(smem_u32(&m1->stg_free[piece]));
@@ -647,7 +688,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
         const uint32_t stage_free_r = mapa_shared(smem_u32(&m0->stage_free), 0);
         for (int t = 0; t < nb; ++t) {
           const int ti = batch0 + t;
-          const int tok = pair + ti * n_pairs;
+          const int item = pair + ti * n_pairs;
           const int n_tiles = warp_uniform(nt[t]);
           if (warp < 4) {
             // ------------------------------------------------------------ correction (thread = head)
@@ -687,7 +728,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
           }
           __syncwarp();
           gt += n_tiles;
-          epilogue_duty(ti, gt - 1, tok);
+          epilogue_duty(ti, gt - 1, item);
           // the P buffer of the last tile staged the output: it is free for the softmax, and 1/l of this
           // token may be replaced, once all 16 warps are through
           if (warp == 4 && lane == 0) {
@@ -761,17 +802,18 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
 #pragma unroll 1
         for (int t = 0; t <= nb; ++t) {                      // pass nb: nothing to fetch, the last token's epilogue is left
           const int ti = batch0 + t;
-          const int tok = pair + ti * n_pairs;
+          const int item = pair + ti * n_pairs;
           const int n_tiles = t < nb ? warp_uniform(nt[t]) : 1;
-          const int32_t* idx_row = p.indices + static_cast<long long>(t < nb ? tok : pair) * p.idx_st;
-          int nxt = sl * kVSlabRows + lane < p.topk ? idx_row[sl * kVSlabRows + lane] : -1;   // row `lane` of the slab
+          const int row0 = t < nb ? warp_uniform(nt[kBatch + t]) * kNT : 0, n_rows = p.topk - row0;
+          const int32_t* idx_row = p.indices + static_cast<long long>(t < nb ? token_of(item) : 0) * p.idx_st + row0;
+          int nxt = sl * kVSlabRows + lane < n_rows ? idx_row[sl * kVSlabRows + lane] : -1;   // row `lane` of the slab
 #pragma unroll 1
           for (int i = 0; i < n_tiles; ++i) {
             if (t < nb) {
               const uint32_t G = gt + i;
               const int row = (nxt >= 0 && nxt < p.s_kv) ? nxt : 0;
               const int jn = (i + 1) * kNT + sl * kVSlabRows + lane;
-              nxt = (i + 1 < n_tiles && jn < p.topk) ? idx_row[jn] : -1;
+              nxt = (i + 1 < n_tiles && jn < n_rows) ? idx_row[jn] : -1;
               if (G >= 1) mbar_wait(v_free, (G - 1) & 1u, abort_flag);
               __syncwarp();
 #pragma unroll
@@ -786,7 +828,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
             // gathers run underneath it
             if (i == 0 && t > 0) {
               __syncwarp();
-              epilogue_duty(ti - 1, gt - 1, tok - n_pairs);
+              epilogue_duty(ti - 1, gt - 1, item - n_pairs);
             }
           }
           if (t < nb) gt += n_tiles;
@@ -811,7 +853,8 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
 
 }  // namespace mla_ring
 
-int launch_sparse_mla_ring(const ftb_sparse_mla_args* a, cudaStream_t st) {
+// n_splits > 1: partial results to part_out / part_lse, and `out` and `lse` of the arguments are left alone
+int launch_sparse_mla_ring(const ftb_sparse_mla_args* a, int n_splits, float* part_out, float* part_lse, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(mla_ring::sparse_mla_ring_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, mla_ring::kSmemBytes);
   if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(sparse_mla_ring)");
   cudaLaunchConfig_t cfg = {};
@@ -844,7 +887,8 @@ int launch_sparse_mla_ring(const ftb_sparse_mla_args* a, cudaStream_t st) {
   // One launch takes at most kBatch tokens per pair, so that every pair finds its tile counts once and runs
   // through its tokens without a stop; a longer batch of query tokens is a sequence of such launches on the
   // stream (a launch boundary every pairs x kBatch tokens costs next to nothing).
-  const long long cap = static_cast<long long>(pairs_dev) * mla_ring::kBatch;
+  const long long items = static_cast<long long>(pairs_dev) * mla_ring::kBatch;
+  const long long cap = items / n_splits > 0 ? items / n_splits : 1;
   // Q: boxes of [h rows x 64 columns] of one token; O: boxes of [32 rows x 64 columns] (a store that
   // reaches past row h is clipped)
   const uint32_t box_h = static_cast<uint32_t>(a->h < 128 ? a->h : 128);
@@ -861,19 +905,24 @@ int launch_sparse_mla_ring(const ftb_sparse_mla_args* a, cudaStream_t st) {
     p.scale_log2 = a->sm_scale * 1.4426950408889634f;
     p.lse_base2 = a->lse_base2;
     p.status = a->status;
+    p.n_splits = n_splits;
+    p.part_lse = part_lse + (n_splits > 1 ? static_cast<size_t>(t0) * n_splits * a->h : 0);
     const void* q0 = static_cast<const __nv_bfloat16*>(a->q) + t0 * a->q_stride_token;
     void* o0 = static_cast<__nv_bfloat16*>(a->out) + t0 * a->out_stride_token;
     CUtensorMap tm_q, tm_o;
     if (!make_tmap_3d(&tm_q, q0, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, mla_ring::kDqk, static_cast<uint64_t>(a->h),
                       static_cast<uint64_t>(n_tok), static_cast<uint64_t>(a->q_stride_head),
                       static_cast<uint64_t>(a->q_stride_token), 64, box_h) ||
-        !make_tmap_3d(&tm_o, o0, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, 512, static_cast<uint64_t>(a->h),
-                      static_cast<uint64_t>(n_tok), static_cast<uint64_t>(a->out_stride_head),
-                      static_cast<uint64_t>(a->out_stride_token), 64, box_h < 32 ? box_h : 32)) {
+        !(n_splits > 1 ? make_tmap_3d(&tm_o, part_out + static_cast<size_t>(t0) * n_splits * a->h * 512, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, 512,
+                                      static_cast<uint64_t>(a->h), static_cast<uint64_t>(n_tok) * n_splits, 512,
+                                      static_cast<uint64_t>(a->h) * 512, 32, box_h < 32 ? box_h : 32)
+                       : make_tmap_3d(&tm_o, o0, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, 512, static_cast<uint64_t>(a->h),
+                                      static_cast<uint64_t>(n_tok), static_cast<uint64_t>(a->out_stride_head),
+                                      static_cast<uint64_t>(a->out_stride_token), 64, box_h < 32 ? box_h : 32))) {
       set_last_error("sparse_mla_ring: cuTensorMapEncodeTiled failed");
       return FTB_ERR_CUDA;
     }
-    const int pairs = pairs_dev < n_tok ? pairs_dev : n_tok;
+    const int pairs = pairs_dev < n_tok * n_splits ? pairs_dev : n_tok * n_splits;
     cfg.gridDim = dim3(static_cast<unsigned>(pairs) * 2u);
     e = cudaLaunchKernelEx(&cfg, mla_ring::sparse_mla_ring_kernel, tm_q, tm_o, p);
     if (e != cudaSuccess) return check_cuda(e, "sparse_mla_ring launch");

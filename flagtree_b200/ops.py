@@ -7,6 +7,7 @@ shared library is missing the call raises.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from typing import Optional, Tuple
 
 import torch
@@ -29,13 +30,27 @@ def _stream_ptr(device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
-def _auto_splits(s_q: int, topk: int, device) -> int:
-    """Split the top-k axis when there are too few query tokens to fill the SMs (decode)."""
-    sms = torch.cuda.get_device_properties(device).multi_processor_count
-    tiles = max(1, (topk + 63) // 64)
-    if 2 * s_q >= sms:
+@functools.lru_cache(maxsize=1024)
+def _plan_splits(s_q: int, h: int, topk: int, pairs: int) -> int:
+    tiles = max(1, (topk + 127) // 128)
+    if s_q >= pairs:
         return 1
-    return int(max(1, min(16, sms // (2 * s_q), tiles)))
+
+    def cost(n):
+        waves = -(-s_q * n // pairs)
+        return 12.0 + waves * (2.0 + 2.2 * -(-tiles // n)) + (5.4 + 0.2 * s_q * n * h / 128 if n > 1 else 0.0)
+
+    return min(range(1, min(16, tiles) + 1), key=cost)
+
+
+def _auto_splits(s_q: int, h: int, topk: int, device) -> int:
+    """Parts into which the top-k axis of every token is cut.
+
+    The persistent kernel runs one item (a token, or a part of one) at a time on each pair of SMs.  Measured on a B200
+    (us): 12 per launch, 2 per item and 2.2 per tile of 128 rows in it; with parts 5.4 for the merge and 0.2 per item of
+    128 heads for the fp32 partials.  topk 2048, 128 heads, whole / in parts: 1 token 49 / 23 (16 parts), 10 tokens 49 / 33 (4),
+    20 tokens 50 / 44 (3), 37 tokens 51 / 55 (2), 74 tokens 54 / 95; 1 token of topk 256: 18.6 / 22."""
+    return _plan_splits(s_q, h, topk, max(1, torch.cuda.get_device_properties(device).multi_processor_count // 2))
 
 
 def _split_workspace(a, s_q: int, h: int, n_splits: int, device):
@@ -71,8 +86,8 @@ def sparse_mla_fwd(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor,
     (third_party/mthreads/python/test/wmma/test_accuracy_musa_vllm_mla.py:571-620) with the
     token table as `indices`.  `sm_scale` defaults to 576**-0.5 (:640 of the same file).
     `check=True` reads back the device status word (one host sync) and raises on a bad index
-    or a device-side timeout.  `num_splits` > 1 splits the top-k axis over several CTAs and merges the
-    partial results (the reference's NUM_KV_SPLITS stage 2); it selects the single-CTA kernel.
+    or a device-side timeout.  `num_splits` > 1 splits the top-k axis over several pairs of CTAs and merges the
+    partial results (the reference's NUM_KV_SPLITS stage 2); None = by the number of tokens.
     """
     _require_cuda(q, kv, indices)
     if kv.dim() == 3:
@@ -112,7 +127,10 @@ def sparse_mla_fwd(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor,
         a.status = status.data_ptr() if status is not None else None
         a.kv_is_fp8 = 0
         a.dbg_scores = _dbg_scores.data_ptr() if _dbg_scores is not None else None
-        _ws = _split_workspace(a, s_q, h1 - h0, int(num_splits) if num_splits else 1, q.device)
+        n_splits = int(num_splits) if num_splits else 1
+        if num_splits is None and algo == 0 and _dbg_scores is None:
+            n_splits = _auto_splits(s_q, h1 - h0, indices.shape[1], q.device)
+        _ws = _split_workspace(a, s_q, h1 - h0, n_splits, q.device)
         with torch.cuda.device(q.device):
             rc = lib.ftb_sparse_mla_fwd(C.byref(a), C.c_void_p(_stream_ptr(q.device)))
         _lib.check(rc, "sparse_mla_fwd")
@@ -213,7 +231,7 @@ def sparse_mla_fwd_paged(q: torch.Tensor, kv_cache: torch.Tensor, kv_scale: torc
     test_accuracy_musa_vllm_mla.py:278-283.  Returns (out [B,n_q,h,512] bf16, lse [B,n_q,h] fp32).
 
     `two_pass`: convert the selected rows to a compact bf16 table first and run the persistent bf16 kernel on
-    it (needs 1156 bytes of scratch per selected row); None = do so when the top-k axis is not split and the
+    it (needs 1156 bytes of scratch per selected row); None = do so when the
     scratch stays below 4 GiB, False = the one-pass kernel that converts while it gathers.
     """
     _require_cuda(q, kv_cache, kv_scale, block_table, context_lens, indices)
@@ -251,14 +269,19 @@ def sparse_mla_fwd_paged(q: torch.Tensor, kv_cache: torch.Tensor, kv_scale: torc
     a.page_size, a.q_per_seq, a.block_table_stride = page_size, n_q, block_table.stride(0)
     a.dbg_scores = None
     if num_splits is None:
-        num_splits = _auto_splits(b * n_q, idx2.shape[1], q.device)
-    _ws = _split_workspace(a, b * n_q, h, int(num_splits), q.device)
-    if int(num_splits) <= 1 and two_pass is not False:
-        need = int(_lib.load().ftb_sparse_mla_dequant_workspace_bytes(b * n_q, idx2.shape[1]))
-        if two_pass or need <= (4 << 30):
-            _ws = torch.empty(need, dtype=torch.uint8, device=q.device)
-            a.workspace, a.workspace_bytes = _ws.data_ptr(), need
-            a.algo_id = 6
+        num_splits = _auto_splits(b * n_q, h, idx2.shape[1], q.device)
+    n_splits = max(1, int(num_splits))
+    lib = _lib.load()
+    rows_bytes = int(lib.ftb_sparse_mla_dequant_workspace_bytes(b * n_q, idx2.shape[1]))
+    if two_pass or (two_pass is None and rows_bytes <= (4 << 30)):
+        # the dequantised rows, then (from a 16-byte boundary) the partial results of a split
+        need = rows_bytes
+        if n_splits > 1:
+            need = (rows_bytes + 15) // 16 * 16 + int(lib.ftb_sparse_mla_workspace_bytes(b * n_q, h, n_splits))
+        _ws = torch.empty(need, dtype=torch.uint8, device=q.device)
+        a.n_splits, a.workspace, a.workspace_bytes, a.algo_id = n_splits, _ws.data_ptr(), need, 6
+    else:
+        _ws = _split_workspace(a, b * n_q, h, n_splits, q.device)
     with torch.cuda.device(q.device):
         rc = _lib.load().ftb_sparse_mla_fwd(C.byref(a), C.c_void_p(_stream_ptr(q.device)))
     _lib.check(rc, "sparse_mla_fwd_paged")

@@ -94,11 +94,12 @@ typedef struct ftb_sparse_mla_args {
 
 FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* args, void* stream);
 FTB_API int64_t ftb_sparse_mla_workspace_bytes(int32_t s_q, int32_t h, int32_t n_splits);
-/* Paged FP8 form, two passes: when `workspace` holds at least this many bytes (16-byte aligned) and
- * n_splits <= 1, the selected rows are first converted to a compact bf16 table (row = token * topk + j,
+/* Paged FP8 form, two passes: when `workspace` holds at least this many bytes (16-byte aligned; with
+ * n_splits > 1 and algo_id 6, rounded up to 16 and followed by ftb_sparse_mla_workspace_bytes()),
+ * the selected rows are first converted to a compact bf16 table (row = token * topk + j,
  * the role of the dequantising loads of decode_attention_int4kv.py:345-450, done once per row instead of
  * inside the attention loop) and the persistent bf16 kernel runs on that table.  algo_id 6 demands this
- * path, algo_id 0 takes it when the workspace allows. */
+ * path, algo_id 0 takes it when the workspace allows and n_splits <= 1. */
 FTB_API int64_t ftb_sparse_mla_dequant_workspace_bytes(int32_t s_q, int32_t topk);
 /* Same operation for callers that cannot allocate device memory (an engine that owns the whole device
  * through its own pool, a sandboxed plugin, a latency path that must stay clear of the allocator).  It has

@@ -406,3 +406,38 @@ def test_paged_context_longer_than_block_table_is_reported():
     for two_pass in (False, True):
         with pytest.raises(RuntimeError, match="BAD_INDEX"):
             sparse_mla_fwd_paged(*args, c.sm_scale, page_size=c.page_size, check=True, num_splits=1, two_pass=two_pass)
+
+
+@pytest.mark.parametrize("s_q,h,topk,splits", [(1, 128, 2048, None), (1, 16, 130, None), (3, 128, 1000, 16), (40, 64, 300, 3),
+                                               (75, 128, 257, 2), (30, 8, 640, 64)])
+def test_parts_of_a_token_on_the_persistent_pairs(s_q, h, topk, splits):
+    """The top-k axis in parts: one tile per part, parts without a tile (short lists, more parts than tiles), more items than
+    pairs, tokens without an entry, trailing entries of no meaning behind the list, few heads, and the automatic choice."""
+    g = torch.Generator().manual_seed(s_q + topk)
+    s_kv = 3000
+    q = torch.randn(s_q, h, 576, generator=g).bfloat16()
+    kv = torch.randn(s_kv, 576, generator=g).bfloat16()
+    idx = torch.stack([torch.randperm(s_kv, generator=g)[:topk] for _ in range(s_q)]).int()
+    if s_q > 2:
+        idx[1, 100:] = -1
+        idx[2, :] = -1
+        idx[0, 3::5] = -1
+    out, lse = sparse_mla_fwd(q.to(DEV), kv.to(DEV), idx.to(DEV), 0.06, check=True, num_splits=splits)
+    ref_out, ref_lse = sparse_mla_fwd_ref(q, kv, idx, 0.06)
+    e_out, e_lse = _errors(out, lse, ref_out, ref_lse)
+    assert e_out <= OUT_ATOL and e_lse <= LSE_RTOL
+    _, lse2 = sparse_mla_fwd(q.to(DEV), kv.to(DEV), idx.to(DEV), 0.06, check=True, num_splits=splits, lse_base2=True)
+    assert torch.allclose(lse2.cpu() * 0.6931471805599453, lse.cpu(), rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("splits,two_pass", [(1, True), (4, True), (4, False), (None, None)])
+def test_paged_forms_agree(splits, two_pass):
+    """Two passes and parts of a token against the one-pass kernel on whole tokens; short contexts leave parts empty.  All forms
+    multiply the same rows rounded to bf16, with fp32 sums in another order: the LSE agrees to some 1e-5, the output to
+    roundings of P and of the result (2^-9 each, of values up to 1)."""
+    c = W.mla_cfg3(batch=3, n_q=2, h=64, topk=300, len_lo=40, len_hi=900)
+    args = (c.q.to(DEV), c.kv_cache.to(DEV), c.kv_scale.to(DEV), c.block_table.to(DEV), c.context_lens.to(DEV), c.indices.to(DEV), c.sm_scale)
+    ref_out, ref_lse = sparse_mla_fwd_paged(*args, page_size=c.page_size, check=True, num_splits=1, two_pass=False)
+    out, lse = sparse_mla_fwd_paged(*args, page_size=c.page_size, check=True, num_splits=splits, two_pass=two_pass)
+    assert (out.float() - ref_out.float()).abs().max().item() <= 1e-2
+    assert ((lse - ref_lse).abs() / ref_lse.abs().clamp(min=1)).max().item() <= 1e-4

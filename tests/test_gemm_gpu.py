@@ -33,6 +33,18 @@ def test_matmul_shapes(m, n, k):
     _check(a, b, f"{m}x{n}x{k}")
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 512, 512), (50, 7168, 2304), (64, 9472, 128), (127, 8, 520), (129, 4160, 2304), (512, 512, 1024),
+                                   (40, 4104, 584), (8, 136, 64), (300, 6152, 1000), (17, 2048, 72)])
+def test_products_with_few_tiles(m, n, k):
+    """Shapes that leave most SMs idle at 128 x 256: narrow tiles (64 and 128 columns, a last one of 8), K in one, two and four
+    parts with K tails and parts of unequal length, one to five row blocks, row counts that are not a multiple of eight."""
+    g = torch.Generator().manual_seed(m + n + k)
+    a = torch.randn(m, k, generator=g).bfloat16()
+    b = torch.randn(k, n, generator=g).bfloat16()
+    c = _check(a, b, f"{m}x{n}x{k}")
+    assert torch.equal(c, matmul(a.to(DEV), b.to(DEV)))
+
+
 @pytest.mark.parametrize("m,n,k", [(4096, 4864, 256), (2048, 9992, 128), (3072, 2560, 192)])
 def test_leftover_tiles_run_as_half_width_steps(m, n, k):
     """Shapes whose tile count leaves a few tiles after the whole waves of a 148-SM GPU: 304 = 4 x 74 + 8 pair

@@ -26,8 +26,28 @@ def _require_cuda(*tensors):
             raise ValueError("Pointer argument cannot be accessed from the device: expected CUDA tensors")
 
 
+# The handle of the current stream, without a Stream object around it where torch has the call.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream_ptr(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return _raw_stream(device.index) if _raw_stream is not None else torch.cuda.current_stream(device).cuda_stream
+
+
+def _launch(fn, args, device, what: str) -> None:
+    """fn(args, stream) on the current stream of `device`, with that device current."""
+    if device.index == torch.cuda.current_device():
+        rc = fn(C.byref(args), C.c_void_p(_stream_ptr(device)))
+    else:
+        with torch.cuda.device(device):
+            rc = fn(C.byref(args), C.c_void_p(_stream_ptr(device)))
+    if rc != 0:
+        _lib.check(rc, what)
+
+
+@functools.lru_cache(maxsize=64)
+def _pairs_of(index: int) -> int:
+    return max(1, torch.cuda.get_device_properties(index).multi_processor_count // 2)
 
 
 @functools.lru_cache(maxsize=1024)
@@ -50,7 +70,7 @@ def _auto_splits(s_q: int, h: int, topk: int, device) -> int:
     (us): 12 per launch, 2 per item and 2.2 per tile of 128 rows in it; with parts 5.4 for the merge and 0.2 per item of
     128 heads for the fp32 partials.  topk 2048, 128 heads, whole / in parts: 1 token 49 / 23 (16 parts), 10 tokens 49 / 33 (4),
     20 tokens 50 / 44 (3), 37 tokens 51 / 55 (2), 74 tokens 54 / 95; 1 token of topk 256: 18.6 / 22."""
-    return _plan_splits(s_q, h, topk, max(1, torch.cuda.get_device_properties(device).multi_processor_count // 2))
+    return _plan_splits(s_q, h, topk, _pairs_of(device.index))
 
 
 def _split_workspace(a, s_q: int, h: int, n_splits: int, device):
@@ -113,27 +133,17 @@ def sparse_mla_fwd(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor,
     lib = _lib.load()
     for h0 in range(0, h, 128):      # more than 128 heads: one launch per block of 128 heads
         h1 = min(h, h0 + 128)
-        qs, os_, ls = q[:, h0:h1], out[:, h0:h1], lse[:, h0:h1]
-        a = _lib.SparseMlaArgs()
-        a.q, a.kv, a.indices = qs.data_ptr(), kv.data_ptr(), indices.data_ptr()
-        a.out, a.lse = os_.data_ptr(), ls.data_ptr()
-        a.s_q, a.h, a.s_kv, a.topk = s_q, h1 - h0, kv.shape[0], indices.shape[1]
-        a.q_stride_token, a.q_stride_head = qs.stride(0), qs.stride(1)
-        a.kv_stride_row = kv.stride(0)
-        a.idx_stride_token = indices.stride(0)
-        a.out_stride_token, a.out_stride_head = os_.stride(0), os_.stride(1)
-        a.lse_stride_token = ls.stride(0)
-        a.sm_scale, a.lse_base2, a.algo_id = float(sm_scale), int(lse_base2), int(algo)
-        a.status = status.data_ptr() if status is not None else None
-        a.kv_is_fp8 = 0
-        a.dbg_scores = _dbg_scores.data_ptr() if _dbg_scores is not None else None
+        qs, os_, ls = (q, out, lse) if h <= 128 else (q[:, h0:h1], out[:, h0:h1], lse[:, h0:h1])
         n_splits = int(num_splits) if num_splits else 1
         if num_splits is None and algo == 0 and _dbg_scores is None:
             n_splits = _auto_splits(s_q, h1 - h0, indices.shape[1], q.device)
+        a = _lib.SparseMlaArgs(
+            qs.data_ptr(), kv.data_ptr(), indices.data_ptr(), os_.data_ptr(), ls.data_ptr(), s_q, h1 - h0, kv.shape[0],
+            indices.shape[1], qs.stride(0), qs.stride(1), kv.stride(0), indices.stride(0), os_.stride(0), os_.stride(1),
+            ls.stride(0), float(sm_scale), int(lse_base2), int(algo), status.data_ptr() if status is not None else None)
+        a.dbg_scores = _dbg_scores.data_ptr() if _dbg_scores is not None else None
         _ws = _split_workspace(a, s_q, h1 - h0, n_splits, q.device)
-        with torch.cuda.device(q.device):
-            rc = lib.ftb_sparse_mla_fwd(C.byref(a), C.c_void_p(_stream_ptr(q.device)))
-        _lib.check(rc, "sparse_mla_fwd")
+        _launch(lib.ftb_sparse_mla_fwd, a, q.device, "sparse_mla_fwd")
     _check_status(status, "sparse_mla_fwd")
     return out, lse
 
@@ -254,20 +264,11 @@ def sparse_mla_fwd_paged(q: torch.Tensor, kv_cache: torch.Tensor, kv_scale: torc
     out = torch.empty(b * n_q, h, D_V, dtype=torch.bfloat16, device=q.device)
     lse = torch.empty(b * n_q, h, dtype=torch.float32, device=q.device)
     status = torch.zeros(1, dtype=torch.int32, device=q.device) if check else None
-    a = _lib.SparseMlaArgs()
-    a.q, a.kv, a.indices, a.out, a.lse = q2.data_ptr(), kv_cache.data_ptr(), idx2.data_ptr(), out.data_ptr(), lse.data_ptr()
-    a.s_q, a.h, a.s_kv, a.topk = b * n_q, h, kv_cache.shape[0] * page_size, idx2.shape[1]
-    a.q_stride_token, a.q_stride_head = q2.stride(0), q2.stride(1)
-    a.kv_stride_row = D_QK
-    a.idx_stride_token = idx2.stride(0)
-    a.out_stride_token, a.out_stride_head = out.stride(0), out.stride(1)
-    a.lse_stride_token = lse.stride(0)
-    a.sm_scale, a.lse_base2, a.algo_id = float(sm_scale), int(lse_base2), 0
-    a.status = status.data_ptr() if status is not None else None
-    a.kv_is_fp8 = 1
-    a.kv_scale, a.block_table, a.context_lens = kv_scale.data_ptr(), block_table.data_ptr(), context_lens.data_ptr()
-    a.page_size, a.q_per_seq, a.block_table_stride = page_size, n_q, block_table.stride(0)
-    a.dbg_scores = None
+    a = _lib.SparseMlaArgs(
+        q2.data_ptr(), kv_cache.data_ptr(), idx2.data_ptr(), out.data_ptr(), lse.data_ptr(), b * n_q, h,
+        kv_cache.shape[0] * page_size, idx2.shape[1], q2.stride(0), q2.stride(1), D_QK, idx2.stride(0), out.stride(0), out.stride(1),
+        lse.stride(0), float(sm_scale), int(lse_base2), 0, status.data_ptr() if status is not None else None, 1, kv_scale.data_ptr(),
+        block_table.data_ptr(), context_lens.data_ptr(), page_size, n_q, block_table.stride(0))
     if num_splits is None:
         num_splits = _auto_splits(b * n_q, h, idx2.shape[1], q.device)
     n_splits = max(1, int(num_splits))
@@ -282,9 +283,7 @@ def sparse_mla_fwd_paged(q: torch.Tensor, kv_cache: torch.Tensor, kv_scale: torc
         a.n_splits, a.workspace, a.workspace_bytes, a.algo_id = n_splits, _ws.data_ptr(), need, 6
     else:
         _ws = _split_workspace(a, b * n_q, h, n_splits, q.device)
-    with torch.cuda.device(q.device):
-        rc = _lib.load().ftb_sparse_mla_fwd(C.byref(a), C.c_void_p(_stream_ptr(q.device)))
-    _lib.check(rc, "sparse_mla_fwd_paged")
+    _launch(_lib.load().ftb_sparse_mla_fwd, a, q.device, "sparse_mla_fwd_paged")
     _check_status(status, "sparse_mla_fwd_paged")
     return out.view(b, n_q, h, D_V), lse.view(b, n_q, h)
 
@@ -338,16 +337,11 @@ def sparse_mla_merge(part_out: torch.Tensor, part_lse: torch.Tensor, *, lse_base
         lse = torch.empty(s_q, h, dtype=torch.float32, device=part_out.device)
     assert out.shape == (s_q, h, D_V) and out.dtype == torch.bfloat16 and out.stride(2) == 1
     assert lse.shape == (s_q, h) and lse.dtype == torch.float32 and lse.stride(1) == 1
-    a = _lib.SparseMlaMergeArgs()
-    a.part_out, a.part_lse, a.out, a.lse = part_out.data_ptr(), part_lse.data_ptr(), out.data_ptr(), lse.data_ptr()
-    a.s_q, a.h, a.n_parts = s_q, h, n_parts
-    a.part_is_fp32, a.lse_base2 = int(part_out.dtype == torch.float32), int(lse_base2)
-    a.part_stride_part, a.part_stride_token, a.part_stride_head = part_out.stride(0), part_out.stride(1), part_out.stride(2)
-    a.lse_stride_part, a.lse_stride_part_token = part_lse.stride(0), part_lse.stride(1)
-    a.out_stride_token, a.out_stride_head, a.lse_stride_token = out.stride(0), out.stride(1), lse.stride(0)
-    with torch.cuda.device(part_out.device):
-        rc = _lib.load().ftb_sparse_mla_merge(C.byref(a), C.c_void_p(_stream_ptr(part_out.device)))
-    _lib.check(rc, "sparse_mla_merge")
+    a = _lib.SparseMlaMergeArgs(
+        part_out.data_ptr(), part_lse.data_ptr(), out.data_ptr(), lse.data_ptr(), s_q, h, n_parts,
+        int(part_out.dtype == torch.float32), int(lse_base2), part_out.stride(0), part_out.stride(1), part_out.stride(2),
+        part_lse.stride(0), part_lse.stride(1), out.stride(0), out.stride(1), lse.stride(0))
+    _launch(_lib.load().ftb_sparse_mla_merge, a, part_out.device, "sparse_mla_merge")
     return out, lse
 
 
@@ -373,14 +367,9 @@ def topk_indices(scores: torch.Tensor, topk: int, lengths: Optional[torch.Tensor
     if out is None:
         out = torch.empty(s_q, topk, dtype=torch.int32, device=scores.device)
     assert out.shape == (s_q, topk) and out.dtype == torch.int32 and out.stride(1) == 1
-    a = _lib.TopkArgs()
-    a.scores, a.out = scores.data_ptr(), out.data_ptr()
-    a.lengths = lengths.data_ptr() if lengths is not None else None
-    a.s_q, a.s_kv, a.topk = s_q, s_kv, int(topk)
-    a.scores_stride_token, a.out_stride_token = scores.stride(0), out.stride(0)
-    with torch.cuda.device(scores.device):
-        rc = _lib.load().ftb_topk_indices(C.byref(a), C.c_void_p(_stream_ptr(scores.device)))
-    _lib.check(rc, "topk_indices")
+    a = _lib.TopkArgs(scores.data_ptr(), lengths.data_ptr() if lengths is not None else None, out.data_ptr(), s_q, s_kv,
+                      int(topk), scores.stride(0), out.stride(0))
+    _launch(_lib.load().ftb_topk_indices, a, scores.device, "topk_indices")
     return out
 
 
@@ -405,15 +394,10 @@ def kv_cache_write_fp8(rows: torch.Tensor, slot_mapping: torch.Tensor, kv_cache:
     num_pages = kv_cache.shape[0]
     ws = torch.empty(int(lib.ftb_kv_cache_write_workspace_bytes(num_pages)), dtype=torch.uint8, device=rows.device)
     status = torch.zeros(1, dtype=torch.int32, device=rows.device) if check else None
-    a = _lib.KvCacheWriteArgs()
-    a.rows, a.slot_mapping, a.kv_cache, a.kv_scale = rows.data_ptr(), slot_mapping.data_ptr(), kv_cache.data_ptr(), kv_scale.data_ptr()
-    a.n_rows, a.num_pages, a.page_size = rows.shape[0], num_pages, page_size
-    a.row_stride = rows.stride(0)
-    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-    a.status = status.data_ptr() if status is not None else None
-    with torch.cuda.device(rows.device):
-        rc = lib.ftb_kv_cache_write_fp8(C.byref(a), C.c_void_p(_stream_ptr(rows.device)))
-    _lib.check(rc, "kv_cache_write_fp8")
+    a = _lib.KvCacheWriteArgs(rows.data_ptr(), slot_mapping.data_ptr(), kv_cache.data_ptr(), kv_scale.data_ptr(), rows.shape[0],
+                              num_pages, page_size, rows.stride(0), ws.data_ptr(), ws.numel(),
+                              status.data_ptr() if status is not None else None)
+    _launch(lib.ftb_kv_cache_write_fp8, a, rows.device, "kv_cache_write_fp8")
     _check_status(status, "kv_cache_write_fp8")
 
 
@@ -445,14 +429,10 @@ def matmul(a: torch.Tensor, b: torch.Tensor, acc_dtype=None, input_precision=Non
 
 
 def _gemm_into(a, b, c, status=None):
-    g = _lib.GemmArgs()
-    g.a, g.b, g.c = a.data_ptr(), b.data_ptr(), c.data_ptr()
-    g.m, g.n, g.k = a.shape[0], b.shape[1], a.shape[1]
-    g.lda, g.ldb, g.ldc = a.stride(0), b.stride(0), c.stride(0)
-    g.status = status.data_ptr() if status is not None else None
-    with torch.cuda.device(a.device):
-        rc = _lib.load().ftb_gemm_bf16(C.byref(g), C.c_void_p(_stream_ptr(a.device)))
-    _lib.check(rc, "matmul")
+    m, k = a.shape
+    g = _lib.GemmArgs(a.data_ptr(), b.data_ptr(), c.data_ptr(), m, b.shape[1], k, a.stride(0), b.stride(0), c.stride(0),
+                      status.data_ptr() if status is not None else None)
+    _launch(_lib.load().ftb_gemm_bf16, g, a.device, "matmul")
 
 
 def matmul_fp8_blockscaled(a: torch.Tensor, a_scale: torch.Tensor, b: torch.Tensor, b_scale: torch.Tensor, *,
@@ -476,16 +456,10 @@ def matmul_fp8_blockscaled(a: torch.Tensor, a_scale: torch.Tensor, b: torch.Tens
     assert b.stride(1) == 1 or b.stride(0) == 1, "b must be contiguous along N or along K"
     if out is None:
         out = torch.empty(m, n, dtype=torch.bfloat16, device=a.device)
-    g = _lib.GemmFp8Args()
-    g.a, g.b, g.c, g.a_scale, g.b_scale = a.data_ptr(), b.data_ptr(), out.data_ptr(), a_scale.data_ptr(), b_scale.data_ptr()
-    g.m, g.n, g.k = m, n, k
-    g.lda, g.ldb, g.ldc = a.stride(0), (b.stride(1) if b_kmajor else b.stride(0)), out.stride(0)
-    g.a_scale_ld, g.b_scale_ld = a_scale.stride(0), b_scale.stride(0)
-    g.status = None
-    g.b_kmajor = 1 if b_kmajor else 0
-    with torch.cuda.device(a.device):
-        rc = _lib.load().ftb_gemm_fp8_blockscaled(C.byref(g), C.c_void_p(_stream_ptr(a.device)))
-    _lib.check(rc, "matmul_fp8_blockscaled")
+    g = _lib.GemmFp8Args(a.data_ptr(), b.data_ptr(), out.data_ptr(), a_scale.data_ptr(), b_scale.data_ptr(), m, n, k,
+                         a.stride(0), b.stride(1) if b_kmajor else b.stride(0), out.stride(0), a_scale.stride(0),
+                         b_scale.stride(0), None, 1 if b_kmajor else 0)
+    _launch(_lib.load().ftb_gemm_fp8_blockscaled, g, a.device, "matmul_fp8_blockscaled")
     return out
 
 

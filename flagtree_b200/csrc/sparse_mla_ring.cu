@@ -102,7 +102,7 @@ struct Misc0 {   // CTA 0
   unsigned long long k_full[kNK];   // one arrival per gather thread (when its copies have landed; the tile load of a Q entry counts on one of them)
   unsigned long long k_free[kNK];   // tcgen05.commit behind the entry's MMAs or its copy to tensor memory
   unsigned long long s_full[2];     // tcgen05.commit
-  unsigned long long s_free[2];     // 8 softmax warps
+  unsigned long long s_free[2];     // softmax warps with heads (8 when h > 96)
   unsigned long long q8_full;       // the token's rope block of Q has landed
   unsigned long long q8_free;       // tcgen05.commit behind the token's last tile
   unsigned long long p_free[2];     // relay warp of CTA 1 (remote arrival)
@@ -121,10 +121,10 @@ struct Misc0 {   // CTA 0
 struct Misc1 {   // CTA 1
   unsigned long long v_full[kNV];   // one arrival per gather thread, when its copies have landed
   unsigned long long v_free[kNV];   // tcgen05.commit
-  unsigned long long p_full[2];     // 8 softmax warps of CTA 0 (remote arrivals, each announcing its bulk copies: 4 KB of P, 128 B of factors)
-  unsigned long long corr_done[2];  // 4 correction warps
+  unsigned long long p_full[2];     // softmax warps with heads of CTA 0 (remote arrivals, each announcing its bulk copies: 4 KB of P, 128 B of factors)
+  unsigned long long corr_done[2];  // correction warps with heads
   unsigned long long pv_done[2];    // tcgen05.commit
-  unsigned long long fin[2];        // 8 softmax warps of CTA 0: 1/l of token t (t % 2) is in place
+  unsigned long long fin[2];        // softmax warps with heads of CTA 0: 1/l of token t (t % 2) is in place
   unsigned long long o_free;        // 16 epilogue warps: the accumulator has been read
   unsigned long long stg_free[8];   // epilogue warp w < 8: its staging piece is free for warp 9 + w
   unsigned long long epi_cnt;       // 16 epilogue warps: the output of the token has left the staging area
@@ -226,12 +226,16 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
   unsigned short* nt = cta == 0 ? m0->nt : m1->nt;
   int* last = cta == 0 ? m0->last : m1->last;
 
+  // 32-row quarters of the 128 head rows that hold heads: the softmax and correction warps of the others have nothing to do
+  const int row_warps = (p.h + 31) >> 5;
+  const bool has_rows = (warp & 3) < row_warps;
+
   if (tid == 0) {
     *abort_flag = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
     if (cta == 0) {
       m0->bad_index = 0;
       for (int i = 0; i < kNK; ++i) { mbar_init(smem_u32(&m0->k_full[i]), 32); mbar_init(smem_u32(&m0->k_free[i]), 1); }
-      for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&m0->s_full[i]), 1); mbar_init(smem_u32(&m0->s_free[i]), 8); }
+      for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&m0->s_full[i]), 1); mbar_init(smem_u32(&m0->s_free[i]), 2 * row_warps); }
       mbar_init(smem_u32(&m0->q8_full), 1);
       mbar_init(smem_u32(&m0->q8_free), 1);
       for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&m0->p_free[i]), 1); mbar_init(smem_u32(&m0->epi_done[i]), 1); }
@@ -239,10 +243,10 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
     } else {
       for (int i = 0; i < kNV; ++i) { mbar_init(smem_u32(&m1->v_full[i]), 64); mbar_init(smem_u32(&m1->v_free[i]), 1); }
       for (int i = 0; i < 2; ++i) {
-        mbar_init(smem_u32(&m1->p_full[i]), 8);
-        mbar_init(smem_u32(&m1->corr_done[i]), 4);
+        mbar_init(smem_u32(&m1->p_full[i]), 2 * row_warps);
+        mbar_init(smem_u32(&m1->corr_done[i]), row_warps);
         mbar_init(smem_u32(&m1->pv_done[i]), 1);
-        mbar_init(smem_u32(&m1->fin[i]), 8);
+        mbar_init(smem_u32(&m1->fin[i]), 2 * row_warps);
       }
       mbar_init(smem_u32(&m1->o_free), 16);
       for (int i = 0; i < 8; ++i) mbar_init(smem_u32(&m1->stg_free[i]), 1);
@@ -331,7 +335,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
     if (cta == 0) {
       // ===================================================================== CTA 0: scores
       const uint32_t k_s = base + kOff0K;
-      if (warp < 8) {
+      if (warp < 8 && has_rows) {
         // -------------------------------------------------------------- softmax (two threads per head row)
         // thread tid: head row = tid % 128 (TMEM lane), columns 64*(tid/128) .. +63 of the tile
         const int rowi = tid & 127;
@@ -382,7 +386,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
               for (int j = 0; j < 32; j += 2) mx = fmaxf(mx, fmaxf(__uint_as_float(sr[q][j]), __uint_as_float(sr[q][j + 1])));
             }
             m0->xchg[b][tid] = mx;
-            named_bar_sync(2, 256);
+            named_bar_sync(2 + (warp & 3), 64);
             mx = fmaxf(mx, m0->xchg[b][tid ^ 128]);
             // Lazy maximum: only move the reference when it grows by more than 2^8, so that the
             // accumulator in the other CTA is rarely rescaled (P stays below 256, exact enough in bf16/fp32).
@@ -433,11 +437,11 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
           }
           gt += n_tiles;
           // end of the token: combine the two halves of every row sum; 1/l goes to CTA 1, LSE is written here
-          named_bar_sync(2, 256);
+          named_bar_sync(2 + (warp & 3), 64);
           m0->xchg[0][tid] = l_run;
-          named_bar_sync(2, 256);
+          named_bar_sync(2 + (warp & 3), 64);
           const float l_tot = l_run + m0->xchg[0][tid ^ 128];
-          named_bar_sync(2, 256);   // xchg[0] may be written again by the first tile of the next token
+          named_bar_sync(2 + (warp & 3), 64);   // xchg[0] may be written again by the first tile of the next token
           if (ch == 0) {
             const float inv_l = (l_tot > 0.0f) ? 1.0f / l_tot : 0.0f;
             st_cluster_f32(invl_remote + ((ti & 1) * 128 + rowi) * 4, inv_l);
@@ -644,8 +648,9 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
           }
           __syncwarp();
         };
+        if (!has_rows && lane == 0) mbar_arrive(smem_u32(&m1->o_free));
 #pragma unroll 1
-        for (int cb = 0; cb < 2; ++cb) {
+        for (int cb = 0; cb < 2 && has_rows; ++cb) {
 #pragma unroll
           for (int c2 = 0; c2 < 2; ++c2) {
             uint32_t acc[32];
@@ -690,7 +695,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
           const int ti = batch0 + t;
           const int item = pair + ti * n_pairs;
           const int n_tiles = warp_uniform(nt[t]);
-          if (warp < 4) {
+          if (warp < 4 && has_rows) {
             // ------------------------------------------------------------ correction (thread = head)
             for (int i = 0; i < n_tiles; ++i) {
               const uint32_t G = gt + i;

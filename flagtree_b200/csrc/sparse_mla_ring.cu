@@ -1,18 +1,17 @@
-// Top-k sparse MLA forward, persistent role-split CTA pairs (bf16 KV), one ring for K and Q.
+// Top-k sparse MLA forward, persistent role-split CTA pairs (bf16 KV).
 //
 // One pair of CTAs (a cluster of 2) walks through query tokens pair, pair + pairs, ...  CTA 0 computes
-// S = Q.K^T (Q in tensor memory, K column blocks from a ring in shared memory filled by cp.async row gathers) and the
+// S = Q.K^T (Q in tensor memory, K column blocks gathered into shared memory by cp.async) and the
 // softmax; P travels to CTA 1 by bulk copies over distributed shared memory; CTA 1 accumulates O += P.V in
 // tensor memory and writes the output.  Every barrier keeps counting across tokens.
 //
-// The ring of CTA 0.  Ten slots of [128 rows x 128 B] hold a stream of entries that the MMA issuer consumes strictly in
-// order: per token eight Q entries (64-column blocks of the token's query rows, fetched by a TMA tile load and moved
-// on to tensor memory by the issuer itself with tcgen05.cp, which runs in order with its MMAs) and then nine K entries per
-// tile of 128 selected rows (one 64-column block each, multiplied by four MMAs).  Entry n lives in slot n % 10; the commit
-// behind an entry frees its slot.  The ninth (rope) block of Q stays in a buffer of its own in shared memory and is
-// multiplied from there: that leaves 256 columns of tensor memory for two score buffers, so that the issuer starts the next
-// tile while the softmax fetches this one (the hand-over of a single buffer cost 550 cycles per tile).  The next token's
-// Q needs no special case: its entries follow the last tile's in the ring, and the token after it is asked into L2.
+// The slots of CTA 0.  Nine slots of [128 rows x 128 B], one per 64-column block: per token the blocks of the token's query
+// rows pass through (fetched by a TMA tile load and moved on to tensor memory by the issuer itself with tcgen05.cp,
+// which runs in order with its MMAs), then a K block per tile of 128 selected rows, multiplied by four MMAs; the commit behind a
+// block frees its slot.  The ninth (rope) block of Q stays in a buffer of its own in shared memory and is multiplied from
+// there: that leaves 256 columns of tensor memory for two score buffers, so that the issuer starts the next tile while the
+// softmax fetches this one (the hand-over of a single buffer cost 550 cycles per tile).  The next token's Q blocks follow the
+// last tile's K blocks into the slots, and the token after it is asked into L2.
 //
 // Gather warps.  One warp per column block of K (nine) and per half slab of V (eight) copies rows with 16-byte cp.async:
 // the lanes keep the tile's row numbers and pass them round with shuffles.  148 SMs fetch random rows at 70 bytes
@@ -21,13 +20,14 @@
 // three schedulers that the MMA issuer is not on.  cp.async writes through the generic proxy, so the issuers fence
 // (fence.proxy.async) between the barrier wait and their MMAs.
 //
-// What bounds it: instruction supply, not memory or the tensor pipe (32 % busy).  Seventeen warps run ten different
-// roles, and a warp that has a scheduler's instruction cache to share runs 5 or more cycles per instruction; fully unrolled
-// role loops with a private copy of the wait loop each (95 KB of code) kept a third of all warps stalled on
-// instruction fetch.  So every role has one rolled loop, the softmax has one path (masked entries become -inf once) with
-// two-wide fp32 instructions, role state is warp-uniform, and the issuer waits for three entries at once (a wait with its
-// fences costs it 350 cycles, twelve MMAs take 768).  740 tokens, 128 heads, topk 2048: 832 -> 1065 TFLOP/s (one launch
-// alone); prefill of 4096 causal tokens, back to back under the power limit: 2247 -> 2036 us; one token: 58.8 -> 50.3 us.
+// What bounds it: instruction supply, not memory or the tensor pipe.  Seventeen warps run ten different roles, and a
+// warp that has a scheduler's instruction cache to share runs 5 or more cycles per instruction; fully unrolled role loops with
+// a private copy of the wait loop each (95 KB of code) kept a third of all warps stalled on instruction fetch.  So every
+// role but the MMA issue has one rolled loop, the softmax has one path (masked entries become -inf once) with two-wide
+// fp32 instructions, loop counts are warp-uniform, and the issuer has constant addresses and waits for three blocks at once.
+// Warps whose 32 head rows hold no head take no part.  One launch alone, 740 tokens, 128 heads, topk 2048: 832 -> 1065
+// TFLOP/s.  Back to back: 4096 causal tokens 2243 -> 2022 us; 1999 tokens of 16 heads 1319 -> 965 us (1159 with all rows
+// at work, 1076 with a ring of ten slots and computed addresses).
 //
 // Few tokens.  A launch may cut the top-k list of every token in parts; an item of work is then a part of a token, its result
 // leaves as fp32 (32 columns per TMA store instead of 64) with a base-2 LSE, and a second kernel merges the parts.  One token
@@ -61,7 +61,7 @@ constexpr int kNChunk = 9;
 constexpr int kNT = 128;                       // gathered rows per tile
 constexpr int kQBlock = 128 * 128;             // 16384: [128 heads x 128 B]
 constexpr int kNQ = 8;                         // 64-column blocks of Q that live in tensor memory; the ninth (rope) stays in shared memory
-constexpr int kNK = 10;                        // ring slots of CTA 0: entry n (a Q block or a K block of a tile) lives in slot n % 10
+constexpr int kNK = kNChunk;                   // slots of CTA 0: column block c of Q or of a tile's K lives in slot c
 constexpr int kKSlot = kNT * 128;              // 16384: [128 rows x 128 B]
 constexpr int kNV = 4;                         // V ring slots: one whole tile, slab s in slot s
 constexpr int kVSlabRows = 32;
@@ -69,11 +69,11 @@ constexpr int kVBlock = kVSlabRows * 128;      // 4096: one 64-column block of a
 constexpr int kVSlab = 8 * kVBlock;            // 32768
 constexpr int kPBuf = 2 * kQBlock;             // 32768: P [128 heads x 128 rows] bf16 as two 64-row blocks
 constexpr int kBatch = 64;                     // tokens whose tile counts are found in one go
-// CTA 0 layout: ring of 10 slots | rope block of Q | P staging | misc.
+// CTA 0 layout: nine slots | rope block of Q | P staging | misc.
 // CTA 1 layout: V ring | P x 2 | misc; between tokens the P buffer of the last tile stages O.
 constexpr int kOff0K = 0;
-constexpr int kOff0Q8 = kOff0K + kNK * kKSlot;             // 163840
-constexpr int kOff0P = kOff0Q8 + kQBlock;                  // 180224
+constexpr int kOff0Q8 = kOff0K + kNK * kKSlot;             // 147456
+constexpr int kOff0P = kOff0Q8 + kQBlock;                  // 163840
 constexpr int kOff0Misc = kOff0P + kPBuf;                  // 212992
 constexpr int kOff1P = kNV * kVSlab;                       // 131072
 constexpr int kOff1Misc = kOff1P + 2 * kPBuf;              // 196608
@@ -139,7 +139,6 @@ struct Misc1 {   // CTA 1
 static_assert(sizeof(Misc0) <= 4096 && sizeof(Misc1) <= 4096, "misc area");
 static_assert(kOff1Misc + 4096 + 1024 <= kSmemBytes, "CTA 1 layout fits");
 static_assert(kNV == kNT / kVSlabRows, "V ring slot index = slab index");
-static_assert(kNK > kNChunk && kNK < 2 * kNChunk, "a ring position advances by one tile with a single wrap test");
 
 // the same value in every lane, made visible to the compiler: loop counts and role state then stay in uniform registers
 __device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
@@ -186,14 +185,6 @@ __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
       : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return r;
 }
-// position of a role in the stream of ring entries: slot = n % kNK, use = n / kNK
-struct RingPos {
-  uint32_t slot, use;
-  __device__ __forceinline__ void advance(uint32_t by) {   // by < kNK
-    slot += by;
-    if (slot >= static_cast<uint32_t>(kNK)) { slot -= kNK; ++use; }
-  }
-};
 // bulk copy local shared memory -> shared memory of another CTA; completes (byte count) on that CTA's barrier
 __device__ __forceinline__ void bulk_copy_to_cluster(uint32_t dst_cluster, uint32_t src_cta, uint32_t bytes, uint32_t bar_cluster) {
   asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -292,10 +283,6 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
   // CTA 0: the nine gather warps, one per column block: the warps 9-19 whose id is not 0 modulo 4, in order (they share no
   // scheduler with the MMA issuer, warp 8)
   const int prod = (warp >= 9 && (warp & 3) != 0) ? (warp - 9) - ((warp - 8) >> 2) : -1;
-  RingPos pos;       // CTA 0, issuer and producers: position in the stream of ring entries
-  pos.slot = (cta == 0 && prod >= 0) ? static_cast<uint32_t>(prod) : 0u;
-  pos.use = 0;
-
   for (int batch0 = 0; batch0 < my_tokens; batch0 += kBatch) {
     const int nb = min(kBatch, my_tokens - batch0);
     // ------------------------------------------------------------------ tiles per token of this batch
@@ -457,77 +444,73 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
       } else if (warp == 8) {
         // -------------------------------------------------------------- ring consumer: Q copies and Q.K^T
         // The whole warp runs the loop and waits; an elected lane (always the same one, so that its commits
-        // cover its MMAs and copies) issues.  Per token: eight Q entries, each moved to its 32 columns of tensor memory by
+        // cover its MMAs and copies) issues.  Per token: eight Q blocks, each moved to its 32 columns of tensor memory by
         // four tcgen05.cp (they run in order behind the MMAs issued before them, so the previous token's last tile
-        // has read the block by then), then nine K entries per tile with four MMAs each.  The commit behind an entry
-        // frees its slot.  The tensor pipe takes four MMAs ahead of the one it executes (256 cycles), while a wait, its
-        // fences and the issue of four MMAs by a lone warp take about 340: so the warp waits for a group of entries
-        // at once, lane by lane, and issues twelve MMAs behind one wait.
+        // has read the block by then), then nine K blocks per tile with four MMAs each.  The commit behind a block
+        // frees its slot.  The tensor pipe takes four MMAs ahead of the one it executes (256 cycles), while a wait and its
+        // fences take a lone warp about 300: so the warp waits for three blocks at once, lane by lane, and issues
+        // twelve MMAs behind one wait.  A block has a slot of its own, so every address of a tile is a constant off the base:
+        // with a ring of ten slots the address arithmetic alone made an MMA cost 82 cycles of issue, against 64 of execution.
         {
           constexpr uint32_t kIdesc = umma_idesc(kFmtBF16, 128, kNT, 0, 0);
           const uint64_t bd0 = smem_desc_sw128(k_s, 16, 1024);
           const uint64_t qd0 = smem_desc_sw128(base + kOff0Q8, 16, 1024);
           const uint32_t bd_lo = static_cast<uint32_t>(bd0), bd_hi = static_cast<uint32_t>(bd0 >> 32);
+          const uint32_t qd_lo = static_cast<uint32_t>(qd0), qd_hi = static_cast<uint32_t>(qd0 >> 32);
           const uint32_t t_q = tmem + kColQ;
           const uint32_t k_full0 = smem_u32(&m0->k_full[0]), k_free0 = smem_u32(&m0->k_free[0]);
-          auto wait_group = [&](uint32_t n) {                // entries pos .. pos + n - 1 (n <= 4): lane l waits for entry l % n
-            RingPos at = pos;
-            at.advance(static_cast<uint32_t>(lane) % n);
-            mbar_wait(k_full0 + at.slot * 8, at.use & 1u, abort_flag);
-            __syncwarp();
-            fence_proxy_async_smem();                        // the rows were written by cp.async (generic proxy)
-            tc_fence_after();
-          };
+          const uint32_t wait_at = k_full0 + (lane % 3) * 8;
+          // uses of a slot before token ti and tile G: slots 0-7 G tiles and ti blocks of Q, slot 8 G tiles
 #pragma unroll 1
           for (int t = 0; t < nb; ++t) {
+            const int ti = batch0 + t;
             const int n_tiles = warp_uniform(nt[t]);
-#pragma unroll 1
-            for (int c0 = 0; c0 < kNQ; c0 += 4) {
-              wait_group(4);
+            mbar_wait(k_full0 + (lane & 7) * 8, (gt + ti) & 1u, abort_flag);
+            __syncwarp();
+            fence_proxy_async_smem();
+            tc_fence_after();
+            if (elect_one()) {
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                if (elect_one()) {
-                  const uint32_t lo = bd_lo + ((pos.slot * kKSlot) >> 4);
+              for (int cc = 0; cc < kNQ; ++cc) {
 #pragma unroll
-                  for (int k = 0; k < 4; ++k) tmem_cp_128x256b(t_q + (c0 + j) * 32 + k * 8, lo + ((k * 32) >> 4), bd_hi);
-                  umma_commit(k_free0 + pos.slot * 8);
-                }
-                __syncwarp();
-                pos.advance(1);
+                for (int k = 0; k < 4; ++k) tmem_cp_128x256b(t_q + cc * 32 + k * 8, bd_lo + ((cc * kKSlot + k * 32) >> 4), bd_hi);
+                umma_commit(k_free0 + cc * 8);
               }
             }
+            __syncwarp();
 #pragma unroll 1
             for (int i = 0; i < n_tiles; ++i) {
               const uint32_t G = gt + i;
-              const uint32_t b = G & 1u;
+              const uint32_t b = G & 1u, par = (G + ti + 1) & 1u;
               const uint32_t t_s = tmem + kColS + b * kNT;
               // score buffer b: the softmax of tile G-2 has copied it to registers
               if (G >= 2) mbar_wait(smem_u32(&m0->s_free[b]), ((G >> 1) & 1u) ^ 1u, abort_flag);
-#pragma unroll 1
-              for (int c0 = 0; c0 < kNChunk; c0 += 3) {
-                if (c0 == 6 && i == 0) mbar_wait(smem_u32(&m0->q8_full), (batch0 + t) & 1u, abort_flag);
-                wait_group(3);
 #pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                  if (elect_one()) {
-                    const uint32_t lo = bd_lo + ((pos.slot * kKSlot) >> 4);
+              for (int c0 = 0; c0 < kNChunk; c0 += 3) {
+                if (c0 == 6 && i == 0) mbar_wait(smem_u32(&m0->q8_full), ti & 1u, abort_flag);
+                mbar_wait(wait_at + c0 * 8, c0 == 6 && lane % 3 == 2 ? b : par, abort_flag);
+                __syncwarp();
+                fence_proxy_async_smem();                    // the rows were written by cp.async (generic proxy)
+                tc_fence_after();
+                if (elect_one()) {
+#pragma unroll
+                  for (int cc = c0; cc < c0 + 3; ++cc) {
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                      const uint64_t bd = (static_cast<uint64_t>(bd_hi) << 32) | (lo + ((k * 32) >> 4));
-                      if (j == 2 && c0 == 6) umma_f16_ss(t_s, qd0 + ((k * 32) >> 4), bd, kIdesc, 1u);
-                      else umma_f16_ts(t_s, t_q + (c0 + j) * 32 + k * 8, bd, kIdesc, (j | k) == 0 ? static_cast<uint32_t>(c0) : 1u);
+                      const uint32_t lo = bd_lo + ((cc * kKSlot + k * 32) >> 4);
+                      if (cc == kNQ) umma_f16_ss_lohi<true>(t_s, qd_lo + ((k * 32) >> 4), qd_hi, lo, bd_hi, kIdesc);
+                      else if (cc == 0 && k == 0) umma_f16_ts_lohi<false>(t_s, t_q, lo, bd_hi, kIdesc);
+                      else umma_f16_ts_lohi<true>(t_s, t_q + cc * 32 + k * 8, lo, bd_hi, kIdesc);
                     }
-                    umma_commit(k_free0 + pos.slot * 8);
+                    umma_commit(k_free0 + cc * 8);
                   }
-                  __syncwarp();
-                  pos.advance(1);
+                  if (c0 == 6) {
+                    umma_commit(smem_u32(&m0->s_full[b]));
+                    if (i == n_tiles - 1) umma_commit(smem_u32(&m0->q8_free));
+                  }
                 }
+                __syncwarp();
               }
-              if (elect_one()) {
-                umma_commit(smem_u32(&m0->s_full[b]));
-                if (i == n_tiles - 1) umma_commit(smem_u32(&m0->q8_free));
-              }
-              __syncwarp();
             }
             gt += n_tiles;
           }
@@ -535,17 +518,17 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
       } else if (prod >= 0) {
         // -------------------------------------------------------------- ring producers
         // Producer c supplies block c of every token's Q (a TMA tile load) and of every tile (32 copies of 16 bytes per lane:
-        // lane l copies piece l % 8 of rows 4 q + l / 8), in the order of the ring: its entries are c, c + 9, c + 18, ...
-        // A slot is free once the commit behind the entry that used it last has arrived (k_free); the parity wait is exact
-        // because the entry ten places back is at most one phase away.  Block c of the token after this one is asked
-        // into L2 when this token's is loaded.
+        // lane l copies piece l % 8 of rows 4 q + l / 8) into slot c.  The slot is free once the commit behind its last use has
+        // arrived (k_free); the parity wait is exact because that use is at most one phase away.  Block c of the token
+        // after this one is asked into L2 when this token's is loaded.
         const int c = prod;
+        const uint32_t k_full = smem_u32(&m0->k_full[c]), k_free = smem_u32(&m0->k_free[c]);
         const __nv_bfloat16* src0 = p.kv + c * 64 + (lane & 7) * 8;
         uint32_t dst0[2];                                    // rows 8 m + 0..3 and 8 m + 4..7 (the 128-byte swizzle goes with row % 8)
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           const int r = 4 * q + (lane >> 3);
-          dst0[q] = k_s + r * 128 + (((lane & 7) ^ r) << 4);
+          dst0[q] = k_s + c * kKSlot + r * 128 + (((lane & 7) ^ r) << 4);
         }
 #pragma unroll 1
         for (int t = 0; t < nb; ++t) {
@@ -560,9 +543,9 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
           {
             uint32_t full, dst;
             if (c < kNQ) {
-              if (pos.use >= 1) mbar_wait(smem_u32(&m0->k_free[pos.slot]), (pos.use - 1) & 1u, abort_flag);
-              full = smem_u32(&m0->k_full[pos.slot]);
-              dst = k_s + pos.slot * kKSlot;
+              if (gt + ti >= 1) mbar_wait(k_free, (gt + ti - 1) & 1u, abort_flag);
+              full = k_full;
+              dst = k_s + c * kKSlot;
             } else {
               if (ti >= 1) mbar_wait(smem_u32(&m0->q8_free), (ti - 1) & 1u, abort_flag);
               full = smem_u32(&m0->q8_full);
@@ -578,7 +561,6 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
               mbar_arrive(full);
             }
             __syncwarp();
-            pos.advance(kNQ);
           }
           // ---- the K entries
 #pragma unroll 1
@@ -598,15 +580,14 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
               nxt[j] = (i + 1 < n_tiles && jn < n_rows) ? idx_row[jn] : -1;
             }
             __syncwarp();
-            if (pos.use >= 1) mbar_wait(smem_u32(&m0->k_free[pos.slot]), (pos.use - 1) & 1u, abort_flag);
-            const uint32_t at = pos.slot * kKSlot;
+            const uint32_t uses = c < kNQ ? G + ti + 1 : G;
+            if (uses >= 1) mbar_wait(k_free, (uses - 1) & 1u, abort_flag);
 #pragma unroll
             for (int q = 0; q < 32; ++q) {
               const int r = __shfl_sync(0xffffffffu, row[q >> 3], (q & 7) * 4 + (lane >> 3));
-              cp_async16(dst0[q & 1] + at + (q >> 1) * 1024, src0 + static_cast<long long>(r) * p.kv_sr);
+              cp_async16(dst0[q & 1] + (q >> 1) * 1024, src0 + static_cast<long long>(r) * p.kv_sr);
             }
-            cp_async_mbar_arrive_noinc(smem_u32(&m0->k_full[pos.slot]));
-            pos.advance(kNChunk);
+            cp_async_mbar_arrive_noinc(k_full);
           }
           gt += n_tiles;
         }

@@ -614,11 +614,12 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
     return FTB_ERR_INVALID;
   }
   // algo 0 = default = 5: persistent role-split CTA pairs (scores in one CTA, values in the other, Q in tensor
-  // memory, one ring for K and Q filled by TMA row gathers); algo 1 = one CTA per (token, output half), which is
-  // also the kernel of the FP8 paged form without a workspace, of the split form and of the diagnostic score tap;
+  // memory, rows gathered by cp.async), whole tokens or parts of them; algo 1 = one CTA per (token, output half), which is
+  // also the kernel of the FP8 paged form without a workspace and of the diagnostic score tap;
   // algo 6 = paged FP8 form: dequantise the selected rows, then the persistent kernel; algo 2 = few heads (h <= 32):
   // one CTA per token, the gathered rows on the rows of the MMA.  Measured at h = 16 / 32 (2048 causal tokens,
-  // topk 2048): 0.89 / 1.14 ms against 0.80 ms of the persistent pairs, so the default keeps the pairs: an MMA with
+  // topk 2048): 0.89 / 1.14 ms against 0.80 ms of the persistent pairs (which have become faster since), so the default
+  // keeps the pairs: an MMA with
   // 16 columns costs what one with 128 costs (its time goes with the 128 rows of the A operand), so putting the
   // heads on the columns saves no tensor time, and this kernel does not overlap its gather with its products.
   if (a->algo_id != 0 && a->algo_id != 1 && a->algo_id != 2 && a->algo_id != 5 && a->algo_id != 6) {

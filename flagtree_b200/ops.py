@@ -31,7 +31,9 @@ _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def _stream_ptr(device) -> int:
-    return _raw_stream(device.index) if _raw_stream is not None else torch.cuda.current_stream(device).cuda_stream
+    if _raw_stream is None or device.index is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    return _raw_stream(device.index)
 
 
 def _launch(fn, args, device, what: str) -> None:
@@ -199,6 +201,8 @@ def sparse_mla_fwd_host(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor
     with torch.cuda.stream(s_in):
         pipe["kv"].copy_(kv, non_blocking=True)
     n_chunks = (s_q + ct - 1) // ct
+    # the parts of a token as the device form would choose them for the whole batch, so that a short last chunk gives the same bits
+    splits = _auto_splits(s_q, h, topk, pipe["kv"].device) if h <= 128 else None
     for i in range(n_chunks):
         b = i & 1
         lo, hi = i * ct, min(s_q, (i + 1) * ct)
@@ -214,7 +218,7 @@ def sparse_mla_fwd_host(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor
             if ev_out[b] is not None:
                 s_c.wait_event(ev_out[b])
             sparse_mla_fwd(pipe["q"][b][:n], pipe["kv"], pipe["idx"][b][:n], sm_scale, out=pipe["out"][b][:n],
-                           lse=pipe["lse"][b][:n])
+                           lse=pipe["lse"][b][:n], num_splits=splits)
             ev_c[b] = s_c.record_event()
         with torch.cuda.stream(s_out):
             s_out.wait_event(ev_c[b])

@@ -441,3 +441,15 @@ def test_paged_forms_agree(splits, two_pass):
     out, lse = sparse_mla_fwd_paged(*args, page_size=c.page_size, check=True, num_splits=splits, two_pass=two_pass)
     assert (out.float() - ref_out.float()).abs().max().item() <= 1e-2
     assert ((lse - ref_lse).abs() / ref_lse.abs().clamp(min=1)).max().item() <= 1e-4
+
+
+@pytest.mark.parametrize("s_q,chunk", [(200, 192), (20, 16)])
+def test_host_buffer_form_with_a_short_last_chunk(s_q, chunk):
+    """A last chunk of fewer tokens than pairs of SMs gives the bits of the device form on the whole batch."""
+    from flagtree_b200 import sparse_mla_fwd_host
+    c = W.mla_cfg2(device="cpu", s_q=s_q, s_kv=1024, h=128, topk=512)
+    out_d, lse_d = sparse_mla_fwd(c.q.to(DEV), c.kv.to(DEV), c.indices.to(DEV), c.sm_scale, check=True)
+    out_h, lse_h = sparse_mla_fwd_host(c.q.pin_memory(), c.kv.pin_memory(), c.indices.pin_memory(), c.sm_scale,
+                                       device=torch.device(DEV), chunk_tokens=chunk)
+    torch.cuda.synchronize()
+    assert torch.equal(out_h, out_d.cpu()) and torch.equal(lse_h, lse_d.cpu())

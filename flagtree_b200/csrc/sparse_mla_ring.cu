@@ -96,6 +96,7 @@ struct Params {
   // the top-k list of a token in n_splits parts, an item of work each; their results go to fp32 partials that are merged later
   int n_splits;
   float* part_lse;     // [s_q, n_splits, h], base 2
+  float max_slack;     // how far (log2) the running maximum may lag behind
 };
 
 struct Misc0 {   // CTA 0
@@ -375,11 +376,12 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
             m0->xchg[b][tid] = mx;
             named_bar_sync(2 + (warp & 3), 64);
             mx = fmaxf(mx, m0->xchg[b][tid ^ 128]);
-            // Lazy maximum: only move the reference when it grows by more than 2^8, so that the
-            // accumulator in the other CTA is rarely rescaled (P stays below 256, exact enough in bf16/fp32).
+            // Lazy maximum: whole tokens only move the reference when it grows by more than 2^8, so that the
+            // accumulator in the other CTA is rarely rescaled (P stays below 256).  Parts of a token, a few tiles each, take
+            // the true maximum: the largest weight is then 1, which bf16 holds exactly.
             const float m_cand = fmaxf(m_run, mx * p.scale_log2);
             float alpha = 1.0f;
-            if (m_cand > m_run + 8.0f || m_run == -INFINITY) {
+            if (m_cand > m_run + p.max_slack || m_run == -INFINITY) {
               alpha = (m_run == -INFINITY) ? 0.0f : fast_exp2(m_run - m_cand);
               m_run = m_cand;
             }
@@ -892,6 +894,7 @@ int launch_sparse_mla_ring(const ftb_sparse_mla_args* a, int n_splits, float* pa
     p.lse_base2 = a->lse_base2;
     p.status = a->status;
     p.n_splits = n_splits;
+    p.max_slack = n_splits > 1 ? 0.0f : 8.0f;
     p.part_lse = part_lse + (n_splits > 1 ? static_cast<size_t>(t0) * n_splits * a->h : 0);
     const void* q0 = static_cast<const __nv_bfloat16*>(a->q) + t0 * a->q_stride_token;
     void* o0 = static_cast<__nv_bfloat16*>(a->out) + t0 * a->out_stride_token;

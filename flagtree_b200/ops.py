@@ -75,6 +75,23 @@ def _auto_splits(s_q: int, h: int, topk: int, device) -> int:
     return _plan_splits(s_q, h, topk, _pairs_of(device.index))
 
 
+def _plan_paged(s_q: int, h: int, topk: int, pairs: int) -> Tuple[int, bool]:
+    """Parts of a token's list in the paged form, and whether the rows are dequantised first.
+
+    Both kernels take the true maximum of a part as the reference of its weights, so the largest weight is exactly 1 in bf16;
+    fewer parts than the SMs could take would only cost precision (relative error against 64 bits, 30 tokens of topk 2048: 4.23e-3
+    whole, 4.12e-3 in 2 parts).  Up to eight tokens whose parts are at most three tiles of 64 rows, the one-pass kernel is
+    the faster one: two launches instead of three (us, one pass / two: 3 tokens of topk 2048 28.7 / 32.0, 8 of 512 24.6 / 28.7;
+    beyond it 8 of 2048 45 / 41, 12 of 512 35 / 31, 32 of 2048 135 / 86)."""
+    if s_q >= pairs:
+        return 1, True
+    tiles = max(1, (topk + 63) // 64)
+    parts = max(1, min(16, pairs // max(1, s_q), tiles))
+    if s_q <= 8 and -(-tiles // parts) <= 3:
+        return parts, False
+    return max(_plan_splits(s_q, h, topk, pairs), min(parts, max(1, (topk + 127) // 128))), True
+
+
 def _split_workspace(a, s_q: int, h: int, n_splits: int, device):
     """Fills the split fields of the argument struct; returns the scratch tensor (kept alive by the caller)."""
     a.n_splits = n_splits
@@ -245,8 +262,8 @@ def sparse_mla_fwd_paged(q: torch.Tensor, kv_cache: torch.Tensor, kv_scale: torc
     test_accuracy_musa_vllm_mla.py:278-283.  Returns (out [B,n_q,h,512] bf16, lse [B,n_q,h] fp32).
 
     `two_pass`: convert the selected rows to a compact bf16 table first and run the persistent bf16 kernel on
-    it (needs 1156 bytes of scratch per selected row); None = do so when the
-    scratch stays below 4 GiB, False = the one-pass kernel that converts while it gathers.
+    it (needs 1156 bytes of scratch per selected row), False = the one-pass kernel that converts while it gathers; None = by the
+    number of tokens, never with more than 4 GiB of scratch, and with a `num_splits` above 1 the one-pass kernel.
     """
     _require_cuda(q, kv_cache, kv_scale, block_table, context_lens, indices)
     assert q.dim() == 4 and indices.dim() == 3 and kv_cache.dim() == 3
@@ -273,12 +290,14 @@ def sparse_mla_fwd_paged(q: torch.Tensor, kv_cache: torch.Tensor, kv_scale: torc
         kv_cache.shape[0] * page_size, idx2.shape[1], q2.stride(0), q2.stride(1), D_QK, idx2.stride(0), out.stride(0), out.stride(1),
         lse.stride(0), float(sm_scale), int(lse_base2), 0, status.data_ptr() if status is not None else None, 1, kv_scale.data_ptr(),
         block_table.data_ptr(), context_lens.data_ptr(), page_size, n_q, block_table.stride(0))
-    if num_splits is None:
-        num_splits = _auto_splits(b * n_q, h, idx2.shape[1], q.device)
-    n_splits = max(1, int(num_splits))
     lib = _lib.load()
     rows_bytes = int(lib.ftb_sparse_mla_dequant_workspace_bytes(b * n_q, idx2.shape[1]))
-    if two_pass or (two_pass is None and rows_bytes <= (4 << 30)):
+    if num_splits is None:
+        n_splits, rows_first = _plan_paged(b * n_q, h, idx2.shape[1], _pairs_of(q.device.index))
+    else:
+        n_splits = max(1, int(num_splits))
+        rows_first = n_splits == 1
+    if two_pass or (two_pass is None and rows_first and rows_bytes <= (4 << 30)):
         # the dequantised rows, then (from a 16-byte boundary) the partial results of a split
         need = rows_bytes
         if n_splits > 1:

@@ -453,3 +453,38 @@ def test_host_buffer_form_with_a_short_last_chunk(s_q, chunk):
                                        device=torch.device(DEV), chunk_tokens=chunk)
     torch.cuda.synchronize()
     assert torch.equal(out_h, out_d.cpu()) and torch.equal(lse_h, lse_d.cpu())
+
+
+def _weight_between_two_bf16_values(s_q, topk):
+    """Lists whose first tile holds a row of score 0 and no value, and whose second tile a row of score 3 / 512 (base 2): its weight
+    2^(3/512) = 1.00407 lies half-way between two bf16 values, and nothing else has any weight."""
+    g = torch.Generator().manual_seed(s_q)
+    q = torch.zeros(s_q, 128, 576)
+    q[:, :, 512] = 1.0
+    kv = torch.zeros(topk, 576)
+    kv[:, 512] = -128.0
+    kv[5, 512] = 0.0
+    kv[200, 512] = 3.0 / 512
+    kv[200, :512] = torch.randint(8, 16, (512,), generator=g) / 8.0          # exact in e4m3
+    w = 2.0 ** (3.0 / 512)
+    return q.bfloat16(), kv, kv[200, :512].double() * w / (1.0 + w)
+
+
+@pytest.mark.parametrize("form", ["dense", "paged"])
+def test_parts_take_the_true_maximum(form):
+    """Parts of two tiles: the reference of the weights follows the maximum, so the largest weight is 1 and exact, and the result is off by
+    its own rounding to bf16 alone (2^-9).  A reference that lags behind gives a weight that is off by another 2^-8."""
+    s_q, topk = (1, 512) if form == "dense" else (32, 512)
+    q, kv, ref = _weight_between_two_bf16_values(s_q, topk)
+    idx = torch.arange(topk, dtype=torch.int32).repeat(s_q, 1)
+    sm_scale = 0.6931471805599453
+    if form == "dense":
+        out, _ = sparse_mla_fwd(q.to(DEV), kv.bfloat16().to(DEV), idx.to(DEV), sm_scale, check=True, num_splits=2)
+    else:
+        cache = kv.to(torch.float8_e4m3fn).view(1, 8, 64, 576).repeat(s_q, 1, 1, 1).view(torch.uint8).view(s_q * 8, 64, 576)
+        table = torch.arange(s_q * 8, dtype=torch.int32).view(s_q, 8)
+        out, _ = sparse_mla_fwd_paged(q.view(s_q, 1, 128, 576).to(DEV), cache.to(DEV), torch.ones(s_q * 8, device=DEV), table.to(DEV),
+                                      torch.full((s_q,), topk, dtype=torch.int32, device=DEV), idx.view(s_q, 1, topk).to(DEV), sm_scale, check=True)
+        out = out[:, 0]
+    err = ((out.double().cpu() - ref) / ref).abs().max().item()
+    assert err <= 2 ** -9 * 1.05, err

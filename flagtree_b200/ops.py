@@ -297,7 +297,7 @@ def sparse_mla_fwd_paged(q: torch.Tensor, kv_cache: torch.Tensor, kv_scale: torc
     else:
         n_splits = max(1, int(num_splits))
         rows_first = n_splits == 1
-    if two_pass or (two_pass is None and rows_first and rows_bytes <= (4 << 30)):
+    if rows_bytes > 0 and (two_pass or (two_pass is None and rows_first and rows_bytes <= (4 << 30))):
         # the dequantised rows, then (from a 16-byte boundary) the partial results of a split
         need = rows_bytes
         if n_splits > 1:

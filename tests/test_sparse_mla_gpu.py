@@ -488,3 +488,12 @@ def test_parts_take_the_true_maximum(form):
         out = out[:, 0]
     err = ((out.double().cpu() - ref) / ref).abs().max().item()
     assert err <= 2 ** -9 * 1.05, err
+
+
+@pytest.mark.parametrize("splits", [None, 1, 4])
+def test_paged_lists_of_no_entry(splits):
+    """topk = 0 is an empty list like one of padding alone: zeros, and a log-sum-exp of -inf."""
+    c = W.mla_cfg3(batch=2, n_q=2, h=16, topk=64, len_lo=40, len_hi=90)
+    out, lse = sparse_mla_fwd_paged(c.q.to(DEV), c.kv_cache.to(DEV), c.kv_scale.to(DEV), c.block_table.to(DEV), c.context_lens.to(DEV),
+                                    c.indices[:, :, :0].contiguous().to(DEV), c.sm_scale, page_size=c.page_size, check=True, num_splits=splits)
+    assert (out == 0).all() and (lse == float("-inf")).all()

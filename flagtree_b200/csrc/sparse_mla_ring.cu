@@ -199,6 +199,22 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
+// Masked entries (-1) fetch a row all the same, which is multiplied by zero: the one that the lane fetched for the tile before, or in
+// the first tile another one of the token's (this function, the rare path: the first row that the list names; `none` if
+// it names none, row 0 for a token and any rows for a part, whose result the merge drops).  With row 0 for all of them, as it used to be,
+// every SM fetched the same 1152 bytes (4096 tokens of topk 65 took longer than of topk 128, 760 us against 329; now 313),
+// and a row 0 that holds no numbers spoiled tokens that never selected it.  Not inline: the roles share an instruction cache.
+__device__ __noinline__ int first_row(const int32_t* idx_row, int n_rows, int s_kv, int none) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int j = 0; j < n_rows; j += 32) {
+    const int v = j + lane < n_rows ? idx_row[j + lane] : -1;
+    const unsigned have = __ballot_sync(0xffffffffu, v >= 0 && v < s_kv);
+    if (have != 0u) return __shfl_sync(0xffffffffu, v, __ffs(static_cast<int>(have)) - 1);
+  }
+  return none;
+}
+
 __global__ void __launch_bounds__(kThreads, 1)
 sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
                          const __grid_constant__ CUtensorMap tm_o, const Params p) {
@@ -565,10 +581,20 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
             __syncwarp();
           }
           // ---- the K entries
+          int row[4], own = -1;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            row[j] = nxt[j] >= 0 && nxt[j] < p.s_kv ? nxt[j] : -1;
+            own = max(own, row[j]);
+          }
+          if (!__all_sync(0xffffffffu, (row[0] | row[1] | row[2] | row[3]) >= 0)) {
+            const int any = first_row(idx_row, last[t] > 0 ? n_rows : 0, p.s_kv, p.n_splits > 1 ? min(static_cast<int>(blockIdx.x * 32 + lane), p.s_kv - 1) : 0);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) row[j] = row[j] >= 0 ? row[j] : own >= 0 ? own : any;
+          }
 #pragma unroll 1
           for (int i = 0; i < n_tiles; ++i) {
             const uint32_t G = gt + i;
-            int row[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const bool ok = nxt[j] >= 0 && nxt[j] < p.s_kv;
@@ -577,7 +603,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
                 const uint32_t v = __ballot_sync(0xffffffffu, ok);
                 if (lane == 0) m0->valid_mask[G & 7][j] = v;
               }
-              row[j] = ok ? nxt[j] : 0;                      // a masked entry fetches row 0 and is multiplied by zero
+              if (ok) row[j] = nxt[j];                       // a masked entry fetches the row before it again and is multiplied by zero
               const int jn = (i + 1) * kNT + 32 * j + lane;
               nxt[j] = (i + 1 < n_tiles && jn < n_rows) ? idx_row[jn] : -1;
             }
@@ -795,11 +821,16 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
           const int row0 = t < nb ? warp_uniform(nt[kBatch + t]) * kNT : 0, n_rows = p.topk - row0;
           const int32_t* idx_row = p.indices + static_cast<long long>(t < nb ? token_of(item) : 0) * p.idx_st + row0;
           int nxt = sl * kVSlabRows + lane < n_rows ? idx_row[sl * kVSlabRows + lane] : -1;   // row `lane` of the slab
+          int row = nxt >= 0 && nxt < p.s_kv ? nxt : -1;
+          if (!__all_sync(0xffffffffu, row >= 0)) {
+            const int any = first_row(idx_row, t < nb && last[t] > 0 ? n_rows : 0, p.s_kv, p.n_splits > 1 ? min(static_cast<int>(blockIdx.x * 32 + lane), p.s_kv - 1) : 0);
+            if (row < 0) row = any;
+          }
 #pragma unroll 1
           for (int i = 0; i < n_tiles; ++i) {
             if (t < nb) {
               const uint32_t G = gt + i;
-              const int row = (nxt >= 0 && nxt < p.s_kv) ? nxt : 0;
+              if (nxt >= 0 && nxt < p.s_kv) row = nxt;
               const int jn = (i + 1) * kNT + sl * kVSlabRows + lane;
               nxt = (i + 1 < n_tiles && jn < n_rows) ? idx_row[jn] : -1;
               if (G >= 1) mbar_wait(v_free, (G - 1) & 1u, abort_flag);

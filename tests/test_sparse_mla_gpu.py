@@ -497,3 +497,27 @@ def test_paged_lists_of_no_entry(splits):
     out, lse = sparse_mla_fwd_paged(c.q.to(DEV), c.kv_cache.to(DEV), c.kv_scale.to(DEV), c.block_table.to(DEV), c.context_lens.to(DEV),
                                     c.indices[:, :, :0].contiguous().to(DEV), c.sm_scale, page_size=c.page_size, check=True, num_splits=splits)
     assert (out == 0).all() and (lse == float("-inf")).all()
+
+
+@pytest.mark.parametrize("splits", [1, 4, 20])
+def test_masked_entries_read_no_foreign_row(splits):
+    """Rows that nobody selects hold NaN patterns, row 0 among them: lists with a ragged tail, with most entries masked (whole slabs and
+    whole tiles among them), with nothing in their first tile, with one entry, and parts without an entry."""
+    g = torch.Generator().manual_seed(splits)
+    s_q, s_kv, topk = 8, 3000, 700
+    kv = torch.full((s_kv, 576), float("nan")).bfloat16()
+    rows = torch.randperm(s_kv - 1, generator=g)[:1500] + 1
+    kv[rows] = torch.randn(1500, 576, generator=g).bfloat16()
+    q = torch.randn(s_q, 128, 576, generator=g).bfloat16()
+    idx = rows[torch.stack([torch.randperm(1500, generator=g)[:topk] for _ in range(s_q)])].int()
+    idx[0, 65:] = -1
+    idx[1, torch.rand(topk, generator=g) < 0.875] = -1
+    idx[2, torch.rand(topk, generator=g) < 0.98] = -1
+    idx[3, :200] = -1
+    idx[4, 1:] = -1
+    idx[5, :-1] = -1
+    idx[6, 40:650] = -1
+    out, lse = sparse_mla_fwd(q.to(DEV), kv.to(DEV), idx.to(DEV), 0.06, check=True, num_splits=splits)
+    ref_out, ref_lse = sparse_mla_fwd_ref(q, torch.nan_to_num(kv.float()).bfloat16(), idx, 0.06)
+    e_out, e_lse = _errors(out, lse, ref_out, ref_lse)
+    assert e_out <= OUT_ATOL and e_lse <= LSE_RTOL

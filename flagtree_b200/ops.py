@@ -116,7 +116,7 @@ def sparse_mla_fwd(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor,
                    sm_scale: Optional[float] = None, d_v: int = D_V, *, lse_base2: bool = False,
                    out: Optional[torch.Tensor] = None, lse: Optional[torch.Tensor] = None,
                    check: bool = False, algo: int = 0, num_splits: Optional[int] = None,
-                   _dbg_scores: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
+                   _dbg_scores: Optional[torch.Tensor] = None, _plan_tokens: Optional[int] = None) -> Tuple[torch.Tensor, torch.Tensor]:
     """Top-k sparse MLA forward.
 
     q [S_q, h, 576] bf16, kv [S_kv, 576] (or [S_kv, 1, 576]) bf16, indices [S_q, topk] int32 with
@@ -155,7 +155,7 @@ def sparse_mla_fwd(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor,
         qs, os_, ls = (q, out, lse) if h <= 128 else (q[:, h0:h1], out[:, h0:h1], lse[:, h0:h1])
         n_splits = int(num_splits) if num_splits else 1
         if num_splits is None and algo == 0 and _dbg_scores is None:
-            n_splits = _auto_splits(s_q, h1 - h0, indices.shape[1], q.device)
+            n_splits = _auto_splits(_plan_tokens or s_q, h1 - h0, indices.shape[1], q.device)
         a = _lib.SparseMlaArgs(
             qs.data_ptr(), kv.data_ptr(), indices.data_ptr(), os_.data_ptr(), ls.data_ptr(), s_q, h1 - h0, kv.shape[0],
             indices.shape[1], qs.stride(0), qs.stride(1), kv.stride(0), indices.stride(0), os_.stride(0), os_.stride(1),
@@ -218,8 +218,6 @@ def sparse_mla_fwd_host(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor
     with torch.cuda.stream(s_in):
         pipe["kv"].copy_(kv, non_blocking=True)
     n_chunks = (s_q + ct - 1) // ct
-    # the parts of a token as the device form would choose them for the whole batch, so that a short last chunk gives the same bits
-    splits = _auto_splits(s_q, h, topk, pipe["kv"].device) if h <= 128 else None
     for i in range(n_chunks):
         b = i & 1
         lo, hi = i * ct, min(s_q, (i + 1) * ct)
@@ -235,7 +233,7 @@ def sparse_mla_fwd_host(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor
             if ev_out[b] is not None:
                 s_c.wait_event(ev_out[b])
             sparse_mla_fwd(pipe["q"][b][:n], pipe["kv"], pipe["idx"][b][:n], sm_scale, out=pipe["out"][b][:n],
-                           lse=pipe["lse"][b][:n], num_splits=splits)
+                           lse=pipe["lse"][b][:n], _plan_tokens=s_q)      # parts of a token as for the whole batch: the same bits
             ev_c[b] = s_c.record_event()
         with torch.cuda.stream(s_out):
             s_out.wait_event(ev_c[b])

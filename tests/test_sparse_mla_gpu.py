@@ -521,3 +521,14 @@ def test_masked_entries_read_no_foreign_row(splits):
     ref_out, ref_lse = sparse_mla_fwd_ref(q, torch.nan_to_num(kv.float()).bfloat16(), idx, 0.06)
     e_out, e_lse = _errors(out, lse, ref_out, ref_lse)
     assert e_out <= OUT_ATOL and e_lse <= LSE_RTOL
+
+
+def test_host_buffer_form_with_a_short_last_chunk_and_many_heads():
+    """The same with two blocks of heads in a launch each: the last chunk of 8 tokens would be cut in parts by itself."""
+    from flagtree_b200 import sparse_mla_fwd_host
+    c = W.mla_cfg2(device="cpu", s_q=80, s_kv=1024, h=160, topk=1024)
+    out_d, lse_d = sparse_mla_fwd(c.q.to(DEV), c.kv.to(DEV), c.indices.to(DEV), c.sm_scale, check=True)
+    out_h, lse_h = sparse_mla_fwd_host(c.q.pin_memory(), c.kv.pin_memory(), c.indices.pin_memory(), c.sm_scale,
+                                       device=torch.device(DEV), chunk_tokens=72)
+    torch.cuda.synchronize()
+    assert torch.equal(out_h, out_d.cpu()) and torch.equal(lse_h, lse_d.cpu())

@@ -464,8 +464,9 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_fwd_kernel(const MlaPa
 // out = sum w_k out_k / sum w_k, and the merged LSE, which the reference does not store.
 // One CTA of 128 threads per (token, head), four columns each: a decode step merges few rows of many parts, so what counts is
 // that the loads of all parts are in flight at once (a warp per row that took one part after the other: 13 us for 3 tokens
-// of 128 heads and 16 parts).
-constexpr int kMergeBatch = 16;
+// of 128 heads and 16 parts).  kBatch parts at a time, the least power of two that holds them all, up to 16: with 16 for every call, 300 tokens
+// of 128 heads and topk 2048 in 2 parts took 817 us on the one-CTA kernel, now 687.
+template <int kBatch>
 __global__ void __launch_bounds__(128) sparse_mla_merge_kernel(const float* __restrict__ part_out,
                                                                const float* __restrict__ part_lse, __nv_bfloat16* out,
                                                                float* lse, int h, int n_splits, long long out_st,
@@ -474,19 +475,24 @@ __global__ void __launch_bounds__(128) sparse_mla_merge_kernel(const float* __re
   const float* lrow = part_lse + static_cast<long long>(token) * n_splits * h + head;
   const float4* src = reinterpret_cast<const float4*>(part_out + (static_cast<long long>(token) * n_splits * h + head) * 512) + threadIdx.x;
   float mx = -INFINITY, wsum = 0.0f;
-  for (int k = 0; k < n_splits; ++k) mx = fmaxf(mx, lrow[static_cast<long long>(k) * h]);
+  if (n_splits > kBatch)
+    for (int k = 0; k < n_splits; ++k) mx = fmaxf(mx, lrow[static_cast<long long>(k) * h]);
   float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  for (int k0 = 0; k0 < n_splits && mx != -INFINITY; k0 += kMergeBatch) {
-    float4 v[kMergeBatch];
-    float w[kMergeBatch];
+  for (int k0 = 0; k0 < n_splits; k0 += kBatch) {
+    float4 v[kBatch];
+    float w[kBatch];
 #pragma unroll
-    for (int k = 0; k < kMergeBatch; ++k) {
+    for (int k = 0; k < kBatch; ++k) {
       const bool in = k0 + k < n_splits;
       w[k] = in ? lrow[static_cast<long long>(k0 + k) * h] : -INFINITY;
       v[k] = in ? __ldcs(src + static_cast<long long>(k0 + k) * h * 128) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
+    if (n_splits <= kBatch) {
 #pragma unroll
-    for (int k = 0; k < kMergeBatch; ++k) {
+      for (int k = 0; k < kBatch; ++k) mx = fmaxf(mx, w[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
       if (w[k] == -INFINITY) continue;
       const float wk = fast_exp2(w[k] - mx);
       wsum += wk;
@@ -661,8 +667,10 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
   // one-pass kernel below converts while it gathers.
   const int64_t split_bytes = ftb_sparse_mla_workspace_bytes(a->s_q, a->h, n_splits);
   auto merge = [&]() {
-    sparse_mla_merge_kernel<<<static_cast<unsigned>(a->s_q * a->h), 128, 0, st>>>(p.part_out, p.part_lse, p.out, p.lse, a->h, n_splits,
-                                                                               p.out_st, p.out_sh, p.lse_st, p.lse_base2);
+    const auto kern = n_splits <= 2 ? sparse_mla_merge_kernel<2> : n_splits <= 4 ? sparse_mla_merge_kernel<4>
+                      : n_splits <= 8 ? sparse_mla_merge_kernel<8> : sparse_mla_merge_kernel<16>;
+    kern<<<static_cast<unsigned>(a->s_q * a->h), 128, 0, st>>>(p.part_out, p.part_lse, p.out, p.lse, a->h, n_splits, p.out_st, p.out_sh,
+                                                             p.lse_st, p.lse_base2);
     return check_cuda(cudaGetLastError(), "sparse_mla_merge launch");
   };
   // With a split, algo 6 wants room for both: the dequantised rows, then the partial results (from a 16-byte boundary).

@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(256) sparse_mla_merge_parts_kernel(const T* __
 namespace ftb {
 void set_last_error(const char* fmt, ...);
 int check_cuda(cudaError_t e, const char* what);
-int launch_sparse_mla_ring(const ftb_sparse_mla_args* a, int n_splits, float* part_out, float* part_lse, cudaStream_t st);
+int launch_sparse_mla_ring(const ftb_sparse_mla_args* a, int n_splits, float* part_out, float* part_lse, float max_slack, cudaStream_t st);
 int launch_sparse_mla_few(const ftb_sparse_mla_args* a, cudaStream_t st);
 }  // namespace ftb
 
@@ -640,7 +640,7 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
   }
   if (a->algo_id == 2) return launch_sparse_mla_few(a, reinterpret_cast<cudaStream_t>(stream));
   if (plain && (a->algo_id == 0 || a->algo_id == 5))
-    return launch_sparse_mla_ring(a, 1, nullptr, nullptr, reinterpret_cast<cudaStream_t>(stream));
+    return launch_sparse_mla_ring(a, 1, nullptr, nullptr, 8.0f, reinterpret_cast<cudaStream_t>(stream));
   MlaParams p;
   memset(&p, 0, sizeof(p));
   p.q = reinterpret_cast<const __nv_bfloat16*>(a->q);
@@ -662,6 +662,12 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
   }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int n_splits = a->n_splits > 0 ? a->n_splits : 1;
+  // parts with at least a tile of the list each: what a caller asks for beyond that would be empty parts (300 tokens of topk 256 and 128
+  // heads in 16 parts 860 us, in the four that hold something 270)
+  auto parts_of = [&](int tile) {
+    const int tiles = (a->topk + tile - 1) / tile;
+    return n_splits < tiles ? n_splits : tiles > 1 ? tiles : 1;
+  };
   // Paged FP8 form with a workspace for the dequantised rows (algo 0 or 6, no split): convert the selected
   // rows once, then run the persistent bf16 kernel on the compact table.  Without such a workspace the
   // one-pass kernel below converts while it gathers.
@@ -706,11 +712,12 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
       b.idx_stride_token = a->topk;
       b.algo_id = 5;
       b.workspace = nullptr; b.workspace_bytes = 0; b.n_splits = 0;
-      if (n_splits == 1) return launch_sparse_mla_ring(&b, 1, nullptr, nullptr, st);
+      if (n_splits == 1) return launch_sparse_mla_ring(&b, 1, nullptr, nullptr, 8.0f, st);
       p.part_out = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(a->workspace) + rows_bytes);
+      n_splits = parts_of(128);
       p.part_lse = p.part_out + static_cast<size_t>(a->s_q) * n_splits * a->h * 512;
-      rc0 = launch_sparse_mla_ring(&b, n_splits, p.part_out, p.part_lse, st);
-      return rc0 != FTB_OK ? rc0 : merge();
+      rc0 = launch_sparse_mla_ring(&b, n_splits, p.part_out, p.part_lse, 0.0f, st);
+      return rc0 != FTB_OK || n_splits == 1 ? rc0 : merge();
     }
   }
   if (n_splits > 1) {
@@ -722,12 +729,20 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
     p.part_lse = p.part_out + static_cast<size_t>(a->s_q) * n_splits * a->h * 512;
   }
   p.n_splits = n_splits;
-  // bf16 rows: the persistent pairs take a part of a token as they take a token (up to as many parts as a pair has room for)
-  if (n_splits > 1 && n_splits <= 64 && !a->kv_is_fp8 && a->dbg_scores == nullptr && (a->algo_id == 0 || a->algo_id == 5) &&
+  // bf16 rows: the persistent pairs take a part of a token as they take a token (up to as many parts as a pair has room for).  algo 5
+  // always does; algo 0, with the true maximum like the one-CTA kernel, where the parts are not short: one-CTA kernel / pairs (us), two
+  // parts of 128 heads, 32 tokens of topk 256 23 / 36, of 512 31 / 38, of 1024 48 / 34, of 2048 80 / 43; 148 tokens of topk 512 in four parts
+  // 167 / 142; 16 heads, 148 tokens of topk 512 in two parts 88 / 44.
+  const bool pairs = a->algo_id == 5 || (a->algo_id == 0 && (a->topk > 512 || (n_splits * 128 <= a->topk && (a->h <= 32 || (a->topk > 256 && a->s_q >= 64)))));
+  if (n_splits > 1 && n_splits <= 64 && !a->kv_is_fp8 && a->dbg_scores == nullptr && pairs &&
       (reinterpret_cast<uintptr_t>(a->workspace) & 15u) == 0) {
-    const int rc0 = launch_sparse_mla_ring(a, n_splits, p.part_out, p.part_lse, st);
-    return rc0 != FTB_OK ? rc0 : merge();
+    n_splits = parts_of(128);
+    p.part_lse = p.part_out + static_cast<size_t>(a->s_q) * n_splits * a->h * 512;
+    const int rc0 = launch_sparse_mla_ring(a, n_splits, p.part_out, p.part_lse, a->algo_id == 5 ? 8.0f : 0.0f, st);
+    return rc0 != FTB_OK || n_splits == 1 ? rc0 : merge();
   }
+  n_splits = p.n_splits = parts_of(kBN);
+  if (n_splits > 1) p.part_lse = p.part_out + static_cast<size_t>(a->s_q) * n_splits * a->h * 512;
   const dim3 grid(static_cast<unsigned>(a->s_q) * 2u * static_cast<unsigned>(n_splits)), block(kThreads);
   cudaError_t e;
   if (a->kv_is_fp8) {

@@ -154,12 +154,13 @@ def sparse_mla_fwd(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor,
         h1 = min(h, h0 + 128)
         qs, os_, ls = (q, out, lse) if h <= 128 else (q[:, h0:h1], out[:, h0:h1], lse[:, h0:h1])
         n_splits = int(num_splits) if num_splits else 1
+        algo_id = int(algo)
         if num_splits is None and algo == 0 and _dbg_scores is None:
-            n_splits = _auto_splits(_plan_tokens or s_q, h1 - h0, indices.shape[1], q.device)
+            n_splits, algo_id = _auto_splits(_plan_tokens or s_q, h1 - h0, indices.shape[1], q.device), 5
         a = _lib.SparseMlaArgs(
             qs.data_ptr(), kv.data_ptr(), indices.data_ptr(), os_.data_ptr(), ls.data_ptr(), s_q, h1 - h0, kv.shape[0],
             indices.shape[1], qs.stride(0), qs.stride(1), kv.stride(0), indices.stride(0), os_.stride(0), os_.stride(1),
-            ls.stride(0), float(sm_scale), int(lse_base2), int(algo), status.data_ptr() if status is not None else None)
+            ls.stride(0), float(sm_scale), int(lse_base2), algo_id, status.data_ptr() if status is not None else None)
         a.dbg_scores = _dbg_scores.data_ptr() if _dbg_scores is not None else None
         _ws = _split_workspace(a, s_q, h1 - h0, n_splits, q.device)
         _launch(lib.ftb_sparse_mla_fwd, a, q.device, "sparse_mla_fwd")

@@ -474,12 +474,12 @@ def _weight_between_two_bf16_values(s_q, topk):
 def test_parts_take_the_true_maximum(form):
     """Parts of two tiles: the reference of the weights follows the maximum, so the largest weight is 1 and exact, and the result is off by
     its own rounding to bf16 alone (2^-9).  A reference that lags behind gives a weight that is off by another 2^-8."""
-    s_q, topk = (1, 512) if form == "dense" else (32, 512)
+    s_q, topk = (1, 1024) if form == "dense" else (32, 512)
     q, kv, ref = _weight_between_two_bf16_values(s_q, topk)
     idx = torch.arange(topk, dtype=torch.int32).repeat(s_q, 1)
     sm_scale = 0.6931471805599453
     if form == "dense":
-        out, _ = sparse_mla_fwd(q.to(DEV), kv.bfloat16().to(DEV), idx.to(DEV), sm_scale, check=True, num_splits=2)
+        out, _ = sparse_mla_fwd(q.to(DEV), kv.bfloat16().to(DEV), idx.to(DEV), sm_scale, check=True, num_splits=4)
     else:
         cache = kv.to(torch.float8_e4m3fn).view(1, 8, 64, 576).repeat(s_q, 1, 1, 1).view(torch.uint8).view(s_q * 8, 64, 576)
         table = torch.arange(s_q * 8, dtype=torch.int32).view(s_q, 8)
@@ -532,3 +532,20 @@ def test_host_buffer_form_with_a_short_last_chunk_and_many_heads():
                                        device=torch.device(DEV), chunk_tokens=72)
     torch.cuda.synchronize()
     assert torch.equal(out_h, out_d.cpu()) and torch.equal(lse_h, lse_d.cpu())
+
+
+@pytest.mark.parametrize("algo", [0, 5])
+@pytest.mark.parametrize("s_q,h,topk,splits", [(40, 64, 300, 3), (75, 128, 257, 2), (4, 128, 513, 5), (20, 32, 256, 2), (9, 32, 255, 2), (5, 33, 512, 4)])
+def test_parts_by_either_kernel(s_q, h, topk, splits, algo):
+    """A given number of parts: the persistent pairs (algo 5, and algo 0 above 512 entries or for few heads) or the one-CTA kernel."""
+    g = torch.Generator().manual_seed(s_q + topk)
+    q = torch.randn(s_q, h, 576, generator=g).bfloat16()
+    kv = torch.randn(2000, 576, generator=g).bfloat16()
+    idx = torch.stack([torch.randperm(2000, generator=g)[:topk] for _ in range(s_q)]).int()
+    idx[1, 100:] = -1
+    idx[2, :] = -1
+    idx[0, 3::5] = -1
+    out, lse = sparse_mla_fwd(q.to(DEV), kv.to(DEV), idx.to(DEV), 0.06, check=True, num_splits=splits, algo=algo)
+    ref_out, ref_lse = sparse_mla_fwd_ref(q, kv, idx, 0.06)
+    e_out, e_lse = _errors(out, lse, ref_out, ref_lse)
+    assert e_out <= OUT_ATOL and e_lse <= LSE_RTOL

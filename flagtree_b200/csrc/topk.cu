@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(kThreads) topk_select_kernel(const Params p) {
 // Rows of at most 65536 scores: persistent CTAs of 1024 threads, one per SM.  Thread t holds the keys of positions
 // t, t + 1024, ... (32 in registers; rows of more than 32768 scores keep the rest in shared memory), so that a vote over a
 // warp is the mask of 32 consecutive positions.  Rows of at most 32768 scores are copied into shared memory one row
-// ahead (one bulk copy, or 4-byte asynchronous copies for rows that are not 16-byte aligned); scores are read from device memory
+// ahead by asynchronous copies; scores are read from device memory
 // once.
 //
 // Bound by instruction issue, so the work per key is kept to a few instructions and no key goes through a shared-memory
@@ -186,19 +186,11 @@ __device__ __forceinline__ int row_len(const Params& p, int row) {
   return max(0, min(len, p.s_kv));
 }
 
-// scores src[0 .. n) -> buf, filled up to `full` with the pattern whose key is 0.  A 16-byte aligned row is one bulk copy that
-// completes on `bar` (after the fence that orders it behind the reads of the row before), its last n % 4 scores and other
-// rows 4-byte copies of the calling threads.
-__device__ __forceinline__ bool is_bulk(const uint32_t* src, int n) { return (reinterpret_cast<uintptr_t>(src) & 15) == 0 && n >= 4; }
-__device__ __forceinline__ void fetch(const uint32_t* src, int n, int full, uint32_t* buf, uint32_t bar) {
-  if (is_bulk(src, n)) {
-    const uint32_t bytes = static_cast<uint32_t>(n & ~3) * 4u;
-    if (threadIdx.x == 0) {
-      fence_proxy_async_smem();
-      mbar_arrive_expect_tx(bar, bytes);
-      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                   ::"r"(smem_u32(buf)), "l"(src), "r"(bytes), "r"(bar) : "memory");
-    }
+// scores src[0 .. n) -> buf, filled up to `full` with the pattern whose key is 0, by asynchronous copies of the calling threads: of 16
+// bytes where the row is aligned
+__device__ __forceinline__ void fetch(const uint32_t* src, int n, int full, uint32_t* buf) {
+  if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+    for (int c = threadIdx.x; c < n >> 2; c += kBigThreads) cp_async16(smem_u32(buf + 4 * c), src + 4 * c);
     const int tail = (n & ~3) + threadIdx.x;
     if (tail < n) cp_async4(buf + tail, src + tail);
   } else {
@@ -221,17 +213,11 @@ __global__ void __launch_bounds__(kBigThreads, 1) topk_select_rows_kernel(const 
   uint32_t* warp_sum = samp + kSampleMax;                                            // [4][32]
   uint32_t* few = warp_sum + 4 * kBigWarps;                                          // [kFew]
   int* ctl = reinterpret_cast<int*>(few + kFew);                                     // [16]
-  __shared__ alignas(8) unsigned long long bulk_bar;
-  __shared__ int abort_flag;                               // a copy that does not arrive within a second (never, on a working device)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t bar = smem_u32(&bulk_bar);
-  uint32_t n_bulk = 0;                                     // bulk copies waited for
-  if (tid == 0) { abort_flag = 0; mbar_init(bar, 1); fence_mbar_init(); }
-  __syncthreads();
 
   auto scores_of = [&](int row) { return reinterpret_cast<const uint32_t*>(p.scores) + static_cast<long long>(row) * p.sc_stride; };
   int row = blockIdx.x;
-  if (!kLong && row < p.s_q) fetch(scores_of(row), row_len(p, row), kHalf, buf, bar);
+  if (!kLong && row < p.s_q) fetch(scores_of(row), row_len(p, row), kHalf, buf);
   for (; row < p.s_q; row += gridDim.x) {
     const int len = row_len(p, row);
     const int k = min(p.topk, len);
@@ -240,7 +226,7 @@ __global__ void __launch_bounds__(kBigThreads, 1) topk_select_rows_kernel(const 
     const bool sampled = k < len && len >= kSampleMinLen;
     uint32_t key[kPerThread];                              // position 1024 i + tid; 0 past the row
     if (kLong) {
-      if (len > kHalf) fetch(src + kHalf, len - kHalf, 0, buf, bar);
+      if (len > kHalf) fetch(src + kHalf, len - kHalf, 0, buf);
       if (sampled && tid < kSample)
         samp[tid] = (to_key(src[static_cast<int>((static_cast<long long>(tid) * len) / kSample) + (tid & 15)]) & ~0xffu) | static_cast<uint32_t>(tid);
 #pragma unroll
@@ -249,10 +235,8 @@ __global__ void __launch_bounds__(kBigThreads, 1) topk_select_rows_kernel(const 
         key[i] = pos < len ? to_key(__ldcs(src + pos)) : 0u;
       }
       cp_async_wait_all();
-      if (len > kHalf && is_bulk(src + kHalf, len - kHalf)) mbar_wait(bar, n_bulk++ & 1u, &abort_flag);
     } else {
       cp_async_wait_all();
-      if (is_bulk(src, len)) mbar_wait(bar, n_bulk++ & 1u, &abort_flag);
       __syncthreads();
 #pragma unroll
       for (int i = 0; i < kPerThread; ++i) {
@@ -266,7 +250,7 @@ __global__ void __launch_bounds__(kBigThreads, 1) topk_select_rows_kernel(const 
     if (tid == 0) { ctl[kCtlLo] = 1; ctl[kCtlHi] = -1; ctl[kCtlFirst] = ctl[kCtlFirst + 1] = 1; ctl[kCtlFirst + 2] = ctl[kCtlFirst + 3] = -1; ctl[kCtlAbove] = 0; ctl[kCtlList] = 0; ctl[kCtlFew] = 0; }
     __syncthreads();
     if (!kLong && row + static_cast<int>(gridDim.x) < p.s_q)
-      fetch(scores_of(row + gridDim.x), row_len(p, row + gridDim.x), kHalf, buf, bar);           // overlaps the selection
+      fetch(scores_of(row + gridDim.x), row_len(p, row + gridDim.x), kHalf, buf);           // overlaps the selection
 
     if (k < len) {
       // the keys of positions kHalf + 1024 i + tid, i < n2: read again from shared memory by every sweep

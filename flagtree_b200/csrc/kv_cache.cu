@@ -436,31 +436,43 @@ __global__ void __launch_bounds__(kRunThreads, 3) run_write_kernel(const Params 
 
 // pages with several runs: their word holds the candidate scale (float bits; counts are far smaller)
 constexpr unsigned int kCandMin = 0x20000000u;
+// CTA b looks after pages b, b + gridDim.x, ...: all their words at once, then the few that rise, a page at a time.
 __global__ void __launch_bounds__(256) page_settle_kernel(const Params p) {
-  const int page0 = blockIdx.x * 8;
-  for (int page = page0; page < min(page0 + 8, p.num_pages); ++page) {
-    const unsigned word = p.cand[page];
-    if (word < kCandMin) continue;
-    const float cand = __uint_as_float(word);
-    const float old = p.scale[page];
-    if (!(cand > old)) continue;                          // the page's scale already covers the new rows
-    __syncthreads();                                      // every thread has read the old scale
-    if (old > 0.0f) requantise(p, page, old, cand, threadIdx.x, 256);
-    if (threadIdx.x == 0) p.scale[page] = cand;
+  __shared__ int rises[256];
+  __shared__ int n_rises;
+  const int tid = threadIdx.x;
+  for (int first = blockIdx.x; first < p.num_pages; first += gridDim.x * 256) {
+    if (tid == 0) n_rises = 0;
+    __syncthreads();
+    const long long mine = first + static_cast<long long>(tid) * gridDim.x;
+    if (mine < p.num_pages) {
+      const unsigned word = p.cand[mine];
+      if (word >= kCandMin && __uint_as_float(word) > p.scale[mine]) rises[atomicAdd(&n_rises, 1)] = static_cast<int>(mine);
+    }
+    __syncthreads();
+    const int n = n_rises;
+    for (int i = 0; i < n; ++i) {
+      const int page = rises[i];
+      const float cand = __uint_as_float(p.cand[page]), old = p.scale[page];
+      if (old > 0.0f) requantise(p, page, old, cand, tid, 256);
+      __syncthreads();                                    // every thread has read the old scale
+      if (tid == 0) p.scale[page] = cand;
+    }
+    __syncthreads();
   }
 }
 
-__global__ void __launch_bounds__(256) row_store_kernel(const Params p) {
+// A warp looks after `per_warp` rows (at most 32, a power of two) and stores those of the pages that the kernel before settled.
+__global__ void __launch_bounds__(256) row_store_kernel(const Params p, int per_warp) {
   const int lane = threadIdx.x & 31;
-  for (int r0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 32; r0 < p.n_rows; r0 += gridDim.x * 256) {
-    const int r = r0 + lane;
-    const int slot = r < p.n_rows ? p.slots[r] : -1;
-    const int page = page_of(p, slot);
-    for (unsigned todo = __ballot_sync(0xffffffffu, page >= 0 && p.cand[page < 0 ? 0 : page] >= kCandMin); todo != 0; todo &= todo - 1) {
-      const int l = __ffs(static_cast<int>(todo)) - 1;
-      const int page_l = __shfl_sync(0xffffffffu, page, l);
-      store_row(p, r0 + l, __shfl_sync(0xffffffffu, slot, l), make_divisor(p.scale[page_l]), lane);
-    }
+  const long long r0 = (static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5)) * per_warp;
+  const int slot = lane < per_warp && r0 + lane < p.n_rows ? p.slots[r0 + lane] : -1;
+  const int page = page_of(p, slot);
+  const unsigned word = page >= 0 ? p.cand[page] : 0u;
+  const float scale = word >= kCandMin ? p.scale[page] : 0.0f;
+  for (unsigned todo = __ballot_sync(0xffffffffu, word >= kCandMin); todo != 0; todo &= todo - 1) {
+    const int l = __ffs(static_cast<int>(todo)) - 1;
+    store_row(p, static_cast<int>(r0) + l, __shfl_sync(0xffffffffu, slot, l), make_divisor(__shfl_sync(0xffffffffu, scale, l)), lane);
   }
 }
 
@@ -516,7 +528,12 @@ extern "C" FTB_API int ftb_kv_cache_write_fp8(const ftb_kv_cache_write_args* a, 
   if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(run_write)");
   kvw::run_count_kernel<<<row_blocks, 256, 0, st>>>(p);
   kvw::run_write_kernel<<<static_cast<unsigned>((static_cast<long long>(a->n_rows) + kvw::kChunk - 1) / kvw::kChunk), kvw::kRunThreads, kvw::kRunSmem, st>>>(p);
-  kvw::page_settle_kernel<<<static_cast<unsigned>((static_cast<long long>(a->num_pages) + 7) / 8), 256, 0, st>>>(p);
-  kvw::row_store_kernel<<<row_blocks < 1184u ? row_blocks : 1184u, 256, 0, st>>>(p);
+  // Pages with several runs.  The settle kernel: eight CTAs per SM, or one per page.  The store kernel: as many rows per warp as keep it at
+  // one wave, up to 32.
+  kvw::page_settle_kernel<<<static_cast<unsigned>(a->num_pages < 1184 ? a->num_pages : 1184), 256, 0, st>>>(p);
+  int per_warp = 1;
+  while (per_warp < 32 && static_cast<long long>(per_warp) * 9472 < a->n_rows) per_warp *= 2;
+  const long long per_cta = 8LL * per_warp;
+  kvw::row_store_kernel<<<static_cast<unsigned>((a->n_rows + per_cta - 1) / per_cta), 256, 0, st>>>(p, per_warp);
   return check_cuda(cudaGetLastError(), "ftb_kv_cache_write_fp8 launch");
 }

@@ -328,17 +328,19 @@ __global__ void __launch_bounds__(kRunThreads, 3) run_write_kernel(const Params 
     float mx = 0.0f;
     for (int i = 0; i < len; ++i) mx = fmaxf(mx, row_amax(p, r + i, lane));
     const float cand = scale_of(warp_max(mx));
-    if (p.cand[page] != 1u) {                             // several runs
+    const unsigned runs = p.cand[page];
+    const float old = p.scale[page];
+    const bool rises = cand > old;
+    // several runs, or a page to requantise that is too much for a warp: to the kernels behind this one
+    if (runs != 1u || (rises && old > 0.0f && p.page_size > kWarpRun)) {
       if (lane == 0) atomicMax(p.cand + page, __float_as_uint(cand));
       continue;
     }
-    const float old = p.scale[page];
-    __syncwarp();
-    if (cand > old) {
-      if (old > 0.0f) requantise(p, page, old, cand, lane, 32);
+    if (rises && old > 0.0f) {
+      requantise(p, page, old, cand, lane, 32);
       __syncwarp();
-      if (lane == 0) p.scale[page] = cand;
     }
+    if (lane == 0 && rises) p.scale[page] = cand;
     const Divisor d = make_divisor(cand > old ? cand : old);
     for (int i = 0; i < len; ++i) store_row(p, r + i, slot_at(r + i), d, lane);
   }

@@ -211,18 +211,20 @@ __device__ __forceinline__ int page_of(const Params& p, int slot) {
   return page < p.num_pages ? page : -1;
 }
 
-// first row of a run: the page changes here.  Pages of more than kMaxRun rows have their runs cut every kMaxRun rows, so
-// that no CTA is left with a long one.
-constexpr int kMaxRun = 256;
+// first row of a run: the page changes here.  Pages of more than kMaxRun rows, what a CTA of run_write_kernel holds, have their runs
+// cut every kMaxRun rows, so that no CTA is left with a long one (65 536 rows in pages of 256: 76 us with runs of 256, 58 now).
+constexpr int kMaxRun = 64;
 __device__ __forceinline__ bool is_head(const Params& p, int r, int page) {
   return r == 0 || page_of(p, p.slots[r - 1]) != page || (p.page_size > kMaxRun && r % kMaxRun == 0);
 }
 
 constexpr int kSmallRows = 1024;
-__global__ void __launch_bounds__(256) small_write_kernel(const Params p) {
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads) small_write_kernel(const Params p) {
+  constexpr int kWarps = kThreads / 32;
   __shared__ int mine[kSmallRows];
   __shared__ int n_mine;
-  __shared__ float wmax[8];
+  __shared__ float wmax[kWarps];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int r0 = blockIdx.x;
   const int slot0 = p.slots[r0];
@@ -235,7 +237,7 @@ __global__ void __launch_bounds__(256) small_write_kernel(const Params p) {
   if (tid == 0) n_mine = 0;
   __syncthreads();
   int earlier = 0;
-  for (int r = tid; r < p.n_rows; r += 256) {
+  for (int r = tid; r < p.n_rows; r += kThreads) {
     if (page_of(p, p.slots[r]) != page) continue;
     if (r < r0) earlier = 1;
     else mine[atomicAdd(&n_mine, 1)] = r;
@@ -243,24 +245,24 @@ __global__ void __launch_bounds__(256) small_write_kernel(const Params p) {
   if (__syncthreads_or(earlier)) return;                  // the CTA of an earlier row has this page
   const int n = n_mine;
   float mx = 0.0f;
-  for (int i = warp; i < n; i += 8) mx = fmaxf(mx, row_amax(p, mine[i], lane));
+  for (int i = warp; i < n; i += kWarps) mx = fmaxf(mx, row_amax(p, mine[i], lane));
   mx = warp_max(mx);
   if (lane == 0) wmax[warp] = mx;
   const float old = p.scale[page];
   __syncthreads();
 #pragma unroll
-  for (int w = 0; w < 8; ++w) mx = fmaxf(mx, wmax[w]);
+  for (int w = 0; w < kWarps; ++w) mx = fmaxf(mx, wmax[w]);
   const float cand = scale_of(mx);
   const float scale = cand > old ? cand : old;
   if (cand > old) {
     if (old > 0.0f) {
-      requantise(p, page, old, cand, tid, 256);
+      requantise(p, page, old, cand, tid, kThreads);
       __syncthreads();
     }
     if (tid == 0) p.scale[page] = cand;
   }
   const Divisor d = make_divisor(scale);
-  for (int i = warp; i < n; i += 8) store_row(p, mine[i], p.slots[mine[i]], d, lane);
+  for (int i = warp; i < n; i += kWarps) store_row(p, mine[i], p.slots[mine[i]], d, lane);
 }
 
 __global__ void __launch_bounds__(256) run_count_kernel(const Params p) {
@@ -519,8 +521,11 @@ extern "C" FTB_API int ftb_kv_cache_write_fp8(const ftb_kv_cache_write_args* a, 
   p.status = a->status;
   // Up to kSmallRows rows: one launch without a workspace instead of five.  A decode step over 37 353 pages spent 24 to 42 us in
   // the settle kernel alone when that had a CTA per page; such a step of 128 rows is 36 us shorter (396 -> 360 us).
-  if (a->n_rows <= kvw::kSmallRows && a->page_size <= kvw::kMaxRun) {
-    kvw::small_write_kernel<<<static_cast<unsigned>(a->n_rows), 256, 0, st>>>(p);
+  // A CTA has a page to itself, so the line also lies where the rows of one page are many: 1024 rows in pages of 256 take it 39 us, the large
+  // path 21 (both with the host's part).  More threads for pages of 128: 20.4 -> 16.2 us.
+  if (a->n_rows <= 64 || (a->n_rows <= kvw::kSmallRows && a->page_size <= 128)) {
+    if (a->n_rows <= 64 || a->page_size <= 64) kvw::small_write_kernel<256><<<static_cast<unsigned>(a->n_rows), 256, 0, st>>>(p);
+    else kvw::small_write_kernel<512><<<static_cast<unsigned>(a->n_rows), 512, 0, st>>>(p);
     return check_cuda(cudaGetLastError(), "ftb_kv_cache_write_fp8 launch");
   }
   cudaError_t e = cudaMemsetAsync(p.cand, 0, static_cast<size_t>(a->num_pages) * 4, st);

@@ -278,13 +278,14 @@ __global__ void __launch_bounds__(256) run_count_kernel(const Params p) {
   if (is_head(p, r, page)) atomicAdd(p.cand + page, 1u);
 }
 
-constexpr int kChunk = 64;                     // rows whose run heads one CTA looks after
+constexpr int kChunk = 64;                     // most rows whose run heads one CTA looks after (kHeads)
 constexpr int kWarpRun = 8;                    // longer runs take the whole CTA
 constexpr int kRunThreads = 512;
 constexpr int kRunWarps = kRunThreads / 32;
 constexpr int kRowVecs = kD / 8;               // 72 pieces of 16 bytes per row
 constexpr int kHeld = 9;                       // pieces a lane keeps in shared memory: a warp holds 4 rows (288 pieces), the CTA 64
 constexpr int kRunSmem = kHeld * kRunThreads * 16;
+template <int kHeads>
 __global__ void __launch_bounds__(kRunThreads, 3) run_write_kernel(const Params p) {
   extern __shared__ uint4 keep[];              // piece x of the run; a thread reads only what it copied itself
   __shared__ int slot_of[2 * kChunk + 1], page_at[2 * kChunk + 1];   // rows c0 - 1 .. c0 + 127: the chunk and what its last run may reach into
@@ -293,7 +294,7 @@ __global__ void __launch_bounds__(kRunThreads, 3) run_write_kernel(const Params 
   __shared__ int n_long, n_short, first_break;
   __shared__ unsigned wmax[kRunWarps];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int c0 = blockIdx.x * kChunk;
+  const int c0 = blockIdx.x * kHeads;
   if (tid <= 2 * kChunk) {
     const int r = c0 - 1 + tid;
     const int slot = r >= 0 && r < p.n_rows ? p.slots[r] : -1;
@@ -309,7 +310,7 @@ __global__ void __launch_bounds__(kRunThreads, 3) run_write_kernel(const Params 
   }
   __syncthreads();
   auto slot_at = [&](int r) { return r - c0 < 2 * kChunk ? slot_of[r - c0 + 1] : p.slots[r]; };
-  if (tid < kChunk && page_at[tid + 1] >= 0 && ((breaks[warp] >> lane) & 1u)) {
+  if (tid < kHeads && page_at[tid + 1] >= 0 && ((breaks[warp] >> lane) & 1u)) {
     // the next break behind this head, if it lies in the window
     int word = warp;
     unsigned rest = lane == 31 ? 0u : breaks[word] & (0xffffffffu << (lane + 1));
@@ -531,10 +532,14 @@ extern "C" FTB_API int ftb_kv_cache_write_fp8(const ftb_kv_cache_write_args* a, 
   cudaError_t e = cudaMemsetAsync(p.cand, 0, static_cast<size_t>(a->num_pages) * 4, st);
   if (e != cudaSuccess) return check_cuda(e, "ftb_kv_cache_write_fp8: cudaMemsetAsync");
   const unsigned row_blocks = static_cast<unsigned>((static_cast<long long>(a->n_rows) + 255) / 256);
-  e = cudaFuncSetAttribute(kvw::run_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kvw::kRunSmem);
+  // Rows per CTA of the write kernel: few enough that one wave holds all CTAs where it can, since the runs of a CTA go one after the other.
+  int heads = 16;
+  while (heads < kvw::kChunk && static_cast<long long>(heads) * 444 < a->n_rows) heads *= 2;
+  const auto run_write = heads == 16 ? kvw::run_write_kernel<16> : heads == 32 ? kvw::run_write_kernel<32> : kvw::run_write_kernel<kvw::kChunk>;
+  e = cudaFuncSetAttribute(run_write, cudaFuncAttributeMaxDynamicSharedMemorySize, kvw::kRunSmem);
   if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(run_write)");
   kvw::run_count_kernel<<<row_blocks, 256, 0, st>>>(p);
-  kvw::run_write_kernel<<<static_cast<unsigned>((static_cast<long long>(a->n_rows) + kvw::kChunk - 1) / kvw::kChunk), kvw::kRunThreads, kvw::kRunSmem, st>>>(p);
+  run_write<<<static_cast<unsigned>((static_cast<long long>(a->n_rows) + heads - 1) / heads), kvw::kRunThreads, kvw::kRunSmem, st>>>(p);
   // Pages with several runs.  The settle kernel: eight CTAs per SM, or one per page.  The store kernel: as many rows per warp as keep it at
   // one wave, up to 32.
   kvw::page_settle_kernel<<<static_cast<unsigned>(a->num_pages < 1184 ? a->num_pages : 1184), 256, 0, st>>>(p);

@@ -186,7 +186,11 @@ def kv_cache_write_fp8_ref(rows: torch.Tensor, slot_mapping: torch.Tensor, kv_ca
     Per touched page: new = max(old, max|new rows of the page| / 448) with the maximum floored at 1e-12; if
     new > old and old > 0 every byte of the page is requantised as e4m3(decode(byte) * old / new); then the new
     rows are stored as e4m3(clamp(x / new, +-448)).  All arithmetic in fp32, divisions IEEE, conversion to e4m3
-    round-to-nearest-even."""
+    round-to-nearest-even.  A NaN has no say in the maximum and is stored as -448, and so is the quotient of two
+    infinities: an infinite row makes its page's scale infinite, and everything finite in the page zero."""
+    def to_e4m3(v):
+        return torch.where(torch.isnan(v), torch.full_like(v, -E4M3_MAX), v.clamp(-E4M3_MAX, E4M3_MAX)).to(torch.float8_e4m3fn).view(torch.uint8)
+
     x = _as_f32(rows)
     slots = slot_mapping.detach().to("cpu").to(torch.int64)
     cache = kv_cache_u8.detach().to("cpu").clone()
@@ -197,7 +201,7 @@ def kv_cache_write_fp8_ref(rows: torch.Tensor, slot_mapping: torch.Tensor, kv_ca
     assert page == page_size
     keep = slots >= 0
     pages = slots[keep] // page_size
-    row_amax = x[keep].abs().amax(dim=1).clamp(min=1e-12)
+    row_amax = torch.where(torch.isnan(x[keep]), torch.zeros(()), x[keep].abs()).amax(dim=1).clamp(min=1e-12)
     cand = torch.zeros(n_pages, dtype=torch.float32)
     cand.scatter_reduce_(0, pages, (row_amax / E4M3_MAX).to(torch.float32), reduce="amax", include_self=True)
     for pg in torch.unique(pages).tolist():
@@ -207,11 +211,10 @@ def kv_cache_write_fp8_ref(rows: torch.Tensor, slot_mapping: torch.Tensor, kv_ca
         if old > 0:
             dec = cache[pg].view(torch.float8_e4m3fn).to(torch.float32)
             re = ((dec * torch.tensor(old, dtype=torch.float32)) / torch.tensor(new, dtype=torch.float32))
-            cache[pg] = re.clamp(-E4M3_MAX, E4M3_MAX).to(torch.float8_e4m3fn).view(torch.uint8)
+            cache[pg] = to_e4m3(re)
         scale[pg] = new
     flat = cache.view(n_pages * page, d)
-    qv = (x[keep] / scale[pages][:, None]).clamp(-E4M3_MAX, E4M3_MAX).to(torch.float8_e4m3fn).view(torch.uint8)
-    flat[slots[keep]] = qv
+    flat[slots[keep]] = to_e4m3(x[keep] / scale[pages][:, None])
     return cache, scale
 
 

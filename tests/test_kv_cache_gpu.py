@@ -129,3 +129,46 @@ def test_write_paths_bit_exact(n, page, order):
     g_cache, g_scale, r_cache, r_scale = _write_both(x.bfloat16(), slots, cache, scale, page)
     assert torch.equal(g_scale, r_scale)
     assert torch.equal(g_cache, r_cache)
+
+
+@pytest.mark.parametrize("n,page,order", [(8, 64, "runs"), (1000, 128, "runs"), (60, 256, "runs"), (1100, 5, "runs"), (1100, 64, "runs"), (1100, 64, "nines"),
+                                          (1100, 64, "halves"), (1100, 512, "runs")])
+def test_rows_that_are_no_numbers(n, page, order):
+    """NaN and infinities on every route: the maximum leaves a NaN out, its byte is that of -448; an infinite row makes the scale of its page
+    infinite.  Runs of up to 8 rows (a warp's), of 9 to 64 (a CTA's, with and without a NaN among its rows), longer ones, pages in two
+    runs, small calls."""
+    g = torch.Generator().manual_seed(n + page)
+    n_pages = -(-n // (9 if order == "nines" else page)) + 1
+    at = torch.arange(n)
+    perm = torch.randperm(n_pages, generator=g)
+    slots = perm[at // 9] * page + at % 9 if order == "nines" else perm[at // page] * page + at % page
+    if order == "halves":
+        half = at % 64 < 32
+        slots = torch.cat([slots[half], slots[~half]])
+    x = torch.randn(n, 576, generator=g)
+    x[torch.rand(n, generator=g) < 0.1, 3] = float("nan")
+    x[torch.rand(n, generator=g) < 0.1, 570] = -float("nan")
+    x[n // 2, :] = float("nan")
+    x[n // 3, 100] = float("inf")
+    x[n - 1, 200] = -float("inf")
+    cache = torch.randint(0, 120, (n_pages, page, 576), generator=g, dtype=torch.uint8)
+    scale = torch.rand(n_pages, generator=g) * 0.01 * (torch.rand(n_pages, generator=g) < 0.5)
+    g_cache, g_scale, r_cache, r_scale = _write_both(x.bfloat16(), slots.int(), cache, scale, page)
+    assert torch.equal(g_scale, r_scale)
+    assert torch.equal(g_cache, r_cache)
+
+
+@pytest.mark.parametrize("n,page", [(1100, 64), (1100, 16), (1100, 8), (1100, 4), (65, 256), (1024, 128), (1025, 128), (2000, 1024)])
+def test_scattered_rows_that_raise_their_pages(n, page):
+    """One-row runs in pages of their own and, above 64 rows to a page, runs that fill pages, all under a scale that rises: pages requantised
+    by a warp, by a CTA and by the kernel behind, and more pages than that kernel has CTAs."""
+    g = torch.Generator().manual_seed(n + page)
+    n_pages = n + 3 if page <= 64 else -(-n // page) + 1
+    perm = torch.randperm(n_pages, generator=g)
+    at = torch.arange(n)
+    slots = perm[at] * page + torch.randint(0, page, (n,), generator=g) if page <= 64 else perm[at // page] * page + at % page
+    cache = torch.randint(0, 120, (n_pages, page, 576), generator=g, dtype=torch.uint8)
+    scale = torch.rand(n_pages, generator=g) * 0.02
+    g_cache, g_scale, r_cache, r_scale = _write_both(torch.randn(n, 576, generator=g).bfloat16(), slots.int(), cache, scale, page)
+    assert torch.equal(g_scale, r_scale)
+    assert torch.equal(g_cache, r_cache)

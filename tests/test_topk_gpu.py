@@ -113,3 +113,22 @@ def test_edges_of_the_row_kernels(s_kv):
     for k in (2048, 1, s_kv - 1):
         got = topk_indices(sc.to(DEV), k, lengths.to(DEV)).cpu()
         assert torch.equal(got, topk_indices_ref(sc, k, lengths)), k
+
+
+@pytest.mark.parametrize("s_q,s_kv", [(300, 33), (7, 1000), (160, 5119), (3, 5121), (150, 6656), (149, 6657), (5, 20001), (150, 32765), (300, 40003)])
+def test_ties_and_lengths_on_every_kernel(s_q, s_kv):
+    """Rows of few values, rows padded with -inf, rows that are short in a long matrix and rows that do not start on a 16-byte boundary, at
+    sizes either side of the lines between the kernels."""
+    g = torch.Generator().manual_seed(s_kv)
+    sc = torch.randn(s_q, s_kv, generator=g)
+    sc[::3] = (sc[::3] * 4).round()
+    sc[1::3] = torch.where(torch.arange(s_kv) < s_kv // 20, sc[1::3], float("-inf"))
+    lengths = torch.randint(0, s_kv + 1, (s_q,), generator=g).int()
+    lengths[::2] = torch.minimum(lengths[::2], torch.randint(1, 6000, (lengths[::2].numel(),), generator=g).int())
+    lengths[:3] = torch.tensor([s_kv, 0, 1])
+    wide = torch.zeros(s_q, s_kv + 5)
+    wide[:, 1:s_kv + 1] = sc
+    for k in (min(512, s_kv), min(2048, s_kv)):
+        ref = topk_indices_ref(sc, k, lengths)
+        assert torch.equal(topk_indices(sc.to(DEV), k, lengths.to(DEV)).cpu(), ref)
+        assert torch.equal(topk_indices(wide.to(DEV)[:, 1:s_kv + 1], k, lengths.to(DEV)).cpu(), ref)

@@ -120,9 +120,12 @@ def load() -> C.CDLL:
                 raise RuntimeError("ftb_topk_args layout differs between the header and the Python mirror")
             lib.ftb_topk_indices.argtypes = [C.POINTER(TopkArgs), C.c_void_p]
             lib.ftb_gemm_bf16.argtypes = [C.POINTER(GemmArgs), C.c_void_p]
+            lib.ftb_gemm_bf16_whole_k.argtypes = [C.POINTER(GemmArgs), C.c_void_p]
+            lib.ftb_gemm_plan.argtypes = [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int32)]
             if lib.ftb_sizeof_gemm_fp8_args() != C.sizeof(GemmFp8Args):
                 raise RuntimeError("ftb_gemm_fp8_args layout differs between the header and the Python mirror")
             lib.ftb_gemm_fp8_blockscaled.argtypes = [C.POINTER(GemmFp8Args), C.c_void_p]
+            lib.ftb_gemm_fp8_blockscaled_whole_k.argtypes = [C.POINTER(GemmFp8Args), C.c_void_p]
             lib.ftb_gemm_rs_workspace_bytes.argtypes = [C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]
             lib.ftb_gemm_rs_ctx_create.argtypes = [C.POINTER(C.c_void_p), C.c_int, C.c_int, C.c_int, C.c_int,
                                                    C.POINTER(C.c_void_p), C.POINTER(C.c_void_p)]

@@ -399,15 +399,15 @@ struct Shape { int ncta, splits; };
 //   64 x 1024 x 7168: 25.4, 18.4, 32.8, 26.6     64 x 8192 x 3584: 18.5, 59 (four waves), 23.4, 23.3
 //   512 x 4096 x 7168: 29.5, -, 38.9, 30.7       1024 x 4096 x 7168: 50.0, -, 39.8, 55.3
 //   2048 x 8192 x 3584: 88, -, 74.6, 150         4096 x 8192 x 28672: 1240, -, 913, 1106
-// A split runs as one wave only: clusters that queue for SMs cost about ten microseconds a wave.
-inline Shape pick_shape(int m, int n, int k, int sms) {
+// A split runs as one wave only: clusters that queue for SMs cost about ten microseconds a wave.  `whole_k` keeps K in one part.
+inline Shape pick_shape(int m, int n, int k, int sms, bool whole_k) {
   const int kb = k / BK;
   Shape best{1, 1};
   long long best_t = -1;
   for (int ncta = 1; ncta <= 2; ++ncta) {
     const long long tiles = static_cast<long long>((m + BM * ncta - 1) / (BM * ncta)) * ((n + 128 * ncta - 1) / (128 * ncta));
     for (int s = 1; s * ncta <= (ncta == 1 ? 8 : 4); s *= 2) {
-      if (s > 1 && (kb < 2 * s || tiles * s * ncta > sms - sms / 8)) break;   // an eighth of the SMs may not host a cluster
+      if (s > 1 && (whole_k || kb < 2 * s || tiles * s * ncta > sms - sms / 8)) break;   // an eighth of the SMs may not host a cluster
       const long long waves = s > 1 ? 1 : (tiles + sms / ncta - 1) / (sms / ncta);
       const long long t = waves * ((kb + s - 1) / s) * (ncta == 1 ? 33 : 50) + (s == 1 ? 0 : s == 2 ? 500 : s == 4 ? 600 : 700);
       if (best_t < 0 || t < best_t) { best_t = t; best = Shape{ncta, s}; }
@@ -417,11 +417,19 @@ inline Shape pick_shape(int m, int n, int k, int sms) {
 }
 
 }  // namespace gemm8
+
+// CTAs per tile and parts of K of a launch
+void plan_gemm_fp8(int m, int n, int k, int sms, int* ctas, int* parts) {
+  const gemm8::Shape s = gemm8::pick_shape(m, n, k, sms, false);
+  *ctas = s.ncta;
+  *parts = s.splits;
+}
+
 }  // namespace ftb
 
 using namespace ftb;
 
-extern "C" FTB_API int ftb_gemm_fp8_blockscaled(const ftb_gemm_fp8_args* g, void* stream) {
+static int gemm_fp8_blockscaled(const ftb_gemm_fp8_args* g, bool whole_k, void* stream) {
   if (!g || !g->a || !g->b || !g->c || !g->a_scale || !g->b_scale) { set_last_error("ftb_gemm_fp8_blockscaled: null pointer"); return FTB_ERR_INVALID; }
   if (g->m <= 0 || g->n <= 0 || g->k <= 0 || (g->k % 128) || (g->n % 128)) {
     set_last_error("ftb_gemm_fp8_blockscaled: need k and n multiples of 128 (scale blocks), got m=%d n=%d k=%d", g->m, g->n, g->k);
@@ -435,7 +443,7 @@ extern "C" FTB_API int ftb_gemm_fp8_blockscaled(const ftb_gemm_fp8_args* g, void
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const gemm8::Shape shape = gemm8::pick_shape(g->m, g->n, g->k, sms);
+  const gemm8::Shape shape = gemm8::pick_shape(g->m, g->n, g->k, sms, whole_k);
   CUtensorMap tm_a, tm_b;
   const bool bkm = g->b_kmajor != 0;
   const int box_m = g->m < gemm8::BM ? (g->m + 7) & ~7 : gemm8::BM;   // whole swizzle atoms of eight rows
@@ -481,3 +489,7 @@ extern "C" FTB_API int ftb_gemm_fp8_blockscaled(const ftb_gemm_fp8_args* g, void
   if (e != cudaSuccess) return check_cuda(e, "gemm_fp8 launch");
   return FTB_OK;
 }
+
+extern "C" FTB_API int ftb_gemm_fp8_blockscaled(const ftb_gemm_fp8_args* g, void* stream) { return gemm_fp8_blockscaled(g, false, stream); }
+
+extern "C" FTB_API int ftb_gemm_fp8_blockscaled_whole_k(const ftb_gemm_fp8_args* g, void* stream) { return gemm_fp8_blockscaled(g, true, stream); }

@@ -138,12 +138,12 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       *reinterpret_cast<uint4*>(p.c + static_cast<long long>(row) * p.ldc + n0 + col) = o;
     }
   };
-  if (p.splits == 1) {
+  if (BN != 64 || p.splits == 1) {
     if (writes) {
 #pragma unroll
       for (int j = 0; j < BN; j += 8) put8(acc + j, j);
     }
-  } else {
+  } else if constexpr (BN == 64) {
     // Every part of K has been multiplied and read from the stages, which become the meeting place: part s gets columns
     // [s cw, (s + 1) cw), as 16-byte pieces with the row fastest.
     cluster_sync_all();
@@ -186,18 +186,15 @@ struct Shape { int bn, splits; };
 // Taken when the persistent kernel would use at most half of the SMs, with the narrowest tile that still is one wave.  Around
 // the line (us, persistent / this one): 512 x 4096 x 2304, 64 tiles of 256, 19.9 / 14.3; 256 x 7168 x 512, 56 tiles, 11.9 / 7.6;
 // above it, at 512 x 7168 (112 tiles), the persistent kernel is at its full rate.  K is split as long as the clusters fit and a
-// part keeps eight K blocks: 128 x 512 x 2304 17.3 / 7.3.
-inline Shape pick_shape(int m, int n, int k, int sms) {
+// part keeps four K blocks: 128 x 512 x 2304 17.3 / 7.3.  Only tiles of 64 columns can be so few; `whole_k` keeps K in one part.
+inline Shape pick_shape(int m, int n, int k, int sms, bool whole_k) {
   const int mb = (m + BM - 1) / BM, kb = (k + BK - 1) / BK;
   if (mb * ((n + 255) / 256) * 2 > sms) return Shape{0, 1};
-  for (int bn = 64; bn <= 128; bn *= 2) {
-    const int tiles = mb * ((n + bn - 1) / bn);
-    if (tiles > sms) continue;
-    int s = 1;
-    while (s < 4 && tiles * s * 2 <= sms - sms / 8 && kb >= 8 * s) s *= 2;   // an eighth of the SMs may not host a cluster
-    return Shape{bn, s};
-  }
-  return Shape{0, 1};
+  const int tiles = mb * ((n + 63) / 64);
+  if (tiles > sms) return Shape{128, 1};                     // at most twice the tiles of 256 columns: one wave
+  int s = 1;
+  while (!whole_k && s < 4 && tiles * s * 2 <= sms - sms / 8 && kb >= 8 * s) s *= 2;   // an eighth of the SMs may not host a cluster
+  return Shape{64, s};
 }
 
 template <int BN>
@@ -239,15 +236,22 @@ static int launch(const void* a, const void* b, void* c, int m, int n, int k, lo
 
 // Takes the product if its shape is one of these; *taken says so.
 int launch_gemm_small(const void* a, const void* b, void* c, int m, int n, int k, long long lda, long long ldb, long long ldc, int* status,
-                      cudaStream_t st, bool* taken) {
+                      bool whole_k, cudaStream_t st, bool* taken) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const gemm_small::Shape s = gemm_small::pick_shape(m, n, k, sms);
+  const gemm_small::Shape s = gemm_small::pick_shape(m, n, k, sms, whole_k);
   *taken = s.bn != 0;
   if (s.bn == 64) return gemm_small::launch<64>(a, b, c, m, n, k, lda, ldb, ldc, s.splits, status, st);
   if (s.bn == 128) return gemm_small::launch<128>(a, b, c, m, n, k, lda, ldb, ldc, s.splits, status, st);
   return FTB_OK;
+}
+
+// Columns of a tile and parts of K of that shape; 0 columns: the persistent kernel's.
+void plan_gemm_small(int m, int n, int k, int sms, int* columns, int* parts) {
+  const gemm_small::Shape s = gemm_small::pick_shape(m, n, k, sms, false);
+  *columns = s.bn;
+  *parts = s.splits;
 }
 
 }  // namespace ftb

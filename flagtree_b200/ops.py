@@ -126,7 +126,8 @@ def sparse_mla_fwd(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor,
     token table as `indices`.  `sm_scale` defaults to 576**-0.5 (:640 of the same file).
     `check=True` reads back the device status word (one host sync) and raises on a bad index
     or a device-side timeout.  `num_splits` > 1 splits the top-k axis over several pairs of CTAs and merges the
-    partial results (the reference's NUM_KV_SPLITS stage 2); None = by the number of tokens.
+    partial results (the reference's NUM_KV_SPLITS stage 2); None = by the number of tokens, so that the bits of a token may
+    depend on how many there are; with `num_splits=1` they do not.
     """
     _require_cuda(q, kv, indices)
     if kv.dim() == 3:
@@ -425,10 +426,12 @@ def kv_cache_write_fp8(rows: torch.Tensor, slot_mapping: torch.Tensor, kv_cache:
 
 # ------------------------------------------------------------------------------------- GEMM
 def matmul(a: torch.Tensor, b: torch.Tensor, acc_dtype=None, input_precision=None, fp8_fast_accum=True,
-           output_dtype=None, *, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+           output_dtype=None, *, out: Optional[torch.Tensor] = None, whole_k: bool = False) -> torch.Tensor:
     """C = A @ B for bf16 operands with fp32 accumulation; same call shape as the reference's
     `triton.ops.matmul` (python/triton/ops/matmul.py:231-236).  Non-contiguous inputs are copied as
-    the reference does (:165-168); the shape check is the reference's assertion (:170)."""
+    the reference does (:165-168); the shape check is the reference's assertion (:170).
+    Products with few tiles add up K in up to four parts, so the bits of a row may depend on the number of rows; with
+    `whole_k` they do not."""
     _require_cuda(a, b)
     if a.stride(0) > 1 and a.stride(1) > 1:
         a = a.contiguous()
@@ -446,22 +449,24 @@ def matmul(a: torch.Tensor, b: torch.Tensor, acc_dtype=None, input_precision=Non
     n = b.shape[1]
     if out is None:
         out = torch.empty(m, n, dtype=torch.bfloat16, device=a.device)
-    _gemm_into(a, b, out)
+    _gemm_into(a, b, out, whole_k=whole_k)
     return out
 
 
-def _gemm_into(a, b, c, status=None):
+def _gemm_into(a, b, c, status=None, whole_k=False):
     m, k = a.shape
     g = _lib.GemmArgs(a.data_ptr(), b.data_ptr(), c.data_ptr(), m, b.shape[1], k, a.stride(0), b.stride(0), c.stride(0),
                       status.data_ptr() if status is not None else None)
-    _launch(_lib.load().ftb_gemm_bf16, g, a.device, "matmul")
+    lib = _lib.load()
+    _launch(lib.ftb_gemm_bf16_whole_k if whole_k else lib.ftb_gemm_bf16, g, a.device, "matmul")
 
 
 def matmul_fp8_blockscaled(a: torch.Tensor, a_scale: torch.Tensor, b: torch.Tensor, b_scale: torch.Tensor, *,
-                           out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                           out: Optional[torch.Tensor] = None, whole_k: bool = False) -> torch.Tensor:
     """C = (A * a_scale) @ (B * b_scale) for e4m3 operands (uint8 or float8_e4m3fn storage) with 1x128 (A) and
     128x128 (B) fp32 block scales; bf16 result.  Operands follow the reference's fp8 matmul convention of
-    raw 8-bit patterns (python/test/unit/operators/test_matmul.py:165-169)."""
+    raw 8-bit patterns (python/test/unit/operators/test_matmul.py:165-169).  Products with few tiles add up K in up to eight
+    parts, so the bits of a row may depend on the number of rows; with `whole_k` they do not."""
     _require_cuda(a, a_scale, b, b_scale)
     for t in (a, b):
         assert t.dtype in (torch.uint8, torch.float8_e4m3fn), "operands must hold e4m3 bytes"
@@ -481,7 +486,8 @@ def matmul_fp8_blockscaled(a: torch.Tensor, a_scale: torch.Tensor, b: torch.Tens
     g = _lib.GemmFp8Args(a.data_ptr(), b.data_ptr(), out.data_ptr(), a_scale.data_ptr(), b_scale.data_ptr(), m, n, k,
                          a.stride(0), b.stride(1) if b_kmajor else b.stride(0), out.stride(0), a_scale.stride(0),
                          b_scale.stride(0), None, 1 if b_kmajor else 0)
-    _launch(_lib.load().ftb_gemm_fp8_blockscaled, g, a.device, "matmul_fp8_blockscaled")
+    lib = _lib.load()
+    _launch(lib.ftb_gemm_fp8_blockscaled_whole_k if whole_k else lib.ftb_gemm_fp8_blockscaled, g, a.device, "matmul_fp8_blockscaled")
     return out
 
 

@@ -50,8 +50,8 @@ def test_fp8_unit_scales_equal_plain_product():
     assert torch.equal(c, (a @ b).bfloat16().float())      # small integers: every partial sum is exact
 
 
-# One shape per choice of the dispatch (tile of one CTA or of a pair, K in 1, 2, 4, 8 parts), each with a remainder in M
-# and, for the pairs, an N that ends in the middle of a 256-column tile.  The sums of the parts of K are added in fp32,
+# Tiles of one CTA with K in 1, 4 and 8 parts and tiles of a pair (the other choices are further down), most with a remainder
+# in M and, for the pairs, an N that ends in the middle of a 256-column tile.  The sums of the parts of K are added in fp32,
 # so the bound is the same as for one part: the bf16 rounding of the result.
 @pytest.mark.parametrize("m,n,k", [(1, 128, 128), (7, 128, 256), (64, 1024, 7168), (130, 512, 2048), (60, 2048, 1024), (33, 3968, 4096),
                                    (129, 8192, 256), (520, 4224, 640), (1025, 8064, 128), (2049, 4224, 384)])
@@ -67,3 +67,26 @@ def test_fp8_tile_shapes_and_parts_of_k(m, n, k, nk):
     ref = deq_a.view(m, k) @ deq_b.view(k, n)
     # 2^-8 of the value for the bf16 result, 2^-17 of the largest value for sums in fp32 in any order
     assert ((c - ref).abs() <= 2 ** -8 * ref.abs() + 2 ** -17 * ref.abs().max()).all()
+
+
+# One shape or two per route of the dispatch on 148 SMs: (columns of a tile, CTAs that share it, parts of K).
+ROUTES = {(128, 1, 1): [(60, 2048, 1024), (130, 512, 1024)], (128, 1, 2): [(40, 8192, 7168)], (128, 1, 4): [(33, 3968, 4096)], (128, 1, 8): [(64, 1024, 7168)],
+          (256, 2, 1): [(1025, 2176, 384), (1030, 3200, 1664)], (256, 2, 2): [(142, 4608, 13824), (162, 4224, 10240), (395, 2304, 15616)]}
+
+
+@pytest.mark.parametrize("m,n,k", [s for shapes in ROUTES.values() for s in shapes])
+@pytest.mark.parametrize("nk", [False, True])
+def test_fp8_every_route(m, n, k, nk):
+    """The result, and the same with K in one part: a row then has the bits that it has in a product of many rows."""
+    g = torch.Generator(device=DEV).manual_seed(m + n + k)
+    a8, a_s = W.quantize_block_e4m3(torch.randn(m + 2048, k, generator=g, device=DEV), 1, 128)
+    b8, b_s = W.quantize_block_e4m3(torch.randn(k, n, generator=g, device=DEV), 128, 128)
+    b = b8.t().contiguous().t() if nk else b8
+    deq_a = a8[:m].view(torch.float8_e4m3fn).double().view(m, k // 128, 128) * a_s[:m].double()[..., None]
+    deq_b = b8.view(torch.float8_e4m3fn).double().view(k // 128, 128, n // 128, 128) * b_s.double()[:, None, :, None]
+    ref = deq_a.view(m, k) @ deq_b.view(k, n)
+    whole = matmul_fp8_blockscaled(a8[:m], a_s[:m], b, b_s, whole_k=True)
+    for c in (matmul_fp8_blockscaled(a8[:m], a_s[:m], b, b_s), whole):
+        # 2^-8 of the value for the bf16 result, 2^-16 of the largest value for sums in fp32 in any order
+        assert ((c.double() - ref).abs() <= 2 ** -8 * ref.abs() + 2 ** -16 * ref.abs().max()).all()
+    assert torch.equal(whole, matmul_fp8_blockscaled(a8, a_s, b, b_s, whole_k=True)[:m])

@@ -36,8 +36,9 @@ def test_matmul_shapes(m, n, k):
 @pytest.mark.parametrize("m,n,k", [(1, 512, 512), (50, 7168, 2304), (64, 9472, 128), (127, 8, 520), (129, 4160, 2304), (512, 512, 1024),
                                    (40, 4104, 584), (8, 136, 64), (300, 6152, 1000), (17, 2048, 72)])
 def test_products_with_few_tiles(m, n, k):
-    """Shapes that leave most SMs idle at 128 x 256: narrow tiles (64 and 128 columns, a last one of 8), K in one, two and four
-    parts with K tails and parts of unequal length, one to five row blocks, row counts that are not a multiple of eight."""
+    """Shapes that leave most SMs idle at 128 x 256: narrow tiles (64 columns, a last one of 8), K in one, two and four
+    parts with K tails and parts of unequal length, one to four row blocks, row counts that are not a multiple of eight; and the
+    persistent kernel just above the line (300 x 6152)."""
     g = torch.Generator().manual_seed(m + n + k)
     a = torch.randn(m, k, generator=g).bfloat16()
     b = torch.randn(k, n, generator=g).bfloat16()
@@ -98,3 +99,23 @@ def test_determinism():
     a = torch.randn(1024, 2304, generator=g).bfloat16().to(DEV)
     b = torch.randn(2304, 1792, generator=g).bfloat16().to(DEV)
     assert torch.equal(matmul(a, b), matmul(a, b))
+
+
+# One shape or two per route of the dispatch on 148 SMs, with tails in M, N and K: (columns of a tile, CTAs that share it, parts of K).
+ROUTES = {(64, 1, 1): [(50, 7168, 2304), (129, 4160, 200)], (64, 1, 2): [(40, 4104, 584), (33, 4096, 2304)], (64, 1, 4): [(17, 2048, 2304), (129, 512, 1096)],
+          (128, 1, 1): [(300, 6136, 1000), (512, 4096, 2304)], (256, 1, 1): [(50, 20488, 584), (128, 19456, 136)], (256, 2, 1): [(700, 6152, 328)]}
+
+
+@pytest.mark.parametrize("m,n,k", [s for shapes in ROUTES.values() for s in shapes])
+def test_every_route(m, n, k):
+    """The result, and the same with K in one part: a row then has the bits that it has in a product of many rows."""
+    g = torch.Generator(device=DEV).manual_seed(m + n + k)
+    a = torch.randn(m, k, generator=g, device=DEV).bfloat16()
+    b = torch.randn(k, n, generator=g, device=DEV).bfloat16()
+    ref = a.double() @ b.double()
+    many = torch.cat([a, torch.randn(2048, k, generator=g, device=DEV).bfloat16()])
+    whole = matmul(a, b, whole_k=True)
+    for c in (matmul(a, b), whole):
+        # 2^-8 of the value for the bf16 result, 2^-16 of the largest value for sums in fp32 in any order
+        assert ((c.double() - ref).abs() <= 2 ** -8 * ref.abs() + 2 ** -16 * ref.abs().max()).all()
+    assert torch.equal(whole, matmul(many, b, whole_k=True)[:m])

@@ -71,6 +71,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
+// After a wait that ran out: loads, copies and MMAs that were issued still land in this CTA's shared and tensor memory and signal its
+// barriers.  64 us is far longer than any of them takes on a working device; the CTA must not leave before.
+__device__ __forceinline__ void drain_after_abort() {
+  for (int i = 0; i < 64; ++i) __nanosleep(1000);
+}
+
 // ---------------------------------------------------------------- cp.async (16-byte rows gather)
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");

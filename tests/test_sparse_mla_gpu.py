@@ -549,3 +549,25 @@ def test_parts_by_either_kernel(s_q, h, topk, splits, algo):
     ref_out, ref_lse = sparse_mla_fwd_ref(q, kv, idx, 0.06)
     e_out, e_lse = _errors(out, lse, ref_out, ref_lse)
     assert e_out <= OUT_ATOL and e_lse <= LSE_RTOL
+
+
+def test_parts_on_two_streams_at_once():
+    """Calls of few tokens on two streams, each with scratch of its own: the bits of the same calls one after the other."""
+    g = torch.Generator(device=DEV).manual_seed(11)
+    calls = []
+    for s_q in (1, 9):
+        q = torch.randn(s_q, 128, 576, generator=g, device=DEV).bfloat16()
+        kv = torch.randn(4000, 576, generator=g, device=DEV).bfloat16()
+        idx = torch.rand(s_q, 4000, generator=g, device=DEV).topk(1500, dim=1).indices.int()
+        calls.append((q, kv, idx, 0.06))
+    alone = [sparse_mla_fwd(*c) for c in calls]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(DEV) for _ in calls]
+    got = [[], []]
+    for _ in range(20):
+        for i, c in enumerate(calls):
+            with torch.cuda.stream(streams[i]):
+                got[i].append(sparse_mla_fwd(*c))
+    torch.cuda.synchronize()
+    for i, (out, lse) in enumerate(alone):
+        assert all(torch.equal(o, out) and torch.equal(l, lse) for o, l in got[i])

@@ -84,3 +84,31 @@ def test_static_scratch_rejects_oversized_problems():
     rc = lib.ftb_sparse_mla_fwd_static_scratch(C.byref(a), None)
     assert rc == _lib.FTB_ERR_INVALID
     assert "built-in" in _lib.last_error()
+
+
+@pytest.mark.parametrize("algo", [0, 5])
+def test_static_scratch_entry_on_the_persistent_pairs(algo):
+    """Lists long enough for the default route: the same bits as with a workspace of the caller, which is checked elsewhere."""
+    from flagtree_b200 import _lib
+    lib = _lib.load()
+    stream = C.c_void_p(torch.cuda.current_stream(DEV).cuda_stream)
+    g = torch.Generator().manual_seed(78)
+    s_q, h, s_kv, topk, n_splits = 5, 128, 2000, 1100, 4
+    q = torch.randn(s_q, h, 576, generator=g).bfloat16().to(DEV)
+    kv = torch.randn(s_kv, 576, generator=g).bfloat16().to(DEV)
+    idx = torch.stack([torch.randperm(s_kv, generator=g)[:topk] for _ in range(s_q)]).int().to(DEV)
+    idx[0, 300:] = -1
+    out = [torch.empty(s_q, h, 512, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    lse = [torch.empty(s_q, h, dtype=torch.float32, device=DEV) for _ in range(2)]
+    ws = torch.empty(int(lib.ftb_sparse_mla_workspace_bytes(s_q, h, n_splits)), dtype=torch.uint8, device=DEV)
+    args = [_args(_lib, q, kv, idx, out[i], lse[i], 0.05, n_splits, w) for i, w in enumerate((ws, None))]
+    for a in args:
+        a.algo_id = algo
+    with torch.cuda.device(DEV):
+        assert lib.ftb_sparse_mla_fwd(C.byref(args[0]), stream) == 0, _lib.last_error()
+        assert lib.ftb_sparse_mla_fwd_static_scratch(C.byref(args[1]), stream) == 0, _lib.last_error()
+    torch.cuda.synchronize()
+    assert torch.equal(out[0], out[1]) and torch.equal(lse[0], lse[1])
+    ref_out, ref_lse = sparse_mla_fwd_ref(q.cpu(), kv.cpu(), idx.cpu(), 0.05)
+    assert (out[1].float().cpu() - ref_out).abs().max().item() <= 2e-2
+    assert ((lse[1].cpu() - ref_lse).abs() / ref_lse.abs().clamp(min=1.0)).max().item() <= 1e-3

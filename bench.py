@@ -185,7 +185,7 @@ def bench_kv_cache_write(args, dev, peaks):
     nbytes = n_rows * (1152 + 576) + n_rows * 4
     return {"workload": f"kv_cache_write_fp8_rows{n_rows}_pages{n_pages}x{page}", "ms": ms, "iters": iters,
             "bytes": nbytes, "gbs": nbytes / (ms * 1e-3) / 1e9, "frac_of_hbm_peak": nbytes / (ms * 1e-3) / 1e9 / peaks["hbm_gbs"],
-            "bound": "hbm", "kernels": "row_amax_kernel + page_settle_kernel + row_store_kernel",
+            "bound": "hbm", "kernels": "run_count_kernel + run_write_kernel + page_settle_kernel + row_store_kernel",
             "l2": "new rows (302 MB) larger than L2"}
 
 

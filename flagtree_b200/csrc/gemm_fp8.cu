@@ -18,11 +18,11 @@
 // Roles (384 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 4-11 promotion/epilogue: warp w takes
 // TMEM lanes 32 (w % 4) .. and half (w / 4 - 1) of the columns, so a thread holds 128 (64) fp32 sums.  Per K block a
 // thread needs one product of two scales: they are fetched from memory a group of four blocks ahead.
-// Measured (TFLOP/s, one GPU, K = 28672, N = 8192): M = 4096 2107, M = 1024 1130; the kernel before (128 x 128 tiles, four
-// promotion warps that fetched their scales when they needed them) 1078 and 912.  Steps of M = 4096: eight promotion
+// Measured, one GPU, K = 28672, N = 8192.  M = 4096 back to back, where the power limit sets the clock: 1064 us a call (1808 TFLOP/s) against
+// 1848 of the kernel before (128 x 128 tiles, four promotion warps that fetched their scales when they needed them).  Launches
+// with pauses between them (TFLOP/s): M = 4096 2107 (before 1078), M = 1024 1130 (912).  Steps of M = 4096 that way: eight promotion
 // warps, scales ahead, single tiles 1269 and pairs 1037; the pair's hand-back of an accumulator as a relaxed remote
 // arrival (a release at cluster scope stalls the warp) 1921; the pieces of neighbouring K blocks as one stream 2107.
-// Back to back for 0.15 s, where the power limit sets the clock: 1064 us a call against 1848 of the kernel before.
 // What bounds it now: with the additions left out 826 us instead of 913, with the tensor-memory loads left out too 680 us
 // (the tensor pipe and the power limit: a library e4m3 GEMM reaches 2960).
 #include <cstring>
@@ -317,7 +317,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                 __syncwarp();
                 if (lane == 0) {
                   if constexpr (NCTA == 1) mbar_arrive(be0 + acc * 8);
-                  else mbar_arrive_cluster_relaxed(be0 + acc * 8);   // nothing but the read that is over depends on it
+                  // Relaxed is enough: what the issuer's MMA may not overtake are the loads of this accumulator, and
+                  // tcgen05.wait::ld has seen them complete in this warp before the lane arrives.  No other write of these
+                  // warps is handed over, and tensor memory is not reached through the generic proxy.
+                  else mbar_arrive_cluster_relaxed(be0 + acc * 8);
                 }
                 ++it;
                 if (kq + j + 1 < kb1) begin_block();

@@ -142,17 +142,8 @@ __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t adesc, uin
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// A operand from tensor memory (128 lanes x 8 columns per K = 16 step, two bf16 per 32-bit column), B from shared memory.
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The same two forms for an unrolled issue loop: the shared-memory descriptor arrives as its two 32-bit
+// For an unrolled issue loop, with A from shared memory or from tensor memory (128 lanes x 8 columns per K = 16 step, two bf16 per
+// 32-bit column): the shared-memory descriptor arrives as its two 32-bit
 // halves (only the low one, which holds the address, changes between steps) and the accumulate flag is a
 // compile-time constant, so that one step costs the issuing thread an integer add or two.  A lone thread
 // runs dependent instructions several cycles apart; a loop that rebuilds 64-bit descriptors per step was
@@ -176,16 +167,6 @@ __device__ __forceinline__ void umma_f16_ss_lohi(uint32_t d_tmem, uint32_t a_lo,
       "mov.b64 bd, {%3, %4};\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], ad, bd, %5, p;\n\t}"
       ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "n"(kAccumulate ? 1 : 0)
-      : "memory");
-}
-// Same with fp8 (e4m3/e5m2) operands: K = 32 per instruction.
-__device__ __forceinline__ void umma_f8_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // The mbarrier gets one arrival when every tcgen05.mma issued so far by this thread has finished.
@@ -227,16 +208,6 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 }
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-// One thread of the even CTA issues the MMA for both CTAs of the pair (M counts both halves).
-__device__ __forceinline__ void umma_f16_ss_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                                 uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
 }
 // Arrival on ONE barrier (shared::cluster address, own or peer CTA) when the pair's MMAs issued so far finish.
 __device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster) {

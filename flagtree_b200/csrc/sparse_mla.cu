@@ -21,7 +21,6 @@
 namespace ftb {
 
 constexpr int kDqk = 576;
-constexpr int kDv = 512;
 constexpr int kNChunk = kDqk / 64;          // 9 column blocks of 64 bf16
 constexpr int kHeadsPerCta = 128;           // MMA M
 constexpr int kBN = 64;                     // gathered rows per tile (MMA N of Q.K^T, K of P.V)
@@ -668,7 +667,7 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
     const int tiles = (a->topk + tile - 1) / tile;
     return n_splits < tiles ? n_splits : tiles > 1 ? tiles : 1;
   };
-  // Paged FP8 form with a workspace for the dequantised rows (algo 0 or 6, no split): convert the selected
+  // Paged FP8 form with a workspace for the dequantised rows (algo 6, or algo 0 without a split): convert the selected
   // rows once, then run the persistent bf16 kernel on the compact table.  Without such a workspace the
   // one-pass kernel below converts while it gathers.
   const int64_t split_bytes = ftb_sparse_mla_workspace_bytes(a->s_q, a->h, n_splits);

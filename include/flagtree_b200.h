@@ -86,7 +86,9 @@ typedef struct ftb_sparse_mla_args {
   /* Split of the top-k axis (for few query tokens, e.g. decode): n_splits > 1 makes every split write a
    * partial result to `workspace` (ftb_sparse_mla_workspace_bytes() bytes of device memory, contents
    * need not be initialised) and a merge kernel combine them, the role of _fwd_kernel_stage2
-   * (test_accuracy_musa_vllm_mla.py:426-477).  0 or 1 = no split, no workspace. */
+   * (test_accuracy_musa_vllm_mla.py:426-477).  0 or 1 = no split, no workspace.  bf16 form: algo_id 5 takes the parts on the
+   * persistent pairs, algo_id 0 on whichever kernel is faster, algo_id 1 on the one-CTA kernel.  Paged FP8 form: the one-CTA kernel,
+   * unless algo_id 6 finds room for both passes (below).  Parts beyond the tiles of a list are left out. */
   int32_t n_splits;
   void* workspace;
   int64_t workspace_bytes;
@@ -99,7 +101,8 @@ FTB_API int64_t ftb_sparse_mla_workspace_bytes(int32_t s_q, int32_t h, int32_t n
  * the selected rows are first converted to a compact bf16 table (row = token * topk + j,
  * the role of the dequantising loads of decode_attention_int4kv.py:345-450, done once per row instead of
  * inside the attention loop) and the persistent bf16 kernel runs on that table.  algo_id 6 demands this
- * path, algo_id 0 takes it when the workspace allows and n_splits <= 1. */
+ * path when n_splits <= 1, algo_id 0 takes it when the workspace allows and n_splits <= 1.  With n_splits > 1 and a
+ * workspace that only holds the partial results, algo_id 6 is the one-pass kernel with a split. */
 FTB_API int64_t ftb_sparse_mla_dequant_workspace_bytes(int32_t s_q, int32_t topk);
 /* Same operation for callers that cannot allocate device memory (an engine that owns the whole device
  * through its own pool, a sandboxed plugin, a latency path that must stay clear of the allocator).  It has

@@ -100,7 +100,8 @@ struct Params {
 };
 
 struct Misc0 {   // CTA 0
-  unsigned long long k_full[kNK];   // one arrival per gather thread (when its copies have landed; the tile load of a Q entry counts on one of them)
+  unsigned long long k_full[kNK];   // one arrival per gather thread (when its copies have landed; the tile load of a Q entry counts on one of them);
+                                    // slot 0 one more, which releases the tile's validity mask
   unsigned long long k_free[kNK];   // tcgen05.commit behind the entry's MMAs or its copy to tensor memory
   unsigned long long s_full[2];     // tcgen05.commit
   unsigned long long s_free[2];     // softmax warps with heads (8 when h > 96)
@@ -242,7 +243,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
     *abort_flag = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
     if (cta == 0) {
       m0->bad_index = 0;
-      for (int i = 0; i < kNK; ++i) { mbar_init(smem_u32(&m0->k_full[i]), 32); mbar_init(smem_u32(&m0->k_free[i]), 1); }
+      for (int i = 0; i < kNK; ++i) { mbar_init(smem_u32(&m0->k_full[i]), i == 0 ? 33 : 32); mbar_init(smem_u32(&m0->k_free[i]), 1); }
       for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&m0->s_full[i]), 1); mbar_init(smem_u32(&m0->s_free[i]), 2 * row_warps); }
       mbar_init(smem_u32(&m0->q8_full), 1);
       mbar_init(smem_u32(&m0->q8_free), 1);
@@ -577,6 +578,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
                              ::"l"(&tm_q), "r"(c * 64), "r"(0), "r"(tok_next) : "memory");
             } else if (c < kNQ) {
               mbar_arrive(full);
+              if (c == 0 && lane == 1) mbar_arrive(full);
             }
             __syncwarp();
           }
@@ -610,6 +612,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
             __syncwarp();
             const uint32_t uses = c < kNQ ? G + ti + 1 : G;
             if (uses >= 1) mbar_wait(k_free, (uses - 1) & 1u, abort_flag);
+            if (c == 0 && lane == 0) mbar_arrive(k_full);    // the arrivals below track the copies; this one releases the mask
 #pragma unroll
             for (int q = 0; q < 32; ++q) {
               const int r = __shfl_sync(0xffffffffu, row[q >> 3], (q & 7) * 4 + (lane >> 3));

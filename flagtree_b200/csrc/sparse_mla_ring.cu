@@ -860,6 +860,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
     __syncthreads();   // nt[] is rewritten by the next batch
   }
 
+  if (*abort_flag) drain_after_abort();
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();            // nobody leaves while the peer may still write or signal this CTA

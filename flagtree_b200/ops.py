@@ -75,6 +75,7 @@ def _auto_splits(s_q: int, h: int, topk: int, device) -> int:
     return _plan_splits(s_q, h, topk, _pairs_of(device.index))
 
 
+@functools.lru_cache(maxsize=1024)
 def _plan_paged(s_q: int, h: int, topk: int, pairs: int) -> Tuple[int, bool]:
     """Parts of a token's list in the paged form, and whether the rows are dequantised first.
 
@@ -291,13 +292,15 @@ def sparse_mla_fwd_paged(q: torch.Tensor, kv_cache: torch.Tensor, kv_scale: torc
         lse.stride(0), float(sm_scale), int(lse_base2), 0, status.data_ptr() if status is not None else None, 1, kv_scale.data_ptr(),
         block_table.data_ptr(), context_lens.data_ptr(), page_size, n_q, block_table.stride(0))
     lib = _lib.load()
-    rows_bytes = int(lib.ftb_sparse_mla_dequant_workspace_bytes(b * n_q, idx2.shape[1]))
     if num_splits is None:
         n_splits, rows_first = _plan_paged(b * n_q, h, idx2.shape[1], _pairs_of(q.device.index))
     else:
         n_splits = max(1, int(num_splits))
         rows_first = n_splits == 1
-    if rows_bytes > 0 and (two_pass or (two_pass is None and rows_first and rows_bytes <= (4 << 30))):
+    rows_bytes = 0
+    if two_pass or (two_pass is None and rows_first):
+        rows_bytes = int(lib.ftb_sparse_mla_dequant_workspace_bytes(b * n_q, idx2.shape[1]))
+    if 0 < rows_bytes and (two_pass or rows_bytes <= (4 << 30)):
         # the dequantised rows, then (from a 16-byte boundary) the partial results of a split
         need = rows_bytes
         if n_splits > 1:

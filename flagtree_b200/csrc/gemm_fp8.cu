@@ -382,9 +382,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       }
     }
   }
-  if (*abort_flag) drain_after_abort();
   tc_fence_before();
   __syncthreads();
+  if (bars->abort_flag) drain_after_abort();
   if (clustered) cluster_sync_all();   // nobody leaves while a peer may still signal or read this CTA
   if (warp == 1) {
     tc_fence_after();

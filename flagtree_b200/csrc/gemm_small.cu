@@ -173,8 +173,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       }
     }
   }
-  if (*abort_flag && !dead) drain_after_abort();
   __syncthreads();
+  if (bars->abort_flag && !dead) drain_after_abort();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem, BN);

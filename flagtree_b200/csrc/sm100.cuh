@@ -74,6 +74,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // After a wait that ran out: loads, copies and MMAs that were issued still land in this CTA's shared and tensor memory and signal its
 // barriers.  64 us is far longer than any of them takes on a working device; the CTA must not leave before.
 __device__ __forceinline__ void drain_after_abort() {
+#pragma unroll 1
   for (int i = 0; i < 64; ++i) __nanosleep(1000);
 }
 

@@ -26,8 +26,8 @@
 // role but the MMA issue has one rolled loop, the softmax has one path (masked entries become -inf once) with two-wide
 // fp32 instructions, loop counts are warp-uniform, and the issuer has constant addresses and waits for three blocks at once.
 // Warps whose 32 head rows hold no head take no part.  One launch alone, 740 tokens, 128 heads, topk 2048: 832 -> 1065
-// TFLOP/s.  Back to back: 4096 causal tokens 2243 -> 2022 us; 1999 tokens of 16 heads 1319 -> 965 us (1159 with all rows
-// at work, 1076 with a ring of ten slots and computed addresses).
+// TFLOP/s.  Back to back, in turn on one box: 4096 causal tokens 2244 -> 1944 us; 1999 tokens of 16 heads 1327 -> 970 us (1159 with all
+// rows at work, 1076 with a ring of ten slots and computed addresses).
 //
 // Few tokens.  A launch may cut the top-k list of every token in parts; an item of work is then a part of a token, its result
 // leaves as fp32 (32 columns per TMA store instead of 64) with a base-2 LSE, and a second kernel merges the parts.  One token
@@ -203,7 +203,7 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
 // Masked entries (-1) fetch a row all the same, which is multiplied by zero: the one that the lane fetched for the tile before, or in
 // the first tile another one of the token's (this function, the rare path: the first row that the list names; `none` if
 // it names none, row 0 for a token and any rows for a part, whose result the merge drops).  With row 0 for all of them, as it used to be,
-// every SM fetched the same 1152 bytes (4096 tokens of topk 65 took longer than of topk 128, 760 us against 329; now 313),
+// every SM fetched the same 1152 bytes (4096 tokens of topk 65 took longer than of topk 128, 761 us against 329; now 335),
 // and a row 0 that holds no numbers spoiled tokens that never selected it.  Not inline: the roles share an instruction cache.
 __device__ __noinline__ int first_row(const int32_t* idx_row, int n_rows, int s_kv, int none) {
   const int lane = threadIdx.x & 31;

@@ -724,6 +724,10 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
       set_last_error("ftb_sparse_mla_fwd: n_splits=%d needs a workspace of ftb_sparse_mla_workspace_bytes() bytes", n_splits);
       return FTB_ERR_INVALID;
     }
+    if (!aligned16(a->workspace)) {                            // the partial results are written and merged 16 bytes at a time
+      set_last_error("ftb_sparse_mla_fwd: the workspace must be 16-byte aligned");
+      return FTB_ERR_INVALID;
+    }
     p.part_out = reinterpret_cast<float*>(a->workspace);
     p.part_lse = p.part_out + static_cast<size_t>(a->s_q) * n_splits * a->h * 512;
   }
@@ -733,8 +737,7 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
   // parts of 128 heads, 32 tokens of topk 256 23 / 36, of 512 31 / 38, of 1024 48 / 34, of 2048 80 / 43; 148 tokens of topk 512 in four parts
   // 167 / 142; 16 heads, 148 tokens of topk 512 in two parts 88 / 44.
   const bool pairs = a->algo_id == 5 || (a->algo_id == 0 && (a->topk > 512 || (n_splits * 128 <= a->topk && (a->h <= 32 || (a->topk > 256 && a->s_q >= 64)))));
-  if (n_splits > 1 && n_splits <= 64 && !a->kv_is_fp8 && a->dbg_scores == nullptr && pairs &&
-      (reinterpret_cast<uintptr_t>(a->workspace) & 15u) == 0) {
+  if (n_splits > 1 && n_splits <= 64 && !a->kv_is_fp8 && a->dbg_scores == nullptr && pairs) {
     n_splits = parts_of(128);
     p.part_lse = p.part_out + static_cast<size_t>(a->s_q) * n_splits * a->h * 512;
     const int rc0 = launch_sparse_mla_ring(a, n_splits, p.part_out, p.part_lse, a->algo_id == 5 ? 8.0f : 0.0f, st);

@@ -84,7 +84,7 @@ typedef struct ftb_sparse_mla_args {
    * [s_q, 128, topk_padded_to_64] raw (unscaled) scores of the one-CTA kernel.  Pass NULL. */
   float* dbg_scores;
   /* Split of the top-k axis (for few query tokens, e.g. decode): n_splits > 1 makes every split write a
-   * partial result to `workspace` (ftb_sparse_mla_workspace_bytes() bytes of device memory, contents
+   * partial result to `workspace` (ftb_sparse_mla_workspace_bytes() bytes of device memory, 16-byte aligned, contents
    * need not be initialised) and a merge kernel combine them, the role of _fwd_kernel_stage2
    * (test_accuracy_musa_vllm_mla.py:426-477).  0 or 1 = no split, no workspace.  bf16 form: algo_id 5 takes the parts on the
    * persistent pairs, algo_id 0 on whichever kernel is faster, algo_id 1 on the one-CTA kernel.  Paged FP8 form: the one-CTA kernel,

@@ -45,3 +45,21 @@ def test_paged_plan_of_few_and_many_tokens():
     assert ops._plan_paged(73, 128, 2048, 74) == (1, True)
     assert ops._plan_paged(128, 128, 2048, 74) == (1, True)
     assert ops._plan_paged(5, 16, 0, 74)[0] == 1
+
+
+@pytest.mark.parametrize("fp8", [0, 1])
+def test_misaligned_split_workspace_is_refused(fp8):
+    """Refused on the host, before anything is launched: the kernels write the partial results 16 bytes at a time."""
+    lib = _lib.load()
+    a = _lib.SparseMlaArgs()
+    a.q = a.kv = a.indices = a.out = a.lse = 4096
+    a.s_q, a.h, a.s_kv, a.topk = 4, 16, 1000, 256
+    a.q_stride_token, a.q_stride_head, a.kv_stride_row, a.idx_stride_token = 16 * 576, 576, 576, 256
+    a.out_stride_token, a.out_stride_head, a.lse_stride_token = 16 * 512, 512, 16
+    a.sm_scale, a.n_splits = 0.05, 4
+    if fp8:
+        a.kv_is_fp8, a.page_size, a.q_per_seq, a.block_table_stride = 1, 64, 1, 16
+        a.kv_scale = a.block_table = a.context_lens = 4096
+    a.workspace, a.workspace_bytes = 4096 + 8, lib.ftb_sparse_mla_workspace_bytes(4, 16, 4)
+    assert lib.ftb_sparse_mla_fwd(C.byref(a), None) == _lib.FTB_ERR_INVALID
+    assert "aligned" in _lib.last_error()

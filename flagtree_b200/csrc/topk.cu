@@ -4,10 +4,12 @@
 //
 // Selection is exact and deterministic: scores are mapped to 32-bit keys whose unsigned order is the order of the
 // floats (-0 below +0, NaN patterns above +inf, as an unsigned compare of the transformed bits gives), the k-th
-// largest key is found, and among the entries equal to that key the lowest positions are taken.  Three kernels, by the length
-// of a row: a radix select that reads the row five times from wherever it is, many rows to an SM (short rows, and those
-// that fit no SM); persistent CTAs that hold a row of at most 32768 scores in registers and read it once; and one for rows of at most
-// 65536 scores.  The floor is device-memory traffic: 4 * s_kv bytes of scores per token (plus 4 * topk bytes of output).
+// largest key is found, and among the entries equal to that key the lowest positions are taken.  Two kernels, by the length
+// of a row: up to 65536 scores a CTA makes a short list of the keys that may be among the k largest and selects in that; longer rows,
+// and lists that no SM has room for, go to a radix select that reads the row five times from wherever it is.  The floor is device-memory
+// traffic: 4 * s_kv bytes of scores per token (plus 4 * topk bytes of output).
+#include <cmath>
+
 #include "sm100.cuh"
 
 namespace ftb {
@@ -17,7 +19,7 @@ int check_cuda(cudaError_t e, const char* what);
 
 namespace topk {
 
-constexpr int kThreads = 512;                              // of the kernel that reads rows from memory
+constexpr int kThreads = 512;                              // of the radix select
 
 struct Params {
   const float* scores;
@@ -166,685 +168,388 @@ __global__ void __launch_bounds__(kThreads) topk_select_kernel(const Params p) {
                        p.out + static_cast<long long>(row) * p.out_stride, &sm);
 }
 
-constexpr int kBigThreads = 1024;                          // of the kernels that hold a row
-constexpr int kBigWarps = kBigThreads / 32;
-
-__device__ __forceinline__ void cp_async4(uint32_t smem_dst, const void* gmem_src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_dst), "l"(gmem_src) : "memory");
-}
-// scores src[0 .. n) -> buf by asynchronous copies of the calling threads, of 16 bytes where the row is aligned
-__device__ __forceinline__ void copy_row(const float* src, int n, float* buf) {
-  const uint32_t dst = smem_u32(buf);
-  if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-    for (int c = threadIdx.x; c < n >> 2; c += kBigThreads) cp_async16(dst + 16 * c, src + 4 * c);
-    const int tail = (n & ~3) + threadIdx.x;
-    if (tail < n) cp_async4(dst + 4 * tail, src + tail);
-  } else {
-    for (int c = threadIdx.x; c < n; c += kBigThreads) cp_async4(dst + 4 * c, src + c);
-  }
-}
 // ---------------------------------------------------------------------------------------------------------------
-// Rows of at most 32768 scores: one persistent CTA of 1024 threads per SM.  The next row travels into shared
-// memory by asynchronous copies while the current one, held as 32 keys per thread in registers, is
-// selected; the scores are read from device memory exactly once.  Thread t owns the 32 consecutive positions
-// 32 t .. 32 t + 31 (read as eight 16-byte pieces in the order piece ^ (t & 7), which keeps the eight lanes of a
-// shared-memory phase on different banks), so the ordered output needs one scan over per-thread counts and a
-// walk over the few set bits of a per-thread mask.
+// Rows up to 65536 scores: one CTA per row, as many CTAs to an SM as fit.
 //
-// Shared-memory atomics retire about one lane per clock, so a histogram over the whole row would cost far more
-// than the row takes to arrive.  A sample of 256 keys therefore brackets the k-th largest key first: the sample
-// is ranked by counting, two thresholds L <= H are picked a few standard deviations of the sample quantile
-// either side of rank k / len, and one sweep over the registers counts A = #{key > H} and builds a 256-bin
-// histogram of key - L over the keys in [L, H].  When A < k <= A + #[L, H] (checked, so a bad sample costs time
-// and never exactness) the k-th largest key lies in one bin of a few keys, which are ranked by counting;
-// otherwise the sweep is repeated over the whole key range.  Bins still crowded (ties, repeated values) go
-// through further 8-bit passes.  The histograms hold one counter per (bin, lane): the atomic adds of a warp fall
-// into 32 different banks whatever the distribution of the scores.
-// ---------------------------------------------------------------------------------------------------------------
-namespace held {
-
-constexpr int kRowMax = 32768;
-constexpr int kPerThread = kRowMax / kBigThreads;          // 32 keys per thread
-constexpr int kSample = 256;
-constexpr int kSampleMinLen = 4096;                        // shorter rows are selected without a bracket
-constexpr int kListMax = 256;                              // a bin of at most this many keys is ranked by counting
-constexpr size_t kBigSmem = static_cast<size_t>(kRowMax) * 4 + 256 * 32 * 4 + 256 * 4 + kSample * 4 + kBigWarps * 4 + 16 * 4 +
-                            2 * kBigThreads * 4 + 2 * kListMax * 4;
-
-enum { kCtlBin = 0, kCtlRemaining, kCtlBinCount, kCtlInside, kCtlAbove, kCtlLo, kCtlHi, kCtlListCount, kCtlThresh, kCtlNeedEq };
-
-// kAligned: every row starts on a 16-byte boundary and s_kv is a multiple of 4
-template <bool kAligned>
-__device__ __forceinline__ void fetch_row(const Params& p, int row, float* buf) {
-  const float* sc = p.scores + static_cast<long long>(row) * p.sc_stride;
-  const uint32_t dst = smem_u32(buf);
-  if constexpr (kAligned) {
-    const int chunks = (row_len(p, row) + 3) >> 2;
-    for (int c = threadIdx.x; c < chunks; c += kBigThreads) cp_async16(dst + 16 * c, sc + 4 * c);
-  } else {
-    const int n = row_len(p, row);
-    for (int c = threadIdx.x; c < n; c += kBigThreads) cp_async4(dst + 4 * c, sc + c);
-  }
-}
-
-// moves nibble s of `bits` to nibble s ^ x (x in 0..7): register order <-> position order of a thread's keys
-__device__ __forceinline__ uint32_t swap_nibbles(uint32_t bits, int x) {
-  if (x & 1) bits = ((bits & 0x0f0f0f0fu) << 4) | ((bits >> 4) & 0x0f0f0f0fu);
-  if (x & 2) bits = ((bits & 0x00ff00ffu) << 8) | ((bits >> 8) & 0x00ff00ffu);
-  if (x & 4) bits = (bits << 16) | (bits >> 16);
-  return bits;
-}
-
-template <bool kAligned>
-__global__ void __launch_bounds__(kBigThreads, 1) topk_select_rows_kernel(const Params p) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float* buf = reinterpret_cast<float*>(smem_raw);                                   // the row in flight
-  int* hist = reinterpret_cast<int*>(smem_raw + static_cast<size_t>(kRowMax) * 4);   // [256 bins][32 lanes]
-  int* bin_total = hist + 256 * 32;                                                  // [256]
-  uint32_t* samp = reinterpret_cast<uint32_t*>(bin_total + 256);                     // [256]
-  uint32_t* warp_sum = samp + kSample;                                               // [32]
-  int* ctl = reinterpret_cast<int*>(warp_sum + kBigWarps);                           // [16]
-  uint32_t* gt_extra = reinterpret_cast<uint32_t*>(ctl + 16);                        // [1024] per owner thread: keys of
-  uint32_t* eq_extra = gt_extra + kBigThreads;                                       // [1024] the last bin above / equal
-  uint32_t* list = eq_extra + kBigThreads;                                           // [kListMax] keys of the last bin
-  int* list_pos = reinterpret_cast<int*>(list + kListMax);                           // [kListMax] and their positions
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int twist = tid & 7;
-  const int pos0 = tid * kPerThread;
-
-  int row = blockIdx.x;
-  if (row < p.s_q) fetch_row<kAligned>(p, row, buf);
-  for (; row < p.s_q; row += gridDim.x) {
-    const int len = row_len(p, row);
-    const int k = min(p.topk, len);
-    const bool sampled = k < len && len >= kSampleMinLen;
-    const int n_valid = max(0, min(kPerThread, len - pos0));
-    const uint32_t valid_pos = n_valid >= 32 ? 0xffffffffu : ((1u << n_valid) - 1u);   // position order
-    cp_async_wait_all();
-    __syncthreads();
-    uint32_t key[kPerThread];
-#pragma unroll
-    for (int s = 0; s < 8; ++s) {
-      const int piece = s ^ twist;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (n_valid > 0) v = *reinterpret_cast<const float4*>(buf + pos0 + 4 * piece);
-      const uint32_t ok = valid_pos >> (4 * piece);          // positions past the row take the lowest key
-      key[4 * s + 0] = (ok & 1u) ? to_key(__float_as_uint(v.x)) : 0u;
-      key[4 * s + 1] = (ok & 2u) ? to_key(__float_as_uint(v.y)) : 0u;
-      key[4 * s + 2] = (ok & 4u) ? to_key(__float_as_uint(v.z)) : 0u;
-      key[4 * s + 3] = (ok & 8u) ? to_key(__float_as_uint(v.w)) : 0u;
-    }
-    if (sampled && tid < kSample) {
-      // the sample number in the low byte makes the sample keys distinct; the bracket does not need exact keys
-      const uint32_t sk = to_key(__float_as_uint(buf[static_cast<int>((static_cast<long long>(tid) * len) >> 8) + (tid & 15)]));
-      samp[tid] = (sk & ~0xffu) | static_cast<uint32_t>(tid);
-    }
-    if (tid == 0) { ctl[kCtlLo] = 0; ctl[kCtlHi] = -1; }
-    __syncthreads();
-    if (row + static_cast<int>(gridDim.x) < p.s_q) fetch_row<kAligned>(p, row + gridDim.x, buf);   // overlaps the selection
-
-    uint32_t above_bits = 0, tie_bits = 0;                 // register order: keys above the last bin, ties of a one-key bin
-    int need_eq = 0;
-    if (k < len) {
-      if (sampled) {
-        // rank of sample s among the 256: four threads count a quarter each
-        const int s_no = tid >> 2, quarter = tid & 3;
-        const uint32_t mine = samp[s_no];
-        int rank = 0;
-#pragma unroll
-        for (int m = 0; m < kSample / 16; ++m) {           // the four threads of a sample read different banks
-          const uint4 v = *reinterpret_cast<const uint4*>(samp + 16 * m + 4 * quarter);
-          rank += (v.x > mine) + (v.y > mine) + (v.z > mine) + (v.w > mine);
-        }
-        rank += __shfl_xor_sync(0xffffffffu, rank, 1);
-        rank += __shfl_xor_sync(0xffffffffu, rank, 2);
-        const float frac = static_cast<float>(k) / static_cast<float>(len);
-        const int centre = static_cast<int>(frac * kSample);
-        const int margin = static_cast<int>(3.5f * sqrtf(kSample * frac * (1.0f - frac))) + 2;
-        if (quarter == 0) {
-          if (rank == centre + margin) ctl[kCtlLo] = static_cast<int>(mine & ~0xffu);   // stays 0 past the sample
-          if (rank == centre - margin) ctl[kCtlHi] = static_cast<int>(mine | 0xffu);    // stays the largest key
-        }
-        __syncthreads();
-      }
-      uint32_t lo = static_cast<uint32_t>(ctl[kCtlLo]), hi = static_cast<uint32_t>(ctl[kCtlHi]);
-      uint32_t cand = 0, prefix = 0, mask = 0;             // cand bit r: key[r] still in the running (register order)
-      int remaining = 0, low_bits = 0, bin_count = 0;
-#pragma unroll 1
-      for (int attempt = 0; attempt < 2; ++attempt) {
-        // first sweep: count the keys above H, histogram key - L over [L, H] in 256 bins
-        const uint32_t range = hi - lo;
-        low_bits = 32 - __clz(range);
-        const int shift = max(low_bits - 8, 0);
-        {
-          int4* h4 = reinterpret_cast<int4*>(hist);
-          h4[tid] = make_int4(0, 0, 0, 0);
-          h4[tid + kBigThreads] = make_int4(0, 0, 0, 0);
-        }
-        __syncthreads();
-        const uint32_t valid_reg = swap_nibbles(valid_pos, twist);
-        int above = 0;
-        cand = 0;
-        if (valid_reg != 0) {
-#pragma unroll
-          for (int r = 0; r < kPerThread; ++r) {
-            const uint32_t rel = key[r] - lo;
-            above += key[r] > hi ? 1 : 0;
-            if (rel <= range && ((valid_reg >> r) & 1u)) {
-              cand |= 1u << r;
-              atomicAdd(&hist[((rel >> shift) << 5) + lane], 1);
-            }
-          }
-        }
-        above = __reduce_add_sync(0xffffffffu, above);
-        if (lane == 0) warp_sum[warp] = static_cast<uint32_t>(above);
-        __syncthreads();
-        {
-          const int bin = tid >> 2, q = tid & 3;
-          int t = 0;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) t += hist[(bin << 5) + ((q * 8 + i + bin) & 31)];
-          t += __shfl_xor_sync(0xffffffffu, t, 1);
-          t += __shfl_xor_sync(0xffffffffu, t, 2);
-          if (q == 0) bin_total[bin] = t;
-        }
-        __syncthreads();
-        if (warp == 0) {
-          const int total_above = static_cast<int>(__reduce_add_sync(0xffffffffu, warp_sum[lane]));
-          int mine = 0;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) mine += bin_total[8 * lane + j];
-          int suffix = mine;                               // keys in this lane's bins and the bins of higher lanes
-#pragma unroll
-          for (int d = 1; d < 32; d <<= 1) {
-            const int v = __shfl_down_sync(0xffffffffu, suffix, d);
-            if (lane + d < 32) suffix += v;
-          }
-          const int inside = __shfl_sync(0xffffffffu, suffix, 0);
-          const int want = k - total_above;                // rank of the k-th largest key inside the bracket
-          if (lane == 0) { ctl[kCtlAbove] = total_above; ctl[kCtlInside] = inside; }
-          const int higher = suffix - mine;
-          if (want > 0 && higher < want && want <= suffix) {
-            int cum = higher;
-            for (int j = 7; j >= 0; --j) {
-              const int h = bin_total[8 * lane + j];
-              if (cum + h >= want) {
-                ctl[kCtlBin] = 8 * lane + j;
-                ctl[kCtlRemaining] = want - cum;
-                ctl[kCtlBinCount] = h;
-                break;
-              }
-              cum += h;
-            }
-          }
-        }
-        __syncthreads();
-        const int total_above = ctl[kCtlAbove];
-        if (total_above < k && k <= total_above + ctl[kCtlInside]) {
-          prefix = static_cast<uint32_t>(ctl[kCtlBin]) << shift;
-          mask = ~((1u << shift) - 1u);                    // bits of key - L fixed so far
-          remaining = ctl[kCtlRemaining];
-          bin_count = ctl[kCtlBinCount];
-          low_bits = shift;
-          break;
-        }
-        lo = 0u; hi = 0xffffffffu;                         // the sample misled: select over the whole key range
-      }
-      // further 8-bit passes while the bin is crowded
-#pragma unroll 1
-      while (low_bits > 0 && bin_count > kListMax) {
-        const int width = min(8, low_bits), shift = low_bits - width;
-        const uint32_t digit_mask = (1u << width) - 1u;
-        {
-          int4* h4 = reinterpret_cast<int4*>(hist);
-          h4[tid] = make_int4(0, 0, 0, 0);
-          h4[tid + kBigThreads] = make_int4(0, 0, 0, 0);
-        }
-        __syncthreads();
-        if (cand != 0) {
-#pragma unroll
-          for (int r = 0; r < kPerThread; ++r) {
-            if ((cand >> r) & 1u) {
-              const uint32_t rel = key[r] - lo;
-              if ((rel & mask) == prefix) atomicAdd(&hist[(((rel >> shift) & digit_mask) << 5) + lane], 1);
-              else cand &= ~(1u << r);
-            }
-          }
-        }
-        __syncthreads();
-        {
-          const int bin = tid >> 2, q = tid & 3;
-          int t = 0;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) t += hist[(bin << 5) + ((q * 8 + i + bin) & 31)];
-          t += __shfl_xor_sync(0xffffffffu, t, 1);
-          t += __shfl_xor_sync(0xffffffffu, t, 2);
-          if (q == 0) bin_total[bin] = t;
-        }
-        __syncthreads();
-        if (warp == 0) {
-          int mine = 0;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) mine += bin_total[8 * lane + j];
-          int suffix = mine;
-#pragma unroll
-          for (int d = 1; d < 32; d <<= 1) {
-            const int v = __shfl_down_sync(0xffffffffu, suffix, d);
-            if (lane + d < 32) suffix += v;
-          }
-          const int higher = suffix - mine;
-          if (higher < remaining && remaining <= suffix) {
-            int cum = higher;
-            for (int j = 7; j >= 0; --j) {
-              const int h = bin_total[8 * lane + j];
-              if (cum + h >= remaining) {
-                ctl[kCtlBin] = 8 * lane + j;
-                ctl[kCtlRemaining] = remaining - cum;
-                ctl[kCtlBinCount] = h;
-                break;
-              }
-              cum += h;
-            }
-          }
-        }
-        __syncthreads();
-        prefix |= static_cast<uint32_t>(ctl[kCtlBin]) << shift;
-        mask |= digit_mask << shift;
-        remaining = ctl[kCtlRemaining];
-        bin_count = ctl[kCtlBinCount];
-        low_bits = shift;
-      }
-      // the last bin [base, top]: keys above it are taken, its own few keys go to a list with their positions and
-      // are ranked by counting: the threshold is the key v with #{keys > v} < remaining <= #{keys >= v}
-      const uint32_t base = lo + prefix;
-      const uint32_t span = min(low_bits == 0 ? 0u : ((1u << low_bits) - 1u), hi - base);   // keys above H were counted apart
-      const uint32_t top = base + span;
-      gt_extra[tid] = 0u;
-      eq_extra[tid] = 0u;
-      if (tid == 0) ctl[kCtlListCount] = 0;
-      __syncthreads();
-      const uint32_t valid_reg = swap_nibbles(valid_pos, twist);
-#pragma unroll
-      for (int r = 0; r < kPerThread; ++r) {
-        above_bits |= key[r] > top ? (1u << r) : 0u;
-        if (key[r] - base <= span && ((valid_reg >> r) & 1u)) {
-          if (low_bits == 0) {
-            tie_bits |= 1u << r;                           // the bin is one key wide: these are the ties
-          } else {
-            const int at = atomicAdd(&ctl[kCtlListCount], 1);
-            list[at] = key[r];
-            list_pos[at] = pos0 + 4 * ((r >> 2) ^ twist) + (r & 3);
-          }
-        }
-      }
-      need_eq = remaining;
-      if (low_bits != 0) {
-        __syncthreads();
-        const int n = ctl[kCtlListCount];
-        if (tid < n) {
-          const uint32_t v = list[tid];
-          int gt = 0, ge = 0;
-          for (int m = 0; m < n; ++m) {
-            const uint32_t o = list[m];
-            gt += o > v ? 1 : 0;
-            ge += o >= v ? 1 : 0;
-          }
-          const int at = list_pos[tid];
-          if (gt < remaining) {
-            if (remaining <= ge) { atomicOr(&eq_extra[at >> 5], 1u << (at & 31)); ctl[kCtlNeedEq] = remaining - gt; }
-            else atomicOr(&gt_extra[at >> 5], 1u << (at & 31));
-          }
-        }
-        __syncthreads();
-        need_eq = ctl[kCtlNeedEq];
-      }
-    } else {
-      // k == len: every position of the row is taken
-      above_bits = swap_nibbles(valid_pos, twist);
-      gt_extra[tid] = 0u;
-      eq_extra[tid] = 0u;
-      need_eq = 0;
-    }
-
-    // per thread the taken keys and the ties as bit masks in position order, one scan over the packed counts
-    // (ties << 16 | taken; neither exceeds 32768), then each thread writes its few positions
-    uint32_t gt_bits = swap_nibbles(above_bits, twist) | gt_extra[tid];
-    uint32_t eq_bits = (swap_nibbles(tie_bits, twist) | eq_extra[tid]) & valid_pos;
-    const uint32_t packed = (static_cast<uint32_t>(__popc(eq_bits)) << 16) | static_cast<uint32_t>(__popc(gt_bits));
-    uint32_t incl = packed;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
-      if (lane >= d) incl += v;
-    }
-    if (lane == 31) warp_sum[warp] = incl;
-    __syncthreads();
-    const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp ? warp_sum[lane] : 0u) + incl - packed;
-    const int gt_before = static_cast<int>(before & 0xffffu), eq_before = static_cast<int>(before >> 16);
-    int eq_take = min(max(need_eq - eq_before, 0), __popc(eq_bits));    // the lowest positions among the ties
-    uint32_t bits = gt_bits;
-    while (eq_take > 0) {
-      const uint32_t lowest = eq_bits & (0u - eq_bits);
-      bits |= lowest;
-      eq_bits ^= lowest;
-      --eq_take;
-    }
-    int32_t* out = p.out + static_cast<long long>(row) * p.out_stride;
-    int write_at = gt_before + min(eq_before, need_eq);
-    while (bits != 0) {
-      out[write_at++] = pos0 + __ffs(static_cast<int>(bits)) - 1;
-      bits &= bits - 1u;
-    }
-    for (int j = k + tid; j < p.topk; j += kBigThreads) out[j] = -1;
-    __syncthreads();                                       // the shared words are reused by the next row
-  }
-}
-
-}  // namespace held
-
-// ---------------------------------------------------------------------------------------------------------------
-// Rows of at most 65536 scores: persistent CTAs of 1024 threads, one per SM.  Thread t holds the keys of positions
-// t, t + 1024, ... below 32768 in registers; the rest of the row lies in shared memory.  A vote over a warp is the mask of 32
-// consecutive positions.  Scores are read from device memory once.
+// A sample of 512 keys gives a lower bound of the k-th largest key, a few standard deviations of the sample quantile on the safe
+// side.  One sweep over the row votes the keys from there on into a mask over the row (four instructions for 32 keys: load,
+// compare, vote, store).  The few positions in the mask, an eighth of the row or so, become a list in ascending order, and
+// their keys are fetched again, out of L2.  The list is counted against four trial values at a time, quantiles of the sample
+// first, then values interpolated between the counts known so far, until 128 candidates are left, which are ranked by
+// counting.  The list is in order, so the taken ones among it are the output as they come.
+// Where a value fills so much of the row that keys equal to the bound would crowd the list, the list takes the keys above it and
+// the ties go to a mask of their own in the same sweep.  A bound that turns out too high, or more keys than the list has room
+// for (both checked), costs time and never exactness: the row is then selected by the radix select, out of L2.
+// A row that fits the list goes there without a sweep.
 //
-// Bound by instruction issue, so the work per key is kept to a few instructions and no key goes through a shared-memory
-// atomic (they retire about one lane per clock).  A sample of 256 keys, ranked by counting, brackets the k-th largest key
-// a few standard deviations of the sample quantile either side (or only from below, where all above fits the list); one
-// sweep counts the keys of the bracket and copies them to a list, an eighth of the row or so.  The list is counted
-// against four trial values at a time, keys of the sample first, then interpolated between the counts known so far (the
-// keys are spread evenly enough there that two or three rounds leave 128 candidates), and the last few are ranked by counting.  A
-// bracket that does not hold the k-th key, or more keys than the list, is not used: the interval is then halved by
-// counting the whole row.  Both are checked, so a bad sample costs time (32 sweeps) and never exactness.  A last sweep
-// votes the taken positions into masks, and one scan over their counts gives every mask its place in the ordered output.
-// 128 rows of 28 000 scores on average out of 65 536 (a decode step): 138 us with the radix select, 28 here; 4096 rows of 33 000 scores
-// 1290 and 579.
+// What bounds it: instruction issue (0.69 a clock and scheduler, a row of 32768 some 40 000) and chains of latencies (sample, bound, sweep, list,
+// keys, trials), which the other CTAs of the SM fill; memory is at a quarter of its rate.  Copying the keys to the list in the sweep itself,
+// instead of voting, took 130 instructions per 128 keys (4096 x 32 768, topk 2048: 293 us; with votes 234, with the tail of the row apart 210).
+// Against persistent CTAs that hold a row in registers and histogram it (us, before / now): 4096 x 32 768 causal 334 / 210, 4096 x 20 001
+// topk 1024 426 / 151, 4096 x 6000 277 / 103, 4096 x 1000 topk 512 85 / 57, 592 rows of 33 000 82 / 35, 592 rows of 32 768 equal scores 52 / 40,
+// 128 rows of up to 65 536 30 / 19, 300 short rows of a matrix of 65 536 columns 44 / 17; slower: 100 rows of 32 768 with topk 16 384 27 / 46.
 // ---------------------------------------------------------------------------------------------------------------
-namespace half_held {
+namespace listed {
 
-constexpr int kHalf = 32768;                               // scores held in registers
-constexpr int kRowMax = 2 * kHalf;
-constexpr int kPerThread = kHalf / kBigThreads;            // 32 keys per thread
-constexpr int kSample = 256;                                // 128 would overflow the list (65536 scores, 2048 wanted: 6100 keys expected above the lower end)
-constexpr int kShortLen = 5120;                            // rows this short are read from memory: 148 rows of 1500 to 6000 scores 29.8 -> 19.1 us
-constexpr int kListPer = 8;
-constexpr int kListMax = kListPer * kBigThreads;
-constexpr int kWords = kRowMax / 32;
+constexpr int kRowMax = 65536;                             // positions in the list are 16-bit words
+constexpr int kSample = 512;
+constexpr float kMargin = 4.5f;                            // standard deviations between the k-th largest key and the bound
+constexpr int kCrowd = 6;                                  // that many keys of the sample more than wanted: many keys equal the bound
 constexpr int kFew = 128;                                  // this many candidates are ranked by counting
-constexpr size_t kBigSmem = (static_cast<size_t>(kHalf) + kListMax + 2 * kWords + kSample + 4 * kBigWarps + kFew + 16) * 4;
+constexpr int kAhead = 16;                                 // loads in flight per lane
+constexpr int kSmemMax = 220 * 1024;                       // dynamic; a few KB of static beside it
 
-enum { kCtlLo = 0, kCtlHi, kCtlFirst, kCtlAbove = kCtlFirst + 4, kCtlList, kCtlFew, kCtlLimit, kCtlNeedEq };
-
-// not inline: it needs none of the registers that hold a row
-__device__ __noinline__ void select_short_row(const uint32_t* sc, int len, int topk, int32_t* out, RowSmem<kBigThreads>* sm) {
-  select_row<kBigThreads>(sc, len, topk, out, sm);
+struct Shape {
+  int room;                                                // list entries
+  int words;                                               // of a mask over the row
+};
+// The list has room for what the bound is expected to let through and four standard deviations more; 0 where that is more than an SM has.
+inline int plan(int s_kv, int topk, bool alone, Shape* shape) {
+  if (s_kv > kRowMax) return 0;
+  const double k = topk < s_kv ? topk : s_kv, n = s_kv < kSample ? s_kv : kSample, frac = k / s_kv;
+  const double r = n * frac + kMargin * std::sqrt(n * frac * (1.0 - frac)) + 3.0 + kCrowd;   // rank of the bound in the sample
+  const int wanted = static_cast<int>((r + 4.0 * std::sqrt(r)) / n * s_kv) + 64, whole = s_kv < 4096 ? s_kv : 4096;
+  shape->words = (s_kv + 31) / 32;
+  shape->room = wanted > s_kv ? s_kv : wanted > whole ? wanted : whole;
+  const int most = (kSmemMax - 8 * shape->words) / 6;
+  if (alone && shape->room > s_kv / 4 && s_kv <= most) shape->room = s_kv;   // the SM's memory is there, and a row as a whole needs no sweep
+  if (shape->room > most) {
+    if (most < 1.1 * r / n * s_kv) return 0;
+    shape->room = most;
+  }
+  shape->room = (shape->room + 3) & ~3;
+  return 8 * shape->words + 6 * shape->room;
 }
 
-__global__ void __launch_bounds__(kBigThreads, 1) topk_select_long_rows_kernel(const Params p) {
-  constexpr int kRankers = kBigThreads / kSample;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  uint32_t* buf = reinterpret_cast<uint32_t*>(smem_raw);         // [kHalf] scores of the second half of the row
-  uint32_t* list = buf + kHalf;                          // [kListMax] keys inside the bracket
-  uint32_t* gt_words = list + kListMax;                                              // [kWords] taken positions
-  uint32_t* eq_words = gt_words + kWords;                                            // [kWords] ties
-  uint32_t* samp = eq_words + kWords;                                                // [kSample]
-  uint32_t* warp_sum = samp + kSample;                                            // [4][32]
-  uint32_t* few = warp_sum + 4 * kBigWarps;                                          // [kFew]
-  int* ctl = reinterpret_cast<int*>(few + kFew);                                     // [16]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int row = blockIdx.x; row < p.s_q; row += gridDim.x) {
-    const int len = row_len(p, row);
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(p.scores) + static_cast<long long>(row) * p.sc_stride;
-    int32_t* out = p.out + static_cast<long long>(row) * p.out_stride;
-    if (len <= kShortLen) {
-      select_short_row(src, len, p.topk, out, reinterpret_cast<RowSmem<kBigThreads>*>(list));
-      __syncthreads();
-      continue;
-    }
-    const int k = min(p.topk, len);
-    uint32_t key[kPerThread];                              // position 1024 i + tid; 0 past the row
-    if (len > kHalf) copy_row(reinterpret_cast<const float*>(src + kHalf), len - kHalf, reinterpret_cast<float*>(buf));
-    // the sample number in the low bits makes the sample keys distinct; the bracket does not need exact keys
-    if (k < len && tid < kSample)
-      samp[tid] = (to_key(src[static_cast<int>((static_cast<long long>(tid) * len) / kSample) + (tid & 15)]) & ~0xffu) | static_cast<uint32_t>(tid);
+// how many of the keys x (of all lanes) are t or more
+__device__ __forceinline__ int count_from(const uint32_t (&x)[kSample / 32], uint32_t t) {
+  int n[4] = {0, 0, 0, 0};
 #pragma unroll
-    for (int i = 0; i < kPerThread; ++i) {
-      const int pos = i * kBigThreads + tid;
-      key[i] = pos < len ? to_key(__ldcs(src + pos)) : 0u;
-    }
-    cp_async_wait_all();
-    if (tid == 0) { ctl[kCtlLo] = 1; ctl[kCtlHi] = -1; ctl[kCtlFirst] = ctl[kCtlFirst + 1] = 1; ctl[kCtlFirst + 2] = ctl[kCtlFirst + 3] = -1; ctl[kCtlAbove] = 0; ctl[kCtlList] = 0; ctl[kCtlFew] = 0; }
-    __syncthreads();
-    if (k < len) {
-      // the keys of positions kHalf + 1024 i + tid, i < n2: read again from shared memory by every sweep
-      const int n2 = max(0, min(kPerThread, (len - kHalf - tid + kBigThreads - 1) / kBigThreads));
-      auto key2 = [&](int i) { return to_key(buf[i * kBigThreads + tid]); };
-      bool use_list = false;
-      uint32_t lo = 0u, hi = 0xffffffffu;                  // the threshold lies in [lo, hi]
-      int c_lo = len, c_hi = 0, want = k;                  // keys >= lo, keys > hi, among those that are counted
-      uint32_t cand[kListPer];
-      // rank of a key of the sample: kRankers threads count a part each
-      const int s_no = tid / kRankers, part = tid % kRankers;
-      const uint32_t mine = samp[s_no];
-      int rank = 0;
-#pragma unroll
-      for (int m = 0; m < kSample / kRankers / 4; ++m) { // the threads of a sample read different banks
-        const uint4 v = *reinterpret_cast<const uint4*>(samp + 4 * kRankers * m + 4 * part);
-        rank += (v.x > mine) + (v.y > mine) + (v.z > mine) + (v.w > mine);
-      }
-#pragma unroll
-      for (int d = 1; d < kRankers; d <<= 1) rank += __shfl_xor_sync(0xffffffffu, rank, d);
-      const float frac = static_cast<float>(k) / static_cast<float>(len);
-      const int centre = static_cast<int>(frac * kSample);
-      const int margin = static_cast<int>(3.5f * sqrtf(kSample * frac * (1.0f - frac))) + 2, step = margin / 3;
-      if (part == 0) {
-        if (rank == centre + margin) ctl[kCtlLo] = static_cast<int>(max(mine & ~0xffu, 1u));   // stays 1 past the sample
-        if (rank == centre - margin) ctl[kCtlHi] = static_cast<int>(mine | 0xffu);             // stays the largest key
-        // the first trial values (past the sample: the ends)
-        if (rank == centre + step) ctl[kCtlFirst] = static_cast<int>(max(mine, 1u));
-        if (rank == centre) ctl[kCtlFirst + 1] = static_cast<int>(max(mine, 1u));
-        if (rank == centre - step) ctl[kCtlFirst + 2] = static_cast<int>(mine);
-        if (rank == centre - margin) ctl[kCtlFirst + 3] = static_cast<int>(mine | 0xffu);
-      }
-      __syncthreads();
-      // no upper end where the list has room for all that lies above the lower one (three quarters of it, as expected)
-      const bool open = (centre + margin) * (len / kSample) <= kListMax * 3 / 4;
-      const uint32_t b_lo = static_cast<uint32_t>(ctl[kCtlLo]), b_hi = open ? 0xffffffffu : static_cast<uint32_t>(ctl[kCtlHi]);
-      const uint32_t range = b_hi - b_lo;                // (a position past the row has key 0, below every bracket)
-      int above = 0, inside = 0;
-#pragma unroll
-      for (int i = 0; i < kPerThread; ++i) inside += key[i] >= b_lo ? 1 : 0;
-      for (int i = 0; i < n2; ++i) inside += key2(i) >= b_lo ? 1 : 0;
-      if (!open) {
-#pragma unroll
-        for (int i = 0; i < kPerThread; ++i) above += key[i] > b_hi ? 1 : 0;
-        for (int i = 0; i < n2; ++i) above += key2(i) > b_hi ? 1 : 0;
-        inside -= above;
-      }
-      above = __reduce_add_sync(0xffffffffu, above);
-      int at = inside;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, at, d);
-        if (lane >= d) at += v;
-      }
-      int first = 0;
-      if (lane == 31) {
-        atomicAdd(&ctl[kCtlAbove], above);
-        first = atomicAdd(&ctl[kCtlList], at);
-      }
-      at += __shfl_sync(0xffffffffu, first, 31) - inside;
-      if (at + inside <= kListMax) {
-#pragma unroll
-        for (int i = 0; i < kPerThread; ++i)
-          if (key[i] - b_lo <= range) list[at++] = key[i];
-        for (int i = 0; i < n2; ++i) {
-            const uint32_t x = key2(i);
-            if (x - b_lo <= range) list[at++] = x;
-          }
-      }
-      __syncthreads();
-      const int n_above = ctl[kCtlAbove], n_list = ctl[kCtlList];
-      if (n_above < k && k <= n_above + n_list) {
-        lo = b_lo; hi = b_hi;
-        c_lo = n_above + n_list; c_hi = n_above;
-      }
-      if (lo == b_lo && n_list <= kListMax) {
-        use_list = true;
-        c_lo = n_list; c_hi = 0; want = k - n_above;
-#pragma unroll
-        for (int j = 0; j < kListPer; ++j) cand[j] = j * kBigThreads + tid < n_list ? list[j * kBigThreads + tid] : 0u;
-      }
-      // c_lo >= want > c_hi at all times
-      if (use_list) {
-        // four trial values at a time: first keys of the sample, then values a little either side of where the threshold lies if
-        // the keys of the interval are spread evenly; every third time they cut the interval in five, whatever the counts say
-        const int in_use = (c_lo + kBigThreads - 1) / kBigThreads;
+  for (int i = 0; i < kSample / 32; ++i) n[i & 3] += x[i] >= t ? 1 : 0;
+  return static_cast<int>(__reduce_add_sync(0xffffffffu, (n[0] + n[1]) + (n[2] + n[3])));
+}
+// `v` with the bits from .. to set as far as at least r of the keys x still reach it: the r-th largest of them, cut off below bit `to`
+__device__ __forceinline__ uint32_t rank_value(const uint32_t (&x)[kSample / 32], int r, uint32_t v, int from, int to) {
 #pragma unroll 1
-        for (int trial = 0; c_lo != want && lo != hi && c_lo - c_hi > kFew; ++trial) {
-          const float share = (static_cast<float>(c_lo - want) + 0.5f) / static_cast<float>(c_lo - c_hi), width = static_cast<float>(hi - lo);
-          uint32_t mid[4], c01 = 0, c23 = 0;
+  for (int b = from; b >= to; --b) {
+    const uint32_t t = v | (1u << b);
+    if (count_from(x, t) >= r) v = t;
+  }
+  return v;
+}
+
+template <int kThr>
+struct Shared {
+  union {
+    RowSmem<kThr> radix;
+    struct {
+      uint32_t samp[kSample];
+      alignas(16) uint32_t few[kFew];
+    };
+  };
+  uint32_t bound;                                          // the list takes the keys from here on (ties: above)
+  uint32_t first[4];                                       // first trial values
+  int ties;
+  uint32_t sums[4][32];
+  int n_few, need_eq;
+  uint32_t limit;
+};
+
+// not inline: the rare path needs registers of its own
+template <int kThr>
+__device__ __noinline__ void select_from_memory(const uint32_t* sc, int len, int topk, int32_t* out, RowSmem<kThr>* sm) {
+  select_row<kThr>(sc, len, topk, out, sm);
+}
+
+// exclusive prefix over the block of a packed count, and its total; `sums` (32 words) must not be in use
+template <int kThr>
+__device__ __forceinline__ uint32_t block_prefix(uint32_t v, uint32_t* sums, uint32_t& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t incl = v;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float at = trial % 3 == 0 ? 0.2f * static_cast<float>(j + 1) : share + (j == 0 ? -0.12f : j == 1 ? -0.03f : j == 2 ? 0.03f : 0.12f);
-            mid[j] = lo + 1u + min(static_cast<uint32_t>(fmaxf(at, 0.0f) * width), hi - lo - 1u);
-            if (trial == 0) mid[j] = min(max(static_cast<uint32_t>(ctl[kCtlFirst + j]), lo + 1u), hi);
-          }
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += o;
+  }
+  if (lane == 31) sums[warp] = incl;
+  __syncthreads();
+  const uint32_t w = lane < kThr / 32 ? sums[lane] : 0u;
+  total = __reduce_add_sync(0xffffffffu, w);
+  return __reduce_add_sync(0xffffffffu, lane < warp ? w : 0u) + incl - v;
+}
+
+template <int kThr, int kBlocks>
+__global__ void __launch_bounds__(kThr, kBlocks) topk_listed_kernel(const Params p, const Shape shape) {
+  constexpr int kWarps = kThr / 32;
+  __shared__ Shared<kThr> sm;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t* gt_words = reinterpret_cast<uint32_t*>(smem_raw);                       // keys in the list
+  uint32_t* eq_words = gt_words + shape.words;                                      // keys that equal the bound
+  uint32_t* keys = eq_words + shape.words;                                          // the list: keys,
+  unsigned short* at_pos = reinterpret_cast<unsigned short*>(keys + shape.room);    // and positions, ascending
+  const int row = blockIdx.x;
+  const int len = row_len(p, row);
+  const int k = min(p.topk, len);
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(p.scores) + static_cast<long long>(row) * p.sc_stride;   // bits: NaN patterns keep theirs
+  int32_t* out = p.out + static_cast<long long>(row) * p.out_stride;
+  for (int j = k + tid; j < p.topk; j += kThr) out[j] = -1;
+  if (k == len) {
+    for (int j = tid; j < len; j += kThr) out[j] = j;
+    return;
+  }
+  const bool whole = len <= shape.room;
+  const int words = (len + 31) >> 5;
+  int n_list = len;
+  if (whole) {
+    for (int i = tid; i < len; i += kThr) {
+      keys[i] = to_key(src[i]);
+      at_pos[i] = static_cast<unsigned short>(i);
+    }
+    __syncthreads();
+  }
+  // ---- the sample: one key from each of 512 stretches, not at the same place of each; a row that is shorter is its own sample
+  for (int t = tid; t < kSample; t += kThr) {
+    const uint32_t stride = static_cast<uint32_t>(len) / kSample;
+    const uint32_t at = len >= kSample ? static_cast<uint32_t>((static_cast<unsigned long long>(t) * len) / kSample) + ((((t * 0x9e3779b1u) >> 16) * stride) >> 16)
+                                       : static_cast<uint32_t>(t);
+    sm.samp[t] = at >= static_cast<uint32_t>(len) ? 0u : whole ? keys[at] : to_key(src[at]);
+  }
+  if (tid < kFew) sm.few[tid] = 0u;
+  if (tid == 0) sm.n_few = 0;
+  __syncthreads();
+  if (warp < 4) {
+    uint32_t x[kSample / 32];
 #pragma unroll
-          for (int j = 0; j < kListPer; ++j)
-            if (j < in_use) {
-              c01 += (cand[j] >= mid[0] ? 1u : 0u) + (cand[j] >= mid[1] ? 65536u : 0u);
-              c23 += (cand[j] >= mid[2] ? 1u : 0u) + (cand[j] >= mid[3] ? 65536u : 0u);
-            }
-          c01 = __reduce_add_sync(0xffffffffu, c01);
-          c23 = __reduce_add_sync(0xffffffffu, c23);
-          uint32_t* sums = warp_sum + (trial & 1) * 2 * kBigWarps;
-          if (lane == 0) { sums[warp] = c01; sums[kBigWarps + warp] = c23; }
-          __syncthreads();
-          c01 = __reduce_add_sync(0xffffffffu, sums[lane]);
-          c23 = __reduce_add_sync(0xffffffffu, sums[kBigWarps + lane]);
-          const int c[4] = {static_cast<int>(c01 & 0xffffu), static_cast<int>(c01 >> 16), static_cast<int>(c23 & 0xffffu), static_cast<int>(c23 >> 16)};
+    for (int i = 0; i < kSample / 32; ++i) x[i] = sm.samp[32 * i + lane];
+    const float n = static_cast<float>(min(len, kSample)), frac = __fdividef(static_cast<float>(k), static_cast<float>(len));
+    const float var = n * frac * (1.0f - frac);
+    const int centre = static_cast<int>(frac * n);
+    const int margin = static_cast<int>(kMargin * var * rsqrtf(var)) + 3, step = margin / 4;         // (0 < k < len: the variance is above zero)
+    const int r = warp == 0 ? centre + margin : warp == 1 ? centre + step : warp == 2 ? centre - step : centre - margin;
+    // the high bits (sign, exponent and five more) will do, unless many keys of the sample share them
+    uint32_t v = rank_value(x, max(r, 1), 0u, 31, 18);
+    if (warp == 0) {
+      int from = count_from(x, v);
+      if (from >= r + kCrowd) {
+        v = rank_value(x, r, v, 17, 0);
+        from = count_from(x, v);
+      }
+      if (lane == 0) {
+        sm.bound = v;
+        sm.ties = v != 0u && from >= r + kCrowd ? 1 : 0;
+      }
+    }
+    if (lane == 0) sm.first[warp] = v;
+  }
+  __syncthreads();
+  const uint32_t bound = sm.bound;
+  const bool ties = !whole && sm.ties != 0;
+  int n_ties = 0;
+  if (!whole) {
+    // ---- the sweep: warp w takes stretches of 32 kAhead positions, w, w + kWarps, ...; word i of the mask is positions 32 i ..
+    const bool plain = !ties && bound > 0x80000000u;       // the usual case, a bound above zero: floats from there on compare by their bits
+    const int lo_bits = static_cast<int>(bound ^ 0x80000000u);
+#pragma unroll 1
+    for (int w0 = warp * kAhead; w0 < words; w0 += kWarps * kAhead) {
+      uint32_t v[kAhead];
+      const uint32_t* at = src + w0 * 32 + lane;
+      const bool inside = (w0 + kAhead) * 32 <= len;
+      if (inside) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {                    // mid and so c in order
-            if (c[j] >= want) { lo = mid[j]; c_lo = c[j]; }
-          }
+        for (int j = 0; j < kAhead; ++j) v[j] = at[32 * j];
+      } else {
 #pragma unroll
-          for (int j = 3; j >= 0; --j) {
-            if (c[j] < want) { hi = mid[j] - 1u; c_hi = c[j]; }
-          }
-        }
-        if (c_lo != want && lo != hi) {                    // few left: the one of which want - c_hi are not smaller
+        for (int j = 0; j < kAhead; ++j) v[j] = (w0 + j) * 32 + lane < len ? at[32 * j] : 0xffffffffu;   // the lowest key
+      }
+      if (plain && inside) {
 #pragma unroll
-          for (int j = 0; j < kListPer; ++j)
-            if (cand[j] >= lo && cand[j] <= hi) few[atomicAdd(&ctl[kCtlFew], 1)] = cand[j];
-          __syncthreads();
-          const int n = c_lo - c_hi, r = want - c_hi;
-          const int which = tid >> 3;                      // eight threads per candidate
-          const uint32_t v = few[which < n ? which : 0];
-          int above_v = 0, from_v = 0;
-          for (int m = tid & 7; m < n; m += 8) {
-            above_v += few[m] > v ? 1 : 0;
-            from_v += few[m] >= v ? 1 : 0;
-          }
-#pragma unroll
-          for (int d = 1; d < 8; d <<= 1) {
-            above_v += __shfl_xor_sync(0xffffffffu, above_v, d);
-            from_v += __shfl_xor_sync(0xffffffffu, from_v, d);
-          }
-          if (which < n && above_v < r && r <= from_v) { ctl[kCtlLimit] = static_cast<int>(v); ctl[kCtlNeedEq] = r - above_v; }
-          __syncthreads();
-          lo = hi = static_cast<uint32_t>(ctl[kCtlLimit]);
-          c_hi = want - ctl[kCtlNeedEq];
+        for (int j = 0; j < kAhead; ++j) {
+          const uint32_t m = __ballot_sync(0xffffffffu, static_cast<int>(v[j]) >= lo_bits);
+          if (lane == 0) gt_words[w0 + j] = m;
         }
       } else {
-#pragma unroll 1
-        for (int trial = 0; c_lo != want && lo != hi; ++trial) {
-          const uint32_t mid = lo + 1u + (hi - lo - 1u) / 2u;
-          int n = 0;
+        const int last = len - w0 * 32 - lane;             // the lane's keys from here on are past the row
 #pragma unroll
-          for (int i = 0; i < kPerThread; ++i) n += key[i] >= mid ? 1 : 0;
-          for (int i = 0; i < n2; ++i) n += key2(i) >= mid ? 1 : 0;
-          n = __reduce_add_sync(0xffffffffu, n);
-          uint32_t* sums = warp_sum + (trial & 1) * kBigWarps;
-          if (lane == 0) sums[warp] = static_cast<uint32_t>(n);
-          __syncthreads();
-          n = static_cast<int>(__reduce_add_sync(0xffffffffu, sums[lane]));
-          if (n >= want) { lo = mid; c_lo = n; }
-          else { hi = mid - 1u; c_hi = n; }
+        for (int j = 0; j < kAhead; ++j) {
+          const uint32_t key = to_key(v[j]);
+          uint32_t m = __ballot_sync(0xffffffffu, key >= bound && 32 * j < last);
+          if (ties) {
+            const uint32_t eq = __ballot_sync(0xffffffffu, key == bound) & m;
+            m ^= eq;
+            if (lane == 0 && w0 + j < words) eq_words[w0 + j] = eq;
+          }
+          if (lane == 0 && w0 + j < words) gt_words[w0 + j] = m;
         }
       }
-      // keys above `limit` are taken, and need_eq of those equal to it
-      const int need_eq = c_lo == want ? 0 : want - c_hi;
-      const uint32_t limit = c_lo == want ? lo - 1u : lo;
-      // word i of 32 positions 1024 i + 32 warp ...: taken, ties
-#pragma unroll
-      for (int i = 0; i < kPerThread; ++i) {
-        const uint32_t m = __ballot_sync(0xffffffffu, key[i] > limit);
-        if (lane == 0) gt_words[i * kBigWarps + warp] = m;
-      }
-#pragma unroll 4
-      for (int i = 0; i < kPerThread; ++i) {
-        const uint32_t m = __ballot_sync(0xffffffffu, i < n2 && key2(i) > limit);
-        if (lane == 0) gt_words[kWords / 2 + i * kBigWarps + warp] = m;
-      }
-      if (need_eq > 0) {
-#pragma unroll
-        for (int i = 0; i < kPerThread; ++i) {
-          const uint32_t m = __ballot_sync(0xffffffffu, key[i] == limit && i * kBigThreads + tid < len);
-          if (lane == 0) eq_words[i * kBigWarps + warp] = m;
-        }
-#pragma unroll 4
-        for (int i = 0; i < kPerThread; ++i) {
-          const uint32_t m = __ballot_sync(0xffffffffu, i < n2 && key2(i) == limit);
-          if (lane == 0) eq_words[kWords / 2 + i * kBigWarps + warp] = m;
-        }
-      }
+    }
+    __syncthreads();
+    // ---- the list: every thread the positions of a few words
+    const int per = (words + kThr - 1) / kThr, w_end = min(words, per * (tid + 1));
+    uint32_t packed = 0, total;
+    for (int w = per * tid; w < w_end; ++w) {
+      packed += static_cast<uint32_t>(__popc(gt_words[w]));
+      if (ties) n_ties += __popc(eq_words[w]);
+    }
+    int at = static_cast<int>(block_prefix<kThr>(packed, sm.sums[0], total));
+    n_list = static_cast<int>(total);
+    if (ties) {
+      uint32_t all;
+      block_prefix<kThr>(static_cast<uint32_t>(n_ties), sm.sums[1], all);
+      n_ties = static_cast<int>(all);
+    }
+    if (n_list > shape.room || n_list + n_ties < k) {      // the sample misled
       __syncthreads();
-      // one scan over the packed counts (ties << 16 | taken), then each thread writes the positions of its words
-      constexpr int kPer = 2;
-      uint32_t g[kPer], e[kPer], packed = 0;
-#pragma unroll
-      for (int j = 0; j < kPer; ++j) {
-        g[j] = gt_words[kPer * tid + j];
-        e[j] = need_eq > 0 ? eq_words[kPer * tid + j] : 0u;
-        packed += (static_cast<uint32_t>(__popc(e[j])) << 16) + static_cast<uint32_t>(__popc(g[j]));
-      }
-      uint32_t incl = packed;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += v;
-      }
-      if (lane == 31) warp_sum[warp] = incl;
-      __syncthreads();
-      uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp ? warp_sum[lane] : 0u) + incl - packed;
-#pragma unroll
-      for (int j = 0; j < kPer; ++j) {
-        const int gt_before = static_cast<int>(before & 0xffffu), eq_before = static_cast<int>(before >> 16);
-        int eq_take = min(max(need_eq - eq_before, 0), __popc(e[j]));                 // the lowest positions among the ties
-        uint32_t bits = g[j], ties = e[j];
-        while (eq_take > 0) {
-          const uint32_t lowest = ties & (0u - ties);
+      select_from_memory<kThr>(src, len, p.topk, out, &sm.radix);
+      return;
+    }
+    if (n_list < k) {
+      // the k-th largest key is the bound itself: the keys above it and the first of the ties
+      const int need_eq = k - n_list;
+      uint32_t mine = 0, all;
+      for (int w = per * tid; w < w_end; ++w) mine += static_cast<uint32_t>(__popc(eq_words[w]));
+      int eq_before = static_cast<int>(block_prefix<kThr>(mine, sm.sums[2], all));
+      int write_at = at + min(eq_before, need_eq);
+      for (int w = per * tid; w < w_end; ++w) {
+        uint32_t bits = gt_words[w], eq = eq_words[w];
+        int take = min(max(need_eq - eq_before, 0), __popc(eq));                     // the lowest positions among the ties
+        eq_before += __popc(eq);
+        while (take > 0) {
+          const uint32_t lowest = eq & (0u - eq);
           bits |= lowest;
-          ties ^= lowest;
-          --eq_take;
+          eq ^= lowest;
+          --take;
         }
-        int write_at = gt_before + min(eq_before, need_eq);
-        const int pos0 = (kPer * tid + j) * 32;
         while (bits != 0) {
-          out[write_at++] = pos0 + __ffs(static_cast<int>(bits)) - 1;
+          out[write_at++] = 32 * w + __ffs(static_cast<int>(bits)) - 1;
           bits &= bits - 1u;
         }
-        before += (static_cast<uint32_t>(__popc(e[j])) << 16) + static_cast<uint32_t>(__popc(g[j]));
       }
-    } else {
-      for (int j = tid; j < len; j += kBigThreads) out[j] = j;                        // every position of the row is taken
+      return;
     }
-    for (int j = k + tid; j < p.topk; j += kBigThreads) out[j] = -1;
-    __syncthreads();                                       // the shared words are reused by the next row
+    for (int w = per * tid; w < w_end; ++w) {
+      uint32_t bits = gt_words[w];
+      while (bits != 0) {
+        at_pos[at++] = static_cast<unsigned short>(32 * w + __ffs(static_cast<int>(bits)) - 1);
+        bits &= bits - 1u;
+      }
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int i = tid; i < n_list; i += kThr) keys[i] = to_key(src[at_pos[i]]);
+    __syncthreads();
+  }
+  // ---- the k-th largest key of the list: keys above `limit` are taken, and need_eq of those equal to it (0: none or all, see below)
+  uint32_t limit, lo = whole ? 0u : ties ? bound + 1u : bound, hi = 0xffffffffu;
+  int need_eq = 0;
+  int c_lo = n_list, c_hi = 0;                             // keys >= lo, keys > hi; c_lo >= k > c_hi at all times
+  // every third time the values cut the interval in five, whatever the counts say
+#pragma unroll 1
+  for (int trial = 0; c_lo != k && lo != hi && c_lo - c_hi > kFew; ++trial) {
+    uint32_t mid[4], c01 = 0, c23 = 0;
+    if (trial == 0) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) mid[j] = min(max(sm.first[j], lo + 1u), hi);
+    } else {
+      const float share = __fdividef(static_cast<float>(c_lo - k) + 0.5f, static_cast<float>(c_lo - c_hi)), width = static_cast<float>(hi - lo);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float cut = trial % 3 == 0 ? 0.2f * static_cast<float>(j + 1) : share + (j == 0 ? -0.12f : j == 1 ? -0.03f : j == 2 ? 0.03f : 0.12f);
+        mid[j] = lo + 1u + min(static_cast<uint32_t>(fmaxf(cut, 0.0f) * width), hi - lo - 1u);
+      }
+    }
+#pragma unroll 4
+    for (int i = tid; i < n_list; i += kThr) {
+      const uint32_t x = keys[i];
+      c01 += (x >= mid[0] ? 1u : 0u) + (x >= mid[1] ? 65536u : 0u);
+      c23 += (x >= mid[2] ? 1u : 0u) + (x >= mid[3] ? 65536u : 0u);
+    }
+    c01 = __reduce_add_sync(0xffffffffu, c01);
+    c23 = __reduce_add_sync(0xffffffffu, c23);
+    uint32_t(*sums)[32] = &sm.sums[(trial & 1) * 2];
+    if (lane == 0) { sums[0][warp] = c01; sums[1][warp] = c23; }
+    __syncthreads();
+    c01 = __reduce_add_sync(0xffffffffu, lane < kWarps ? sums[0][lane] : 0u);
+    c23 = __reduce_add_sync(0xffffffffu, lane < kWarps ? sums[1][lane] : 0u);
+    const int c[4] = {static_cast<int>(c01 & 0xffffu), static_cast<int>(c01 >> 16), static_cast<int>(c23 & 0xffffu), static_cast<int>(c23 >> 16)};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (c[j] >= k && mid[j] > lo) { lo = mid[j]; c_lo = c[j]; }
+      if (c[j] < k && mid[j] <= hi) { hi = mid[j] - 1u; c_hi = c[j]; }
+    }
+  }
+  if (c_lo != k && lo != hi) {                             // few left: the one of which k - c_hi are not smaller
+    for (int i0 = warp * 32; i0 < n_list; i0 += kThr) {
+      const int i = i0 + lane;
+      const uint32_t x = i < n_list ? keys[i] : 0u;
+      const bool in = i < n_list && x >= lo && x <= hi;
+      const uint32_t m = __ballot_sync(0xffffffffu, in);
+      if (m != 0u) {
+        int at = 0;
+        if (lane == 0) at = atomicAdd(&sm.n_few, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+        if (in) sm.few[at] = x;
+      }
+    }
+    __syncthreads();
+    const int total = c_lo - c_hi, r = k - c_hi;
+    constexpr int kRankers = kThr / kFew;                  // threads per candidate
+    const int which = tid / kRankers;
+    const uint32_t v = sm.few[which];
+    int above = 0, from = 0;
+    for (int m = (tid % kRankers) * 4; m < total; m += kRankers * 4) {               // (past the last candidate: 0, below every key of the list)
+      const uint4 o = *reinterpret_cast<const uint4*>(&sm.few[m]);
+      above += (o.x > v) + (o.y > v) + (o.z > v) + (o.w > v);
+      from += (o.x >= v) + (o.y >= v) + (o.z >= v) + (o.w >= v);
+    }
+#pragma unroll
+    for (int d = 1; d < kRankers; d <<= 1) {
+      above += __shfl_xor_sync(0xffffffffu, above, d);
+      from += __shfl_xor_sync(0xffffffffu, from, d);
+    }
+    if (which < total && above < r && r <= from) { sm.limit = v; sm.need_eq = r == from ? 0 : r - above; }
+    __syncthreads();
+    need_eq = sm.need_eq;
+    limit = need_eq == 0 ? sm.limit - 1u : sm.limit;       // all that equal the limit are taken: those above the key before it
+  } else {
+    need_eq = c_lo == k ? 0 : k - c_hi;
+    limit = need_eq == 0 ? lo - 1u : lo;
+  }
+  // ---- the output: every warp a stretch of the list, first counted, then written
+  const int stretch = ((n_list + 32 * kWarps - 1) / (32 * kWarps)) * 32, i_begin = warp * stretch, i_end = min(n_list, i_begin + stretch);
+  int taken = 0, equal = 0;
+#pragma unroll 4
+  for (int i = i_begin + lane; i < i_end; i += 32) {
+    const uint32_t x = keys[i];
+    taken += x > limit ? 1 : 0;
+    if (need_eq != 0) equal += x == limit ? 1 : 0;
+  }
+  taken = static_cast<int>(__reduce_add_sync(0xffffffffu, taken));
+  equal = static_cast<int>(__reduce_add_sync(0xffffffffu, equal));
+  __syncthreads();                                         // the trials have read `sums`
+  if (lane == 0) { sm.sums[0][warp] = static_cast<uint32_t>(taken); sm.sums[1][warp] = static_cast<uint32_t>(equal); }
+  __syncthreads();
+  int write_at = static_cast<int>(__reduce_add_sync(0xffffffffu, lane < warp ? sm.sums[0][lane] : 0u));
+  int eq_left = need_eq - static_cast<int>(__reduce_add_sync(0xffffffffu, lane < warp ? sm.sums[1][lane] : 0u));
+  write_at += need_eq - max(eq_left, 0);                   // the ties of the warps before
+  const uint32_t lower = (1u << lane) - 1u;
+  for (int i0 = i_begin; i0 < i_end; i0 += 32) {
+    const int i = i0 + lane;
+    const uint32_t x = i < i_end ? keys[i] : 0u;
+    bool take = i < i_end && x > limit;
+    if (need_eq != 0) {
+      const bool tie = i < i_end && x == limit;
+      const uint32_t m = __ballot_sync(0xffffffffu, tie);
+      take = take || (tie && __popc(m & lower) < eq_left);
+      eq_left -= __popc(m);
+    }
+    const uint32_t m = __ballot_sync(0xffffffffu, take);
+    if (take) out[write_at + __popc(m & lower)] = at_pos[i];
+    write_at += __popc(m);
   }
 }
 
-}  // namespace half_held
+}  // namespace listed
 
 }  // namespace topk
 }  // namespace ftb
@@ -866,19 +571,20 @@ extern "C" FTB_API int ftb_topk_indices(const ftb_topk_args* a, void* stream) {
   int dev = 0, sm_count = 0;
   if (int rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice")) return rc;
   if (int rc = check_cuda(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev), "SM count")) return rc;
-  // Short rows go to the radix select, many to an SM, up to where the persistent CTAs pass it (us, radix / persistent): 4096 rows of 1000
-  // scores 84 / 332, of 4000 190 / 318, of 6000 275 / 317, of 8192 341 / 307; 148 rows of 4000 12 / 13, of 5001 14 / 16, of 6000 17 / 17.
-  const bool short_rows = a->s_kv <= 5120 || (a->s_kv <= 6656 && a->s_q > sm_count);
-  if (!short_rows && a->s_kv <= topk::half_held::kRowMax) {
-    const bool held = a->s_kv <= topk::held::kRowMax;
-    const bool aligned = (a->s_kv & 3) == 0 && (a->scores_stride_token & 3) == 0 && (reinterpret_cast<uintptr_t>(a->scores) & 15) == 0;
-    const auto kernel = !held ? topk::half_held::topk_select_long_rows_kernel
-                              : aligned ? topk::held::topk_select_rows_kernel<true> : topk::held::topk_select_rows_kernel<false>;
-    const size_t smem = held ? topk::held::kBigSmem : topk::half_held::kBigSmem;
-    if (int rc = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-                            "topk shared memory")) return rc;
-    const unsigned grid = static_cast<unsigned>(a->s_q < sm_count ? a->s_q : sm_count);
-    kernel<<<grid, topk::kBigThreads, smem, st>>>(p);
+  // A row to an SM: as many threads as its sweep keeps busy (us, 512 threads / 1024: 148 rows of 4000 14.4 / 17.1, 128 of up to 65536 20.7 / 19.3,
+  // one of 32768 14.4 / 13.6).  More rows: six small CTAs to an SM hide their chains better, three larger ones keep fewer lists and rows
+  // in flight (256 threads / 512: 4096 rows of 1000 56 / 79, of 6000 103 / 134, of 20001 151 / 159, of 32768 236 / 210; 592 of 33000 35 / 41;
+  // 600 of 32768 with topk 8192 101 / 76).
+  const bool alone = a->s_q <= sm_count;
+  topk::listed::Shape shape;
+  const int smem = topk::listed::plan(a->s_kv, a->topk, alone, &shape);
+  if (smem > 0) {
+    const bool small = alone ? a->s_kv <= 8192 : a->topk <= 4096 && (a->s_kv <= 24576 || a->s_q <= 6 * sm_count);
+    const auto kernel = alone ? (small ? topk::listed::topk_listed_kernel<512, 1> : topk::listed::topk_listed_kernel<1024, 1>)
+                              : (small ? topk::listed::topk_listed_kernel<256, 6> : topk::listed::topk_listed_kernel<512, 3>);
+    const unsigned threads = alone ? (small ? 512 : 1024) : (small ? 256 : 512);
+    if (int rc = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, topk::listed::kSmemMax), "topk shared memory")) return rc;
+    kernel<<<static_cast<unsigned>(a->s_q), threads, smem, st>>>(p, shape);
   } else {
     topk::topk_select_kernel<<<static_cast<unsigned>(a->s_q), topk::kThreads, 0, st>>>(p);
   }

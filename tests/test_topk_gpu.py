@@ -132,3 +132,37 @@ def test_ties_and_lengths_on_every_kernel(s_q, s_kv):
         ref = topk_indices_ref(sc, k, lengths)
         assert torch.equal(topk_indices(sc.to(DEV), k, lengths.to(DEV)).cpu(), ref)
         assert torch.equal(topk_indices(wide.to(DEV)[:, 1:s_kv + 1], k, lengths.to(DEV)).cpu(), ref)
+
+
+@pytest.mark.parametrize("rows,s_kv,topk", [(3, 511, 100), (3, 512, 100), (3, 513, 512), (2, 4096, 64), (2, 4097, 64), (5, 8192, 2048),
+                                            (5, 8193, 2048), (2, 65536, 2048), (2, 65536, 30000), (3, 32768, 16384), (200, 5001, 512),
+                                            (200, 3000, 2999), (150, 12001, 5000), (900, 24577, 65), (160, 65535, 1)])
+@pytest.mark.parametrize("values", ["plain", "crowded", "negative"])
+def test_lists_of_candidates(rows, s_kv, topk, values):
+    """Both sides of every rule of the dispatch and of the list: rows that are their own sample, that fit the list as a whole, that fill an
+    SM or share one; keys whose bound is a value that fills much of the row; bounds below zero; an unaligned view; short and empty rows."""
+    g = torch.Generator().manual_seed(rows + s_kv + topk)
+    wide = torch.randn(rows, s_kv + 3, generator=g)
+    if values == "crowded":
+        wide = wide.clamp(-0.5, 0.5).mul(4).round()
+    elif values == "negative":
+        wide = -wide.abs() - 1e-30
+    lengths = torch.full((rows,), s_kv, dtype=torch.int32)
+    if rows >= 5:
+        lengths[1:5] = torch.tensor([0, min(topk, s_kv), min(topk + 1, s_kv), s_kv // 3])
+    got = topk_indices(wide.to(DEV)[:, 1:1 + s_kv], topk, lengths.to(DEV)).cpu()
+    assert torch.equal(got, topk_indices_ref(wide[:, 1:1 + s_kv], topk, lengths))
+
+
+@pytest.mark.parametrize("top", [0.0, 1e6, -1e6])
+def test_sample_that_misleads(top):
+    """The sampled positions hold values unlike the rest: a bound that is too high, or a list that overflows, sends the row to the radix select."""
+    g = torch.Generator().manual_seed(31)
+    s_kv, t = 40000, torch.arange(512)
+    at = t * s_kv // 512 + ((((t * 0x9E3779B1) & 0xFFFFFFFF) >> 16) * (s_kv // 512) >> 16)
+    sc = torch.randn(4, s_kv, generator=g)
+    sc[:, at] = top
+    sc[1] = sc[1].abs()
+    sc[2] = -sc[2].abs()
+    got = topk_indices(sc.to(DEV), 2048).cpu()
+    assert torch.equal(got, topk_indices_ref(sc, 2048))

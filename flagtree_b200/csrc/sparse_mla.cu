@@ -582,7 +582,20 @@ namespace ftb {
 void set_last_error(const char* fmt, ...);
 int check_cuda(cudaError_t e, const char* what);
 int launch_sparse_mla_ring(const ftb_sparse_mla_args* a, int n_splits, float* part_out, float* part_lse, float max_slack, cudaStream_t st);
-int launch_sparse_mla_few(const ftb_sparse_mla_args* a, cudaStream_t st);
+int launch_sparse_mla_few(const ftb_sparse_mla_args* a, int n_splits, float* part_out, float* part_lse, float max_slack, cudaStream_t st);
+
+// The persistent kernels: up to 64 heads on the columns of the MMA, one CTA per item; more on its rows, a pair of CTAs per item.
+// The two add in the same order, so that the choice is not to be seen in the bits.  More than 64 heads in groups of 64, an item
+// each, are the faster form while a CTA has one item of at most 16 tiles (us, pairs / groups, 128 heads, topk 2048: 1 token 21.2 / 14.7,
+// 8 tokens 27.3 / 18.8, 32 tokens 48 / 39; 74 tokens of topk 512 24.7 / 22.3, of topk 2048 51 / 58).
+static int launch_persistent(const ftb_sparse_mla_args* a, int n_splits, float* part_out, float* part_lse, float max_slack, cudaStream_t st) {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long long groups = (a->h + 63) / 64, tiles = (a->topk + 63) / 64;
+  const bool few = a->h <= 64 || (a->s_q * groups * n_splits <= sms && tiles <= 16LL * n_splits);
+  return (few ? launch_sparse_mla_few : launch_sparse_mla_ring)(a, n_splits, part_out, part_lse, max_slack, st);
+}
 }  // namespace ftb
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -618,15 +631,10 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
     set_last_error("ftb_sparse_mla_fwd: kv row stride must be a multiple of 8 elements");
     return FTB_ERR_INVALID;
   }
-  // algo 0 = default = 5: persistent role-split CTA pairs (scores in one CTA, values in the other, Q in tensor
-  // memory, rows gathered by cp.async), whole tokens or parts of them; algo 1 = one CTA per (token, output half), which is
-  // also the kernel of the FP8 paged form without a workspace and of the diagnostic score tap;
-  // algo 6 = paged FP8 form: dequantise the selected rows, then the persistent kernel; algo 2 = few heads (h <= 32):
-  // one CTA per token, the gathered rows on the rows of the MMA.  Measured at h = 16 / 32 (2048 causal tokens,
-  // topk 2048): 0.89 / 1.14 ms against 0.80 ms of the persistent pairs (which have become faster since), so the default
-  // keeps the pairs: an MMA with
-  // 16 columns costs what one with 128 costs (its time goes with the 128 rows of the A operand), so putting the
-  // heads on the columns saves no tensor time, and this kernel does not overlap its gather with its products.
+  // algo 0 = default = 5: the persistent kernels (launch_persistent above), whole tokens or parts of them; algo 1 = one CTA per
+  // (token, output half), which is also the kernel of the FP8 paged form without a workspace and of the diagnostic score tap;
+  // algo 6 = paged FP8 form: dequantise the selected rows, then the persistent kernels; algo 2 = the kernel for few heads (h <= 32) with the
+  // true maximum as the reference of the weights.
   if (a->algo_id != 0 && a->algo_id != 1 && a->algo_id != 2 && a->algo_id != 5 && a->algo_id != 6) {
     set_last_error("ftb_sparse_mla_fwd: unknown algo_id %d (0 = default, 1, 2, 5, 6)", a->algo_id);
     return FTB_ERR_INVALID;
@@ -637,9 +645,9 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
     set_last_error("ftb_sparse_mla_fwd: algo 2 serves the bf16 form without splits for at most 32 heads");
     return FTB_ERR_INVALID;
   }
-  if (a->algo_id == 2) return launch_sparse_mla_few(a, reinterpret_cast<cudaStream_t>(stream));
+  if (a->algo_id == 2) return launch_sparse_mla_few(a, 1, nullptr, nullptr, 0.0f, reinterpret_cast<cudaStream_t>(stream));
   if (plain && (a->algo_id == 0 || a->algo_id == 5))
-    return launch_sparse_mla_ring(a, 1, nullptr, nullptr, 8.0f, reinterpret_cast<cudaStream_t>(stream));
+    return launch_persistent(a, 1, nullptr, nullptr, 8.0f, reinterpret_cast<cudaStream_t>(stream));
   MlaParams p;
   memset(&p, 0, sizeof(p));
   p.q = reinterpret_cast<const __nv_bfloat16*>(a->q);
@@ -711,11 +719,11 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
       b.idx_stride_token = a->topk;
       b.algo_id = 5;
       b.workspace = nullptr; b.workspace_bytes = 0; b.n_splits = 0;
-      if (n_splits == 1) return launch_sparse_mla_ring(&b, 1, nullptr, nullptr, 8.0f, st);
+      if (n_splits == 1) return launch_persistent(&b, 1, nullptr, nullptr, 8.0f, st);
       p.part_out = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(a->workspace) + rows_bytes);
       n_splits = parts_of(128);
       p.part_lse = p.part_out + static_cast<size_t>(a->s_q) * n_splits * a->h * 512;
-      rc0 = launch_sparse_mla_ring(&b, n_splits, p.part_out, p.part_lse, 0.0f, st);
+      rc0 = launch_persistent(&b, n_splits, p.part_out, p.part_lse, 0.0f, st);
       return rc0 != FTB_OK || n_splits == 1 ? rc0 : merge();
     }
   }
@@ -740,7 +748,7 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
   if (n_splits > 1 && n_splits <= 64 && !a->kv_is_fp8 && a->dbg_scores == nullptr && pairs) {
     n_splits = parts_of(128);
     p.part_lse = p.part_out + static_cast<size_t>(a->s_q) * n_splits * a->h * 512;
-    const int rc0 = launch_sparse_mla_ring(a, n_splits, p.part_out, p.part_lse, a->algo_id == 5 ? 8.0f : 0.0f, st);
+    const int rc0 = launch_persistent(a, n_splits, p.part_out, p.part_lse, a->algo_id == 5 ? 8.0f : 0.0f, st);
     return rc0 != FTB_OK || n_splits == 1 ? rc0 : merge();
   }
   n_splits = p.n_splits = parts_of(kBN);

@@ -118,13 +118,15 @@ struct Misc0 {   // CTA 0
   unsigned short nt[2 * kBatch];    // per item of the current batch: number of tiles, first tile
   int last[kBatch];                 // entries of its list up to the last that is not negative
   float xchg[2][256];               // row maximum / row sum exchange between the two threads of a head row
-  alignas(16) float alpha_stage[128]; // rescale factors of a tile on their way to CTA 1 (sent with P)
+  alignas(16) float2 alpha_stage[128]; // rescale factors of a tile's halves on their way to CTA 1 (sent with P)
 };
 struct Misc1 {   // CTA 1
   unsigned long long v_full[kNV];   // one arrival per gather thread, when its copies have landed
   unsigned long long v_free[kNV];   // tcgen05.commit
-  unsigned long long p_full[2];     // softmax warps with heads of CTA 0 (remote arrivals, each announcing its bulk copies: 4 KB of P, 128 B of factors)
+  unsigned long long p_full[2];     // softmax warps with heads of CTA 0 (remote arrivals, each announcing its bulk copies: 4 KB of P, 256 B of factors)
   unsigned long long corr_done[2];  // correction warps with heads
+  unsigned long long half_done[4];  // per correction warp: tcgen05.commit behind the first half of a tile whose second half moves one of its maxima
+  unsigned long long half_corr[4];  // the warp: its rows of the accumulator are ready for that second half
   unsigned long long pv_done[2];    // tcgen05.commit
   unsigned long long fin[2];        // softmax warps with heads of CTA 0: 1/l of token t (t % 2) is in place
   unsigned long long o_free;        // 16 epilogue warps: the accumulator has been read
@@ -132,10 +134,10 @@ struct Misc1 {   // CTA 1
   unsigned long long epi_cnt;       // 16 epilogue warps: the output of the token has left the staging area
   uint32_t tmem_base;
   int abort_flag;
-  int pad[2];
+  uint32_t late[2];                 // a byte per correction warp: does the second half of the tile move one of its maxima?
   unsigned short nt[2 * kBatch];
   int last[kBatch];
-  alignas(16) float alpha[2][128];  // rescale factor of the tile (two buffers), written by bulk copies from CTA 0
+  alignas(16) float2 alpha[2][128];  // rescale factors of the halves of a tile (two buffers), written by bulk copies from CTA 0
   float inv_l[2][128];              // final 1/l of token t (t % 2)
 };
 static_assert(sizeof(Misc0) <= 4096 && sizeof(Misc1) <= 4096, "misc area");
@@ -146,6 +148,17 @@ static_assert(kNV == kNT / kVSlabRows, "V ring slot index = slab index");
 __device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+// does the predicate hold for any of the threads of the barrier?
+__device__ __forceinline__ bool named_bar_any(int id, int nthreads, bool pred) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %3, 0;\n\t"
+      "bar.red.or.pred q, %1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r) : "r"(id), "r"(nthreads), "r"(pred ? 1u : 0u) : "memory");
+  return r != 0u;
 }
 __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
@@ -177,6 +190,14 @@ __device__ __forceinline__ float2 ffma2(float a0, float a1, float2 b, float2 c) 
       "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
       "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
       : "=f"(r.x), "=f"(r.y) : "f"(a0), "f"(a1), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+__device__ __forceinline__ float2 fmul2(float2 a, float b) {
+  float2 r;
+  asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
+      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %4};\n\t"
+      "mul.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b));
   return r;
 }
 __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
@@ -254,10 +275,12 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
       for (int i = 0; i < 2; ++i) {
         mbar_init(smem_u32(&m1->p_full[i]), 2 * row_warps);
         mbar_init(smem_u32(&m1->corr_done[i]), row_warps);
+        m1->late[i] = 0;
         mbar_init(smem_u32(&m1->pv_done[i]), 1);
         mbar_init(smem_u32(&m1->fin[i]), 2 * row_warps);
       }
       mbar_init(smem_u32(&m1->o_free), 16);
+      for (int i = 0; i < 4; ++i) { mbar_init(smem_u32(&m1->half_done[i]), 1); mbar_init(smem_u32(&m1->half_corr[i]), 1); }
       for (int i = 0; i < 8; ++i) mbar_init(smem_u32(&m1->stg_free[i]), 1);
       mbar_init(smem_u32(&m1->epi_cnt), 16);
     }
@@ -297,6 +320,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
   // items (tokens, or parts of tokens) of this pair: pair, pair + n_pairs, ...  (the host launches no more pairs than items)
   auto token_of = [&](int item) { return p.n_splits == 1 ? item : item / p.n_splits; };
   const int my_tokens = (p.s_q * p.n_splits - pair + n_pairs - 1) / n_pairs;
+  uint32_t n_late = 0;   // CTA 1: tiles so far whose second half moved a maximum, of a correction warp (the issuer: a bit of it per warp)
   uint32_t gt = 0;   // tiles processed before the current token: every role counts the same way
   // CTA 0: the nine gather warps, one per column block: the warps 9-19 whose id is not 0 modulo 4, in order (they share no
   // scheduler with the MMA issuer, warp 8)
@@ -358,7 +382,8 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
           const int n_tiles = warp_uniform(nt[t]);
           // 1/l and the `fin` barrier of parity ti % 2 were last used by token ti - 2: its epilogue is over
           if (ti >= 2) mbar_wait(smem_u32(&m0->epi_done[ti & 1]), ((ti >> 1) - 1) & 1u, abort_flag);
-          float m_run = -INFINITY, l_run = 0.0f;
+          float m_run = -INFINITY;
+          float2 l01 = make_float2(0.0f, 0.0f), l23 = l01;   // sums of the weights, by groups of 16 columns of this thread's 64
           for (int i = 0; i < n_tiles; ++i) {
             const uint32_t G = gt + i;
             const int b = G & 1;
@@ -390,59 +415,97 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
 #pragma unroll
               for (int j = 0; j < 32; j += 2) mx = fmaxf(mx, fmaxf(__uint_as_float(sr[q][j]), __uint_as_float(sr[q][j + 1])));
             }
-            m0->xchg[b][tid] = mx;
-            named_bar_sync(2 + (warp & 3), 64);
-            mx = fmaxf(mx, m0->xchg[b][tid ^ 128]);
             // Lazy maximum: with a slack of 8 the reference only moves when it grows by more than 2^8, so that the
             // accumulator in the other CTA is rarely rescaled (P stays below 256).  Without slack it follows the true
-            // maximum: the largest weight is then 1, which bf16 holds exactly.
-            const float m_cand = fmaxf(m_run, mx * p.scale_log2);
-            float alpha = 1.0f;
-            if (m_cand > m_run + p.max_slack || m_run == -INFINITY) {
-              alpha = (m_run == -INFINITY) ? 0.0f : fast_exp2(m_run - m_cand);
-              m_run = m_cand;
+            // maximum: the largest weight is then 1, which bf16 holds exactly.  The first tile sets it as a whole; later the two
+            // halves of a tile (64 rows: the tile of the kernel for few heads) move it one after the other, and the sums below add in
+            // that kernel's order: the bits of a head do not depend on how many heads the call has.
+            auto move_to = [&](float top) {
+              const float m_cand = fmaxf(m_run, top * p.scale_log2);
+              float a = 1.0f;
+              if (m_cand > m_run + p.max_slack || m_run == -INFINITY) {
+                a = (m_run == -INFINITY) ? 0.0f : fast_exp2(m_run - m_cand);
+                m_run = m_cand;
+              }
+              return a;
+            };
+            float alpha_a = 1.0f, alpha_b = 1.0f, m_mine = m_run;
+            // (the two warps of 32 rows agree; only then do they exchange their maxima)
+            const bool moves = named_bar_any(2 + (warp & 3), 64, mx * p.scale_log2 > m_run + p.max_slack || m_run == -INFINITY);
+            if (moves) {
+              m0->xchg[b][tid] = mx;
+              named_bar_sync(2 + (warp & 3), 64);
+              const float other = m0->xchg[b][tid ^ 128];
+              alpha_a = move_to(i == 0 ? fmaxf(mx, other) : ch == 0 ? mx : other);
+              m_mine = m_run;
+              if (i != 0) alpha_b = move_to(ch == 0 ? other : mx);
+              if (ch != 0) m_mine = m_run;
+              l01 = fmul2(l01, alpha_a);
+              l23 = fmul2(l23, alpha_a);
+              if (ch != 0) {
+                l01 = fmul2(l01, alpha_b);
+                l23 = fmul2(l23, alpha_b);
+              }
             }
-            const float m_use = (m_run == -INFINITY) ? 0.0f : m_run;
+            const float m_use = (m_mine == -INFINITY) ? 0.0f : m_mine;
+            float sum16[4];
+            const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), neg_m2 = make_float2(-m_use, -m_use);
+            uint32_t pk[2][16];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+#pragma unroll
+              for (int g = 0; g < 2; ++g) {
+                float2 e[8];
+#pragma unroll
+                for (int j = 0; j < 16; j += 2) {
+                  const float2 x = ffma2(__uint_as_float(sr[q][16 * g + j]), __uint_as_float(sr[q][16 * g + j + 1]), scale2, neg_m2);
+                  e[j >> 1] = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+                  pk[q][8 * g + (j >> 1)] = pack_bf16x2(e[j >> 1].x, e[j >> 1].y);
+                }
+                // columns j and j + 8, then + 4, + 2, + 1
+#pragma unroll
+                for (int j = 0; j < 4; ++j) e[j] = fadd2(e[j], e[j + 4]);
+                e[0] = fadd2(e[0], e[2]);
+                e[1] = fadd2(e[1], e[3]);
+                e[0] = fadd2(e[0], e[1]);
+                sum16[2 * q + g] = e[0].x + e[0].y;
+              }
+            }
+            // The weights wait in registers, so that the way of the tile before (its copies to CTA 1 and the report back, about
+            // 1500 cycles) is hidden by the exponentials of this one.
             // P buffer b of CTA 1 was last read by P.V of tile G-2
             if (G >= 2) mbar_wait(smem_u32(&m0->p_free[b]), ((G - 2) >> 1) & 1u, abort_flag);
             // the staging area is single: CTA 1 reports as soon as the copies of the tile before have landed
             if (G >= 1) mbar_wait(smem_u32(&m0->stage_free), (G - 1) & 1u, abort_flag);
-            float2 psum2 = make_float2(0.0f, 0.0f);
-            const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), neg_m2 = make_float2(-m_use, -m_use);
             // this thread's 64 columns are block `ch` of the P buffer: row rowi, eight 16-byte chunks
             const uint32_t p_row = p_local + ch * kQBlock + rowi * 128;
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              uint32_t pk[16];
-#pragma unroll
-              for (int j = 0; j < 32; j += 2) {
-                const float2 x = ffma2(__uint_as_float(sr[q][j]), __uint_as_float(sr[q][j + 1]), scale2, neg_m2);
-                const float2 e = make_float2(fast_exp2(x.x), fast_exp2(x.y));
-                psum2 = fadd2(psum2, e);
-                pk[j >> 1] = pack_bf16x2(e.x, e.y);
+            for (int c = 0; c < 8; ++c)
+              st_shared_v4(p_row + ((c ^ (rowi & 7)) << 4), pk[c >> 2][4 * (c & 3)], pk[c >> 2][4 * (c & 3) + 1], pk[c >> 2][4 * (c & 3) + 2], pk[c >> 2][4 * (c & 3) + 3]);
+            l01 = fadd2(l01, make_float2(sum16[0], sum16[1]));
+            l23 = fadd2(l23, make_float2(sum16[2], sum16[3]));
+            if (ch == 0) {
+              if (moves) {
+                l01 = fmul2(l01, alpha_b);
+                l23 = fmul2(l23, alpha_b);
               }
-#pragma unroll
-              for (int c = 0; c < 4; ++c) {
-                const int chunk = q * 4 + c;
-                st_shared_v4(p_row + ((chunk ^ (rowi & 7)) << 4), pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
-              }
+              m0->alpha_stage[rowi] = make_float2(alpha_a, alpha_b);
             }
-            l_run = l_run * alpha + (psum2.x + psum2.y);
-            if (ch == 0) m0->alpha_stage[rowi] = alpha;
             fence_proxy_async_smem();   // the bulk copies read this warp's rows through the async proxy
             __syncwarp();
             if (lane == 0) {
               // this warp's 32 rows of block ch are 4 KB in a row, here and in CTA 1; the warps of block 0 also
               // send the rescale factors of their 32 rows
               const uint32_t off = ch * kQBlock + lane_base * 128;
-              mbar_arrive_expect_tx_cluster(p_full_r[b], 32 * 128 + (ch == 0 ? 128 : 0));
+              mbar_arrive_expect_tx_cluster(p_full_r[b], 32 * 128 + (ch == 0 ? 256 : 0));
               bulk_copy_to_cluster(p_remote + b * kPBuf + off, p_local + off, 32 * 128, p_full_r[b]);
               if (ch == 0)
-                bulk_copy_to_cluster(alpha_remote + (b * 128 + lane_base) * 4, smem_u32(&m0->alpha_stage[lane_base]), 128, p_full_r[b]);
+                bulk_copy_to_cluster(alpha_remote + (b * 128 + lane_base) * 8, smem_u32(&m0->alpha_stage[lane_base]), 256, p_full_r[b]);
             }
           }
           gt += n_tiles;
           // end of the token: combine the two halves of every row sum; 1/l goes to CTA 1, LSE is written here
+          const float l_run = (l01.x + l01.y) + (l23.x + l23.y);
           named_bar_sync(2 + (warp & 3), 64);
           m0->xchg[0][tid] = l_run;
           named_bar_sync(2 + (warp & 3), 64);
@@ -714,10 +777,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
               const int b = G & 1;
               mbar_wait(smem_u32(&m1->p_full[b]), (G >> 1) & 1u, abort_flag);
               if (tid == 0) mbar_arrive_cluster_relaxed(stage_free_r);   // the copies have read CTA 0's staging area
-              const float a = m1->alpha[b][tid];
-              const bool need = (i > 0) && (a != 1.0f);
-              if (__any_sync(0xffffffffu, need)) {
-                mbar_wait(smem_u32(&m1->pv_done[(G - 1) & 1]), ((G - 1) >> 1) & 1u, abort_flag);
+              auto rescale = [&](float a) {
                 tc_fence_after();
 #pragma unroll 1
                 for (int c0 = 0; c0 < 512; c0 += 32) {
@@ -730,10 +790,25 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
                 }
                 tmem_wait_st();
                 tc_fence_before();
+              };
+              const float a = m1->alpha[b][tid].x, a_late = m1->alpha[b][tid].y;
+              if (__any_sync(0xffffffffu, (i > 0) && (a != 1.0f))) {
+                mbar_wait(smem_u32(&m1->pv_done[(G - 1) & 1]), ((G - 1) >> 1) & 1u, abort_flag);
+                rescale(a);
               }
+              // the second half of the tile may move a maximum once more: the issuer then stops between the halves
+              const bool late = __any_sync(0xffffffffu, a_late != 1.0f);
+              if (lane == 0) reinterpret_cast<uint8_t*>(&m1->late[b])[warp] = late ? 1 : 0;
               // P arrived through the async proxy (bulk copy), which is also how the MMA reads it: no proxy fence
               __syncwarp();
               if (lane == 0) mbar_arrive(smem_u32(&m1->corr_done[b]));
+              if (late) {
+                mbar_wait(smem_u32(&m1->half_done[warp]), n_late & 1u, abort_flag);
+                rescale(a_late);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&m1->half_corr[warp]));
+                ++n_late;
+              }
             }
           } else if (warp == 4 && lane == 0) {
             // ------------------------------------------------------------ relay: P buffer free -> CTA 0
@@ -774,6 +849,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
               const uint32_t ph = G & 1u;
               mbar_wait(smem_u32(&m1->corr_done[b]), (G >> 1) & 1u, abort_flag);
               tc_fence_after();
+              const uint32_t late = m1->late[b];
               const uint32_t a_lo = ad_lo + ((b * kPBuf) >> 4);
 #pragma unroll 1
               for (int sl = 0; sl < kNV; ++sl) {
@@ -793,8 +869,22 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
                                   kk == 0 ? static_cast<uint32_t>(i | sl) : 1u);
                   }
                   umma_commit(v_free0 + sl * 8);
+                  if (sl == 1 && late != 0u) {
+                    for (int w = 0; w < 4; ++w)
+                      if ((late >> (8 * w)) & 1u) umma_commit(smem_u32(&m1->half_done[w]));
+                  }
                 }
                 __syncwarp();
+                if (sl == 1 && late != 0u) {
+#pragma unroll 1
+                  for (int w = 0; w < 4; ++w) {
+                    if ((late >> (8 * w)) & 1u) {
+                      mbar_wait(smem_u32(&m1->half_corr[w]), (n_late >> w) & 1u, abort_flag);
+                      n_late ^= 1u << w;
+                    }
+                  }
+                  tc_fence_after();
+                }
               }
               if (elect_one()) umma_commit(smem_u32(&m1->pv_done[b]));
               __syncwarp();

@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 import functools
+import math
 from typing import Optional, Tuple
 
 import torch
@@ -55,12 +56,24 @@ def _pairs_of(index: int) -> int:
 @functools.lru_cache(maxsize=1024)
 def _plan_splits(s_q: int, h: int, topk: int, pairs: int) -> int:
     tiles = max(1, (topk + 127) // 128)
-    if s_q >= pairs:
-        return 1
 
-    def cost(n):
+    def pairs_cost(n):
         waves = -(-s_q * n // pairs)
         return 12.0 + waves * (2.0 + 2.2 * -(-tiles // n)) + (5.4 + 0.2 * s_q * n * h / 128 if n > 1 else 0.0)
+
+    # one CTA per item of up to 64 heads: the library takes that kernel for more heads while every CTA has one item of at most 16 tiles
+    groups, rows64 = -(-h // 64), max(1, (topk + 63) // 64)
+    start, per_tile = (6.0, 1.03) if h <= 16 else (8.0, 1.13) if h <= 32 else (8.6, 1.4)
+
+    def ctas_cost(n):
+        waves = -(-s_q * groups * n // (2 * pairs))
+        if h > 64 and (waves > 1 or rows64 > 16 * n):
+            return math.inf
+        return start + waves * (1.0 + per_tile * -(-rows64 // n)) + (1.0 + 0.35 * s_q * n * h / 1000 if n > 1 else 0.0)
+
+    def cost(n):
+        device = pairs_cost(n) if h > 64 and ctas_cost(n) == math.inf else ctas_cost(n)
+        return max(device, 21.5 if n > 1 else 16.0), device      # calls in a row take at least what the host needs: one launch, or two and a workspace
 
     return min(range(1, min(16, tiles) + 1), key=cost)
 
@@ -68,10 +81,12 @@ def _plan_splits(s_q: int, h: int, topk: int, pairs: int) -> int:
 def _auto_splits(s_q: int, h: int, topk: int, device) -> int:
     """Parts into which the top-k axis of every token is cut.
 
-    The persistent kernel runs one item (a token, or a part of one) at a time on each pair of SMs.  Measured on a B200
-    (us): 12 per launch, 2 per item and 2.2 per tile of 128 rows in it; with parts 5.4 for the merge and 0.2 per item of
-    128 heads for the fp32 partials.  topk 2048, 128 heads, whole / in parts: 1 token 49 / 23 (16 parts), 10 tokens 49 / 33 (4),
-    20 tokens 50 / 44 (3), 37 tokens 51 / 55 (2), 74 tokens 54 / 95; 1 token of topk 256: 18.6 / 22."""
+    The persistent kernels run one item (a token, or a part of one) at a time: up to 64 heads on an SM, more on a pair of SMs, or while
+    there are SMs for it as an item per 64 heads.  Measured on a B200 (device us, in a captured graph).  An SM: 7 per launch, 1 per item
+    and 1.03 per tile of 64 rows in it with 16 heads (9 and 1.4 with 64), with parts 1 for the merge and 0.35 per 1000 fp32 rows of 512; topk 2048,
+    16 heads, whole / in parts: 1 token 40 / 10.6 (16 parts), 16 tokens 40.5 / 13.3 (8), 74 tokens 41 / 26 (2), 148 tokens 42 / 45.  A pair: 12 per
+    launch, 2 per item, 2.2 per tile of 128 rows; with parts 5.4 and 0.2 per item.  The host takes 16 for a call with one launch and
+    21.5 for one in parts, so that lists which an SM is through with by then stay whole (1 token of topk 256: 16 against 22)."""
     return _plan_splits(s_q, h, topk, _pairs_of(device.index))
 
 

@@ -96,3 +96,27 @@ def test_more_than_32_heads_are_refused():
     idx = torch.zeros(1, 4, dtype=torch.int32, device=DEV)
     with pytest.raises((RuntimeError, ValueError)):
         sparse_mla_fwd(q, kv, idx, 0.1, algo=2)
+
+
+@pytest.mark.parametrize("h,s_q,topk", [(16, 160, 200), (32, 40, 1000), (64, 9, 64), (100, 5, 700), (128, 60, 130)])
+@pytest.mark.parametrize("steps", [False, True])
+def test_bits_of_a_head_do_not_depend_on_the_heads_of_the_call(h, s_q, topk, steps):
+    """The kernel for few heads, its groups of 64 and the pairs for many add in the same order: equal bits, also where maxima move in either
+    half of a tile of the pairs (`steps`), where whole tiles are masked, and for tokens that select nothing."""
+    g = torch.Generator().manual_seed(h + s_q + topk)
+    s_kv = 1500
+    q = torch.randn(s_q, h, 576, generator=g).bfloat16().to(DEV)
+    kv = torch.randn(s_kv, 576, generator=g)
+    if steps:
+        kv *= torch.linspace(0.1, 20.0, s_kv)[:, None]
+    kv = kv.bfloat16().to(DEV)
+    idx = torch.stack([torch.randperm(s_kv, generator=g)[:topk] for _ in range(s_q)]).int().sort(dim=1).values
+    idx[1, :] = -1
+    idx[2, :64] = -1
+    idx[3, 1::2] = -1
+    idx[4, 40:] = -1
+    idx = idx.to(DEV)
+    reps = 1 + (400 + s_q - 1) // s_q                       # so many tokens that all heads of a call with more than 64 go to the pairs
+    many, lse_many = sparse_mla_fwd(q.repeat(reps, 128 // h + 1, 1)[:, :128].contiguous(), kv, idx.repeat(reps, 1), 0.05, check=True, num_splits=1)
+    out, lse = sparse_mla_fwd(q, kv, idx, 0.05, check=True, num_splits=1)
+    assert torch.equal(out, many[:s_q, :h]) and torch.equal(lse, lse_many[:s_q, :h])

@@ -27,8 +27,11 @@ def _require_cuda(*tensors):
             raise ValueError("Pointer argument cannot be accessed from the device: expected CUDA tensors")
 
 
-# The handle of the current stream, without a Stream object around it where torch has the call.
+# The handle of the current stream and the current device, without a Stream object and the initialisation check around them where
+# torch has the calls.  (A call of a small shape is bound by the host: what a tensor is asked for costs 0.05 to 0.2 us each time, a tensor 1.5 to 2.4,
+# so the functions below ask for all strides at once and check no tensor that they made themselves.)
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
 
 
 def _stream_ptr(device) -> int:
@@ -39,11 +42,11 @@ def _stream_ptr(device) -> int:
 
 def _launch(fn, args, device, what: str) -> None:
     """fn(args, stream) on the current stream of `device`, with that device current."""
-    if device.index == torch.cuda.current_device():
-        rc = fn(C.byref(args), C.c_void_p(_stream_ptr(device)))
+    if device.index == _current_device():
+        rc = fn(C.byref(args), _stream_ptr(device))
     else:
         with torch.cuda.device(device):
-            rc = fn(C.byref(args), C.c_void_p(_stream_ptr(device)))
+            rc = fn(C.byref(args), _stream_ptr(device))
     if rc != 0:
         _lib.check(rc, what)
 
@@ -114,7 +117,7 @@ def _split_workspace(a, s_q: int, h: int, n_splits: int, device):
     if n_splits <= 1:
         a.workspace, a.workspace_bytes = None, 0
         return None
-    nbytes = int(_lib.load().ftb_sparse_mla_workspace_bytes(s_q, h, n_splits))
+    nbytes = s_q * n_splits * h * (D_V + 1) * 4              # ftb_sparse_mla_workspace_bytes()
     ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
     a.workspace, a.workspace_bytes = ws.data_ptr(), nbytes
     return ws
@@ -150,22 +153,28 @@ def sparse_mla_fwd(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor,
         assert kv.shape[1] == 1, "latent KV has a single shared head"
         kv = kv[:, 0, :]
     assert q.dim() == 3 and kv.dim() == 2 and indices.dim() == 2, "expected q[S_q,h,576], kv[S_kv,576], indices[S_q,topk]"
-    assert q.dtype == torch.bfloat16 and kv.dtype == torch.bfloat16, "q and kv must be bf16"
+    bf16, device = torch.bfloat16, q.device
+    assert q.dtype == bf16 and kv.dtype == bf16, "q and kv must be bf16"
     assert indices.dtype == torch.int32, "indices must be int32"
-    assert q.shape[2] == D_QK and kv.shape[1] == D_QK, "q/k head dim must be 576 (512 latent + 64 rope)"
+    (s_q, h, d_q), (s_kv, d_k), (s_i, topk) = q.shape, kv.shape, indices.shape
+    (q_st, q_sh, q_sd), (kv_sr, kv_sd), (i_st, i_sd) = q.stride(), kv.stride(), indices.stride()
+    assert d_q == D_QK and d_k == D_QK, "q/k head dim must be 576 (512 latent + 64 rope)"
     assert d_v == D_V, "v head dim must be 512"
-    assert indices.shape[0] == q.shape[0]
-    assert q.stride(2) == 1 and kv.stride(1) == 1 and indices.stride(1) == 1, "innermost dimension must be contiguous"
-    s_q, h, _ = q.shape
+    assert s_i == s_q
+    assert q_sd == 1 and kv_sd == 1 and i_sd == 1, "innermost dimension must be contiguous"
     if sm_scale is None:
         sm_scale = D_QK ** -0.5
     if out is None:
-        out = torch.empty(s_q, h, D_V, dtype=torch.bfloat16, device=q.device)
+        out = torch.empty(s_q, h, D_V, dtype=bf16, device=device)
+    else:
+        assert out.shape == (s_q, h, D_V) and out.dtype == bf16 and out.stride(2) == 1
     if lse is None:
-        lse = torch.empty(s_q, h, dtype=torch.float32, device=q.device)
-    assert out.shape == (s_q, h, D_V) and out.dtype == torch.bfloat16 and out.stride(2) == 1
-    assert lse.shape == (s_q, h) and lse.dtype == torch.float32 and lse.stride(1) == 1
-    status = torch.zeros(1, dtype=torch.int32, device=q.device) if check else None
+        lse = torch.empty(s_q, h, dtype=torch.float32, device=device)
+    else:
+        assert lse.shape == (s_q, h) and lse.dtype == torch.float32 and lse.stride(1) == 1
+    o_st, o_sh, _ = out.stride()
+    l_st = lse.stride(0)
+    status = torch.zeros(1, dtype=torch.int32, device=device) if check else None
     lib = _lib.load()
     for h0 in range(0, h, 128):      # more than 128 heads: one launch per block of 128 heads
         h1 = min(h, h0 + 128)
@@ -173,14 +182,15 @@ def sparse_mla_fwd(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor,
         n_splits = int(num_splits) if num_splits else 1
         algo_id = int(algo)
         if num_splits is None and algo == 0 and _dbg_scores is None:
-            n_splits, algo_id = _auto_splits(_plan_tokens or s_q, h1 - h0, indices.shape[1], q.device), 5
+            n_splits, algo_id = _auto_splits(_plan_tokens or s_q, h1 - h0, topk, device), 5
         a = _lib.SparseMlaArgs(
-            qs.data_ptr(), kv.data_ptr(), indices.data_ptr(), os_.data_ptr(), ls.data_ptr(), s_q, h1 - h0, kv.shape[0],
-            indices.shape[1], qs.stride(0), qs.stride(1), kv.stride(0), indices.stride(0), os_.stride(0), os_.stride(1),
-            ls.stride(0), float(sm_scale), int(lse_base2), algo_id, status.data_ptr() if status is not None else None)
-        a.dbg_scores = _dbg_scores.data_ptr() if _dbg_scores is not None else None
-        _ws = _split_workspace(a, s_q, h1 - h0, n_splits, q.device)
-        _launch(lib.ftb_sparse_mla_fwd, a, q.device, "sparse_mla_fwd")
+            qs.data_ptr(), kv.data_ptr(), indices.data_ptr(), os_.data_ptr(), ls.data_ptr(), s_q, h1 - h0, s_kv, topk,
+            q_st, q_sh, kv_sr, i_st, o_st, o_sh, l_st, float(sm_scale), int(lse_base2), algo_id,
+            status.data_ptr() if status is not None else None)
+        if _dbg_scores is not None:
+            a.dbg_scores = _dbg_scores.data_ptr()
+        _ws = _split_workspace(a, s_q, h1 - h0, n_splits, device)
+        _launch(lib.ftb_sparse_mla_fwd, a, device, "sparse_mla_fwd")
     _check_status(status, "sparse_mla_fwd")
     return out, lse
 
@@ -283,50 +293,64 @@ def sparse_mla_fwd_paged(q: torch.Tensor, kv_cache: torch.Tensor, kv_scale: torc
     """
     _require_cuda(q, kv_cache, kv_scale, block_table, context_lens, indices)
     assert q.dim() == 4 and indices.dim() == 3 and kv_cache.dim() == 3
-    assert q.dtype == torch.bfloat16
+    bf16, int32, device = torch.bfloat16, torch.int32, q.device
+    assert q.dtype == bf16
     assert kv_cache.dtype in (torch.uint8, torch.float8_e4m3fn), "kv_cache must hold e4m3 bytes"
-    assert kv_cache.shape[1] == page_size and kv_cache.shape[2] == D_QK and kv_cache.is_contiguous()
-    assert kv_scale.dtype == torch.float32 and kv_scale.numel() == kv_cache.shape[0] and kv_scale.is_contiguous()
-    assert block_table.dtype == torch.int32 and context_lens.dtype == torch.int32 and indices.dtype == torch.int32
-    assert block_table.stride(1) == 1 and context_lens.is_contiguous()
-    assert d_v == D_V and q.shape[3] == D_QK
-    b, n_q, h, _ = q.shape
+    num_pages, rows_per_page, d_k = kv_cache.shape
+    assert rows_per_page == page_size and d_k == D_QK and kv_cache.is_contiguous()
+    assert kv_scale.dtype == torch.float32 and kv_scale.numel() == num_pages and kv_scale.is_contiguous()
+    assert block_table.dtype == int32 and context_lens.dtype == int32 and indices.dtype == int32
+    bt_stride, bt_inner = block_table.stride()
+    assert bt_inner == 1 and context_lens.is_contiguous()
+    b, n_q, h, d_q = q.shape
+    i_b, i_q, topk = indices.shape
+    assert d_v == D_V and d_q == D_QK
     assert h <= 128, "at most 128 heads per call in the paged form"
-    assert indices.shape[:2] == (b, n_q) and block_table.shape[0] == b and context_lens.shape[0] == b
-    q2 = q.reshape(b * n_q, h, D_QK)
-    idx2 = indices.reshape(b * n_q, indices.shape[2])
-    assert q2.stride(2) == 1 and idx2.stride(1) == 1
+    assert i_b == b and i_q == n_q and block_table.shape[0] == b and context_lens.shape[0] == b
+    s_q = b * n_q
+    if q.is_contiguous():
+        q2, q_st, q_sh = q, h * D_QK, D_QK
+    else:
+        q2 = q.reshape(s_q, h, D_QK)
+        q_st, q_sh, q_sd = q2.stride()
+        assert q_sd == 1
+    if indices.is_contiguous():
+        idx2, i_st = indices, topk
+    else:
+        idx2 = indices.reshape(s_q, topk)
+        i_st, i_sd = idx2.stride()
+        assert i_sd == 1
     if sm_scale is None:
         sm_scale = D_QK ** -0.5
-    out = torch.empty(b * n_q, h, D_V, dtype=torch.bfloat16, device=q.device)
-    lse = torch.empty(b * n_q, h, dtype=torch.float32, device=q.device)
-    status = torch.zeros(1, dtype=torch.int32, device=q.device) if check else None
+    out = torch.empty(b, n_q, h, D_V, dtype=bf16, device=device)
+    lse = torch.empty(b, n_q, h, dtype=torch.float32, device=device)
+    status = torch.zeros(1, dtype=int32, device=device) if check else None
     a = _lib.SparseMlaArgs(
-        q2.data_ptr(), kv_cache.data_ptr(), idx2.data_ptr(), out.data_ptr(), lse.data_ptr(), b * n_q, h,
-        kv_cache.shape[0] * page_size, idx2.shape[1], q2.stride(0), q2.stride(1), D_QK, idx2.stride(0), out.stride(0), out.stride(1),
-        lse.stride(0), float(sm_scale), int(lse_base2), 0, status.data_ptr() if status is not None else None, 1, kv_scale.data_ptr(),
-        block_table.data_ptr(), context_lens.data_ptr(), page_size, n_q, block_table.stride(0))
+        q2.data_ptr(), kv_cache.data_ptr(), idx2.data_ptr(), out.data_ptr(), lse.data_ptr(), s_q, h,
+        num_pages * page_size, topk, q_st, q_sh, D_QK, i_st, h * D_V, D_V, h, float(sm_scale), int(lse_base2), 0,
+        status.data_ptr() if status is not None else None, 1, kv_scale.data_ptr(),
+        block_table.data_ptr(), context_lens.data_ptr(), page_size, n_q, bt_stride)
     lib = _lib.load()
     if num_splits is None:
-        n_splits, rows_first = _plan_paged(b * n_q, h, idx2.shape[1], _pairs_of(q.device.index))
+        n_splits, rows_first = _plan_paged(s_q, h, topk, _pairs_of(device.index))
     else:
         n_splits = max(1, int(num_splits))
         rows_first = n_splits == 1
     rows_bytes = 0
     if two_pass or (two_pass is None and rows_first):
-        rows_bytes = int(lib.ftb_sparse_mla_dequant_workspace_bytes(b * n_q, idx2.shape[1]))
+        rows_bytes = int(lib.ftb_sparse_mla_dequant_workspace_bytes(s_q, topk))
     if 0 < rows_bytes and (two_pass or rows_bytes <= (4 << 30)):
         # the dequantised rows, then (from a 16-byte boundary) the partial results of a split
         need = rows_bytes
         if n_splits > 1:
-            need = (rows_bytes + 15) // 16 * 16 + int(lib.ftb_sparse_mla_workspace_bytes(b * n_q, h, n_splits))
-        _ws = torch.empty(need, dtype=torch.uint8, device=q.device)
+            need = (rows_bytes + 15) // 16 * 16 + int(lib.ftb_sparse_mla_workspace_bytes(s_q, h, n_splits))
+        _ws = torch.empty(need, dtype=torch.uint8, device=device)
         a.n_splits, a.workspace, a.workspace_bytes, a.algo_id = n_splits, _ws.data_ptr(), need, 6
     else:
-        _ws = _split_workspace(a, b * n_q, h, n_splits, q.device)
-    _launch(_lib.load().ftb_sparse_mla_fwd, a, q.device, "sparse_mla_fwd_paged")
+        _ws = _split_workspace(a, s_q, h, n_splits, device)
+    _launch(lib.ftb_sparse_mla_fwd, a, device, "sparse_mla_fwd_paged")
     _check_status(status, "sparse_mla_fwd_paged")
-    return out.view(b, n_q, h, D_V), lse.view(b, n_q, h)
+    return out, lse
 
 
 def decode_attention_fwd(q, k_buffer, v_buffer, o, req_to_token, b_seq_len, attn_logits=None,
@@ -368,21 +392,24 @@ def sparse_mla_merge(part_out: torch.Tensor, part_lse: torch.Tensor, *, lse_base
     `sparse_mla_fwd` with `shard_indices(indices, lo, hi)`, the parts are all-gathered, this merges them."""
     _require_cuda(part_out, part_lse)
     assert part_out.dim() == 4 and part_lse.dim() == 3 and part_out.shape[3] == D_V
-    assert part_out.dtype in (torch.bfloat16, torch.float32) and part_lse.dtype == torch.float32
+    is_fp32, device = part_out.dtype == torch.float32, part_out.device
+    assert (is_fp32 or part_out.dtype == torch.bfloat16) and part_lse.dtype == torch.float32
     n_parts, s_q, h, _ = part_out.shape
     assert part_lse.shape == (n_parts, s_q, h)
-    assert part_out.stride(3) == 1 and part_lse.stride(2) == 1, "innermost dimension must be contiguous"
+    (p_sp, p_st, p_sh, p_sd), (l_sp, l_st, l_sd) = part_out.stride(), part_lse.stride()
+    assert p_sd == 1 and l_sd == 1, "innermost dimension must be contiguous"
     if out is None:
-        out = torch.empty(s_q, h, D_V, dtype=torch.bfloat16, device=part_out.device)
+        out = torch.empty(s_q, h, D_V, dtype=torch.bfloat16, device=device)
+    else:
+        assert out.shape == (s_q, h, D_V) and out.dtype == torch.bfloat16 and out.stride(2) == 1
     if lse is None:
-        lse = torch.empty(s_q, h, dtype=torch.float32, device=part_out.device)
-    assert out.shape == (s_q, h, D_V) and out.dtype == torch.bfloat16 and out.stride(2) == 1
-    assert lse.shape == (s_q, h) and lse.dtype == torch.float32 and lse.stride(1) == 1
-    a = _lib.SparseMlaMergeArgs(
-        part_out.data_ptr(), part_lse.data_ptr(), out.data_ptr(), lse.data_ptr(), s_q, h, n_parts,
-        int(part_out.dtype == torch.float32), int(lse_base2), part_out.stride(0), part_out.stride(1), part_out.stride(2),
-        part_lse.stride(0), part_lse.stride(1), out.stride(0), out.stride(1), lse.stride(0))
-    _launch(_lib.load().ftb_sparse_mla_merge, a, part_out.device, "sparse_mla_merge")
+        lse = torch.empty(s_q, h, dtype=torch.float32, device=device)
+    else:
+        assert lse.shape == (s_q, h) and lse.dtype == torch.float32 and lse.stride(1) == 1
+    o_st, o_sh, _ = out.stride()
+    a = _lib.SparseMlaMergeArgs(part_out.data_ptr(), part_lse.data_ptr(), out.data_ptr(), lse.data_ptr(), s_q, h, n_parts, int(is_fp32),
+                                int(lse_base2), p_sp, p_st, p_sh, l_sp, l_st, o_st, o_sh, lse.stride(0))
+    _launch(_lib.load().ftb_sparse_mla_merge, a, device, "sparse_mla_merge")
     return out, lse
 
 
@@ -401,16 +428,20 @@ def topk_indices(scores: torch.Tensor, topk: int, lengths: Optional[torch.Tensor
     +inf, ties to the lower position.  The reference builds index lists for its block-sparse ops on the device
     in the same spirit (python/triton/ops/blocksparse/matmul.py:117-127)."""
     _require_cuda(scores, lengths)
-    assert scores.dim() == 2 and scores.dtype == torch.float32 and scores.stride(1) == 1
-    s_q, s_kv = scores.shape
+    assert scores.dim() == 2 and scores.dtype == torch.float32
+    (s_q, s_kv), (sc_stride, sc_inner), device = scores.shape, scores.stride(), scores.device
+    assert sc_inner == 1
     if lengths is not None:
         assert lengths.dtype == torch.int32 and lengths.shape == (s_q,) and lengths.is_contiguous()
     if out is None:
-        out = torch.empty(s_q, topk, dtype=torch.int32, device=scores.device)
-    assert out.shape == (s_q, topk) and out.dtype == torch.int32 and out.stride(1) == 1
+        out = torch.empty(s_q, topk, dtype=torch.int32, device=device)
+        out_stride = topk
+    else:
+        assert out.shape == (s_q, topk) and out.dtype == torch.int32 and out.stride(1) == 1
+        out_stride = out.stride(0)
     a = _lib.TopkArgs(scores.data_ptr(), lengths.data_ptr() if lengths is not None else None, out.data_ptr(), s_q, s_kv,
-                      int(topk), scores.stride(0), out.stride(0))
-    _launch(_lib.load().ftb_topk_indices, a, scores.device, "topk_indices")
+                      int(topk), sc_stride, out_stride)
+    _launch(_lib.load().ftb_topk_indices, a, device, "topk_indices")
     return out
 
 
@@ -426,19 +457,20 @@ def kv_cache_write_fp8(rows: torch.Tensor, slot_mapping: torch.Tensor, kv_cache:
     a page that holds nothing yet.  A page's scale only grows: max(old, max|new rows| / 448); when it grows for
     a page that already held rows, those bytes are requantised to the new scale first."""
     _require_cuda(rows, slot_mapping, kv_cache, kv_scale)
-    assert rows.dim() == 2 and rows.shape[1] == D_QK and rows.dtype == torch.bfloat16 and rows.stride(1) == 1
-    assert slot_mapping.dtype == torch.int32 and slot_mapping.shape == (rows.shape[0],) and slot_mapping.is_contiguous()
+    assert rows.dim() == 2 and rows.dtype == torch.bfloat16 and kv_cache.dim() == 3
+    (n, d), (row_stride, row_inner), device = rows.shape, rows.stride(), rows.device
+    assert d == D_QK and row_inner == 1
+    assert slot_mapping.dtype == torch.int32 and slot_mapping.shape == (n,) and slot_mapping.is_contiguous()
+    num_pages, rows_per_page, d = kv_cache.shape
     assert kv_cache.dtype in (torch.uint8, torch.float8_e4m3fn) and kv_cache.is_contiguous()
-    assert kv_cache.dim() == 3 and kv_cache.shape[1] == page_size and kv_cache.shape[2] == D_QK
-    assert kv_scale.dtype == torch.float32 and kv_scale.shape == (kv_cache.shape[0],) and kv_scale.is_contiguous()
-    lib = _lib.load()
-    num_pages = kv_cache.shape[0]
-    ws = torch.empty(int(lib.ftb_kv_cache_write_workspace_bytes(num_pages)), dtype=torch.uint8, device=rows.device)
-    status = torch.zeros(1, dtype=torch.int32, device=rows.device) if check else None
-    a = _lib.KvCacheWriteArgs(rows.data_ptr(), slot_mapping.data_ptr(), kv_cache.data_ptr(), kv_scale.data_ptr(), rows.shape[0],
-                              num_pages, page_size, rows.stride(0), ws.data_ptr(), ws.numel(),
-                              status.data_ptr() if status is not None else None)
-    _launch(lib.ftb_kv_cache_write_fp8, a, rows.device, "kv_cache_write_fp8")
+    assert rows_per_page == page_size and d == D_QK
+    assert kv_scale.dtype == torch.float32 and kv_scale.shape == (num_pages,) and kv_scale.is_contiguous()
+    ws_bytes = 4 * num_pages                                 # ftb_kv_cache_write_workspace_bytes()
+    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=device)
+    status = torch.zeros(1, dtype=torch.int32, device=device) if check else None
+    a = _lib.KvCacheWriteArgs(rows.data_ptr(), slot_mapping.data_ptr(), kv_cache.data_ptr(), kv_scale.data_ptr(), n,
+                              num_pages, page_size, row_stride, ws.data_ptr(), ws_bytes, status.data_ptr() if status is not None else None)
+    _launch(_lib.load().ftb_kv_cache_write_fp8, a, device, "kv_cache_write_fp8")
     _check_status(status, "kv_cache_write_fp8")
 
 
@@ -451,23 +483,23 @@ def matmul(a: torch.Tensor, b: torch.Tensor, acc_dtype=None, input_precision=Non
     Products with few tiles add up K in up to four parts, so the bits of a row may depend on the number of rows; with
     `whole_k` they do not."""
     _require_cuda(a, b)
-    if a.stride(0) > 1 and a.stride(1) > 1:
-        a = a.contiguous()
-    if b.stride(0) > 1 and b.stride(1) > 1:
-        b = b.contiguous()
-    assert a.shape[1] == b.shape[0], "incompatible dimensions"
+    (a_s0, a_s1), (b_s0, b_s1), (m, k), (k_b, n) = a.stride(), b.stride(), a.shape, b.shape
+    assert k == k_b, "incompatible dimensions"
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16, "bf16 operands only"
     assert acc_dtype in (None, torch.float32), "bf16 inputs accumulate in fp32"
     assert output_dtype in (None, torch.bfloat16)
-    if a.stride(1) != 1:
-        a = a.contiguous()
-    if b.stride(1) != 1:
-        b = b.contiguous()
-    m, k = a.shape
-    n = b.shape[1]
+    if a_s1 != 1:
+        a, a_s0 = a.contiguous(), k
+    if b_s1 != 1:
+        b, b_s0 = b.contiguous(), n
+    device = a.device
     if out is None:
-        out = torch.empty(m, n, dtype=torch.bfloat16, device=a.device)
-    _gemm_into(a, b, out, whole_k=whole_k)
+        out, c_s0 = torch.empty(m, n, dtype=torch.bfloat16, device=device), n
+    else:
+        c_s0 = out.stride(0)
+    g = _lib.GemmArgs(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, a_s0, b_s0, c_s0, None)
+    lib = _lib.load()
+    _launch(lib.ftb_gemm_bf16_whole_k if whole_k else lib.ftb_gemm_bf16, g, device, "matmul")
     return out
 
 
@@ -488,22 +520,21 @@ def matmul_fp8_blockscaled(a: torch.Tensor, a_scale: torch.Tensor, b: torch.Tens
     _require_cuda(a, a_scale, b, b_scale)
     for t in (a, b):
         assert t.dtype in (torch.uint8, torch.float8_e4m3fn), "operands must hold e4m3 bytes"
-    assert a.shape[1] == b.shape[0], "incompatible dimensions"
-    m, k = a.shape
-    n = b.shape[1]
+    (m, k), (k_b, n), (a_s0, a_s1), (b_s0, b_s1) = a.shape, b.shape, a.stride(), b.stride()
+    (as_st, as_inner), (bs_st, bs_inner) = a_scale.stride(), b_scale.stride()
+    assert k == k_b, "incompatible dimensions"
     assert k % 128 == 0 and n % 128 == 0, "k and n must be multiples of the 128-wide scale blocks"
     assert a_scale.shape == (m, k // 128) and b_scale.shape == (k // 128, n // 128)
     assert a_scale.dtype == torch.float32 and b_scale.dtype == torch.float32
-    assert a.stride(1) == 1 and a_scale.stride(1) == 1 and b_scale.stride(1) == 1
+    assert a_s1 == 1 and as_inner == 1 and bs_inner == 1
     # b may be a [K, N] row-major matrix or the transposed view `w.t()` of a weight kept as [N, K] (K contiguous),
     # which the tensor cores read as the K-major operand
-    b_kmajor = b.stride(1) != 1
-    assert b.stride(1) == 1 or b.stride(0) == 1, "b must be contiguous along N or along K"
+    b_kmajor = b_s1 != 1
+    assert b_s1 == 1 or b_s0 == 1, "b must be contiguous along N or along K"
     if out is None:
         out = torch.empty(m, n, dtype=torch.bfloat16, device=a.device)
     g = _lib.GemmFp8Args(a.data_ptr(), b.data_ptr(), out.data_ptr(), a_scale.data_ptr(), b_scale.data_ptr(), m, n, k,
-                         a.stride(0), b.stride(1) if b_kmajor else b.stride(0), out.stride(0), a_scale.stride(0),
-                         b_scale.stride(0), None, 1 if b_kmajor else 0)
+                         a_s0, b_s1 if b_kmajor else b_s0, out.stride(0), as_st, bs_st, None, 1 if b_kmajor else 0)
     lib = _lib.load()
     _launch(lib.ftb_gemm_fp8_blockscaled_whole_k if whole_k else lib.ftb_gemm_fp8_blockscaled, g, a.device, "matmul_fp8_blockscaled")
     return out

@@ -632,7 +632,7 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
     return FTB_ERR_INVALID;
   }
   // algo 0 = default = 5: the persistent kernels (launch_persistent above), whole tokens or parts of them; algo 1 = one CTA per
-  // (token, output half), which is also the kernel of the FP8 paged form without a workspace and of the diagnostic score tap;
+  // (token, output half), which is also the kernel of the diagnostic score tap;
   // algo 6 = paged FP8 form: dequantise the selected rows, then the persistent kernels; algo 2 = the kernel for few heads (h <= 32) with the
   // true maximum as the reference of the weights.
   if (a->algo_id != 0 && a->algo_id != 1 && a->algo_id != 2 && a->algo_id != 5 && a->algo_id != 6) {
@@ -675,9 +675,9 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
     const int tiles = (a->topk + tile - 1) / tile;
     return n_splits < tiles ? n_splits : tiles > 1 ? tiles : 1;
   };
-  // Paged FP8 form with a workspace for the dequantised rows (algo 6, or algo 0 without a split): convert the selected
-  // rows once, then run the persistent bf16 kernel on the compact table.  Without such a workspace the
-  // one-pass kernel below converts while it gathers.
+  // Paged FP8 form: by default (algo 0 with the true maximum, algo 5 with the lazy one) the kernel for few heads converts the rows while it
+  // gathers them, 64 heads at a time; with algo 6 and a workspace for them the selected rows are converted once, and the
+  // persistent kernels run on the compact table (128 tokens of 128 heads, topk 2048: @F1@); algo 1 is the one-CTA kernel.
   const int64_t split_bytes = ftb_sparse_mla_workspace_bytes(a->s_q, a->h, n_splits);
   auto merge = [&]() {
     const auto kern = n_splits <= 2 ? sparse_mla_merge_kernel<2> : n_splits <= 4 ? sparse_mla_merge_kernel<4>
@@ -689,17 +689,16 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
   // With a split, algo 6 wants room for both: the dequantised rows, then the partial results (from a 16-byte boundary).
   const int64_t rows_bytes = (ftb_sparse_mla_dequant_workspace_bytes(a->s_q, a->topk) + 15) / 16 * 16;
   if (a->kv_is_fp8 && a->dbg_scores == nullptr &&
-      (n_splits == 1 ? (a->algo_id == 0 || a->algo_id == 6)
-                     : (a->algo_id == 6 && a->workspace_bytes >= rows_bytes + split_bytes))) {
+      a->algo_id == 6 && (n_splits == 1 || a->workspace_bytes >= rows_bytes + split_bytes)) {
     const int64_t need = ftb_sparse_mla_dequant_workspace_bytes(a->s_q, a->topk);
     const bool have = a->workspace != nullptr && a->workspace_bytes >= need && need > 0 &&
                       (reinterpret_cast<uintptr_t>(a->workspace) & 15u) == 0 &&
                       static_cast<long long>(a->s_q) * a->topk < (1LL << 31);
-    if (a->algo_id == 6 && !have) {
+    if (!have) {
       set_last_error("ftb_sparse_mla_fwd: algo 6 needs a 16-byte aligned workspace of ftb_sparse_mla_dequant_workspace_bytes() bytes");
       return FTB_ERR_INVALID;
     }
-    if (have) {
+    {
       p.topk = a->topk;
       __nv_bfloat16* table = reinterpret_cast<__nv_bfloat16*>(a->workspace);
       int32_t* idx2 = reinterpret_cast<int32_t*>(reinterpret_cast<uint8_t*>(a->workspace) +
@@ -745,6 +744,12 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
   // parts of 128 heads, 32 tokens of topk 256 23 / 36, of 512 31 / 38, of 1024 48 / 34, of 2048 80 / 43; 148 tokens of topk 512 in four parts
   // 167 / 142; 16 heads, 148 tokens of topk 512 in two parts 88 / 44.
   const bool pairs = a->algo_id == 5 || (a->algo_id == 0 && (a->topk > 512 || (n_splits * 128 <= a->topk && (a->h <= 32 || (a->topk > 256 && a->s_q >= 64)))));
+  if (a->kv_is_fp8 && a->dbg_scores == nullptr && a->algo_id != 1 && n_splits <= 64) {
+    n_splits = parts_of(128);
+    if (n_splits > 1) p.part_lse = p.part_out + static_cast<size_t>(a->s_q) * n_splits * a->h * 512;
+    const int rc0 = launch_sparse_mla_few(a, n_splits, p.part_out, p.part_lse, a->algo_id == 5 ? 8.0f : 0.0f, st);
+    return rc0 != FTB_OK || n_splits == 1 ? rc0 : merge();
+  }
   if (n_splits > 1 && n_splits <= 64 && !a->kv_is_fp8 && a->dbg_scores == nullptr && pairs) {
     n_splits = parts_of(128);
     p.part_lse = p.part_out + static_cast<size_t>(a->s_q) * n_splits * a->h * 512;

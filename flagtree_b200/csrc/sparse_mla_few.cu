@@ -29,6 +29,8 @@
 // moved to the gather warps 741 / 920, two issuers 512 / 719, the first reference from two tiles 525 / 759.  Device time of few tokens in parts,
 // pairs / here: 1 token of 16 heads 17.0 / 11.3, 74 tokens of 64 heads 45.6 / 40.0, 1 token of 128 heads 21.2 / 14.7, 16 of them 29.9 / 25.5.
 // Every wait is bounded; a wait that runs out sets the abort flag, after which every later wait returns at once.
+#include <cuda_fp8.h>
+
 #include <cstring>
 
 #include "sm100.cuh"
@@ -52,16 +54,21 @@ constexpr int kGather = 4;                     // gather warps, 16 rows of a til
 constexpr int kThirds = 3;                    // a tile's columns arrive, and are multiplied, in three parts
 constexpr int kBatch = 64;                     // items per CTA and launch
 
-template <int NH>
+template <int NH, bool kFp8>
 struct Shape {
   static constexpr int kGroups = NH == 64 ? 2 : 1;              // softmax groups of four warps
   static constexpr int kHeads = NH / kGroups;                   // heads per group
-  // warps: softmax, the MMA issuers (four apart: one scheduler), gather (on schedulers that the issuers are not on).  A set of gather warps waits for its copies to land;
-  // with two sets every slot has one of its own.  (64 heads: two sets would leave the softmax too few registers.)
+  // Warps: softmax, the MMA issuers, gather.  bf16 rows: four gather warps on schedulers that the issuers (four apart: one scheduler) are not
+  // on; they wait for their copies to land, and with two sets of them every slot has one of its own (64 heads: two sets would leave the
+  // softmax too few registers).  e4m3 rows: the issuers in a warpgroup of their own, then eight warps that convert; with 64 heads registers
+  // move to the softmax: 640 x 96 at launch = 61440 >= 8 x 32 x 128 + 4 x 32 x 56 + 8 x 32 x 80 = 60416.
   static constexpr int kSets = kGroups == 2 ? 1 : 2;
-  static constexpr int kIssuer = 4 * kGroups;
-  static constexpr int kThreads = (kIssuer + (kSets == 2 ? 11 : 6)) * 32;
+  static constexpr int kIssuer = 4 * kGroups, kValueIssuer = kIssuer + (kFp8 ? 1 : 4), kConvert0 = kIssuer + 4, kConverts = 8;
+  static constexpr int kThreads = (kFp8 ? kConvert0 + kConverts : kIssuer + (kSets == 2 ? 11 : 6)) * 32;
+  static constexpr bool kSplitRegs = kFp8 && kGroups == 2;
+  static constexpr int kRegsSoftmax = 128, kRegsIssue = 56, kRegsConvert = 80;
   __device__ static int producer(int warp) {
+    if (kFp8) return warp - kConvert0;
     const int w = warp - kIssuer;
     return w >= 1 && (w & 3) != 0 ? w - 1 - (w >> 2) : -1;
   }
@@ -73,7 +80,7 @@ struct Shape {
 };
 
 struct Params {
-  const __nv_bfloat16* kv;
+  const void* kv;      // bf16 rows, or e4m3 pages
   long long kv_sr;
   const int32_t* indices;
   __nv_bfloat16* out;
@@ -87,6 +94,12 @@ struct Params {
   float* part_out;     // [s_q, n_splits, h, 512] fp32
   float* part_lse;     // [s_q, n_splits, h], base 2
   float max_slack;     // how far (log2) the reference may lag behind the running maximum
+  // e4m3 pages
+  const float* kv_scale;
+  const int32_t* block_table;
+  const int32_t* context_lens;
+  int page_size, q_per_seq;
+  long long bt_stride;
 };
 
 struct Misc {
@@ -99,7 +112,7 @@ struct Misc {
   uint32_t tmem_base;
   int abort_flag;
   int bad_index;
-  uint32_t valid_mask[kSlots][kGather];  // 16 rows each
+  alignas(16) uint16_t valid_mask[kSlots][4];   // 16 rows each
   unsigned short nt[2 * kBatch];       // per item: number of tiles, first tile
   int last[kBatch];                    // entries of its list up to the last that is not negative
   alignas(16) float neg_ref[64];       // minus the reference of a head (log2), 0 where it has none yet
@@ -182,10 +195,10 @@ __device__ __noinline__ int first_row(const int32_t* idx_row, int n_rows, int s_
   return none;
 }
 
-template <int NH>
-__global__ void __launch_bounds__(Shape<NH>::kThreads, 1)
+template <int NH, bool kFp8>
+__global__ void __launch_bounds__(Shape<NH, kFp8>::kThreads, 1)
 sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Params p) {
-  using Sh = Shape<NH>;
+  using Sh = Shape<NH, kFp8>;
   constexpr int kHeads = Sh::kHeads;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -201,7 +214,7 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
     misc->abort_flag = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
     misc->bad_index = 0;
     for (int i = 0; i < kSlots; ++i) {
-      for (int j = 0; j < kThirds; ++j) mbar_init(smem_u32(&misc->k_full[i][j]), kGather);
+      for (int j = 0; j < kThirds; ++j) mbar_init(smem_u32(&misc->k_full[i][j]), kFp8 ? Sh::kConverts : kGather);
       for (int j = 0; j < kGather; ++j) mbar_init(smem_u32(&misc->k_free[i][j]), 1);
       mbar_init(smem_u32(&misc->s_full[i]), 1);
       mbar_init(smem_u32(&misc->p_full[i]), 4 * Sh::kGroups);
@@ -264,7 +277,7 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
   const int prod = Sh::producer(warp);
   const int group = warp < 4 ? 0 : warp < 4 * Sh::kGroups ? 1 : -1;
 
-  if (group >= 0) {
+  auto softmax = [&]() {
     // ------------------------------------------------------------------ softmax and epilogue
     const int q4 = warp & 3, pw = group * 4 + q4, h0 = group * kHeads;
     const bool active = lane < 16;                         // the lanes that hold a key
@@ -290,7 +303,7 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
         const uint32_t s = G & 1u, ph = (G >> 1) & 1u;
         mbar_wait(smem_u32(&misc->s_full[s]), ph, abort_flag);
         tc_fence_after();
-        const bool valid = active && ((misc->valid_mask[s][q4] >> lane) & 1u) != 0u;
+        const bool valid = active && ((static_cast<uint32_t>(misc->valid_mask[s][q4]) >> lane) & 1u) != 0u;
         const uint32_t t_s = tmem_addr(tmem, q4 * 32, Sh::kColS + s * NH + h0);
         uint32_t sr[kHeads];
         tmem_ld(t_s, sr);
@@ -327,7 +340,7 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
             // the first reference is the maximum of two tiles (the tile of the kernel for many heads)
             mbar_wait(smem_u32(&misc->s_full[s ^ 1u]), ((G + 1) >> 1) & 1u, abort_flag);
             tc_fence_after();
-            const bool valid1 = active && ((misc->valid_mask[s ^ 1u][q4] >> lane) & 1u) != 0u;
+            const bool valid1 = active && ((static_cast<uint32_t>(misc->valid_mask[s ^ 1u][q4]) >> lane) & 1u) != 0u;
             uint32_t sr1[kHeads];
             tmem_ld(tmem_addr(tmem, q4 * 32, Sh::kColS + (s ^ 1u) * NH + h0), sr1);
             tmem_wait_ld();
@@ -469,7 +482,8 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
         }
       }
     }
-  } else if (warp == Sh::kIssuer) {
+  };
+  auto scores = [&]() {
     // ------------------------------------------------------------------ S^T = K . Q^T (whole warp, an elected lane issues)
     // (no proxy fence between a wait and its MMAs, where it would cost 300 cycles: those who wrote the operands have executed it)
     constexpr uint32_t kIdesc = umma_idesc(kFmtBF16, kNT, NH, 0, 0);     // A = K rows (K-major), B = Q (K-major)
@@ -509,7 +523,8 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
         }
       }
     }
-  } else if (warp == Sh::kIssuer + 4) {
+  };
+  auto values = [&]() {
     // ------------------------------------------------------------------ O^T += V^T . P^T: a warp of its own, so that the one product's
     // waits do not hold up the other (the tensor pipe takes four MMAs ahead, less than a wait takes)
     constexpr uint32_t kIdesc = umma_idesc(kFmtBF16, 128, NH, 1, 1);     // A = V^T (MN-major), B = P^T (MN-major)
@@ -539,11 +554,26 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
         __syncwarp();
       }
     }
-  } else if (prod >= 0) {
+  };
+  auto load_q = [&](int t) {                               // Q of an item, when the scores of the item before are through; a whole warp
+    const int item = first_item + t * n_ctas, next = item + n_ctas, tok_next = token_of(next);
+    const uint32_t full = smem_u32(&misc->q_full);
+    if (t >= 1) mbar_wait(smem_u32(&misc->q_free), (t - 1) & 1u, abort_flag);
+    if (lane == 0) mbar_arrive_expect_tx(full, static_cast<uint32_t>(min(p.h, NH) * 128 * kNChunk));   // rows past the last head arrive as zeros
+    __syncwarp();
+    if (lane < kNChunk) {
+      tma_load_3d(q_s + lane * Sh::kQBlock, &tm_q, full, lane * 64, (item / p.n_splits) % p.n_groups * NH, token_of(item));
+      if (tok_next < p.s_q)
+        asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
+                     ::"l"(&tm_q), "r"(lane * 64), "r"((next / p.n_splits) % p.n_groups * NH), "r"(tok_next) : "memory");
+    }
+    __syncwarp();
+  };
+  auto gather = [&]() {
     // ------------------------------------------------------------------ gather: rows 16 prod .. 16 prod + 15 of every tile
     // 36 copies of 16 bytes per lane: lane l copies piece l % 8 of every 64-column block of rows 4 j + l / 8
     const int w = prod & 3, set = prod >> 2;               // set: of the tiles with this remainder modulo kSets
-    const __nv_bfloat16* src0 = p.kv + (lane & 7) * 8;
+    const __nv_bfloat16* src0 = static_cast<const __nv_bfloat16*>(p.kv) + (lane & 7) * 8;
     uint32_t dst0[2];                                      // of rows 0..3 and 4..7 (the 128-byte swizzle goes with row % 8)
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
@@ -556,21 +586,7 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
       const int tok = token_of(first_item + t * n_ctas);
       const int n_tiles = warp_uniform(misc->nt[t]), row0 = warp_uniform(misc->nt[kBatch + t]) * kNT, n_rows = p.topk - row0;
       const int32_t* idx_row = p.indices + static_cast<long long>(tok) * p.idx_st + row0;
-      if (prod == 0) {
-        // this warp loads Q as well, when the scores of the item before are through
-        const int item = first_item + t * n_ctas, next = item + n_ctas, tok_next = token_of(next);
-        const uint32_t full = smem_u32(&misc->q_full);
-        if (t >= 1) mbar_wait(smem_u32(&misc->q_free), (t - 1) & 1u, abort_flag);
-        if (lane == 0) mbar_arrive_expect_tx(full, static_cast<uint32_t>(min(p.h, NH) * 128 * kNChunk));   // rows past the last head arrive as zeros
-        __syncwarp();
-        if (lane < kNChunk) {
-          tma_load_3d(q_s + lane * Sh::kQBlock, &tm_q, full, lane * 64, (item / p.n_splits) % p.n_groups * NH, tok);
-          if (tok_next < p.s_q)
-            asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
-                         ::"l"(&tm_q), "r"(lane * 64), "r"((next / p.n_splits) % p.n_groups * NH), "r"(tok_next) : "memory");
-        }
-        __syncwarp();
-      }
+      if (prod == 0) load_q(t);                            // this warp loads Q as well
       const int i0 = static_cast<int>((set - G0) & (Sh::kSets - 1u));
       int j0 = i0 * kNT + 16 * w + (lane & 15);            // (both halves of the warp hold the same 16 rows)
       int nxt = i0 < n_tiles && j0 < n_rows ? idx_row[j0] : -1;
@@ -593,7 +609,7 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
         for (int q = 0; q < 4; ++q) src[q] = src0 + static_cast<long long>(__shfl_sync(0xffffffffu, row, 4 * q + (lane >> 3))) * p.kv_sr;
         if (G >= kSlots) mbar_wait(smem_u32(&misc->k_free[s][w]), ((G >> 1) - 1) & 1u, abort_flag);
         __syncwarp();
-        if (lane == 0) misc->valid_mask[s][w] = mask;      // (released by the arrivals below)
+        if (lane == 0) misc->valid_mask[s][w] = static_cast<uint16_t>(mask);   // (released by the arrivals below)
 #pragma unroll
         for (int j = 0; j < kThirds; ++j) {
 #pragma unroll
@@ -615,6 +631,125 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
       }
       G0 += n_tiles;
     }
+  };
+  auto convert = [&]() {
+    // ------------------------------------------------------------------ gather of e4m3 rows: rows 8 w .. 8 w + 7 of every tile, four lanes to a row
+    // The 576 bytes of a row are nine pieces of 16 bytes per lane, in registers a tile ahead: the page of the tile after that and the
+    // list entry of the next one are on their way too, so that no load is waited for.  A piece becomes 16 values times the scale of
+    // their page, rounded to bf16.  Rows that are masked are zeros.
+    const int w = prod, r = 8 * w + (lane >> 2), c4 = lane & 3;
+    const uint32_t dst0 = base + r * 128 + (((2 * c4) ^ (r & 7)) << 4), dst1 = base + r * 128 + (((2 * c4 + 1) ^ (r & 7)) << 4);
+    const uint8_t* cache = static_cast<const uint8_t*>(p.kv) + c4 * 16;
+    // where the list entries stand: item, tile within it
+    int ct = -1, ci = 0, cn = 0, c_left = 0, c_seq = 0, c_ctx = 0;
+    const int32_t* c_idx = nullptr;
+    int logical = -1, l_seq = 0, l_ctx = 0;                // of the tile after the next
+    int page = -1, in_page = 0;                            // of the next tile: -1 for no row, -2 for an entry of no meaning
+    uint4 raw[9];                                          // of this tile
+    float scale = 0.0f;
+    bool ok = false;
+    auto next_entry = [&]() {
+      if (ci == cn && ct < nb) {
+        ci = cn = 0;
+        if (++ct < nb) {
+          const int tok = token_of(first_item + ct * n_ctas), row0 = misc->nt[kBatch + ct] * kNT;
+          cn = misc->nt[ct];
+          c_left = p.topk - row0 - r;
+          c_idx = p.indices + static_cast<long long>(tok) * p.idx_st + row0 + r;
+          c_seq = tok / p.q_per_seq;
+          c_ctx = p.context_lens[c_seq];
+        }
+      }
+      logical = ct < nb && ci * kNT < c_left ? c_idx[ci * kNT] : -1;
+      l_seq = c_seq;
+      l_ctx = c_ctx;
+      ++ci;
+    };
+    auto next_page = [&]() {
+      page = logical < -1 ? -2 : -1;
+      if (logical >= 0 && logical < l_ctx) {
+        const int at = logical / p.page_size;
+        in_page = logical - at * p.page_size;
+        page = -2;                                         // a context length longer than the table's row
+        if (at < p.bt_stride) {
+          page = p.block_table[l_seq * p.bt_stride + at];
+          if (page < 0) page = -2;
+        }
+      }
+    };
+    auto next_rows = [&]() {
+      const int row = page * p.page_size + in_page;
+      ok = page >= 0 && row >= 0 && row < p.s_kv;
+      if (page == -2 || (page >= 0 && !ok)) misc->bad_index = 1;      // reported, never read
+      scale = ok ? p.kv_scale[page] : 0.0f;
+      const uint4* src = reinterpret_cast<const uint4*>(cache + static_cast<long long>(ok ? row : 0) * p.kv_sr);
+#pragma unroll
+      for (int k = 0; k < 9; ++k) raw[k] = ok ? src[4 * k] : make_uint4(0u, 0u, 0u, 0u);
+    };
+    next_entry();
+    next_page();
+    next_entry();
+    next_rows();
+    next_page();
+    next_entry();
+    uint32_t G = 0;
+#pragma unroll 1
+    for (int t = 0; t < nb; ++t) {
+      const int n_tiles = warp_uniform(misc->nt[t]);
+      if (w == 0) load_q(t);
+#pragma unroll 1
+      for (int i = 0; i < n_tiles; ++i, ++G) {
+        const uint32_t s = G & 1u;
+        const uint32_t rows = __ballot_sync(0xffffffffu, ok);          // bit 4 r: row r
+        const uint32_t mask = __ballot_sync(0xffffffffu, lane < 8 && ((rows >> (4 * (lane & 7))) & 1u) != 0u);
+        if (G >= kSlots) mbar_wait(smem_u32(&misc->k_free[s][w >> 1]), ((G >> 1) - 1) & 1u, abort_flag);
+        __syncwarp();
+        if (lane == 0) reinterpret_cast<uint8_t*>(&misc->valid_mask[s][0])[w] = static_cast<uint8_t>(mask);   // (released by the arrivals below)
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+          const uint32_t in[4] = {raw[k].x, raw[k].y, raw[k].z, raw[k].w};
+          uint32_t o[8];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const __half2_raw lo = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(in[j] & 0xffffu), __NV_E4M3);
+            const __half2_raw hi = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(in[j] >> 16), __NV_E4M3);
+            const float2 flo = __half22float2(*reinterpret_cast<const __half2*>(&lo)), fhi = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+            o[2 * j] = pack_bf16x2(flo.x * scale, flo.y * scale);
+            o[2 * j + 1] = pack_bf16x2(fhi.x * scale, fhi.y * scale);
+          }
+          const uint32_t off = s * kSlot + k * kBlock;
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst0 + off), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst1 + off), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]) : "memory");
+        }
+        fence_proxy_async_smem();                          // the MMAs read the rows through the async proxy
+        __syncwarp();
+        if (lane == 0) {
+#pragma unroll
+          for (int j = 0; j < kThirds; ++j) mbar_arrive(smem_u32(&misc->k_full[s][j]));
+        }
+        next_rows();
+        next_page();
+        next_entry();
+      }
+    }
+  };
+  if constexpr (kFp8) {
+    if (group >= 0) {
+      if constexpr (Sh::kSplitRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Sh::kRegsSoftmax));
+      softmax();
+    } else if (warp < Sh::kConvert0) {
+      if constexpr (Sh::kSplitRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Sh::kRegsIssue));
+      if (warp == Sh::kIssuer) scores();
+      else if (warp == Sh::kValueIssuer) values();
+    } else {
+      if constexpr (Sh::kSplitRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Sh::kRegsConvert));
+      convert();
+    }
+  } else {
+    if (group >= 0) softmax();
+    else if (warp == Sh::kIssuer) scores();
+    else if (warp == Sh::kValueIssuer) values();
+    else if (prod >= 0) gather();
   }
 
   if (*abort_flag) drain_after_abort();
@@ -630,12 +765,12 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
   }
 }
 
-template <int NH>
+template <int NH, bool kFp8>
 static int launch_nh(const ftb_sparse_mla_args* a, Params p, cudaStream_t st) {
-  using Sh = Shape<NH>;
+  using Sh = Shape<NH, kFp8>;
   constexpr int smem = Sh::kOffMisc + static_cast<int>(sizeof(Misc)) + 1024;
   static_assert(smem <= 227 * 1024, "shared memory of an SM");
-  auto kern = sparse_mla_few_heads_kernel<NH>;
+  auto kern = sparse_mla_few_heads_kernel<NH, kFp8>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(sparse_mla few heads)");
   int dev = 0, sms = 0;
@@ -679,7 +814,7 @@ static int launch_nh(const ftb_sparse_mla_args* a, Params p, cudaStream_t st) {
 int launch_sparse_mla_few(const ftb_sparse_mla_args* a, int n_splits, float* part_out, float* part_lse, float max_slack, cudaStream_t st) {
   mla_few::Params p;
   memset(&p, 0, sizeof(p));
-  p.kv = reinterpret_cast<const __nv_bfloat16*>(a->kv);
+  p.kv = a->kv;
   p.kv_sr = a->kv_stride_row;
   p.h = a->h; p.s_kv = a->s_kv; p.topk = a->topk;
   p.idx_st = a->idx_stride_token; p.out_st = a->out_stride_token; p.out_sh = a->out_stride_head; p.lse_st = a->lse_stride_token;
@@ -691,9 +826,16 @@ int launch_sparse_mla_few(const ftb_sparse_mla_args* a, int n_splits, float* par
   p.part_lse = part_lse;
   p.max_slack = max_slack;
   p.n_groups = (a->h + 63) / 64;
-  if (a->h <= 16) return mla_few::launch_nh<16>(a, p, st);
-  if (a->h <= 32) return mla_few::launch_nh<32>(a, p, st);
-  return mla_few::launch_nh<64>(a, p, st);
+  if (a->kv_is_fp8) {
+    p.kv_scale = a->kv_scale; p.block_table = a->block_table; p.context_lens = a->context_lens;
+    p.page_size = a->page_size; p.q_per_seq = a->q_per_seq; p.bt_stride = a->block_table_stride;
+    if (a->h <= 16) return mla_few::launch_nh<16, true>(a, p, st);
+    if (a->h <= 32) return mla_few::launch_nh<32, true>(a, p, st);
+    return mla_few::launch_nh<64, true>(a, p, st);
+  }
+  if (a->h <= 16) return mla_few::launch_nh<16, false>(a, p, st);
+  if (a->h <= 32) return mla_few::launch_nh<32, false>(a, p, st);
+  return mla_few::launch_nh<64, false>(a, p, st);
 }
 
 }  // namespace ftb

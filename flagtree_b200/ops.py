@@ -287,9 +287,9 @@ def sparse_mla_fwd_paged(q: torch.Tensor, kv_cache: torch.Tensor, kv_scale: torc
     Physical row = block_table[b, p // page] * page + p % page, the addressing rule of
     test_accuracy_musa_vllm_mla.py:278-283.  Returns (out [B,n_q,h,512] bf16, lse [B,n_q,h] fp32).
 
-    `two_pass`: convert the selected rows to a compact bf16 table first and run the persistent bf16 kernel on
-    it (needs 1156 bytes of scratch per selected row), False = the one-pass kernel that converts while it gathers; None = by the
-    number of tokens, never with more than 4 GiB of scratch, and with a `num_splits` above 1 the one-pass kernel.
+    The rows are converted while they are gathered.  `two_pass`: convert the selected rows to a compact bf16 table first and run the
+    persistent bf16 kernels on it (needs 1156 bytes of scratch per selected row; a whole token then has the same bits).  With parts of a
+    token, and with `two_pass` False, the weights follow the true maximum, otherwise a lazy one.
     """
     _require_cuda(q, kv_cache, kv_scale, block_table, context_lens, indices)
     assert q.dim() == 4 and indices.dim() == 3 and kv_cache.dim() == 3
@@ -336,10 +336,8 @@ def sparse_mla_fwd_paged(q: torch.Tensor, kv_cache: torch.Tensor, kv_scale: torc
     else:
         n_splits = max(1, int(num_splits))
         rows_first = n_splits == 1
-    rows_bytes = 0
-    if two_pass or (two_pass is None and rows_first):
-        rows_bytes = int(lib.ftb_sparse_mla_dequant_workspace_bytes(s_q, topk))
-    if 0 < rows_bytes and (two_pass or rows_bytes <= (4 << 30)):
+    rows_bytes = int(lib.ftb_sparse_mla_dequant_workspace_bytes(s_q, topk)) if two_pass else 0
+    if rows_bytes > 0:
         # the dequantised rows, then (from a 16-byte boundary) the partial results of a split
         need = rows_bytes
         if n_splits > 1:
@@ -347,6 +345,8 @@ def sparse_mla_fwd_paged(q: torch.Tensor, kv_cache: torch.Tensor, kv_scale: torc
         _ws = torch.empty(need, dtype=torch.uint8, device=device)
         a.n_splits, a.workspace, a.workspace_bytes, a.algo_id = n_splits, _ws.data_ptr(), need, 6
     else:
+        if two_pass is None and rows_first and n_splits == 1:
+            a.algo_id = 5                                    # many tokens, or told to keep them whole: the lazy maximum
         _ws = _split_workspace(a, s_q, h, n_splits, device)
     _launch(lib.ftb_sparse_mla_fwd, a, device, "sparse_mla_fwd_paged")
     _check_status(status, "sparse_mla_fwd_paged")

@@ -120,3 +120,26 @@ def test_bits_of_a_head_do_not_depend_on_the_heads_of_the_call(h, s_q, topk, ste
     many, lse_many = sparse_mla_fwd(q.repeat(reps, 128 // h + 1, 1)[:, :128].contiguous(), kv, idx.repeat(reps, 1), 0.05, check=True, num_splits=1)
     out, lse = sparse_mla_fwd(q, kv, idx, 0.05, check=True, num_splits=1)
     assert torch.equal(out, many[:s_q, :h]) and torch.equal(lse, lse_many[:s_q, :h])
+
+
+@pytest.mark.parametrize("h", [1, 16, 32, 64, 100, 128])
+@pytest.mark.parametrize("batch,n_q,topk,page", [(3, 2, 300, 64), (160, 1, 65, 16), (2, 1, 64, 64), (5, 3, 1000, 7)])
+def test_paged_rows_converted_in_the_gather(h, batch, n_q, topk, page):
+    """e4m3 pages: whole tokens have the bits of the two-pass form (the same values, multiplied and added in the same order), parts of them its
+    values; contexts shorter than the lists, padding inside a list, entries past the context, pages of odd sizes, several items per CTA."""
+    from flagtree_b200 import sparse_mla_fwd_paged
+    c = W.mla_cfg3(batch=batch, n_q=n_q, h=h, topk=topk, len_lo=30, len_hi=1500, page_size=page)
+    c.indices[0, 0, 3::5] = -1
+    c.indices[1, 0, :] = -1
+    c.indices[-1, -1, 7] = 1 << 20                           # past the context: padding
+    args = [t.to(DEV) for t in (c.q, c.kv_cache, c.kv_scale, c.block_table, c.context_lens, c.indices)]
+    out, lse = sparse_mla_fwd_paged(*args, c.sm_scale, page_size=page, check=True, num_splits=1)
+    ref_out, ref_lse = sparse_mla_fwd_paged(*args, c.sm_scale, page_size=page, check=True, num_splits=1, two_pass=True)
+    assert torch.equal(out, ref_out) and torch.equal(lse, ref_lse)
+    for kw in (dict(), dict(num_splits=3), dict(num_splits=1, two_pass=False)):
+        o, l = sparse_mla_fwd_paged(*args, c.sm_scale, page_size=page, check=True, **kw)
+        fin = torch.isfinite(ref_lse)
+        assert torch.equal(torch.isfinite(l), fin)
+        # P and the result are rounded to bf16 (2^-9 each) from another reference maximum and with sums in another order
+        assert (o.float() - ref_out.float()).abs().max().item() <= 2 ** -7 * max(1.0, ref_out.abs().max().item())
+        assert ((l[fin] - ref_lse[fin]).abs() <= 1e-5 * ref_lse[fin].abs().clamp(min=1)).all()

@@ -677,7 +677,8 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
   };
   // Paged FP8 form: by default (algo 0 with the true maximum, algo 5 with the lazy one) the kernel for few heads converts the rows while it
   // gathers them, 64 heads at a time; with algo 6 and a workspace for them the selected rows are converted once, and the
-  // persistent kernels run on the compact table (128 tokens of 128 heads, topk 2048: @F1@); algo 1 is the one-CTA kernel.
+  // persistent kernels run on the compact table (128 tokens of 128 heads, topk 2048: 148 us against 105 for the table and
+  // 106 for the kernel on it; 3 tokens 18.2 against 22.4, and 26.8 with algo 1); algo 1 is the one-CTA kernel.
   const int64_t split_bytes = ftb_sparse_mla_workspace_bytes(a->s_q, a->h, n_splits);
   auto merge = [&]() {
     const auto kern = n_splits <= 2 ? sparse_mla_merge_kernel<2> : n_splits <= 4 ? sparse_mla_merge_kernel<4>

@@ -644,7 +644,7 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
     int ct = -1, ci = 0, cn = 0, c_left = 0, c_seq = 0, c_ctx = 0;
     const int32_t* c_idx = nullptr;
     int logical = -1, l_seq = 0, l_ctx = 0;                // of the tile after the next
-    int page = -1, in_page = 0;                            // of the next tile: -1 for no row, -2 for an entry of no meaning
+    int page = 0, in_page = -1;                            // of the next tile; in_page -1 for no row, -2 for an entry of no meaning
     uint4 raw[9];                                          // of this tile
     float scale = 0.0f;
     bool ok = false;
@@ -666,21 +666,22 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
       ++ci;
     };
     auto next_page = [&]() {
-      page = logical < -1 ? -2 : -1;
+      // (nothing here may look at the page: it is on its way)
+      in_page = logical < -1 ? -2 : -1;
       if (logical >= 0 && logical < l_ctx) {
         const int at = logical / p.page_size;
-        in_page = logical - at * p.page_size;
-        page = -2;                                         // a context length longer than the table's row
         if (at < p.bt_stride) {
+          in_page = logical - at * p.page_size;
           page = p.block_table[l_seq * p.bt_stride + at];
-          if (page < 0) page = -2;
+        } else {
+          in_page = -2;                                    // a context length longer than the table's row
         }
       }
     };
     auto next_rows = [&]() {
       const int row = page * p.page_size + in_page;
-      ok = page >= 0 && row >= 0 && row < p.s_kv;
-      if (page == -2 || (page >= 0 && !ok)) misc->bad_index = 1;      // reported, never read
+      ok = in_page >= 0 && page >= 0 && row >= 0 && row < p.s_kv;
+      if (in_page == -2 || (in_page >= 0 && !ok)) misc->bad_index = 1;      // reported, never read
       scale = ok ? p.kv_scale[page] : 0.0f;
       const uint4* src = reinterpret_cast<const uint4*>(cache + static_cast<long long>(ok ? row : 0) * p.kv_sr);
 #pragma unroll

@@ -65,11 +65,12 @@ typedef struct ftb_sparse_mla_args {
   int64_t lse_stride_token;
   float sm_scale;
   int32_t lse_base2;        /* 0: lse = log sum exp(s);  1: log2 sum 2^(s*log2 e)            */
-  int32_t algo_id;          /* 0 = default = 5; 1 = one CTA per (token, output half); 2 = few heads
-                               (h <= 32, bf16 form without splits): one CTA per token, scores
-                               transposed; 5 = persistent role-split CTA pairs that walk through the
-                               tokens (scores in one CTA, values in the other); 6 = paged FP8 form
-                               only: dequantise the selected rows, then the persistent kernel    */
+  int32_t algo_id;          /* 0 = default; 1 = one CTA per (token, output half); 2 = the kernel for few
+                               heads with the true maximum (h <= 32, bf16 form without splits); 5 = the
+                               persistent kernels with the lazy maximum: up to 64 heads, and few tokens of
+                               more, on single CTAs, else on CTA pairs (0 = 5 for whole tokens of the bf16
+                               form); 6 = paged FP8 form only: convert the selected rows to a table, then the
+                               persistent kernels                                                */
   int32_t* status;          /* optional device int32: kernels OR-in a non-zero FTB_ERR_* code */
   /* Paged FP8 form (kv_is_fp8 != 0): physical row = block_table[seq, p / page] * page + p % page,
    * the rule of test_accuracy_musa_vllm_mla.py:278-283.  Query token t belongs to sequence
@@ -87,8 +88,9 @@ typedef struct ftb_sparse_mla_args {
    * partial result to `workspace` (ftb_sparse_mla_workspace_bytes() bytes of device memory, 16-byte aligned, contents
    * need not be initialised) and a merge kernel combine them, the role of _fwd_kernel_stage2
    * (test_accuracy_musa_vllm_mla.py:426-477).  0 or 1 = no split, no workspace.  bf16 form: algo_id 5 takes the parts on the
-   * persistent pairs, algo_id 0 on whichever kernel is faster, algo_id 1 on the one-CTA kernel.  Paged FP8 form: the one-CTA kernel,
-   * unless algo_id 6 finds room for both passes (below).  Parts beyond the tiles of a list are left out. */
+   * persistent kernels, algo_id 0 on whichever kernel is faster, algo_id 1 on the one-CTA kernel.  Paged FP8 form: algo_id 1 on the
+   * one-CTA kernel, algo_id 6 as below, else on the kernel for few heads, which converts the rows while it gathers them (parts and
+   * algo_id 0 with the true maximum, algo_id 5 without a split with the lazy one).  Parts beyond the tiles of a list are left out. */
   int32_t n_splits;
   void* workspace;
   int64_t workspace_bytes;
@@ -96,13 +98,12 @@ typedef struct ftb_sparse_mla_args {
 
 FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* args, void* stream);
 FTB_API int64_t ftb_sparse_mla_workspace_bytes(int32_t s_q, int32_t h, int32_t n_splits);
-/* Paged FP8 form, two passes: when `workspace` holds at least this many bytes (16-byte aligned; with
- * n_splits > 1 and algo_id 6, rounded up to 16 and followed by ftb_sparse_mla_workspace_bytes()),
+/* Paged FP8 form, two passes (algo_id 6): `workspace` holds at least this many bytes (16-byte aligned; with
+ * n_splits > 1 rounded up to 16 and followed by ftb_sparse_mla_workspace_bytes()),
  * the selected rows are first converted to a compact bf16 table (row = token * topk + j,
  * the role of the dequantising loads of decode_attention_int4kv.py:345-450, done once per row instead of
- * inside the attention loop) and the persistent bf16 kernel runs on that table.  algo_id 6 demands this
- * path when n_splits <= 1, algo_id 0 takes it when the workspace allows and n_splits <= 1.  With n_splits > 1 and a
- * workspace that only holds the partial results, algo_id 6 is the one-pass kernel with a split. */
+ * inside the attention loop) and the persistent bf16 kernels run on that table.  With n_splits > 1 and a
+ * workspace that only holds the partial results, algo_id 6 converts while it gathers. */
 FTB_API int64_t ftb_sparse_mla_dequant_workspace_bytes(int32_t s_q, int32_t topk);
 /* Same operation for callers that cannot allocate device memory (an engine that owns the whole device
  * through its own pool, a sandboxed plugin, a latency path that must stay clear of the allocator).  It has

@@ -27,6 +27,7 @@
 // (the tensor pipe and the power limit: a library e4m3 GEMM reaches 2960).
 #include <cstring>
 
+#include "launch.cuh"
 #include "sm100.cuh"
 #include "tmap.cuh"
 
@@ -134,8 +135,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   const int kb0 = static_cast<int>(static_cast<long long>(p.kb_total) * split / p.splits);
   const int kb1 = static_cast<int>(static_cast<long long>(p.kb_total) * (split + 1) / p.splits);
 
+  const bool one_each = p.n_tiles <= n_groups;
+  if (one_each) griddep_launch();
   if (tid == 0) {
-    bars->abort_flag = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(smem_u32(&bars->full[s]), 1);
       mbar_init(smem_u32(&bars->empty[s]), 1);
@@ -148,6 +150,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     tma_prefetch_desc(&tm_a);
     tma_prefetch_desc(&tm_b);
   }
+  griddep_wait();
+  if (tid == 0) bars->abort_flag = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
   __syncthreads();
   // an earlier launch on this status word failed: leave at once, the whole cluster on the reading of its CTA 0
   if (clustered) {
@@ -384,6 +388,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   }
   tc_fence_before();
   __syncthreads();
+  if (!one_each) griddep_launch();     // (behind the barrier: one thread of a CTA speaks for all)
   if (bars->abort_flag) drain_after_abort();
   if (clustered) cluster_sync_all();   // nobody leaves while a peer may still signal or read this CTA
   if (warp == 1) {
@@ -479,17 +484,8 @@ static int gemm_fp8_blockscaled(const ftb_gemm_fp8_args* g, bool whole_k, void* 
   const int cl = shape.ncta * shape.splits;
   // persistent groups; with a split every cluster computes one tile and leaves
   const int groups = shape.splits > 1 ? p.n_tiles : (p.n_tiles < sms / shape.ncta ? p.n_tiles : sms / shape.ncta);
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = cl; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3(static_cast<unsigned>(groups) * cl);
-  cfg.blockDim = dim3(gemm8::THREADS);
-  cfg.dynamicSmemBytes = gemm8::SMEM_BYTES;
-  cfg.stream = reinterpret_cast<cudaStream_t>(stream);
-  cfg.attrs = attr;
-  cfg.numAttrs = cl > 1 ? 1 : 0;
-  e = cudaLaunchKernelEx(&cfg, kern, tm_a, tm_b, p);
+  e = launch_overlapped(kern, static_cast<unsigned>(groups) * cl, gemm8::THREADS, gemm8::SMEM_BYTES, reinterpret_cast<cudaStream_t>(stream),
+                        static_cast<unsigned>(cl), tm_a, tm_b, p);
   if (e != cudaSuccess) return check_cuda(e, "gemm_fp8 launch");
   return FTB_OK;
 }

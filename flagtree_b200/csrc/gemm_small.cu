@@ -11,6 +11,7 @@
 // Roles (192 threads): warp 0 TMA producer, warp 1 MMA issuer (owns TMEM), warps 2-5 epilogue (TMEM lanes 32 (warp % 4) ..).
 #include <cstring>
 
+#include "launch.cuh"
 #include "sm100.cuh"
 #include "tmap.cuh"
 
@@ -61,8 +62,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   const int m_blk = tile / p.n_blocks, n0 = (tile - m_blk * p.n_blocks) * BN;
   const int kb0 = p.kb_total * split / p.splits, kb1 = p.kb_total * (split + 1) / p.splits;
 
+  griddep_launch();
   if (tid == 0) {
-    bars->abort_flag = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
     for (int s = 0; s < STAGES; ++s) { mbar_init(smem_u32(&bars->full[s]), 1); mbar_init(smem_u32(&bars->empty[s]), 1); }
     mbar_init(smem_u32(&bars->acc_full), 1);
     fence_mbar_init();
@@ -74,6 +75,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     tmem_relinquish();
     tc_fence_before();
   }
+  griddep_wait();
+  if (tid == 0) bars->abort_flag = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
   __syncthreads();
   tc_fence_after();
   // an earlier launch on this status word failed: nothing is loaded or multiplied (every wait returns at once) and nothing written
@@ -220,17 +223,8 @@ static int launch(const void* a, const void* b, void* c, int m, int n, int k, lo
   p.status = status;
   cudaError_t e = cudaFuncSetAttribute(gemm_small_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::SMEM_BYTES);
   if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(gemm_small)");
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(splits); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3(static_cast<unsigned>((m + BM - 1) / BM * p.n_blocks * splits));
-  cfg.blockDim = dim3(THREADS);
-  cfg.dynamicSmemBytes = Cfg<BN>::SMEM_BYTES;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = splits > 1 ? 1 : 0;
-  return check_cuda(cudaLaunchKernelEx(&cfg, gemm_small_kernel<BN>, tm_a, tm_b, p), "gemm_small launch");
+  return check_cuda(launch_overlapped(gemm_small_kernel<BN>, static_cast<unsigned>((m + BM - 1) / BM * p.n_blocks * splits), THREADS, Cfg<BN>::SMEM_BYTES, st,
+                                      static_cast<unsigned>(splits), tm_a, tm_b, p), "gemm_small launch");
 }
 
 }  // namespace gemm_small

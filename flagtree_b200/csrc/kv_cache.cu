@@ -29,6 +29,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "launch.cuh"
 #include "../../include/flagtree_b200.h"
 
 namespace ftb {
@@ -225,6 +226,8 @@ __global__ void __launch_bounds__(kThreads) small_write_kernel(const Params p) {
   __shared__ int mine[kSmallRows];
   __shared__ int n_mine;
   __shared__ float wmax[kWarps];
+  griddep_launch();
+  griddep_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int r0 = blockIdx.x;
   const int slot0 = p.slots[r0];
@@ -266,6 +269,8 @@ __global__ void __launch_bounds__(kThreads) small_write_kernel(const Params p) {
 }
 
 __global__ void __launch_bounds__(256) run_count_kernel(const Params p) {
+  griddep_launch();
+  griddep_wait();
   const int r = blockIdx.x * 256 + threadIdx.x;
   if (r >= p.n_rows) return;
   const int slot = p.slots[r];
@@ -293,6 +298,8 @@ __global__ void __launch_bounds__(kRunThreads, 3) run_write_kernel(const Params 
   __shared__ int long_head[kChunk / kWarpRun + 1], long_len[kChunk / kWarpRun + 1], short_head[kChunk], short_len[kChunk];
   __shared__ int n_long, n_short, first_break;
   __shared__ unsigned wmax[kRunWarps];
+  griddep_launch();
+  griddep_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int c0 = blockIdx.x * kHeads;
   if (tid <= 2 * kChunk) {
@@ -445,6 +452,8 @@ constexpr unsigned int kCandMin = 0x20000000u;
 __global__ void __launch_bounds__(256) page_settle_kernel(const Params p) {
   __shared__ int rises[256];
   __shared__ int n_rises;
+  griddep_launch();
+  griddep_wait();
   const int tid = threadIdx.x;
   for (int first = blockIdx.x; first < p.num_pages; first += gridDim.x * 256) {
     if (tid == 0) n_rises = 0;
@@ -469,6 +478,8 @@ __global__ void __launch_bounds__(256) page_settle_kernel(const Params p) {
 
 // A warp looks after `per_warp` rows (at most 32, a power of two) and stores those of the pages that the kernel before settled.
 __global__ void __launch_bounds__(256) row_store_kernel(const Params p, int per_warp) {
+  griddep_launch();
+  griddep_wait();
   const int lane = threadIdx.x & 31;
   const long long r0 = (static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5)) * per_warp;
   const int slot = lane < per_warp && r0 + lane < p.n_rows ? p.slots[r0 + lane] : -1;
@@ -525,9 +536,9 @@ extern "C" FTB_API int ftb_kv_cache_write_fp8(const ftb_kv_cache_write_args* a, 
   // A CTA has a page to itself, so the line also lies where the rows of one page are many: 1024 rows in pages of 256 take it 39 us, the large
   // path 21 (both with the host's part).  More threads for pages of 128: 20.4 -> 16.2 us.
   if (a->n_rows <= 64 || (a->n_rows <= kvw::kSmallRows && a->page_size <= 128)) {
-    if (a->n_rows <= 64 || a->page_size <= 64) kvw::small_write_kernel<256><<<static_cast<unsigned>(a->n_rows), 256, 0, st>>>(p);
-    else kvw::small_write_kernel<512><<<static_cast<unsigned>(a->n_rows), 512, 0, st>>>(p);
-    return check_cuda(cudaGetLastError(), "ftb_kv_cache_write_fp8 launch");
+    const bool narrow = a->n_rows <= 64 || a->page_size <= 64;
+    return check_cuda(launch_overlapped(narrow ? kvw::small_write_kernel<256> : kvw::small_write_kernel<512>, static_cast<unsigned>(a->n_rows), narrow ? 256 : 512, 0,
+                                        st, 1, p), "ftb_kv_cache_write_fp8 launch");
   }
   cudaError_t e = cudaMemsetAsync(p.cand, 0, static_cast<size_t>(a->num_pages) * 4, st);
   if (e != cudaSuccess) return check_cuda(e, "ftb_kv_cache_write_fp8: cudaMemsetAsync");
@@ -539,14 +550,15 @@ extern "C" FTB_API int ftb_kv_cache_write_fp8(const ftb_kv_cache_write_args* a, 
   const auto run_write = heads == 16 ? kvw::run_write_kernel<16> : heads == 32 ? kvw::run_write_kernel<32> : kvw::run_write_kernel<kvw::kChunk>;
   e = cudaFuncSetAttribute(run_write, cudaFuncAttributeMaxDynamicSharedMemorySize, kvw::kRunSmem);
   if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(run_write)");
-  kvw::run_count_kernel<<<row_blocks, 256, 0, st>>>(p);
-  run_write<<<static_cast<unsigned>((static_cast<long long>(a->n_rows) + heads - 1) / heads), kvw::kRunThreads, kvw::kRunSmem, st>>>(p);
+  e = launch_overlapped(kvw::run_count_kernel, row_blocks, 256, 0, st, 1, p);
+  if (e == cudaSuccess)
+    e = launch_overlapped(run_write, static_cast<unsigned>((static_cast<long long>(a->n_rows) + heads - 1) / heads), kvw::kRunThreads, kvw::kRunSmem, st, 1, p);
   // Pages with several runs.  The settle kernel: eight CTAs per SM, or one per page.  The store kernel: as many rows per warp as keep it at
   // one wave, up to 32.
-  kvw::page_settle_kernel<<<static_cast<unsigned>(a->num_pages < 1184 ? a->num_pages : 1184), 256, 0, st>>>(p);
+  if (e == cudaSuccess) e = launch_overlapped(kvw::page_settle_kernel, static_cast<unsigned>(a->num_pages < 1184 ? a->num_pages : 1184), 256, 0, st, 1, p);
   int per_warp = 1;
   while (per_warp < 32 && static_cast<long long>(per_warp) * 9472 < a->n_rows) per_warp *= 2;
   const long long per_cta = 8LL * per_warp;
-  kvw::row_store_kernel<<<static_cast<unsigned>((a->n_rows + per_cta - 1) / per_cta), 256, 0, st>>>(p, per_warp);
-  return check_cuda(cudaGetLastError(), "ftb_kv_cache_write_fp8 launch");
+  if (e == cudaSuccess) e = launch_overlapped(kvw::row_store_kernel, static_cast<unsigned>((a->n_rows + per_cta - 1) / per_cta), 256, 0, st, 1, p, per_warp);
+  return check_cuda(e, "ftb_kv_cache_write_fp8 launch");
 }

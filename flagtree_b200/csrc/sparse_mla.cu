@@ -15,6 +15,7 @@
 //         the tile has finished (the rope block and a block of the other output half).
 #include <cuda_fp8.h>
 
+#include "launch.cuh"
 #include "sm100.cuh"
 #include "../../include/flagtree_b200.h"
 
@@ -101,6 +102,8 @@ __device__ __forceinline__ int resolve_row(const MlaParams& p, int token, int lo
 // `out_idx[r]` is r, or -1 for padding and for positions at or past the context length.  The bf16 kernels
 // then run on the compact table with these indices.
 __global__ void __launch_bounds__(256) mla_dequant_rows_kernel(const MlaParams p, __nv_bfloat16* table, int32_t* out_idx) {
+  griddep_launch();
+  griddep_wait();
   const int lane = threadIdx.x & 31;
   const long long n_rows = static_cast<long long>(p.s_q) * p.topk;
   const uint8_t* kvp = reinterpret_cast<const uint8_t*>(p.kv);
@@ -465,11 +468,18 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_fwd_kernel(const MlaPa
 // that the loads of all parts are in flight at once (a warp per row that took one part after the other: 13 us for 3 tokens
 // of 128 heads and 16 parts).  kBatch parts at a time, the least power of two that holds them all, up to 16: with 16 for every call, 300 tokens
 // of 128 heads and topk 2048 in 2 parts took 817 us on the one-CTA kernel, now 687.
+// (not __ldcs, which the compiler may move above the wait for the kernel before)
+__device__ __forceinline__ float4 ld_once(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  return v;
+}
 template <int kBatch>
-__global__ void __launch_bounds__(128) sparse_mla_merge_kernel(const float* __restrict__ part_out,
-                                                               const float* __restrict__ part_lse, __nv_bfloat16* out,
+__global__ void __launch_bounds__(128) sparse_mla_merge_kernel(const float* part_out, const float* part_lse, __nv_bfloat16* out,
                                                                float* lse, int h, int n_splits, long long out_st,
                                                                long long out_sh, long long lse_st, int lse_base2) {
+  griddep_launch();
+  griddep_wait();
   const int token = blockIdx.x / h, head = blockIdx.x - token * h;
   const float* lrow = part_lse + static_cast<long long>(token) * n_splits * h + head;
   const float4* src = reinterpret_cast<const float4*>(part_out + (static_cast<long long>(token) * n_splits * h + head) * 512) + threadIdx.x;
@@ -484,7 +494,7 @@ __global__ void __launch_bounds__(128) sparse_mla_merge_kernel(const float* __re
     for (int k = 0; k < kBatch; ++k) {
       const bool in = k0 + k < n_splits;
       w[k] = in ? lrow[static_cast<long long>(k0 + k) * h] : -INFINITY;
-      v[k] = in ? __ldcs(src + static_cast<long long>(k0 + k) * h * 128) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      v[k] = in ? ld_once(src + static_cast<long long>(k0 + k) * h * 128) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
     if (n_splits <= kBatch) {
 #pragma unroll
@@ -514,11 +524,13 @@ __global__ void __launch_bounds__(128) sparse_mla_merge_kernel(const float* __re
 // (T = bf16, what ftb_sparse_mla_fwd writes, or fp32), its log-sum-exp `part_lse + k * lps + token * lts + head`
 // (natural log, or base 2 when lse_base2; -inf = the part saw no valid row).  One warp per (token, head).
 template <typename T>
-__global__ void __launch_bounds__(256) sparse_mla_merge_parts_kernel(const T* __restrict__ part_out, const float* __restrict__ part_lse,
+__global__ void __launch_bounds__(256) sparse_mla_merge_parts_kernel(const T* part_out, const float* part_lse,
                                                                      __nv_bfloat16* out, float* lse, int s_q, int h, int n_parts,
                                                                      long long ps, long long ts, long long hs, long long lps,
                                                                      long long lts, long long out_st, long long out_sh,
                                                                      long long lse_st, int lse_base2) {
+  griddep_launch();
+  griddep_wait();
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (w >= s_q * h) return;
@@ -683,9 +695,8 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
   auto merge = [&]() {
     const auto kern = n_splits <= 2 ? sparse_mla_merge_kernel<2> : n_splits <= 4 ? sparse_mla_merge_kernel<4>
                       : n_splits <= 8 ? sparse_mla_merge_kernel<8> : sparse_mla_merge_kernel<16>;
-    kern<<<static_cast<unsigned>(a->s_q * a->h), 128, 0, st>>>(p.part_out, p.part_lse, p.out, p.lse, a->h, n_splits, p.out_st, p.out_sh,
-                                                             p.lse_st, p.lse_base2);
-    return check_cuda(cudaGetLastError(), "sparse_mla_merge launch");
+    return check_cuda(launch_overlapped(kern, static_cast<unsigned>(a->s_q * a->h), 128, 0, st, 1, p.part_out, p.part_lse, p.out, p.lse, a->h, n_splits,
+                                        p.out_st, p.out_sh, p.lse_st, p.lse_base2), "sparse_mla_merge launch");
   };
   // With a split, algo 6 wants room for both: the dequantised rows, then the partial results (from a 16-byte boundary).
   const int64_t rows_bytes = (ftb_sparse_mla_dequant_workspace_bytes(a->s_q, a->topk) + 15) / 16 * 16;
@@ -706,8 +717,7 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
                                                 static_cast<size_t>(a->s_q) * a->topk * kDqk * 2);
       const long long n_rows = static_cast<long long>(a->s_q) * a->topk;
       const unsigned blocks = static_cast<unsigned>(n_rows / 8 < 148 * 16 ? (n_rows + 7) / 8 : 148 * 16);
-      mla_dequant_rows_kernel<<<blocks, 256, 0, st>>>(p, table, idx2);
-      int rc0 = check_cuda(cudaGetLastError(), "mla_dequant_rows launch");
+      int rc0 = check_cuda(launch_overlapped(mla_dequant_rows_kernel, blocks, 256, 0, st, 1, p, table, idx2), "mla_dequant_rows launch");
       if (rc0 != FTB_OK) return rc0;
       ftb_sparse_mla_args b = *a;
       b.kv = table;
@@ -859,14 +869,15 @@ extern "C" FTB_API int ftb_sparse_mla_merge(const ftb_sparse_mla_merge_args* a, 
   const int warps = a->s_q * a->h;
   const unsigned blocks = static_cast<unsigned>((static_cast<long long>(warps) * 32 + 255) / 256);
   __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(a->out);
+  cudaError_t e;
   if (a->part_is_fp32) {
-    sparse_mla_merge_parts_kernel<float><<<blocks, 256, 0, st>>>(reinterpret_cast<const float*>(a->part_out), a->part_lse, out, a->lse, a->s_q, a->h,
-        a->n_parts, a->part_stride_part, a->part_stride_token, a->part_stride_head, a->lse_stride_part, a->lse_stride_part_token,
-        a->out_stride_token, a->out_stride_head, a->lse_stride_token, a->lse_base2);
+    e = launch_overlapped(sparse_mla_merge_parts_kernel<float>, blocks, 256, 0, st, 1, reinterpret_cast<const float*>(a->part_out), a->part_lse, out, a->lse,
+                          a->s_q, a->h, a->n_parts, a->part_stride_part, a->part_stride_token, a->part_stride_head, a->lse_stride_part,
+                          a->lse_stride_part_token, a->out_stride_token, a->out_stride_head, a->lse_stride_token, a->lse_base2);
   } else {
-    sparse_mla_merge_parts_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(a->part_out), a->part_lse, out, a->lse,
-        a->s_q, a->h, a->n_parts, a->part_stride_part, a->part_stride_token, a->part_stride_head, a->lse_stride_part,
-        a->lse_stride_part_token, a->out_stride_token, a->out_stride_head, a->lse_stride_token, a->lse_base2);
+    e = launch_overlapped(sparse_mla_merge_parts_kernel<__nv_bfloat16>, blocks, 256, 0, st, 1, reinterpret_cast<const __nv_bfloat16*>(a->part_out), a->part_lse,
+                          out, a->lse, a->s_q, a->h, a->n_parts, a->part_stride_part, a->part_stride_token, a->part_stride_head, a->lse_stride_part,
+                          a->lse_stride_part_token, a->out_stride_token, a->out_stride_head, a->lse_stride_token, a->lse_base2);
   }
-  return check_cuda(cudaGetLastError(), "sparse_mla_merge launch");
+  return check_cuda(e, "sparse_mla_merge launch");
 }

@@ -33,6 +33,7 @@
 
 #include <cstring>
 
+#include "launch.cuh"
 #include "sm100.cuh"
 #include "tmap.cuh"
 #include "../../include/flagtree_b200.h"
@@ -210,8 +211,9 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = warp_uniform(tid >> 5);
 
+  const bool one_each = p.s_q * p.n_splits * p.n_groups <= static_cast<int>(gridDim.x);   // items
+  if (one_each) griddep_launch();
   if (tid == 0) {
-    misc->abort_flag = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
     misc->bad_index = 0;
     for (int i = 0; i < kSlots; ++i) {
       for (int j = 0; j < kThirds; ++j) mbar_init(smem_u32(&misc->k_full[i][j]), kFp8 ? Sh::kConverts : kGather);
@@ -224,6 +226,8 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
     mbar_init(smem_u32(&misc->o_free), 4 * Sh::kGroups);
     fence_mbar_init();
   }
+  griddep_wait();
+  if (tid == 0) misc->abort_flag = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
   __syncthreads();
   if (misc->abort_flag) return;   // an earlier launch on this status word failed: do nothing
   if (warp == Sh::kIssuer) {
@@ -756,6 +760,7 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
   if (*abort_flag) drain_after_abort();
   tc_fence_before();
   __syncthreads();
+  if (!one_each) griddep_launch();               // (behind the barrier: one thread of a CTA speaks for all)
   if (warp == Sh::kIssuer) {
     tc_fence_after();
     tmem_dealloc(tmem, Sh::kCols);
@@ -801,8 +806,7 @@ static int launch_nh(const ftb_sparse_mla_args* a, Params p, cudaStream_t st) {
       return FTB_ERR_CUDA;
     }
     const long long n = static_cast<long long>(p.s_q) * per_token;
-    kern<<<static_cast<unsigned>(n < sms ? n : sms), Sh::kThreads, smem, st>>>(tm_q, p);
-    e = cudaGetLastError();
+    e = launch_overlapped(kern, static_cast<unsigned>(n < sms ? n : sms), Sh::kThreads, smem, st, 1, tm_q, p);
     if (e != cudaSuccess) return check_cuda(e, "sparse_mla few heads launch");
   }
   return FTB_OK;

@@ -46,6 +46,7 @@
 // modulo 4).  CTA 1: 0-3 correction, 4 relay, 8 MMA issuer, 9-16 V producers, 0-7 and 9-16 epilogue.
 // Every wait is bounded; a wait that runs out sets the abort flag, after which every later wait returns at
 // once and the status word reports a timeout.
+#include "launch.cuh"
 #include "sm100.cuh"
 #include "tmap.cuh"
 
@@ -260,8 +261,9 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
   const int row_warps = (p.h + 31) >> 5;
   const bool has_rows = (warp & 3) < row_warps;
 
+  const bool one_each = p.s_q * p.n_splits <= n_pairs;         // items
+  if (one_each) griddep_launch();
   if (tid == 0) {
-    *abort_flag = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
     if (cta == 0) {
       m0->bad_index = 0;
       for (int i = 0; i < kNK; ++i) { mbar_init(smem_u32(&m0->k_full[i]), i == 0 ? 33 : 32); mbar_init(smem_u32(&m0->k_free[i]), 1); }
@@ -286,6 +288,8 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
     }
     fence_mbar_init();
   }
+  griddep_wait();
+  if (tid == 0) *abort_flag = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
   __syncthreads();
   cluster_sync_all();
   // An earlier launch on this status word failed: leave at once.  The two CTAs of a pair read the word at
@@ -953,6 +957,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
   if (*abort_flag) drain_after_abort();
   tc_fence_before();
   __syncthreads();
+  if (!one_each) griddep_launch();               // (behind the barrier: one thread of a CTA speaks for all)
   cluster_sync_all();            // nobody leaves while the peer may still write or signal this CTA
   if (warp == 8) {
     tc_fence_after();
@@ -972,14 +977,16 @@ int launch_sparse_mla_ring(const ftb_sparse_mla_args* a, int n_splits, float* pa
   cudaError_t e = cudaFuncSetAttribute(mla_ring::sparse_mla_ring_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, mla_ring::kSmemBytes);
   if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(sparse_mla_ring)");
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   cfg.blockDim = dim3(mla_ring::kThreads);
   cfg.dynamicSmemBytes = mla_ring::kSmemBytes;
   cfg.stream = st;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 1;                            // (of the occupancy query; the launches take both)
   // as many pairs as the device holds at once (one per pair of SMs that can host a cluster), cached per device
   static int pairs_of_device[64] = {0};
   int dev = 0;
@@ -1039,6 +1046,7 @@ int launch_sparse_mla_ring(const ftb_sparse_mla_args* a, int n_splits, float* pa
     }
     const int pairs = pairs_dev < n_tok * n_splits ? pairs_dev : n_tok * n_splits;
     cfg.gridDim = dim3(static_cast<unsigned>(pairs) * 2u);
+    cfg.numAttrs = 2;
     e = cudaLaunchKernelEx(&cfg, mla_ring::sparse_mla_ring_kernel, tm_q, tm_o, p);
     if (e != cudaSuccess) return check_cuda(e, "sparse_mla_ring launch");
   }

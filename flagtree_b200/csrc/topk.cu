@@ -10,6 +10,7 @@
 // traffic: 4 * s_kv bytes of scores per token (plus 4 * topk bytes of output).
 #include <cmath>
 
+#include "launch.cuh"
 #include "sm100.cuh"
 
 namespace ftb {
@@ -162,6 +163,8 @@ __device__ __forceinline__ void select_row(const uint32_t* sc, int len, int topk
 // One CTA per row, four to an SM.
 __global__ void __launch_bounds__(kThreads) topk_select_kernel(const Params p) {
   __shared__ RowSmem<kThreads> sm;
+  griddep_launch();
+  griddep_wait();
   const int row = blockIdx.x;
   const int len = row_len(p, row);
   select_row<kThreads>(reinterpret_cast<const uint32_t*>(p.scores) + static_cast<long long>(row) * p.sc_stride, len, p.topk,   // bits: NaN patterns keep theirs
@@ -199,6 +202,7 @@ constexpr int kFew = 128;                                  // this many candidat
 constexpr int kAhead = 16;                                 // loads in flight per lane
 constexpr int kSmemMax = 220 * 1024;                       // dynamic; a few KB of static beside it
 
+constexpr int kSmemAlone = 116 * 1024;                     // of a row that has an SM to itself: no second CTA beside it, whenever it comes (launch.cuh)
 struct Shape {
   int room;                                                // list entries
   int words;                                               // of a mask over the row
@@ -288,6 +292,8 @@ __global__ void __launch_bounds__(kThr, kBlocks) topk_listed_kernel(const Params
   uint32_t* eq_words = gt_words + shape.words;                                      // keys that equal the bound
   uint32_t* keys = eq_words + shape.words;                                          // the list: keys,
   unsigned short* at_pos = reinterpret_cast<unsigned short*>(keys + shape.room);    // and positions, ascending
+  griddep_launch();
+  griddep_wait();
   const int row = blockIdx.x;
   const int len = row_len(p, row);
   const int k = min(p.topk, len);
@@ -577,16 +583,15 @@ extern "C" FTB_API int ftb_topk_indices(const ftb_topk_args* a, void* stream) {
   // 600 of 32768 with topk 8192 101 / 76).
   const bool alone = a->s_q <= sm_count;
   topk::listed::Shape shape;
-  const int smem = topk::listed::plan(a->s_kv, a->topk, alone, &shape);
+  int smem = topk::listed::plan(a->s_kv, a->topk, alone, &shape);
   if (smem > 0) {
     const bool small = alone ? a->s_kv <= 8192 : a->topk <= 4096 && (a->s_kv <= 24576 || a->s_q <= 6 * sm_count);
     const auto kernel = alone ? (small ? topk::listed::topk_listed_kernel<512, 1> : topk::listed::topk_listed_kernel<1024, 1>)
                               : (small ? topk::listed::topk_listed_kernel<256, 6> : topk::listed::topk_listed_kernel<512, 3>);
+    if (alone && smem < topk::listed::kSmemAlone) smem = topk::listed::kSmemAlone;
     const unsigned threads = alone ? (small ? 512 : 1024) : (small ? 256 : 512);
     if (int rc = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, topk::listed::kSmemMax), "topk shared memory")) return rc;
-    kernel<<<static_cast<unsigned>(a->s_q), threads, smem, st>>>(p, shape);
-  } else {
-    topk::topk_select_kernel<<<static_cast<unsigned>(a->s_q), topk::kThreads, 0, st>>>(p);
+    return check_cuda(launch_overlapped(kernel, static_cast<unsigned>(a->s_q), threads, smem, st, 1, p, shape), "ftb_topk_indices launch");
   }
-  return check_cuda(cudaGetLastError(), "ftb_topk_indices launch");
+  return check_cuda(launch_overlapped(topk::topk_select_kernel, static_cast<unsigned>(a->s_q), topk::kThreads, 0, st, 1, p), "ftb_topk_indices launch");
 }

@@ -68,17 +68,19 @@ constexpr int kNV = 4;                         // V ring slots: one whole tile, 
 constexpr int kVSlabRows = 32;
 constexpr int kVBlock = kVSlabRows * 128;      // 4096: one 64-column block of a slab
 constexpr int kVSlab = 8 * kVBlock;            // 32768
-constexpr int kPBuf = 2 * kQBlock;             // 32768: P [128 heads x 128 rows] bf16 as two 64-row blocks
+// 32768: P [128 heads x 128 rows] bf16, without a swizzle: 8 of the rows (16 bytes) of all heads are 2048 bytes in a row, so that what a
+// softmax warp sends with one instruction lies in a row
+constexpr int kPBuf = 2 * kQBlock;
+constexpr int kPChunk = 128 * 16;
 constexpr int kBatch = 64;                     // tokens whose tile counts are found in one go
-// CTA 0 layout: nine slots | rope block of Q | P staging | misc.
+// CTA 0 layout: nine slots | rope block of Q | misc.
 // CTA 1 layout: V ring | P x 2 | misc; between tokens the P buffer of the last tile stages O.
 constexpr int kOff0K = 0;
 constexpr int kOff0Q8 = kOff0K + kNK * kKSlot;             // 147456
-constexpr int kOff0P = kOff0Q8 + kQBlock;                  // 163840
-constexpr int kOff0Misc = kOff0P + kPBuf;                  // 212992
+constexpr int kOff0Misc = kOff0Q8 + kQBlock;               // 163840
 constexpr int kOff1P = kNV * kVSlab;                       // 131072
 constexpr int kOff1Misc = kOff1P + 2 * kPBuf;              // 196608
-constexpr int kSmemBytes = kOff0Misc + 4096 + 1024;        // the larger of the two + misc + alignment slack
+constexpr int kSmemBytes = kOff1Misc + 4096 + 1024;        // the larger of the two + misc + alignment slack
 constexpr int kThreads = 640;                  // 20 warps
 constexpr int kWarps = kThreads / 32;
 constexpr uint32_t kColQ = 0;                  // TMEM columns of CTA 0: Q (256), then two score buffers of 128
@@ -109,7 +111,6 @@ struct Misc0 {   // CTA 0
   unsigned long long q8_full;       // the token's rope block of Q has landed
   unsigned long long q8_free;       // tcgen05.commit behind the token's last tile
   unsigned long long p_free[2];     // relay warp of CTA 1 (remote arrival)
-  unsigned long long stage_free;    // correction warp 0 of CTA 1 (remote arrival): P and the factors of the tile have landed there
   unsigned long long epi_done[2];   // CTA 1 (remote arrival): the epilogue of token t (t % 2) is over
   uint32_t tmem_base;
   int abort_flag;
@@ -119,7 +120,6 @@ struct Misc0 {   // CTA 0
   unsigned short nt[2 * kBatch];    // per item of the current batch: number of tiles, first tile
   int last[kBatch];                 // entries of its list up to the last that is not negative
   float xchg[2][256];               // row maximum / row sum exchange between the two threads of a head row
-  alignas(16) float2 alpha_stage[128]; // rescale factors of a tile's halves on their way to CTA 1 (sent with P)
 };
 struct Misc1 {   // CTA 1
   unsigned long long v_full[kNV];   // one arrival per gather thread, when its copies have landed
@@ -142,7 +142,7 @@ struct Misc1 {   // CTA 1
   float inv_l[2][128];              // final 1/l of token t (t % 2)
 };
 static_assert(sizeof(Misc0) <= 4096 && sizeof(Misc1) <= 4096, "misc area");
-static_assert(kOff1Misc + 4096 + 1024 <= kSmemBytes, "CTA 1 layout fits");
+static_assert(kOff0Misc + 4096 + 1024 <= kSmemBytes, "CTA 0 layout fits");
 static_assert(kNV == kNT / kVSlabRows, "V ring slot index = slab index");
 
 // the same value in every lane, made visible to the compiler: loop counts and role state then stay in uniform registers
@@ -209,10 +209,33 @@ __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
       : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return r;
 }
-// bulk copy local shared memory -> shared memory of another CTA; completes (byte count) on that CTA's barrier
-__device__ __forceinline__ void bulk_copy_to_cluster(uint32_t dst_cluster, uint32_t src_cta, uint32_t bytes, uint32_t bar_cluster) {
-  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst_cluster), "r"(src_cta), "r"(bytes), "r"(bar_cluster) : "memory");
+// stores to the shared memory of another CTA that count their bytes on a barrier there
+__device__ __forceinline__ void st_async_v4(uint32_t dst_cluster, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t bar_cluster) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+               ::"r"(dst_cluster), "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar_cluster) : "memory");
+}
+__device__ __forceinline__ void st_async_v2(uint32_t dst_cluster, uint32_t a, uint32_t b, uint32_t bar_cluster) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];"
+               ::"r"(dst_cluster), "r"(a), "r"(b), "r"(bar_cluster) : "memory");
+}
+// mbar_wait on a barrier whose bytes come from the other CTA of the cluster
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  const uint32_t t0 = static_cast<uint32_t>(clock());
+#pragma unroll 1
+  for (;;) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity), "r"(kWaitSleepNs) : "memory");
+    if (ok != 0u) return true;
+    if (*abort_flag) return false;
+    if (static_cast<uint32_t>(clock()) - t0 > kWaitLimitCycles) {
+      *abort_flag = 1;
+      return false;
+    }
+  }
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // waits until the bulk stores of this thread have read their shared-memory source (the global writes
@@ -271,7 +294,6 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
       mbar_init(smem_u32(&m0->q8_full), 1);
       mbar_init(smem_u32(&m0->q8_free), 1);
       for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&m0->p_free[i]), 1); mbar_init(smem_u32(&m0->epi_done[i]), 1); }
-      mbar_init(smem_u32(&m0->stage_free), 1);
     } else {
       for (int i = 0; i < kNV; ++i) { mbar_init(smem_u32(&m1->v_full[i]), 64); mbar_init(smem_u32(&m1->v_free[i]), 1); }
       for (int i = 0; i < 2; ++i) {
@@ -374,11 +396,10 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
         const int rowi = tid & 127;
         const int ch = tid >> 7;
         const uint32_t p_remote = mapa_shared(base + kOff1P, 1);
-        const uint32_t p_local = base + kOff0P;
         const uint32_t alpha_remote = mapa_shared(smem_u32(&m1->alpha[0][0]), 1);
         const uint32_t invl_remote = mapa_shared(smem_u32(&m1->inv_l[0][0]), 1);
-        const uint32_t p_full_r[2] = {mapa_shared(smem_u32(&m1->p_full[0]), 1), mapa_shared(smem_u32(&m1->p_full[1]), 1)};
-        const uint32_t fin_r[2] = {mapa_shared(smem_u32(&m1->fin[0]), 1), mapa_shared(smem_u32(&m1->fin[1]), 1)};
+        const uint32_t p_full_r = mapa_shared(smem_u32(&m1->p_full[0]), 1);
+        const uint32_t fin_r = mapa_shared(smem_u32(&m1->fin[0]), 1);
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32);
         for (int t = 0; t < nb; ++t) {
           const int ti = batch0 + t;
@@ -475,36 +496,23 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
                 sum16[2 * q + g] = e[0].x + e[0].y;
               }
             }
-            // The weights wait in registers, so that the way of the tile before (its copies to CTA 1 and the report back, about
-            // 1500 cycles) is hidden by the exponentials of this one.
             // P buffer b of CTA 1 was last read by P.V of tile G-2
             if (G >= 2) mbar_wait(smem_u32(&m0->p_free[b]), ((G - 2) >> 1) & 1u, abort_flag);
-            // the staging area is single: CTA 1 reports as soon as the copies of the tile before have landed
-            if (G >= 1) mbar_wait(smem_u32(&m0->stage_free), (G - 1) & 1u, abort_flag);
-            // this thread's 64 columns are block `ch` of the P buffer: row rowi, eight 16-byte chunks
-            const uint32_t p_row = p_local + ch * kQBlock + rowi * 128;
+            // The weights go there straight from the registers, 512 bytes in a row per instruction, and count themselves on p_full (the
+            // arrival that announces them carries no release).  A staging area and bulk copies cost every tile a proxy fence of 400 to 1400
+            // cycles in the softmax, which is the longest stage; 16-byte stores into swizzled rows cost more than that.
+            if (lane == 0) mbar_arrive_expect_tx_cluster(p_full_r + b * 8, 32 * 128 + (ch == 0 ? 256 : 0));
+            __syncwarp();
+            const uint32_t p_row = p_remote + b * kPBuf + ch * 8 * kPChunk + rowi * 16;
 #pragma unroll
             for (int c = 0; c < 8; ++c)
-              st_shared_v4(p_row + ((c ^ (rowi & 7)) << 4), pk[c >> 2][4 * (c & 3)], pk[c >> 2][4 * (c & 3) + 1], pk[c >> 2][4 * (c & 3) + 2], pk[c >> 2][4 * (c & 3) + 3]);
+              st_async_v4(p_row + c * kPChunk, pk[c >> 2][4 * (c & 3)], pk[c >> 2][4 * (c & 3) + 1], pk[c >> 2][4 * (c & 3) + 2], pk[c >> 2][4 * (c & 3) + 3], p_full_r + b * 8);
+            if (ch == 0) st_async_v2(alpha_remote + (b * 128 + rowi) * 8, __float_as_uint(alpha_a), __float_as_uint(alpha_b), p_full_r + b * 8);
             l01 = fadd2(l01, make_float2(sum16[0], sum16[1]));
             l23 = fadd2(l23, make_float2(sum16[2], sum16[3]));
-            if (ch == 0) {
-              if (moves) {
-                l01 = fmul2(l01, alpha_b);
-                l23 = fmul2(l23, alpha_b);
-              }
-              m0->alpha_stage[rowi] = make_float2(alpha_a, alpha_b);
-            }
-            fence_proxy_async_smem();   // the bulk copies read this warp's rows through the async proxy
-            __syncwarp();
-            if (lane == 0) {
-              // this warp's 32 rows of block ch are 4 KB in a row, here and in CTA 1; the warps of block 0 also
-              // send the rescale factors of their 32 rows
-              const uint32_t off = ch * kQBlock + lane_base * 128;
-              mbar_arrive_expect_tx_cluster(p_full_r[b], 32 * 128 + (ch == 0 ? 256 : 0));
-              bulk_copy_to_cluster(p_remote + b * kPBuf + off, p_local + off, 32 * 128, p_full_r[b]);
-              if (ch == 0)
-                bulk_copy_to_cluster(alpha_remote + (b * 128 + lane_base) * 8, smem_u32(&m0->alpha_stage[lane_base]), 256, p_full_r[b]);
+            if (ch == 0 && moves) {
+              l01 = fmul2(l01, alpha_b);
+              l23 = fmul2(l23, alpha_b);
             }
           }
           gt += n_tiles;
@@ -525,7 +533,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
             }
           }
           __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(fin_r[ti & 1]);
+          if (lane == 0) mbar_arrive_cluster(fin_r + (ti & 1) * 8);
         }
       } else if (warp == 8) {
         // -------------------------------------------------------------- ring consumer: Q copies and Q.K^T
@@ -694,7 +702,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
       // ===================================================================== CTA 1: values
       const uint32_t v_s = base;
       const uint32_t p_s = base + kOff1P;
-      const uint32_t epi_done_r[2] = {mapa_shared(smem_u32(&m0->epi_done[0]), 0), mapa_shared(smem_u32(&m0->epi_done[1]), 0)};
+      const uint32_t epi_done_r = mapa_shared(smem_u32(&m0->epi_done[0]), 0);
       // ---------------------------------------------------------------- epilogue duty (16 warps: 0-7 and 9-16)
       // warp -> TMEM lane quarter warp % 4 (head rows 32q .. 32q+31) and column group g (output columns
       // 128g .. 128g+127): warps 0-3 g = 0, 4-7 g = 1, 9-12 g = 2, 13-16 g = 3.  A warp works alone: it
@@ -768,8 +776,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
         }
       };
       if (warp < 8) {
-        const uint32_t p_free_r[2] = {mapa_shared(smem_u32(&m0->p_free[0]), 0), mapa_shared(smem_u32(&m0->p_free[1]), 0)};
-        const uint32_t stage_free_r = mapa_shared(smem_u32(&m0->stage_free), 0);
+        const uint32_t p_free_r = mapa_shared(smem_u32(&m0->p_free[0]), 0);
         for (int t = 0; t < nb; ++t) {
           const int ti = batch0 + t;
           const int item = pair + ti * n_pairs;
@@ -779,8 +786,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
             for (int i = 0; i < n_tiles; ++i) {
               const uint32_t G = gt + i;
               const int b = G & 1;
-              mbar_wait(smem_u32(&m1->p_full[b]), (G >> 1) & 1u, abort_flag);
-              if (tid == 0) mbar_arrive_cluster_relaxed(stage_free_r);   // the copies have read CTA 0's staging area
+              mbar_wait_cluster(smem_u32(&m1->p_full[b]), (G >> 1) & 1u, abort_flag);
               auto rescale = [&](float a) {
                 tc_fence_after();
 #pragma unroll 1
@@ -819,7 +825,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
             for (int i = 0; i + 1 < n_tiles; ++i) {
               const uint32_t G = gt + i;
               mbar_wait(smem_u32(&m1->pv_done[G & 1]), (G >> 1) & 1u, abort_flag);
-              mbar_arrive_cluster_relaxed(p_free_r[G & 1]);
+              mbar_arrive_cluster_relaxed(p_free_r + (G & 1) * 8);
             }
           }
           __syncwarp();
@@ -829,15 +835,15 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
           // token may be replaced, once all 16 warps are through
           if (warp == 4 && lane == 0) {
             mbar_wait(smem_u32(&m1->epi_cnt), ti & 1u, abort_flag);
-            mbar_arrive_cluster_relaxed(p_free_r[(gt - 1) & 1]);
-            mbar_arrive_cluster_relaxed(epi_done_r[ti & 1]);
+            mbar_arrive_cluster_relaxed(p_free_r + ((gt - 1) & 1) * 8);
+            mbar_arrive_cluster_relaxed(epi_done_r + (ti & 1) * 8);
           }
         }
       } else if (warp == 8) {
         // -------------------------------------------------------------- P.V issuer (whole warp, an elected lane issues)
         {
           constexpr uint32_t kIdesc = umma_idesc(kFmtBF16, 128, 256, 0, 1);
-          const uint64_t ad0 = smem_desc_sw128(p_s, 16, 1024);
+          const uint64_t ad0 = smem_desc_sw128(p_s, kPChunk, 128) & ~(static_cast<uint64_t>(7) << 61);   // no swizzle: 8 x 16-byte matrices, the next along K a chunk on, the next of heads 128 bytes on
           const uint64_t bd0 = smem_desc_sw128(v_s, kVBlock, 1024);
           const uint32_t ad_lo = static_cast<uint32_t>(ad0), ad_hi = static_cast<uint32_t>(ad0 >> 32);
           const uint32_t bd_lo = static_cast<uint32_t>(bd0), bd_hi = static_cast<uint32_t>(bd0 >> 32);
@@ -862,13 +868,13 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
                 tc_fence_after();
                 if (elect_one()) {
                   // slab sl = 16-row steps 2 sl and 2 sl + 1 of the tile
-                  const uint32_t alo = a_lo + (((sl >> 1) * kQBlock + (sl & 1) * 64) >> 4);
+                  const uint32_t alo = a_lo + ((sl * 4 * kPChunk) >> 4);
                   const uint32_t blo = bd_lo + ((sl * kVSlab) >> 4);
 #pragma unroll
                   for (int kk = 0; kk < 2; ++kk) {
 #pragma unroll
                     for (int hv = 0; hv < 2; ++hv)
-                      umma_f16_ss(tmem + hv * 256, (static_cast<uint64_t>(ad_hi) << 32) | (alo + ((kk * 32) >> 4)),
+                      umma_f16_ss(tmem + hv * 256, (static_cast<uint64_t>(ad_hi) << 32) | (alo + ((kk * 2 * kPChunk) >> 4)),
                                   (static_cast<uint64_t>(bd_hi) << 32) | (blo + ((hv * 4 * kVBlock + kk * 2048) >> 4)), kIdesc,
                                   kk == 0 ? static_cast<uint32_t>(i | sl) : 1u);
                   }

@@ -563,9 +563,10 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
     const int item = first_item + t * n_ctas, next = item + n_ctas, tok_next = token_of(next);
     const uint32_t full = smem_u32(&misc->q_full);
     if (t >= 1) mbar_wait(smem_u32(&misc->q_free), (t - 1) & 1u, abort_flag);
-    if (lane == 0) mbar_arrive_expect_tx(full, static_cast<uint32_t>(min(p.h, NH) * 128 * kNChunk));   // rows past the last head arrive as zeros
+    const bool live = !__any_sync(0xffffffffu, *abort_flag);   // (after a wait that ran out nothing is announced or loaded any more)
+    if (lane == 0 && live) mbar_arrive_expect_tx(full, static_cast<uint32_t>(min(p.h, NH) * 128 * kNChunk));   // rows past the last head arrive as zeros
     __syncwarp();
-    if (lane < kNChunk) {
+    if (lane < kNChunk && live) {
       tma_load_3d(q_s + lane * Sh::kQBlock, &tm_q, full, lane * 64, (item / p.n_splits) % p.n_groups * NH, token_of(item));
       if (tok_next < p.s_q)
         asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"

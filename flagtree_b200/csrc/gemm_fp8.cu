@@ -15,7 +15,7 @@
 // Split K (S > 1, for grids that would leave SMs idle): the S CTAs (or pairs) of a cluster multiply S parts of K; the
 // fp32 partial tiles meet in shared memory over DSMEM, every part adds up 1/S of the columns in a fixed order and
 // writes them: no workspace, no second launch, no atomics.
-// Roles (384 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 4-11 promotion/epilogue: warp w takes
+// Roles (384 threads): warp 0 TMA producer (single tiles: of A, and warp 2 of B), warp 1 MMA issuer + TMEM owner, warps 4-11 promotion/epilogue: warp w takes
 // TMEM lanes 32 (w % 4) .. and half (w / 4 - 1) of the columns, so a thread holds 128 (64) fp32 sums.  Per K block a
 // thread needs one product of two scales: they are fetched from memory a group of four blocks ahead.
 // Measured, one GPU, K = 28672, N = 8192.  M = 4096 back to back, where the power limit sets the clock: 1064 us a call (1808 TFLOP/s) against
@@ -23,7 +23,10 @@
 // with pauses between them (TFLOP/s): M = 4096 2107 (before 1078), M = 1024 1130 (912).  Steps of M = 4096 that way: eight promotion
 // warps, scales ahead, single tiles 1269 and pairs 1037; the pair's hand-back of an accumulator as a relaxed remote
 // arrival (a release at cluster scope stalls the warp) 1921; the pieces of neighbouring K blocks as one stream 2107.
-// What bounds it now: with the additions left out 826 us instead of 913, with the tensor-memory loads left out too 680 us
+// Single tiles: 64 x 8192 x 3584 back to back 13.1 -> 12.3 us a call (29 MB, 4.4 us) with A and B loaded by two warps, two K blocks per wait
+// of the issuer, and one commit that tells both the producer and the promotion warps.  With pairs the same commit made M = 4096
+// slower (1119 us), so those keep their two.  What is left of the 12.3 is the fill of the pipeline and 64 columns of B per SM.
+// What bounds M = 4096 now: with the additions left out 826 us instead of 913, with the tensor-memory loads left out too 680 us
 // (the tensor pipe and the power limit: a library e4m3 GEMM reaches 2960).
 #include <cstring>
 
@@ -61,7 +64,7 @@ struct Params {
 struct Bars {
   unsigned long long full[STAGES];
   unsigned long long empty[STAGES];
-  unsigned long long blk_full[4];
+  unsigned long long blk_full[4];      // pairs only
   unsigned long long blk_empty[4];
   uint32_t tmem_base;
   int abort_flag;
@@ -139,7 +142,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   if (one_each) griddep_launch();
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(smem_u32(&bars->full[s]), 1);
+      mbar_init(smem_u32(&bars->full[s]), NCTA == 1 ? 2 : 1);   // A and B apart
       mbar_init(smem_u32(&bars->empty[s]), 1);
     }
     for (int a = 0; a < NACC; ++a) {
@@ -189,7 +192,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
 
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsFew));
-    if (warp == 0) {
+    if (warp == 0 || (NCTA == 1 && warp == 2)) {
+      // Single tiles: A by one warp, B by another, since a turn with two loads takes a lone thread 410 cycles, more than the MMAs' 256.
+      const bool is_b = warp == 2;
       if (lane == 0) {
         uint32_t s = 0, ph = 1;
         for (int t = group; t < p.n_tiles; t += n_groups) {
@@ -202,10 +207,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
             const uint32_t a_dst = base + s * STAGE_BYTES;
             if constexpr (NCTA == 1) {
               const uint32_t full = smem_u32(&bars->full[s]);
-              mbar_arrive_expect_tx(full, p.stage_tx);
-              tma_load_2d(a_dst, &tm_a, full, kb * BK, m_blk * BM);
-              if constexpr (B_KMAJOR) tma_load_2d(a_dst + A_BYTES, &tm_b, full, kb * BK, n0);
-              else tma_load_2d(a_dst + A_BYTES, &tm_b, full, n0, kb * BK);
+              const int x = is_b && !B_KMAJOR ? n0 : kb * BK, y = !is_b ? m_blk * BM : B_KMAJOR ? n0 : kb * BK;
+              mbar_arrive_expect_tx(full, is_b ? B_BYTES : p.stage_tx - B_BYTES);
+              tma_load_2d(is_b ? a_dst + A_BYTES : a_dst, is_b ? &tm_b : &tm_a, full, x, y);
             } else {
               // both CTAs' loads are counted on the even CTA's barrier; that CTA announces the total
               const uint32_t full = mapa_shared(smem_u32(&bars->full[s]), leader);
@@ -230,28 +234,62 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       constexpr uint32_t kBStep = (B_KMAJOR ? 32 : 4096) >> 4;   // 32 bytes of K, or 32 k-rows
       const uint16_t mask = static_cast<uint16_t>(3u << leader);
       const uint32_t full0 = smem_u32(&bars->full[0]), empty0 = smem_u32(&bars->empty[0]);
-      const uint32_t bf0 = smem_u32(&bars->blk_full[0]), be0 = smem_u32(&bars->blk_empty[0]);
+      const uint32_t be0 = smem_u32(&bars->blk_empty[0]);
       uint32_t s = 0, ph = 0, it = 0;   // it: K blocks issued so far = accumulator uses
       for (int t = group; t < p.n_tiles; t += n_groups) {
         bool live = true;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const uint32_t acc = it % NACC;
-          live = mbar_wait(full0 + s * 8, ph, abort_flag) && mbar_wait(be0 + acc * 8, ((it / NACC) & 1u) ^ 1u, abort_flag);
-          live = __all_sync(0xffffffffu, live);
-          if (!live) break;
-          tc_fence_after();
-          if (elect_one()) {
-            const uint32_t a_lo = ad_lo0 + ((s * STAGE_BYTES) >> 4), b_lo = bd_lo0 + ((s * STAGE_BYTES) >> 4);
-            const uint32_t d = tmem + acc * BN;
-            umma_f8_lohi<NCTA, false>(d, a_lo, ad_hi, b_lo, bd_hi, kIdesc);
+        if constexpr (NCTA == 1) {
+          // Two K blocks at a time, the stages and the accumulators waited for by different lanes at once: a wait costs the warp 120 cycles and a
+          // commit 60, the MMAs of a block take 256.  The one commit of a block frees its stage and hands its accumulator over: the promotion
+          // warps follow the stage's phase, which cannot run away from them, as block it + STAGES is not issued before it + 2 is promoted.
+          static_assert(STAGES % 2 == 0 && STAGES > NACC, "both blocks in one phase, accumulators reused before stages");
+          for (int kb = kb0; kb < kb1;) {
+            const int n = min(kb1 - kb, s % 2 == 0 ? 2 : 1);
+            const uint32_t which = n == 2 ? (lane >> 1) & 1u : 0u, acc = (it + which) % NACC;
+            live = (lane & 1) ? mbar_wait(be0 + acc * 8, (((it + which) / NACC) & 1u) ^ 1u, abort_flag) : mbar_wait(full0 + (s + which) * 8, ph, abort_flag);
+            live = __all_sync(0xffffffffu, live);
+            if (!live) break;
+            tc_fence_after();
+            if (elect_one()) {
 #pragma unroll
-            for (int k = 1; k < BK / 32; ++k)
-              umma_f8_lohi<NCTA, true>(d, a_lo + ((k * 32) >> 4), ad_hi, b_lo + k * kBStep, bd_hi, kIdesc);
-            commit_all<NCTA>(empty0 + s * 8, mask);
-            commit_all<NCTA>(bf0 + acc * 8, mask);
+              for (int j = 0; j < 2; ++j) {
+                if (j == n) break;
+                const uint32_t a_lo = ad_lo0 + (((s + j) * STAGE_BYTES) >> 4), b_lo = bd_lo0 + (((s + j) * STAGE_BYTES) >> 4);
+                const uint32_t acc_j = (it + j) % NACC, d = tmem + acc_j * BN;
+                umma_f8_lohi<NCTA, false>(d, a_lo, ad_hi, b_lo, bd_hi, kIdesc);
+#pragma unroll
+                for (int k = 1; k < BK / 32; ++k)
+                  umma_f8_lohi<NCTA, true>(d, a_lo + ((k * 32) >> 4), ad_hi, b_lo + k * kBStep, bd_hi, kIdesc);
+                commit_all<NCTA>(empty0 + (s + j) * 8, mask);
+              }
+            }
+            __syncwarp();
+            kb += n;
+            it += n;
+            s += n;
+            if (s == STAGES) { s = 0; ph ^= 1u; }
           }
-          __syncwarp();
-          if (++s == STAGES) { s = 0; ph ^= 1u; }
+        } else {
+          const uint32_t bf0 = smem_u32(&bars->blk_full[0]);
+          for (int kb = kb0; kb < kb1; ++kb, ++it) {
+            const uint32_t acc = it % NACC;
+            live = mbar_wait(full0 + s * 8, ph, abort_flag) && mbar_wait(be0 + acc * 8, ((it / NACC) & 1u) ^ 1u, abort_flag);
+            live = __all_sync(0xffffffffu, live);
+            if (!live) break;
+            tc_fence_after();
+            if (elect_one()) {
+              const uint32_t a_lo = ad_lo0 + ((s * STAGE_BYTES) >> 4), b_lo = bd_lo0 + ((s * STAGE_BYTES) >> 4);
+              const uint32_t d = tmem + acc * BN;
+              umma_f8_lohi<NCTA, false>(d, a_lo, ad_hi, b_lo, bd_hi, kIdesc);
+#pragma unroll
+              for (int k = 1; k < BK / 32; ++k)
+                umma_f8_lohi<NCTA, true>(d, a_lo + ((k * 32) >> 4), ad_hi, b_lo + k * kBStep, bd_hi, kIdesc);
+              commit_all<NCTA>(empty0 + s * 8, mask);
+              commit_all<NCTA>(bf0 + acc * 8, mask);
+            }
+            __syncwarp();
+            if (++s == STAGES) { s = 0; ph ^= 1u; }
+          }
         }
         if (!live) break;
       }
@@ -265,7 +303,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     const int lg = warp & 3, half = (warp >> 2) - 1;
     const uint32_t tacc = tmem_addr(tmem, lg * 32, half * COLS);
     const uint32_t be0 = NCTA == 1 ? smem_u32(&bars->blk_empty[0]) : mapa_shared(smem_u32(&bars->blk_empty[0]), leader);
-    uint32_t it = 0;
+    uint32_t it = 0, st = 0, st_ph = 0;       // K blocks so far; the stage that the next one goes through
     for (int t = group; t < p.n_tiles; t += n_groups) {
       int m_blk, n_blk;
       coords(t, m_blk, n_blk);
@@ -294,7 +332,12 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       uint32_t v[2][32];
       auto begin_block = [&]() {
         const uint32_t acc = it % NACC;
-        mbar_wait(smem_u32(&bars->blk_full[acc]), (it / NACC) & 1u, abort_flag);
+        if constexpr (NCTA == 1) {
+          mbar_wait(smem_u32(&bars->empty[st]), st_ph, abort_flag);
+          if (++st == STAGES) { st = 0; st_ph ^= 1u; }
+        } else {
+          mbar_wait(smem_u32(&bars->blk_full[acc]), (it / NACC) & 1u, abort_flag);
+        }
         __syncwarp();
         tc_fence_after();
         tmem_ld32(tacc + acc * BN, v[0]);

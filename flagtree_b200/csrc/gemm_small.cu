@@ -5,10 +5,11 @@
 // however deep its pipeline.  So the tile is 128 x 64 or 128 x 128, one tile per CTA, and where even those are few the K axis is
 // split over the CTAs of a cluster: their fp32 partial tiles meet in shared memory over DSMEM, every part adds up its
 // share of the columns in a fixed order and writes them (no workspace, no second launch, no atomics).
-// Measured (us, weights cold in L2, persistent kernel -> this one): 50 x 7168 x 2304 19.2 -> 12.1, 1 x 512 x 2304 15.4 -> 7.0 (four
+// Measured (us, weights cold in L2, persistent kernel -> this one): 50 x 7168 x 2304 19.2 -> 12.1 (back to back 10.1; 9.4 with A and B loaded
+// by two warps and two K blocks per wait of the issuer), 1 x 512 x 2304 15.4 -> 7.0 (four
 // parts), 128 x 4096 x 1152 13.4 -> 8.6, 512 x 4096 x 2304 19.9 -> 14.3.  The floor of the first is 5.2 (33 MB); what is left is
 // launch, the fill of the pipeline and 64 columns per SM at 64 bytes per clock.
-// Roles (192 threads): warp 0 TMA producer, warp 1 MMA issuer (owns TMEM), warps 2-5 epilogue (TMEM lanes 32 (warp % 4) ..).
+// Roles (224 threads): warps 0 and 6 TMA producers, warp 1 MMA issuer (owns TMEM), warps 2-5 epilogue (TMEM lanes 32 (warp % 4) ..).
 #include <cstring>
 
 #include "launch.cuh"
@@ -25,7 +26,7 @@ namespace gemm_small {
 constexpr int BM = 128, BK = 64;
 constexpr int A_BYTES = BM * BK * 2;          // 16384
 constexpr int B_BLOCK_BYTES = BK * 128;       // 8192: 64 k-rows x 64 columns
-constexpr int THREADS = 192;
+constexpr int THREADS = 224;
 template <int BN> struct Cfg {
   static constexpr int STAGES = BN == 64 ? 8 : 6;
   static constexpr int STAGE_BYTES = A_BYTES + BN / 64 * B_BLOCK_BYTES;
@@ -34,7 +35,7 @@ template <int BN> struct Cfg {
 
 struct Params {
   int m, n, n_blocks, kb_total, splits;
-  uint32_t stage_tx;
+  uint32_t stage_tx;          // bytes of A per stage
   __nv_bfloat16* c;
   long long ldc;
   int* status;
@@ -64,7 +65,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 
   griddep_launch();
   if (tid == 0) {
-    for (int s = 0; s < STAGES; ++s) { mbar_init(smem_u32(&bars->full[s]), 1); mbar_init(smem_u32(&bars->empty[s]), 1); }
+    for (int s = 0; s < STAGES; ++s) { mbar_init(smem_u32(&bars->full[s]), 2); mbar_init(smem_u32(&bars->empty[s]), 1); }
     mbar_init(smem_u32(&bars->acc_full), 1);
     fence_mbar_init();
     tma_prefetch_desc(&tm_a);
@@ -84,16 +85,21 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   const uint32_t tmem = bars->tmem_base;
 
   float acc[BN];
-  if (warp == 0) {
+  if (warp == 0 || warp == 6) {
+    // B by one warp, A by another: a turn with all loads takes a lone thread longer than the MMAs of a K block
     if (lane == 0) {
       uint32_t s = 0, ph = 1;
       for (int kb = kb0; kb < kb1 && !dead; ++kb) {
         if (!mbar_wait(smem_u32(&bars->empty[s]), ph, abort_flag)) break;
         const uint32_t dst = base + s * STAGE_BYTES, full = smem_u32(&bars->full[s]);
-        mbar_arrive_expect_tx(full, p.stage_tx);
+        if (warp == 0) {
+          mbar_arrive_expect_tx(full, BN / 64 * B_BLOCK_BYTES);
 #pragma unroll
-        for (int j = 0; j < BN / 64; ++j) tma_load_2d(dst + A_BYTES + j * B_BLOCK_BYTES, &tm_b, full, n0 + j * 64, kb * BK);
-        tma_load_2d(dst, &tm_a, full, kb * BK, m_blk * BM);
+          for (int j = 0; j < BN / 64; ++j) tma_load_2d(dst + A_BYTES + j * B_BLOCK_BYTES, &tm_b, full, n0 + j * 64, kb * BK);
+        } else {
+          mbar_arrive_expect_tx(full, p.stage_tx);
+          tma_load_2d(dst, &tm_a, full, kb * BK, m_blk * BM);
+        }
         if (++s == STAGES) { s = 0; ph ^= 1u; }
       }
     }
@@ -101,20 +107,30 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   } else if (warp == 1) {
     constexpr uint32_t kIdesc = umma_idesc(kFmtBF16, BM, BN, 0, 1);
     const uint64_t ad = smem_desc_sw128(base, 16, 1024), bd = smem_desc_sw128(base + A_BYTES, B_BLOCK_BYTES, 1024);
+    // Two K blocks at a time, their barriers waited for by different lanes: a wait, an election and a commit cost the warp about 250 cycles
+    // between the MMAs of a block, which take 130 to 200.
+    const uint32_t full0 = smem_u32(&bars->full[0]), empty0 = smem_u32(&bars->empty[0]);
     uint32_t s = 0, ph = 0;
-    for (int kb = kb0; kb < kb1 && !dead; ++kb) {
-      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->full[s]), ph, abort_flag))) break;
+    static_assert(STAGES % 2 == 0, "both blocks in one phase");
+    for (int kb = kb0; kb < kb1 && !dead; kb += 2) {
+      const bool two = kb + 1 < kb1;
+      if (!__all_sync(0xffffffffu, mbar_wait(full0 + (s + (two ? lane & 1 : 0)) * 8, ph, abort_flag))) break;
       tc_fence_after();
       if (elect_one()) {
-        const uint64_t off = (s * STAGE_BYTES) >> 4;
 #pragma unroll
-        for (int k = 0; k < BK / 16; ++k)
-          umma_f16_ss(tmem, ad + off + ((k * 32) >> 4), bd + off + ((k * 2048) >> 4), kIdesc, k == 0 ? (kb > kb0 ? 1u : 0u) : 1u);
-        umma_commit(smem_u32(&bars->empty[s]));
-        if (kb + 1 == kb1) umma_commit(smem_u32(&bars->acc_full));
+        for (int j = 0; j < 2; ++j) {
+          if (j == 1 && !two) break;
+          const uint64_t off = ((s + j) * STAGE_BYTES) >> 4;
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k)
+            umma_f16_ss(tmem, ad + off + ((k * 32) >> 4), bd + off + ((k * 2048) >> 4), kIdesc, j == 0 && k == 0 ? (kb > kb0 ? 1u : 0u) : 1u);
+          if (kb + j + 1 == kb1) umma_commit(smem_u32(&bars->acc_full));
+          else umma_commit(empty0 + (s + j) * 8);
+        }
       }
       __syncwarp();
-      if (++s == STAGES) { s = 0; ph ^= 1u; }
+      s += 2;
+      if (s == STAGES) { s = 0; ph ^= 1u; }
     }
   } else {
     if (!dead) mbar_wait(smem_u32(&bars->acc_full), 0, abort_flag);
@@ -132,7 +148,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   }
 
   const int row_in = (warp & 3) * 32 + lane, row = m_blk * BM + row_in;
-  const bool writes = warp >= 2 && row < p.m && !*abort_flag;
+  const bool epilogue = warp >= 2 && warp < 6, writes = epilogue && row < p.m && !*abort_flag;
   auto put8 = [&](const float* f, int col) {                // n is a multiple of 8
     if (n0 + col < p.n) {
       uint4 o;
@@ -151,7 +167,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     // [s cw, (s + 1) cw), as 16-byte pieces with the row fastest.
     cluster_sync_all();
     const int cw = BN / p.splits;
-    if (warp >= 2) {
+    if (epilogue) {
 #pragma unroll
       for (int c4 = 0; c4 < BN / 4; ++c4) {
         const int to = c4 * 4 / cw;
@@ -217,7 +233,7 @@ static int launch(const void* a, const void* b, void* c, int m, int n, int k, lo
   p.n_blocks = (n + BN - 1) / BN;
   p.kb_total = (k + BK - 1) / BK;
   p.splits = splits;
-  p.stage_tx = static_cast<uint32_t>(box_m * BK * 2 + BN / 64 * B_BLOCK_BYTES);
+  p.stage_tx = static_cast<uint32_t>(box_m * BK * 2);
   p.c = static_cast<__nv_bfloat16*>(c);
   p.ldc = ldc;
   p.status = status;

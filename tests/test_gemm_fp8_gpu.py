@@ -57,6 +57,17 @@ def test_fp8_unit_scales_equal_plain_product():
                                    (129, 8192, 256), (520, 4224, 640), (1025, 8064, 128), (2049, 4224, 384)])
 @pytest.mark.parametrize("nk", [False, True])
 def test_fp8_tile_shapes_and_parts_of_k(m, n, k, nk):
+    _check_fp8(m, n, k, nk)
+
+
+# Single tiles take two K blocks per wait: odd counts in one part and in unequal parts (7 and 13 in four), and CTAs with two tiles
+# (19 200 columns, 150 tiles), whose second one begins in the middle of such a pair of stages.
+@pytest.mark.parametrize("m,n,k", [(64, 1024, 384), (50, 512, 896), (33, 3968, 1664), (64, 19200, 384), (128, 19200, 640)])
+def test_fp8_odd_counts_of_k_blocks(m, n, k):
+    _check_fp8(m, n, k, False)
+
+
+def _check_fp8(m, n, k, nk):
     g = torch.Generator(device=DEV).manual_seed(m + n + k)
     a8, a_s = W.quantize_block_e4m3(torch.randn(m, k, generator=g, device=DEV), 1, 128)
     b8, b_s = W.quantize_block_e4m3(torch.randn(k, n, generator=g, device=DEV), 128, 128)

@@ -46,6 +46,14 @@ def test_products_with_few_tiles(m, n, k):
     assert torch.equal(c, matmul(a.to(DEV), b.to(DEV)))
 
 
+@pytest.mark.parametrize("k", [64, 192, 448, 832, 1096])
+@pytest.mark.parametrize("m,n", [(50, 1024), (128, 9472)])
+def test_narrow_tiles_with_odd_counts_of_k_blocks(m, n, k):
+    """The narrow tiles take two K blocks per wait: counts of 1, 3, 7, 13 and 18 (the last one short), in one part and split unequally."""
+    g = torch.Generator().manual_seed(m + n + k)
+    _check(torch.randn(m, k, generator=g).bfloat16(), torch.randn(k, n, generator=g).bfloat16(), f"{m}x{n}x{k}")
+
+
 @pytest.mark.parametrize("m,n,k", [(4096, 4864, 256), (2048, 9992, 128), (3072, 2560, 192)])
 def test_leftover_tiles_run_as_half_width_steps(m, n, k):
     """Shapes whose tile count leaves a few tiles after the whole waves of a 148-SM GPU: 304 = 4 x 74 + 8 pair

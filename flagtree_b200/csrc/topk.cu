@@ -34,6 +34,10 @@ __device__ __forceinline__ uint32_t to_key(uint32_t u) {
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
+__device__ __forceinline__ float to_float(uint32_t key) {
+  return __uint_as_float((key & 0x80000000u) ? key & 0x7fffffffu : ~key);
+}
+
 __device__ __forceinline__ int row_len(const Params& p, int row) {
   const int len = p.lengths != nullptr ? p.lengths[row] : p.s_kv;
   return max(0, min(len, p.s_kv));
@@ -179,7 +183,10 @@ __global__ void __launch_bounds__(kThreads) topk_select_kernel(const Params p) {
 // compare, vote, store).  The few positions in the mask, an eighth of the row or so, become a list in ascending order, and
 // their keys are fetched again, out of L2.  The list is counted against four trial values at a time, quantiles of the sample
 // first, then values interpolated between the counts known so far, until 128 candidates are left, which are ranked by
-// counting.  The list is in order, so the taken ones among it are the output as they come.
+// counting.  A lane works out one of the four values and what its count means: with all four in every thread a trial took a lone row 1900
+// cycles for four keys a thread.  Interpolated are the floats, not the keys, whose density doubles with every power of two
+// towards zero (100 rows of 32 768, topk 16 384, the median: 46 -> 24 us).
+// The list is in order, so the taken ones among it are the output as they come.
 // Where a value fills so much of the row that keys equal to the bound would crowd the list, the list takes the keys above it and
 // the ties go to a mask of their own in the same sweep.  A bound that turns out too high, or more keys than the list has room
 // for (both checked), costs time and never exactness: the row is then selected by the radix select, out of L2.
@@ -188,9 +195,10 @@ __global__ void __launch_bounds__(kThreads) topk_select_kernel(const Params p) {
 // What bounds it: instruction issue (0.69 a clock and scheduler, a row of 32768 some 40 000) and chains of latencies (sample, bound, sweep, list,
 // keys, trials), which the other CTAs of the SM fill; memory is at a quarter of its rate.  Copying the keys to the list in the sweep itself,
 // instead of voting, took 130 instructions per 128 keys (4096 x 32 768, topk 2048: 293 us; with votes 234, with the tail of the row apart 210).
-// Against persistent CTAs that hold a row in registers and histogram it (us, before / now): 4096 x 32 768 causal 334 / 210, 4096 x 20 001
-// topk 1024 426 / 151, 4096 x 6000 277 / 103, 4096 x 1000 topk 512 85 / 57, 592 rows of 33 000 82 / 35, 592 rows of 32 768 equal scores 52 / 40,
-// 128 rows of up to 65 536 30 / 19, 300 short rows of a matrix of 65 536 columns 44 / 17; slower: 100 rows of 32 768 with topk 16 384 27 / 46.
+// Against persistent CTAs that hold a row in registers and histogram it (us, before / now): 4096 x 32 768 causal 334 / 205, 4096 x 20 001
+// topk 1024 426 / 120, 4096 x 6000 277 / 98, 4096 x 4000 topk 512 189 / 65, 4096 x 1000 topk 512 83 / 51, 592 rows of 33 000 82 / 36,
+// 592 rows of 32 768 equal scores 52 / 40, 128 rows of up to 65 536 30 / 17, 300 short rows of a matrix of 65 536 columns 44 / 16, one row of
+// 32 768 13.1 / 11.5, of 4000 11.2 / 7.8; level or up to 8 % slower: rows of 32 768 with topk 4096 and more (148: 14.9 / 15.5, 4096 with 16 384: 588 / 648).
 // ---------------------------------------------------------------------------------------------------------------
 namespace listed {
 
@@ -207,16 +215,19 @@ struct Shape {
   int room;                                                // list entries
   int words;                                               // of a mask over the row
 };
-// The list has room for what the bound is expected to let through and four standard deviations more; 0 where that is more than an SM has.
+// The list has room for what the bound is expected to let through and four standard deviations more (never less for a longer row); 0 where
+// that is more than an SM has.  A row is taken whole, without a sweep, where it is short or most of it would pass the bound (us,
+// whole / swept: 4096 rows of 4000, topk 512 89 / 65, topk 2048 88 / 90; of 2000, topk 512 68 / 62, topk 1024 70 / 72; one row of 2000, topk 512 6.0 / 6.7,
+// of 3000 7.3 / 7.0; 148 rows with an SM each, of 8192 topk 4096 9.9 / 11.8, of 12 000 topk 4096 12.9 / 12.6, of 20 000 topk 2048 17.4 / 12.2).
 inline int plan(int s_kv, int topk, bool alone, Shape* shape) {
   if (s_kv > kRowMax) return 0;
   const double k = topk < s_kv ? topk : s_kv, n = s_kv < kSample ? s_kv : kSample, frac = k / s_kv;
   const double r = n * frac + kMargin * std::sqrt(n * frac * (1.0 - frac)) + 3.0 + kCrowd;   // rank of the bound in the sample
-  const int wanted = static_cast<int>((r + 4.0 * std::sqrt(r)) / n * s_kv) + 64, whole = s_kv < 4096 ? s_kv : 4096;
+  const int wanted = static_cast<int>((r + 4.0 * std::sqrt(r)) / n * s_kv) + 64;
   shape->words = (s_kv + 31) / 32;
-  shape->room = wanted > s_kv ? s_kv : wanted > whole ? wanted : whole;
   const int most = (kSmemMax - 8 * shape->words) / 6;
-  if (alone && shape->room > s_kv / 4 && s_kv <= most) shape->room = s_kv;   // the SM's memory is there, and a row as a whole needs no sweep
+  const bool whole = s_kv <= (alone ? 2048 : 1024) || (wanted > 0.6 * s_kv && s_kv <= (alone ? most : 4096));
+  shape->room = whole || wanted > s_kv ? s_kv : wanted;
   if (shape->room > most) {
     if (most < 1.1 * r / n * s_kv) return 0;
     shape->room = most;
@@ -308,6 +319,7 @@ __global__ void __launch_bounds__(kThr, kBlocks) topk_listed_kernel(const Params
   const int words = (len + 31) >> 5;
   int n_list = len;
   if (whole) {
+#pragma unroll 8
     for (int i = tid; i < len; i += kThr) {
       keys[i] = to_key(src[i]);
       at_pos[i] = static_cast<unsigned short>(i);
@@ -450,20 +462,25 @@ __global__ void __launch_bounds__(kThr, kBlocks) topk_listed_kernel(const Params
   int need_eq = 0;
   int c_lo = n_list, c_hi = 0;                             // keys >= lo, keys > hi; c_lo >= k > c_hi at all times
   // every third time the values cut the interval in five, whatever the counts say
+  int trial = 0;
+  const int tj = lane & 3;                                 // a lane works out one of the four values, and what its count means
 #pragma unroll 1
-  for (int trial = 0; c_lo != k && lo != hi && c_lo - c_hi > kFew; ++trial) {
-    uint32_t mid[4], c01 = 0, c23 = 0;
+  for (; c_lo != k && lo != hi && c_lo - c_hi > kFew; ++trial) {
+    uint32_t own;
     if (trial == 0) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) mid[j] = min(max(sm.first[j], lo + 1u), hi);
+      own = tj == 0 ? min(sm.first[0], sm.first[1]) : sm.first[tj];                  // (the first may have more bits)
     } else {
-      const float share = __fdividef(static_cast<float>(c_lo - k) + 0.5f, static_cast<float>(c_lo - c_hi)), width = static_cast<float>(hi - lo);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float cut = trial % 3 == 0 ? 0.2f * static_cast<float>(j + 1) : share + (j == 0 ? -0.12f : j == 1 ? -0.03f : j == 2 ? 0.03f : 0.12f);
-        mid[j] = lo + 1u + min(static_cast<uint32_t>(fmaxf(cut, 0.0f) * width), hi - lo - 1u);
-      }
+      const float share = __fdividef(static_cast<float>(c_lo - k) + 0.5f, static_cast<float>(c_lo - c_hi));
+      const float f_lo = to_float(lo), f_width = to_float(hi) - f_lo;                // not finite where an end is an infinity or a NaN
+      const bool even = trial % 3 == 0;
+      const float cut = fmaxf(even ? 0.2f * static_cast<float>(tj + 1) : share + (tj == 0 ? -0.12f : tj == 1 ? -0.03f : tj == 2 ? 0.03f : 0.12f), 0.0f);
+      own = !even && f_width < 3.0e38f ? to_key(__float_as_uint(f_lo + cut * f_width))
+                                       : lo + 1u + min(static_cast<uint32_t>(cut * static_cast<float>(hi - lo)), hi - lo - 1u);
     }
+    own = min(max(own, lo + 1u), hi);                      // ascending in tj
+    uint32_t mid[4], c01 = 0, c23 = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) mid[j] = __shfl_sync(0xffffffffu, own, j);
 #pragma unroll 4
     for (int i = tid; i < n_list; i += kThr) {
       const uint32_t x = keys[i];
@@ -477,12 +494,13 @@ __global__ void __launch_bounds__(kThr, kBlocks) topk_listed_kernel(const Params
     __syncthreads();
     c01 = __reduce_add_sync(0xffffffffu, lane < kWarps ? sums[0][lane] : 0u);
     c23 = __reduce_add_sync(0xffffffffu, lane < kWarps ? sums[1][lane] : 0u);
-    const int c[4] = {static_cast<int>(c01 & 0xffffu), static_cast<int>(c01 >> 16), static_cast<int>(c23 & 0xffffu), static_cast<int>(c23 >> 16)};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (c[j] >= k && mid[j] > lo) { lo = mid[j]; c_lo = c[j]; }
-      if (c[j] < k && mid[j] <= hi) { hi = mid[j] - 1u; c_hi = c[j]; }
-    }
+    const uint32_t c_two = tj < 2 ? c01 : c23;
+    const int c = static_cast<int>((tj & 1) ? c_two >> 16 : c_two & 0xffffu);
+    const int reach = __popc(__ballot_sync(0xffffffffu, c >= k) & 15u);              // values that k keys or more reach: the first ones
+    const int below = __shfl_sync(0xffffffffu, c, max(reach - 1, 0)), past = __shfl_sync(0xffffffffu, c, min(reach, 3));
+    const uint32_t at_below = __shfl_sync(0xffffffffu, own, max(reach - 1, 0)), at_past = __shfl_sync(0xffffffffu, own, min(reach, 3));
+    if (reach > 0) { lo = at_below; c_lo = below; }
+    if (reach < 4) { hi = at_past - 1u; c_hi = past; }
   }
   if (c_lo != k && lo != hi) {                             // few left: the one of which k - c_hi are not smaller
     for (int i0 = warp * 32; i0 < n_list; i0 += kThr) {
@@ -503,7 +521,7 @@ __global__ void __launch_bounds__(kThr, kBlocks) topk_listed_kernel(const Params
     const int which = tid / kRankers;
     const uint32_t v = sm.few[which];
     int above = 0, from = 0;
-    for (int m = (tid % kRankers) * 4; m < total; m += kRankers * 4) {               // (past the last candidate: 0, below every key of the list)
+    for (int m = warp * (32 / kRankers) < total ? (tid % kRankers) * 4 : total; m < total; m += kRankers * 4) {   // (past the last candidate: 0, below every key of the list)
       const uint4 o = *reinterpret_cast<const uint4*>(&sm.few[m]);
       above += (o.x > v) + (o.y > v) + (o.z > v) + (o.w > v);
       from += (o.x >= v) + (o.y >= v) + (o.z >= v) + (o.w >= v);
@@ -532,11 +550,11 @@ __global__ void __launch_bounds__(kThr, kBlocks) topk_listed_kernel(const Params
   }
   taken = static_cast<int>(__reduce_add_sync(0xffffffffu, taken));
   equal = static_cast<int>(__reduce_add_sync(0xffffffffu, equal));
-  __syncthreads();                                         // the trials have read `sums`
-  if (lane == 0) { sm.sums[0][warp] = static_cast<uint32_t>(taken); sm.sums[1][warp] = static_cast<uint32_t>(equal); }
+  uint32_t(*sums)[32] = &sm.sums[(trial & 1) * 2];         // not those of the last trial, which another warp may still read
+  if (lane == 0) { sums[0][warp] = static_cast<uint32_t>(taken); sums[1][warp] = static_cast<uint32_t>(equal); }
   __syncthreads();
-  int write_at = static_cast<int>(__reduce_add_sync(0xffffffffu, lane < warp ? sm.sums[0][lane] : 0u));
-  int eq_left = need_eq - static_cast<int>(__reduce_add_sync(0xffffffffu, lane < warp ? sm.sums[1][lane] : 0u));
+  int write_at = static_cast<int>(__reduce_add_sync(0xffffffffu, lane < warp ? sums[0][lane] : 0u));
+  int eq_left = need_eq - static_cast<int>(__reduce_add_sync(0xffffffffu, lane < warp ? sums[1][lane] : 0u));
   write_at += need_eq - max(eq_left, 0);                   // the ties of the warps before
   const uint32_t lower = (1u << lane) - 1u;
   for (int i0 = i_begin; i0 < i_end; i0 += 32) {
@@ -581,11 +599,16 @@ extern "C" FTB_API int ftb_topk_indices(const ftb_topk_args* a, void* stream) {
   // one of 32768 14.4 / 13.6).  More rows: six small CTAs to an SM hide their chains better, three larger ones keep fewer lists and rows
   // in flight (256 threads / 512: 4096 rows of 1000 56 / 79, of 6000 103 / 134, of 20001 151 / 159, of 32768 236 / 210; 592 of 33000 35 / 41;
   // 600 of 32768 with topk 8192 101 / 76).
-  const bool alone = a->s_q <= sm_count;
+  // Lists so long that an SM holds one count as rows alone (600 rows of 32 768 with topk 16 384: 512 threads 136, 1024 96).
+  bool alone = a->s_q <= sm_count;
   topk::listed::Shape shape;
   int smem = topk::listed::plan(a->s_kv, a->topk, alone, &shape);
+  if (!alone && smem > topk::listed::kSmemMax / 2) {
+    alone = true;
+    smem = topk::listed::plan(a->s_kv, a->topk, alone, &shape);
+  }
   if (smem > 0) {
-    const bool small = alone ? a->s_kv <= 8192 : a->topk <= 4096 && (a->s_kv <= 24576 || a->s_q <= 6 * sm_count);
+    const bool small = alone ? a->s_kv <= 8192 : a->topk <= 4096 && (a->s_kv <= 24576 || (a->s_q <= 6 * sm_count && a->topk <= 2048));
     const auto kernel = alone ? (small ? topk::listed::topk_listed_kernel<512, 1> : topk::listed::topk_listed_kernel<1024, 1>)
                               : (small ? topk::listed::topk_listed_kernel<256, 6> : topk::listed::topk_listed_kernel<512, 3>);
     if (alone && smem < topk::listed::kSmemAlone) smem = topk::listed::kSmemAlone;

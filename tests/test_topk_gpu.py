@@ -154,6 +154,17 @@ def test_lists_of_candidates(rows, s_kv, topk, values):
     assert torch.equal(got, topk_indices_ref(wide[:, 1:1 + s_kv], topk, lengths))
 
 
+@pytest.mark.parametrize("rows,s_kv,topk", [(2, 2048, 512), (2, 2049, 512), (150, 1024, 300), (150, 1025, 300), (150, 4096, 2400), (150, 4097, 2400),
+                                            (150, 32768, 16384), (4, 20000, 9000), (4, 20000, 10000), (900, 24577, 2049)])
+@pytest.mark.parametrize("values", ["plain", "huge"])
+def test_whole_rows_and_long_lists(rows, s_kv, topk, values):
+    """Both sides of the lines between rows taken whole and rows swept, and lists that fill an SM; scores among which an interval of the
+    search ends in an infinity or is wider than the largest float."""
+    g = torch.Generator().manual_seed(rows + s_kv + topk + 1)
+    sc = torch.randn(rows, s_kv, generator=g) * (2e38 if values == "huge" else 1.0)
+    assert torch.equal(topk_indices(sc.to(DEV), topk).cpu(), topk_indices_ref(sc, topk))
+
+
 @pytest.mark.parametrize("top", [0.0, 1e6, -1e6])
 def test_sample_that_misleads(top):
     """The sampled positions hold values unlike the rest: a bound that is too high, or a list that overflows, sends the row to the radix select."""

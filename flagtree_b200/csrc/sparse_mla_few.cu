@@ -28,6 +28,12 @@
 // tiles in thirds and 16 rows freed at a time 780 / 974 (each turn of the issuer cost 330 cycles, most of it the proxy fence), the fence
 // moved to the gather warps 741 / 920, two issuers 512 / 719, the first reference from two tiles 525 / 759.  Device time of few tokens in parts,
 // pairs / here: 1 token of 16 heads 17.0 / 11.3, 74 tokens of 64 heads 45.6 / 40.0, 1 token of 128 heads 21.2 / 14.7, 16 of them 29.9 / 25.5.
+// Taken back: the weights written while the warps vote on the references through an mbarrier 517 -> 549 / 733 -> 772 (its wait costs more
+// than the named barrier); pairs of CTAs that share the rows of a token's two head groups 186 -> 190 (a decode step).
+//
+// e4m3 pages (kFp8).  The gather warps resolve the page table, load a row's bytes, convert them to bf16 times the page's scale
+// (as the dequantised table had them) and write the same slots, so nothing goes through a table in memory.  128 tokens of 128 heads, topk 2048: dequantisation and
+// attention one after the other 212 us, here 149; three tokens in parts 23 -> 19 (one-pass kernel of one CTA 28.7).
 // Every wait is bounded; a wait that runs out sets the abort flag, after which every later wait returns at once.
 #include <cuda_fp8.h>
 

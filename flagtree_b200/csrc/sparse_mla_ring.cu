@@ -2,7 +2,7 @@
 //
 // One pair of CTAs (a cluster of 2) walks through query tokens pair, pair + pairs, ...  CTA 0 computes
 // S = Q.K^T (Q in tensor memory, K column blocks gathered into shared memory by cp.async) and the
-// softmax; P travels to CTA 1 by bulk copies over distributed shared memory; CTA 1 accumulates O += P.V in
+// softmax; P travels to CTA 1 by asynchronous stores over distributed shared memory; CTA 1 accumulates O += P.V in
 // tensor memory and writes the output.  Every barrier keeps counting across tokens.
 //
 // The slots of CTA 0.  Nine slots of [128 rows x 128 B], one per 64-column block: per token the blocks of the token's query
@@ -26,8 +26,7 @@
 // role but the MMA issue has one rolled loop, the softmax has one path (masked entries become -inf once) with two-wide
 // fp32 instructions, loop counts are warp-uniform, and the issuer has constant addresses and waits for three blocks at once.
 // Warps whose 32 head rows hold no head take no part.  One launch alone, 740 tokens, 128 heads, topk 2048: 832 -> 1065
-// TFLOP/s.  Back to back, in turn on one box: 4096 causal tokens 2244 -> 1944 us; 1999 tokens of 16 heads 1327 -> 970 us (1159 with all
-// rows at work, 1076 with a ring of ten slots and computed addresses).
+// TFLOP/s.  Back to back, in turn on one box: 4096 causal tokens 2244 -> 1944 us, with the weights sent straight from registers 1881.
 //
 // Few tokens.  A launch may cut the top-k list of every token in parts; an item of work is then a part of a token, its result
 // leaves as fp32 (32 columns per TMA store instead of 64) with a base-2 LSE, and a second kernel merges the parts.  One token
@@ -35,9 +34,9 @@
 // half sectors.)
 //
 // Softmax: two threads per head row; the running maximum moves only when it grows by more than 2^8, so that
-// the accumulator in CTA 1 is rarely rescaled.  P (bf16) and the rescale factors go to a staging area and
-// from there to CTA 1 with bulk copies that complete on CTA 1's barrier; the arrival that announces them
-// carries no release (the data travels with the copies), which keeps the softmax warps from stalling.
+// the accumulator in CTA 1 is rarely rescaled.  P (bf16) and the rescale factors go from registers to
+// CTA 1 with st.async, which count on CTA 1's barrier; the arrival that announces them
+// carries no release (the data travels with the stores), which keeps the softmax warps from stalling.
 //
 // The number of tiles of an item (last non-negative index, rounded up to 128 rows, at least one) is
 // found for 64 items at a time by all warps of a CTA, with CTA barriers between.
@@ -124,7 +123,7 @@ struct Misc0 {   // CTA 0
 struct Misc1 {   // CTA 1
   unsigned long long v_full[kNV];   // one arrival per gather thread, when its copies have landed
   unsigned long long v_free[kNV];   // tcgen05.commit
-  unsigned long long p_full[2];     // softmax warps with heads of CTA 0 (remote arrivals, each announcing its bulk copies: 4 KB of P, 256 B of factors)
+  unsigned long long p_full[2];     // softmax warps with heads of CTA 0 (remote arrivals, each announcing what it sends: 4 KB of P, 256 B of factors)
   unsigned long long corr_done[2];  // correction warps with heads
   unsigned long long half_done[4];  // per correction warp: tcgen05.commit behind the first half of a tile whose second half moves one of its maxima
   unsigned long long half_corr[4];  // the warp: its rows of the accumulator are ready for that second half
@@ -138,7 +137,7 @@ struct Misc1 {   // CTA 1
   uint32_t late[2];                 // a byte per correction warp: does the second half of the tile move one of its maxima?
   unsigned short nt[2 * kBatch];
   int last[kBatch];
-  alignas(16) float2 alpha[2][128];  // rescale factors of the halves of a tile (two buffers), written by bulk copies from CTA 0
+  alignas(16) float2 alpha[2][128];  // rescale factors of the halves of a tile (two buffers), sent by CTA 0
   float inv_l[2][128];              // final 1/l of token t (t % 2)
 };
 static_assert(sizeof(Misc0) <= 4096 && sizeof(Misc1) <= 4096, "misc area");
@@ -809,7 +808,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
               // the second half of the tile may move a maximum once more: the issuer then stops between the halves
               const bool late = __any_sync(0xffffffffu, a_late != 1.0f);
               if (lane == 0) reinterpret_cast<uint8_t*>(&m1->late[b])[warp] = late ? 1 : 0;
-              // P arrived through the async proxy (bulk copy), which is also how the MMA reads it: no proxy fence
+              // (no proxy fence for P here: the issuer, which waits for this arrival, executes one before the first MMA of the tile)
               __syncwarp();
               if (lane == 0) mbar_arrive(smem_u32(&m1->corr_done[b]));
               if (late) {

@@ -11,7 +11,8 @@
 // MMAs take 512 cycles for it where the single tile's take 256, and the operand reads of a 128 x 128 MMA alone
 // need the whole shared-memory bandwidth (32 KB in 256 cycles at 128 B per cycle) with the TMA writes on top.  So
 // the pair is the shape for large M and the single tile the one for small M, where the weight's bytes are the
-// bound and a finer grid matters.
+// bound and a finer grid matters.  An SM takes in about 64 bytes per clock, A included, so a K-major weight is cut finer still, into
+// tiles of 64 columns (NB), while every tile finds an SM (the row-major one would need another swizzle for 64-byte rows).
 // Split K (S > 1, for grids that would leave SMs idle): the S CTAs (or pairs) of a cluster multiply S parts of K; the
 // fp32 partial tiles meet in shared memory over DSMEM, every part adds up 1/S of the columns in a fixed order and
 // writes them: no workspace, no second launch, no atomics.
@@ -25,7 +26,7 @@
 // arrival (a release at cluster scope stalls the warp) 1921; the pieces of neighbouring K blocks as one stream 2107.
 // Single tiles: 64 x 8192 x 3584 back to back 13.1 -> 12.3 us a call (29 MB, 4.4 us) with A and B loaded by two warps, two K blocks per wait
 // of the issuer, and one commit that tells both the producer and the promotion warps.  With pairs the same commit made M = 4096
-// slower (1119 us), so those keep their two.  What is left of the 12.3 is the fill of the pipeline and 64 columns of B per SM.
+// slower (1119 us), so those keep their two.  With tiles of 64 columns 10.6, 2.9 TB/s; what is left is launch, prologue and the fill of the pipeline.
 // What bounds M = 4096 now: with the additions left out 826 us instead of 913, with the tensor-memory loads left out too 680 us
 // (the tensor pipe and the power limit: a library e4m3 GEMM reaches 2960).
 #include <cstring>
@@ -117,12 +118,13 @@ __device__ __forceinline__ void fma_x2(float2& acc, uint32_t v0, uint32_t v1, fl
       : "+f"(acc.x), "+f"(acc.y) : "r"(v0), "r"(v1), "f"(s));
 }
 
-template <int NCTA, bool B_KMAJOR>
+template <int NCTA, bool B_KMAJOR, int NB = 128>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const Params p) {
-  constexpr int BN = 128 * NCTA;          // columns of the tile = fp32 columns of one TMEM accumulator
+  constexpr int BN = NB * NCTA;           // columns of the tile = fp32 columns of one TMEM accumulator
   constexpr int COLS = BN / 2;            // columns of a promotion thread
-  constexpr uint32_t NACC = 512 / BN;     // accumulators in flight: all of tensor memory
+  constexpr uint32_t NACC = BN == 256 ? 2 : 4;     // accumulators in flight
+  static_assert(NB == 128 || (NCTA == 1 && B_KMAJOR), "narrow tiles: the K-major operand of a single CTA");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
@@ -200,7 +202,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         for (int t = group; t < p.n_tiles; t += n_groups) {
           int m_blk, n_blk;
           coords(t, m_blk, n_blk);
-          const int n0 = n_blk * BN + cta * 128;
+          const int n0 = n_blk * BN + cta * NB;
           bool live = true;
           for (int kb = kb0; kb < kb1; ++kb) {
             if (!mbar_wait(smem_u32(&bars->empty[s]), ph, abort_flag)) { live = false; break; }
@@ -208,7 +210,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
             if constexpr (NCTA == 1) {
               const uint32_t full = smem_u32(&bars->full[s]);
               const int x = is_b && !B_KMAJOR ? n0 : kb * BK, y = !is_b ? m_blk * BM : B_KMAJOR ? n0 : kb * BK;
-              mbar_arrive_expect_tx(full, is_b ? B_BYTES : p.stage_tx - B_BYTES);
+              mbar_arrive_expect_tx(full, is_b ? NB * BK : p.stage_tx - NB * BK);
               tma_load_2d(is_b ? a_dst + A_BYTES : a_dst, is_b ? &tm_b : &tm_a, full, x, y);
             } else {
               // both CTAs' loads are counted on the even CTA's barrier; that CTA announces the total
@@ -330,7 +332,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       // next K block, at a block's end) is on its way from tensor memory.
       constexpr int NP = COLS / 32;
       uint32_t v[2][32];
-      auto begin_block = [&]() {
+      auto begin_block = [&](int buf) {
         const uint32_t acc = it % NACC;
         if constexpr (NCTA == 1) {
           mbar_wait(smem_u32(&bars->empty[st]), st_ph, abort_flag);
@@ -340,9 +342,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         }
         __syncwarp();
         tc_fence_after();
-        tmem_ld32(tacc + acc * BN, v[0]);
+        tmem_ld32(tacc + acc * BN, v[buf]);
       };
-      begin_block();
+      begin_block(0);
 #pragma unroll 1
       for (int kq = kb0; kq < kb1; kq += 4) {
         float sc[4];
@@ -355,9 +357,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
             const uint32_t acc = it % NACC;
 #pragma unroll
             for (int c = 0; c < NP; ++c) {
-              tmem_wait_ld_regs(v[c & 1]);
+              const int now = (j * NP + c) & 1;
+              tmem_wait_ld_regs(v[now]);
               if (c + 1 < NP) {
-                tmem_ld32(tacc + acc * BN + (c + 1) * 32, v[(c + 1) & 1]);
+                tmem_ld32(tacc + acc * BN + (c + 1) * 32, v[now ^ 1]);
               } else {
                 // everything of this accumulator is in registers: hand it back
                 tc_fence_before();
@@ -370,10 +373,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                   else mbar_arrive_cluster_relaxed(be0 + acc * 8);
                 }
                 ++it;
-                if (kq + j + 1 < kb1) begin_block();
+                if (kq + j + 1 < kb1) begin_block(now ^ 1);
               }
 #pragma unroll
-              for (int e = 0; e < 16; ++e) fma_x2(accf[c * 16 + e], v[c & 1][2 * e], v[c & 1][2 * e + 1], sc[j]);
+              for (int e = 0; e < 16; ++e) fma_x2(accf[c * 16 + e], v[now][2 * e], v[now][2 * e + 1], sc[j]);
             }
           }
         }
@@ -459,7 +462,9 @@ inline Shape pick_shape(int m, int n, int k, int sms, bool whole_k) {
   for (int ncta = 1; ncta <= 2; ++ncta) {
     const long long tiles = static_cast<long long>((m + BM * ncta - 1) / (BM * ncta)) * ((n + 128 * ncta - 1) / (128 * ncta));
     for (int s = 1; s * ncta <= (ncta == 1 ? 8 : 4); s *= 2) {
-      if (s > 1 && (whole_k || kb < 2 * s || tiles * s * ncta > sms - sms / 8)) break;   // an eighth of the SMs may not host a cluster
+      // an eighth of the SMs may not host a cluster, a little more not one of eight CTAs (64 x 1920 x 7168 in 120 CTAs 11.7 us, 64 x 2048 x 7168
+      // in 128 21.2, in four parts 12.3)
+      if (s > 1 && (whole_k || kb < 2 * s || tiles * s * ncta > (s == 8 ? sms * 13 / 16 : sms - sms / 8))) break;
       const long long waves = s > 1 ? 1 : (tiles + sms / ncta - 1) / (sms / ncta);
       const long long t = waves * ((kb + s - 1) / s) * (ncta == 1 ? 33 : 50) + (s == 1 ? 0 : s == 2 ? 500 : s == 4 ? 600 : 700);
       if (best_t < 0 || t < best_t) { best_t = t; best = Shape{ncta, s}; }
@@ -467,14 +472,22 @@ inline Shape pick_shape(int m, int n, int k, int sms, bool whole_k) {
   }
   return best;
 }
+// Tiles of 64 columns instead of 128 (K-major weights): where they, too, find an SM each.  The parts of K stay those of 128 columns, so that
+// a product has the same bits in both layouts of the weight.  us, 128 / 64 columns: 64 x 1024 x 1024 5.8 / 5.1, 64 x 8192 x 3584 12.0 / 10.6,
+// 384 x 3072 x 7168 22.7 / 18.4, 64 x 2048 x 7168 in four parts 12.3 / 10.8.
+inline bool narrow(const Shape& s, int m, int n, int sms) {
+  const long long tiles = static_cast<long long>((m + BM - 1) / BM) * (n / 64);
+  return s.ncta == 1 && s.splits <= 4 && tiles * s.splits <= (s.splits > 1 ? sms - sms / 8 : sms);
+}
 
 }  // namespace gemm8
 
-// CTAs per tile and parts of K of a launch
-void plan_gemm_fp8(int m, int n, int k, int sms, int* ctas, int* parts) {
+// columns of a tile, CTAs per tile and parts of K of a launch
+void plan_gemm_fp8(int m, int n, int k, bool b_kmajor, int sms, int* columns, int* ctas, int* parts) {
   const gemm8::Shape s = gemm8::pick_shape(m, n, k, sms, false);
   *ctas = s.ncta;
   *parts = s.splits;
+  *columns = b_kmajor && gemm8::narrow(s, m, n, sms) ? 64 : 128 * s.ncta;
 }
 
 }  // namespace ftb
@@ -498,14 +511,15 @@ static int gemm_fp8_blockscaled(const ftb_gemm_fp8_args* g, bool whole_k, void* 
   const gemm8::Shape shape = gemm8::pick_shape(g->m, g->n, g->k, sms, whole_k);
   CUtensorMap tm_a, tm_b;
   const bool bkm = g->b_kmajor != 0;
+  const int nb = bkm && gemm8::narrow(shape, g->m, g->n, sms) ? 64 : 128;
   const int box_m = g->m < gemm8::BM ? (g->m + 7) & ~7 : gemm8::BM;   // whole swizzle atoms of eight rows
   if (!make_tmap_2d(&tm_a, g->a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, g->m, g->k, g->lda, box_m, 128) ||
-      !(bkm ? make_tmap_2d(&tm_b, g->b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, g->n, g->k, g->ldb, 128, 128)
+      !(bkm ? make_tmap_2d(&tm_b, g->b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, g->n, g->k, g->ldb, nb, 128)
             : make_tmap_2d(&tm_b, g->b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, g->k, g->n, g->ldb, gemm8::BK, 128))) {
     set_last_error("ftb_gemm_fp8_blockscaled: cuTensorMapEncodeTiled failed");
     return FTB_ERR_CUDA;
   }
-  const int bm = gemm8::BM * shape.ncta, bn = 128 * shape.ncta;
+  const int bm = gemm8::BM * shape.ncta, bn = nb * shape.ncta;
   gemm8::Params p;
   memset(&p, 0, sizeof(p));
   p.m = g->m; p.n = g->n; p.k = g->k;
@@ -514,14 +528,14 @@ static int gemm_fp8_blockscaled(const ftb_gemm_fp8_args* g, bool whole_k, void* 
   p.n_tiles = p.m_blocks * p.n_blocks;
   p.kb_total = g->k / gemm8::BK;
   p.splits = shape.splits;
-  p.stage_tx = static_cast<uint32_t>(box_m * gemm8::BK + gemm8::B_BYTES);
+  p.stage_tx = static_cast<uint32_t>(box_m * gemm8::BK + nb * gemm8::BK);
   p.a_scale = g->a_scale; p.b_scale = g->b_scale;
   p.lda_s = g->a_scale_ld; p.ldb_s = g->b_scale_ld;
   p.c = reinterpret_cast<__nv_bfloat16*>(g->c);
   p.ldc = g->ldc;
   p.status = g->status;
   auto kern = shape.ncta == 2 ? (bkm ? gemm8::gemm_fp8_kernel<2, true> : gemm8::gemm_fp8_kernel<2, false>)
-                              : (bkm ? gemm8::gemm_fp8_kernel<1, true> : gemm8::gemm_fp8_kernel<1, false>);
+                              : nb == 64 ? gemm8::gemm_fp8_kernel<1, true, 64> : (bkm ? gemm8::gemm_fp8_kernel<1, true> : gemm8::gemm_fp8_kernel<1, false>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm8::SMEM_BYTES);
   if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(gemm_fp8)");
   const int cl = shape.ncta * shape.splits;

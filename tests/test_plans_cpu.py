@@ -29,6 +29,13 @@ def test_gpu_tests_reach_every_route(fp8, routes):
     assert seen <= set(routes)
 
 
+def test_gpu_tests_reach_the_narrow_tiles_of_a_k_major_weight():
+    for route, shapes in test_gemm_fp8_gpu.ROUTES_NK.items():
+        for m, n, k in shapes:
+            assert _plan(2, m, n, k) == route, (m, n, k)
+            assert _plan(1, m, n, k)[1:] == route[1:]                     # the same parts of K in both layouts
+
+
 def test_plan_arguments_are_checked():
     plan = (C.c_int32 * 3)()
     lib = _lib.load()

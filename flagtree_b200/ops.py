@@ -95,13 +95,12 @@ def _auto_splits(s_q: int, h: int, topk: int, device) -> int:
 
 @functools.lru_cache(maxsize=1024)
 def _plan_paged(s_q: int, h: int, topk: int, pairs: int) -> Tuple[int, bool]:
-    """Parts of a token's list in the paged form, and whether the rows are dequantised first.
+    """Parts of a token's list in the paged form, and whether a token kept whole follows the lazy maximum.
 
-    Both kernels take the true maximum of a part as the reference of its weights, so the largest weight is exactly 1 in bf16;
+    Parts take the true maximum as the reference of their weights, so the largest weight is exactly 1 in bf16;
     fewer parts than the SMs could take would only cost precision (relative error against 64 bits, 30 tokens of topk 2048: 4.23e-3
-    whole, 4.12e-3 in 2 parts).  Up to eight tokens whose parts are at most three tiles of 64 rows, the one-pass kernel is
-    the faster one: two launches instead of three (us, one pass / two: 3 tokens of topk 2048 28.7 / 32.0, 8 of 512 24.6 / 28.7;
-    beyond it 8 of 2048 45 / 41, 12 of 512 35 / 31, 32 of 2048 135 / 86)."""
+    whole, 4.12e-3 in 2 parts).  Up to eight tokens whose parts are at most three tiles of 64 rows are cut into as many parts as there are
+    pairs of SMs for (3 tokens of topk 2048 in 16 parts: 18.7 us on the device)."""
     if s_q >= pairs:
         return 1, True
     tiles = max(1, (topk + 63) // 64)

@@ -11,8 +11,8 @@
 // MMAs take 512 cycles for it where the single tile's take 256, and the operand reads of a 128 x 128 MMA alone
 // need the whole shared-memory bandwidth (32 KB in 256 cycles at 128 B per cycle) with the TMA writes on top.  So
 // the pair is the shape for large M and the single tile the one for small M, where the weight's bytes are the
-// bound and a finer grid matters.  An SM takes in about 64 bytes per clock, A included, so a K-major weight is cut finer still, into
-// tiles of 64 columns (NB), while every tile finds an SM (the row-major one would need another swizzle for 64-byte rows).
+// bound and a finer grid matters.  An SM takes in about 64 bytes per clock, A included, so the weight is cut finer still, into
+// tiles of 64 columns (NB), while every tile finds an SM; a row-major weight then lies in 64-byte rows under the 64-byte swizzle.
 // Split K (S > 1, for grids that would leave SMs idle): the S CTAs (or pairs) of a cluster multiply S parts of K; the
 // fp32 partial tiles meet in shared memory over DSMEM, every part adds up 1/S of the columns in a fixed order and
 // writes them: no workspace, no second launch, no atomics.
@@ -124,7 +124,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   constexpr int BN = NB * NCTA;           // columns of the tile = fp32 columns of one TMEM accumulator
   constexpr int COLS = BN / 2;            // columns of a promotion thread
   constexpr uint32_t NACC = BN == 256 ? 2 : 4;     // accumulators in flight
-  static_assert(NB == 128 || (NCTA == 1 && B_KMAJOR), "narrow tiles: the K-major operand of a single CTA");
+  static_assert(NB == 128 || (NCTA == 1 && NB == 64), "narrow tiles: of a single CTA");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
@@ -230,10 +230,12 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       // the whole warp runs the loop and waits, an elected lane (always the same one) issues
       constexpr uint32_t kIdesc = umma_idesc(kFmtE4M3, BM * NCTA, BN, 0, B_KMAJOR ? 0 : 1);
       const uint64_t ad0 = smem_desc_sw128(base, 16, 1024);
-      const uint64_t bd0 = B_KMAJOR ? smem_desc_sw128(base + A_BYTES, 16, 1024) : smem_desc_sw128(base + A_BYTES, B_BYTES, 1024);
+      // row-major B: eight k-rows of NB bytes are a swizzle atom, of 128-byte rows or of 64-byte rows (mode 4 instead of 2)
+      const uint64_t bd0 = B_KMAJOR ? smem_desc_sw128(base + A_BYTES, 16, 1024)
+                                    : smem_desc_sw128(base + A_BYTES, NB * BK, 8 * NB) ^ (NB == 64 ? static_cast<uint64_t>(6) << 61 : 0);
       const uint32_t ad_lo0 = static_cast<uint32_t>(ad0), ad_hi = static_cast<uint32_t>(ad0 >> 32);
       const uint32_t bd_lo0 = static_cast<uint32_t>(bd0), bd_hi = static_cast<uint32_t>(bd0 >> 32);
-      constexpr uint32_t kBStep = (B_KMAJOR ? 32 : 4096) >> 4;   // 32 bytes of K, or 32 k-rows
+      constexpr uint32_t kBStep = (B_KMAJOR ? 32 : 32 * NB) >> 4;   // 32 bytes of K, or 32 k-rows
       const uint16_t mask = static_cast<uint16_t>(3u << leader);
       const uint32_t full0 = smem_u32(&bars->full[0]), empty0 = smem_u32(&bars->empty[0]);
       const uint32_t be0 = smem_u32(&bars->blk_empty[0]);
@@ -472,9 +474,9 @@ inline Shape pick_shape(int m, int n, int k, int sms, bool whole_k) {
   }
   return best;
 }
-// Tiles of 64 columns instead of 128 (K-major weights): where they, too, find an SM each.  The parts of K stay those of 128 columns, so that
-// a product has the same bits in both layouts of the weight.  us, 128 / 64 columns: 64 x 1024 x 1024 5.8 / 5.1, 64 x 8192 x 3584 12.0 / 10.6,
-// 384 x 3072 x 7168 22.7 / 18.4, 64 x 2048 x 7168 in four parts 12.3 / 10.8.
+// Tiles of 64 columns instead of 128, with the same parts of K (and bits): where they, too, find an SM each.
+// us, 128 / 64 columns: 64 x 1024 x 1024 5.8 / 5.1, 64 x 8192 x 3584 12.0 / 10.6 (row-major weight 12.1 / 10.8), 384 x 3072 x 7168 22.7 / 18.4,
+// 64 x 2048 x 7168 in four parts 12.3 / 10.8.
 inline bool narrow(const Shape& s, int m, int n, int sms) {
   const long long tiles = static_cast<long long>((m + BM - 1) / BM) * (n / 64);
   return s.ncta == 1 && s.splits <= 4 && tiles * s.splits <= (s.splits > 1 ? sms - sms / 8 : sms);
@@ -482,12 +484,12 @@ inline bool narrow(const Shape& s, int m, int n, int sms) {
 
 }  // namespace gemm8
 
-// columns of a tile, CTAs per tile and parts of K of a launch
-void plan_gemm_fp8(int m, int n, int k, bool b_kmajor, int sms, int* columns, int* ctas, int* parts) {
+// columns of a tile (`halved`: with the rule above), CTAs per tile and parts of K of a launch
+void plan_gemm_fp8(int m, int n, int k, bool halved, int sms, int* columns, int* ctas, int* parts) {
   const gemm8::Shape s = gemm8::pick_shape(m, n, k, sms, false);
   *ctas = s.ncta;
   *parts = s.splits;
-  *columns = b_kmajor && gemm8::narrow(s, m, n, sms) ? 64 : 128 * s.ncta;
+  *columns = halved && gemm8::narrow(s, m, n, sms) ? 64 : 128 * s.ncta;
 }
 
 }  // namespace ftb
@@ -511,11 +513,12 @@ static int gemm_fp8_blockscaled(const ftb_gemm_fp8_args* g, bool whole_k, void* 
   const gemm8::Shape shape = gemm8::pick_shape(g->m, g->n, g->k, sms, whole_k);
   CUtensorMap tm_a, tm_b;
   const bool bkm = g->b_kmajor != 0;
-  const int nb = bkm && gemm8::narrow(shape, g->m, g->n, sms) ? 64 : 128;
+  const int nb = gemm8::narrow(shape, g->m, g->n, sms) ? 64 : 128;
   const int box_m = g->m < gemm8::BM ? (g->m + 7) & ~7 : gemm8::BM;   // whole swizzle atoms of eight rows
   if (!make_tmap_2d(&tm_a, g->a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, g->m, g->k, g->lda, box_m, 128) ||
       !(bkm ? make_tmap_2d(&tm_b, g->b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, g->n, g->k, g->ldb, nb, 128)
-            : make_tmap_2d(&tm_b, g->b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, g->k, g->n, g->ldb, gemm8::BK, 128))) {
+            : make_tmap_2d(&tm_b, g->b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, g->k, g->n, g->ldb, gemm8::BK, nb,
+                           nb == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B))) {
     set_last_error("ftb_gemm_fp8_blockscaled: cuTensorMapEncodeTiled failed");
     return FTB_ERR_CUDA;
   }
@@ -535,7 +538,8 @@ static int gemm_fp8_blockscaled(const ftb_gemm_fp8_args* g, bool whole_k, void* 
   p.ldc = g->ldc;
   p.status = g->status;
   auto kern = shape.ncta == 2 ? (bkm ? gemm8::gemm_fp8_kernel<2, true> : gemm8::gemm_fp8_kernel<2, false>)
-                              : nb == 64 ? gemm8::gemm_fp8_kernel<1, true, 64> : (bkm ? gemm8::gemm_fp8_kernel<1, true> : gemm8::gemm_fp8_kernel<1, false>);
+              : nb == 64      ? (bkm ? gemm8::gemm_fp8_kernel<1, true, 64> : gemm8::gemm_fp8_kernel<1, false, 64>)
+                              : (bkm ? gemm8::gemm_fp8_kernel<1, true> : gemm8::gemm_fp8_kernel<1, false>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm8::SMEM_BYTES);
   if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(gemm_fp8)");
   const int cl = shape.ncta * shape.splits;

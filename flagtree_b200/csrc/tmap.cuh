@@ -25,9 +25,9 @@ inline EncodeTiledFn get_encode_tiled() {
 }
 
 // 2-D row-major tensor [rows, cols] of `elem_bytes`-wide elements with `ld` elements between rows;
-// box = [box_rows, box_cols]; 128B swizzle (box_cols * elem_bytes must be 128).
+// box = [box_rows, box_cols]; 128B swizzle, or 64B (box_cols * elem_bytes must be that many).
 inline bool make_tmap_2d(CUtensorMap* out, const void* base, CUtensorMapDataType dt, int elem_bytes, uint64_t rows,
-                         uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_cols) {
+                         uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_cols, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
   EncodeTiledFn fn = get_encode_tiled();
   if (fn == nullptr) return false;
   cuuint64_t dims[2] = {cols, rows};
@@ -35,7 +35,7 @@ inline bool make_tmap_2d(CUtensorMap* out, const void* base, CUtensorMapDataType
   cuuint32_t box[2] = {box_cols, box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(out, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
 

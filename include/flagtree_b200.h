@@ -212,7 +212,8 @@ FTB_API int ftb_gemm_bf16(const ftb_gemm_args* args, void* stream);
  * bits of a row may depend on how many rows are multiplied with it.  This form always takes K in one part, in order: a row
  * of the result has the same bits whatever m is. */
 FTB_API int ftb_gemm_bf16_whole_k(const ftb_gemm_args* args, void* stream);
-/* How ftb_gemm_bf16 (fp8 = 0) or ftb_gemm_fp8_blockscaled (fp8 = 1; 2: with b_kmajor) would compute a product on a device of `sms` SMs (host only):
+/* How ftb_gemm_bf16 (fp8 = 0) or ftb_gemm_fp8_blockscaled (fp8 = 1; 2: after few tiles of 128 columns have been halved,
+ * which changes no bits) would compute a product on a device of `sms` SMs (host only):
  * plan[0] = columns of a tile, plan[1] = CTAs that share a tile, plan[2] = parts of K. */
 FTB_API int ftb_gemm_plan(int fp8, int m, int n, int k, int sms, int32_t plan[3]);
 FTB_API int ftb_sizeof_gemm_args(void);

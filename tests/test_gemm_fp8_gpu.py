@@ -85,14 +85,15 @@ ROUTES = {(128, 1, 1): [(60, 2048, 1024), (130, 512, 1024)], (128, 1, 2): [(40, 
           (256, 2, 1): [(1025, 2176, 384), (1030, 3200, 1664)], (256, 2, 2): [(142, 4608, 13824), (162, 4224, 10240), (395, 2304, 15616)]}
 
 
-# The same for a weight kept as [N, K], whose single tiles may have 64 columns: both sides of that line, each with an odd count of K blocks.
-ROUTES_NK = {(64, 1, 1): [(60, 2048, 1024), (1, 128, 384), (128, 9472, 384), (257, 3072, 640)], (64, 1, 4): [(64, 2048, 7168), (100, 1920, 3456)],
-             (128, 1, 1): [(128, 9600, 384)], (128, 1, 4): [(33, 3968, 4096)], (128, 1, 8): [(64, 1920, 7168)]}
+# The same after few single tiles have been halved to 64 columns: both sides of that line, some with an odd count of K blocks.
+ROUTES_HALVED = {(64, 1, 1): [(60, 2048, 1024), (1, 128, 384), (128, 9472, 384), (257, 3072, 640)], (64, 1, 4): [(64, 2048, 7168), (100, 1920, 3456)],
+                 (128, 1, 1): [(128, 9600, 384)], (128, 1, 4): [(33, 3968, 4096)], (128, 1, 8): [(64, 1920, 7168)]}
 
 
-@pytest.mark.parametrize("m,n,k", [s for shapes in ROUTES_NK.values() for s in shapes])
-def test_fp8_every_route_of_a_k_major_weight(m, n, k):
-    _check_fp8(m, n, k, True)
+@pytest.mark.parametrize("m,n,k", [s for shapes in ROUTES_HALVED.values() for s in shapes])
+@pytest.mark.parametrize("nk", [False, True])
+def test_fp8_every_route_of_halved_tiles(m, n, k, nk):
+    _check_fp8(m, n, k, nk)
 
 
 @pytest.mark.parametrize("m,n,k", [(64, 1024, 1024), (64, 2048, 7168), (100, 9472, 384), (128, 9600, 384), (64, 1920, 7168)])

@@ -29,11 +29,11 @@ def test_gpu_tests_reach_every_route(fp8, routes):
     assert seen <= set(routes)
 
 
-def test_gpu_tests_reach_the_narrow_tiles_of_a_k_major_weight():
-    for route, shapes in test_gemm_fp8_gpu.ROUTES_NK.items():
+def test_gpu_tests_reach_the_halved_tiles():
+    for route, shapes in test_gemm_fp8_gpu.ROUTES_HALVED.items():
         for m, n, k in shapes:
             assert _plan(2, m, n, k) == route, (m, n, k)
-            assert _plan(1, m, n, k)[1:] == route[1:]                     # the same parts of K in both layouts
+            assert _plan(1, m, n, k)[1:] == route[1:]                     # the same parts of K
 
 
 def test_plan_arguments_are_checked():

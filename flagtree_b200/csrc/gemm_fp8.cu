@@ -159,7 +159,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   if (tid == 0) bars->abort_flag = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
   __syncthreads();
   // an earlier launch on this status word failed: leave at once, the whole cluster on the reading of its CTA 0
-  if (clustered) {
+  if (clustered && p.status != nullptr) {
     cluster_sync_all();
     uint32_t leave;
     asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(leave) : "r"(mapa_shared(smem_u32(&bars->abort_flag), 0)) : "memory");

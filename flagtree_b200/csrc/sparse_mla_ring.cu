@@ -312,11 +312,11 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
   griddep_wait();
   if (tid == 0) *abort_flag = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
   __syncthreads();
-  cluster_sync_all();
   // An earlier launch on this status word failed: leave at once.  The two CTAs of a pair read the word at
   // different moments (another pair of this launch may report in between), so CTA 1 takes CTA 0's reading:
   // a CTA that went on alone would signal barriers in the shared memory of a partner that has left.
-  {
+  if (p.status != nullptr) {
+    cluster_sync_all();
     uint32_t leave;
     asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(leave) : "r"(mapa_shared(smem_u32(&m0->abort_flag), 0)) : "memory");
     if (leave != 0u) {

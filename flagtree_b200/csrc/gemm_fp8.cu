@@ -47,6 +47,9 @@ constexpr int A_BYTES = BM * BK;          // 16384
 constexpr int B_BYTES = BK * 128;         // 16384: 128 columns per CTA in both shapes
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+// Pairs without a split: where the promotion warps turn their rows round before they write them (4096 x 8192 x 28672 1060 -> 1046 us, 384 x 8192 x 1024
+// 10.3 -> 9.1).  The others do without: it comes off the L1 that holds their scales (64 x 8192 x 16384 29.8 -> 32.1).
+constexpr int BOX_BYTES = 8 * 4096;
 constexpr int THREADS = 384;             // launched with 168 registers each: 8 x 32 x 224 + 4 x 32 x 56 = 384 x 168
 constexpr int kRegsMany = 224, kRegsFew = 56;
 constexpr int kGroupM = 8;                // row blocks of a super-row of tiles (both operands are re-used out of L2)
@@ -130,6 +133,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (base - raw_addr);
   Bars* bars = reinterpret_cast<Bars*>(sm + STAGES * STAGE_BYTES);
+  static_assert(sizeof(Bars) <= 256, "boxes behind the barriers");
+  const uint32_t boxes = base + STAGES * STAGE_BYTES + 256;
   volatile int* abort_flag = &bars->abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool clustered = NCTA * p.splits > 1;
@@ -384,7 +389,14 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         }
       }
       if (p.splits == 1) {
-        if (row_ok && col_ok) {
+        if constexpr (NCTA == 2) {
+#pragma unroll
+          for (int c0 = 0; c0 < COLS; c0 += 64)
+            store_rows_bf16(boxes + (warp - 4) * 4096, p.c, p.ldc, m_blk * BM + lg * 32, p.m, n0 + c0, p.n, [&](int ch) {
+              const float2* f = accf + c0 / 2 + 4 * ch;
+              return make_uint4(pack_bf16x2(f[0].x, f[0].y), pack_bf16x2(f[1].x, f[1].y), pack_bf16x2(f[2].x, f[2].y), pack_bf16x2(f[3].x, f[3].y));
+            });
+        } else if (row_ok && col_ok) {
           __nv_bfloat16* orow = p.c + static_cast<long long>(row) * p.ldc + n0;
 #pragma unroll
           for (int j = 0; j < COLS / 2; j += 4) {
@@ -540,12 +552,13 @@ static int gemm_fp8_blockscaled(const ftb_gemm_fp8_args* g, bool whole_k, void* 
   auto kern = shape.ncta == 2 ? (bkm ? gemm8::gemm_fp8_kernel<2, true> : gemm8::gemm_fp8_kernel<2, false>)
               : nb == 64      ? (bkm ? gemm8::gemm_fp8_kernel<1, true, 64> : gemm8::gemm_fp8_kernel<1, false, 64>)
                               : (bkm ? gemm8::gemm_fp8_kernel<1, true> : gemm8::gemm_fp8_kernel<1, false>);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm8::SMEM_BYTES);
+  const int smem = gemm8::SMEM_BYTES + (shape.ncta == 2 && shape.splits == 1 ? gemm8::BOX_BYTES : 0);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(gemm_fp8)");
   const int cl = shape.ncta * shape.splits;
   // persistent groups; with a split every cluster computes one tile and leaves
   const int groups = shape.splits > 1 ? p.n_tiles : (p.n_tiles < sms / shape.ncta ? p.n_tiles : sms / shape.ncta);
-  e = launch_overlapped(kern, static_cast<unsigned>(groups) * cl, gemm8::THREADS, gemm8::SMEM_BYTES, reinterpret_cast<cudaStream_t>(stream),
+  e = launch_overlapped(kern, static_cast<unsigned>(groups) * cl, gemm8::THREADS, smem, reinterpret_cast<cudaStream_t>(stream),
                         static_cast<unsigned>(cl), tm_a, tm_b, p);
   if (e != cudaSuccess) return check_cuda(e, "gemm_fp8 launch");
   return FTB_OK;

@@ -290,4 +290,29 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// A warp writes 32 rows of 64 columns of a row-major bf16 matrix, of which lane l has row l in registers: `piece(ch)` gives columns 8 ch .. of it.
+// They turn round in `box` (4096 bytes of shared memory, the warp's own), so that eight lanes write 128 bytes of a row: stored straight
+// from the registers every 16-byte piece is a line of its own.  (row0, col0): the first element; rows and columns from
+// `rows` and `cols` on are left out (`cols` is a multiple of 8).
+template <class Piece>
+__device__ __forceinline__ void store_rows_bf16(uint32_t box, __nv_bfloat16* c, long long ldc, int row0, int rows, int col0, int cols, Piece piece) {
+  const int lane = threadIdx.x & 31;
+  auto at = [&](int r, int ch) { return box + r * 128 + ((ch ^ (r & 7)) << 4); };
+  __syncwarp();                                    // the box has been read
+#pragma unroll
+  for (int ch = 0; ch < 8; ++ch) {
+    const uint4 o = piece(ch);
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at(lane, ch)), "r"(o.x), "r"(o.y), "r"(o.z), "r"(o.w) : "memory");
+  }
+  __syncwarp();
+  const int ch = lane & 7, col = col0 + 8 * ch;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = 4 * i + (lane >> 3);
+    uint4 o;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w) : "r"(at(r, ch)) : "memory");
+    if (row0 + r < rows && col < cols) *reinterpret_cast<uint4*>(c + static_cast<long long>(row0 + r) * ldc + col) = o;
+  }
+}
+
 }  // namespace ftb

@@ -47,8 +47,9 @@ constexpr int A_BYTES = BM * BK;          // 16384
 constexpr int B_BYTES = BK * 128;         // 16384: 128 columns per CTA in both shapes
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
-// Pairs without a split: where the promotion warps turn their rows round before they write them (4096 x 8192 x 28672 1060 -> 1046 us, 384 x 8192 x 1024
-// 10.3 -> 9.1).  The others do without: it comes off the L1 that holds their scales (64 x 8192 x 16384 29.8 -> 32.1).
+// Where the promotion warps turn their rows round before they write them (4096 x 8192 x 28672 1060 -> 1046 us, 384 x 8192 x 1024 10.3 -> 9.1): of its
+// own for pairs without a split; a single tile of a CTA has its stages free by then (384 x 6144 x 1024 8.1 -> 6.9, 128 x 6144 x 3584 11.2 -> 10.6).
+// Singles with boxes of their own lost more than that with a long K: they come off the L1 that holds the scales (64 x 8192 x 16384 29.8 -> 32.1).
 constexpr int BOX_BYTES = 8 * 4096;
 constexpr int THREADS = 384;             // launched with 168 registers each: 8 x 32 x 224 + 4 x 32 x 56 = 384 x 168
 constexpr int kRegsMany = 224, kRegsFew = 56;
@@ -389,10 +390,12 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         }
       }
       if (p.splits == 1) {
-        if constexpr (NCTA == 2) {
+        if (NCTA == 2 || (one_each && p.m >= 32)) {        // (a few rows are a few pieces)
+          const uint32_t box = (NCTA == 2 ? boxes : base) + (warp - 4) * 4096;
+          constexpr int P = COLS >= 64 ? 8 : 4;
 #pragma unroll
-          for (int c0 = 0; c0 < COLS; c0 += 64)
-            store_rows_bf16(boxes + (warp - 4) * 4096, p.c, p.ldc, m_blk * BM + lg * 32, p.m, n0 + c0, p.n, [&](int ch) {
+          for (int c0 = 0; c0 < COLS; c0 += 8 * P)
+            store_rows_bf16<P>(box, p.c, p.ldc, m_blk * BM + lg * 32, p.m, n0 + c0, p.n, [&](int ch) {
               const float2* f = accf + c0 / 2 + 4 * ch;
               return make_uint4(pack_bf16x2(f[0].x, f[0].y), pack_bf16x2(f[1].x, f[1].y), pack_bf16x2(f[2].x, f[2].y), pack_bf16x2(f[3].x, f[3].y));
             });

@@ -290,25 +290,26 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
-// A warp writes 32 rows of 64 columns of a row-major bf16 matrix, of which lane l has row l in registers: `piece(ch)` gives columns 8 ch .. of it.
-// They turn round in `box` (4096 bytes of shared memory, the warp's own), so that eight lanes write 128 bytes of a row: stored straight
+// A warp writes 32 rows of 8 P columns of a row-major bf16 matrix, of which lane l has row l in registers: `piece(ch)` gives columns 8 ch .. of it.
+// They turn round in `box` (512 P bytes of shared memory, the warp's own), so that P lanes write 16 P bytes of a row: stored straight
 // from the registers every 16-byte piece is a line of its own.  (row0, col0): the first element; rows and columns from
 // `rows` and `cols` on are left out (`cols` is a multiple of 8).
-template <class Piece>
+template <int P, class Piece>
 __device__ __forceinline__ void store_rows_bf16(uint32_t box, __nv_bfloat16* c, long long ldc, int row0, int rows, int col0, int cols, Piece piece) {
+  static_assert(P == 4 || P == 8, "64 or 128 bytes of a row");
   const int lane = threadIdx.x & 31;
-  auto at = [&](int r, int ch) { return box + r * 128 + ((ch ^ (r & 7)) << 4); };
+  auto at = [&](int r, int ch) { return box + r * (16 * P) + ((ch ^ (P == 8 ? r & 7 : (r >> 1) & 3)) << 4); };
   __syncwarp();                                    // the box has been read
 #pragma unroll
-  for (int ch = 0; ch < 8; ++ch) {
+  for (int ch = 0; ch < P; ++ch) {
     const uint4 o = piece(ch);
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at(lane, ch)), "r"(o.x), "r"(o.y), "r"(o.z), "r"(o.w) : "memory");
   }
   __syncwarp();
-  const int ch = lane & 7, col = col0 + 8 * ch;
+  const int ch = lane % P, col = col0 + 8 * ch;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int r = 4 * i + (lane >> 3);
+  for (int i = 0; i < P; ++i) {
+    const int r = i * (32 / P) + lane / P;
     uint4 o;
     asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w) : "r"(at(r, ch)) : "memory");
     if (row0 + r < rows && col < cols) *reinterpret_cast<uint4*>(c + static_cast<long long>(row0 + r) * ldc + col) = o;

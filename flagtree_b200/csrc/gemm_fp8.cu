@@ -19,7 +19,7 @@
 // Roles (384 threads): warp 0 TMA producer (single tiles: of A, and warp 2 of B), warp 1 MMA issuer + TMEM owner, warps 4-11 promotion/epilogue: warp w takes
 // TMEM lanes 32 (w % 4) .. and half (w / 4 - 1) of the columns, so a thread holds 128 (64) fp32 sums.  Per K block a
 // thread needs one product of two scales: they are fetched from memory a group of four blocks ahead.
-// Measured, one GPU, K = 28672, N = 8192.  M = 4096 back to back, where the power limit sets the clock: 1064 us a call (1808 TFLOP/s) against
+// Measured, one GPU, K = 28672, N = 8192.  M = 4096 back to back, where the power limit sets the clock: 1048 us a call (1836 TFLOP/s) against
 // 1848 of the kernel before (128 x 128 tiles, four promotion warps that fetched their scales when they needed them).  Launches
 // with pauses between them (TFLOP/s): M = 4096 2107 (before 1078), M = 1024 1130 (912).  Steps of M = 4096 that way: eight promotion
 // warps, scales ahead, single tiles 1269 and pairs 1037; the pair's hand-back of an accumulator as a relaxed remote

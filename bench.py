@@ -158,7 +158,7 @@ def bench_mla_decode_fp8(args, dev, peaks):
             "tflops": flops / (ms * 1e-3) / 1e12, "bytes": nbytes, "gbs": nbytes / (ms * 1e-3) / 1e9,
             "frac_of_bf16_peak": flops / (ms * 1e-3) / 1e12 / peaks["bf16_tflops"],
             "frac_of_hbm_peak": nbytes / (ms * 1e-3) / 1e9 / peaks["hbm_gbs"],
-            "l2": "gathered rows (151 MB) larger than L2", "kernel": "mla_dequant_rows_kernel + persistent sparse-MLA kernel"}
+            "l2": "gathered rows (151 MB) larger than L2", "kernel": "sparse_mla_few_heads_kernel (rows converted in the gather)"}
 
 
 def bench_kv_cache_write(args, dev, peaks):

@@ -106,6 +106,7 @@ struct Params {
   const int32_t* block_table;
   const int32_t* context_lens;
   int page_size, q_per_seq;
+  int tok0;            // the launch's first token, counted over the call: sequences go by the latter
   long long bt_stride;
 };
 
@@ -667,7 +668,7 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
           cn = misc->nt[ct];
           c_left = p.topk - row0 - r;
           c_idx = p.indices + static_cast<long long>(tok) * p.idx_st + row0 + r;
-          c_seq = tok / p.q_per_seq;
+          c_seq = (p.tok0 + tok) / p.q_per_seq;
           c_ctx = p.context_lens[c_seq];
         }
       }
@@ -797,6 +798,7 @@ static int launch_nh(const ftb_sparse_mla_args* a, Params p, cudaStream_t st) {
   float* const part_lse = p.part_lse;
   for (long long t0 = 0; t0 < a->s_q; t0 += cap) {
     p.s_q = static_cast<int>(a->s_q - t0 < cap ? a->s_q - t0 : cap);
+    p.tok0 = static_cast<int>(t0);
     p.indices = a->indices + t0 * a->idx_stride_token;
     p.lse = a->lse + t0 * a->lse_stride_token;
     p.out = static_cast<__nv_bfloat16*>(a->out) + t0 * a->out_stride_token;

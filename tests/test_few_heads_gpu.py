@@ -143,3 +143,42 @@ def test_paged_rows_converted_in_the_gather(h, batch, n_q, topk, page):
         # P and the result are rounded to bf16 (2^-9 each) from another reference maximum and with sums in another order
         assert (o.float() - ref_out.float()).abs().max().item() <= 2 ** -7 * max(1.0, ref_out.abs().max().item())
         assert ((l[fin] - ref_lse[fin]).abs() <= 1e-5 * ref_lse[fin].abs().clamp(min=1)).all()
+
+
+def _paged_algo(args, sm_scale, page_size, algo, splits):
+    """The paged form through the C ABI, with a kernel and a number of parts of the caller's choice."""
+    import ctypes as C
+    from flagtree_b200 import _lib
+    q, cache, scale, table, lens, idx = args
+    b, n_q, h, _ = q.shape
+    topk = idx.shape[2]
+    lib = _lib.load()
+    out = torch.empty(b, n_q, h, 512, dtype=torch.bfloat16, device=DEV)
+    lse = torch.empty(b, n_q, h, dtype=torch.float32, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    a = _lib.SparseMlaArgs(q.data_ptr(), cache.data_ptr(), idx.data_ptr(), out.data_ptr(), lse.data_ptr(), b * n_q, h, cache.shape[0] * page_size,
+                           topk, h * 576, 576, 576, topk, h * 512, 512, h, sm_scale, 0, algo, status.data_ptr(), 1, scale.data_ptr(),
+                           table.data_ptr(), lens.data_ptr(), page_size, n_q, table.stride(0))
+    ws = torch.empty(max(1, lib.ftb_sparse_mla_workspace_bytes(b * n_q, h, splits)), dtype=torch.uint8, device=DEV)
+    a.n_splits, a.workspace, a.workspace_bytes = splits, ws.data_ptr(), ws.numel()
+    assert lib.ftb_sparse_mla_fwd(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0, _lib.last_error()
+    torch.cuda.synchronize()
+    assert status.item() == 0
+    return out, lse
+
+
+@pytest.mark.parametrize("h", [16, 64, 128])
+@pytest.mark.parametrize("batch,topk,splits", [(3, 2048, 16), (2, 512, 8), (5, 300, 3), (4, 130, 1), (1, 1000, 40)])
+def test_paged_parts_have_the_weights_of_the_one_cta_kernel(h, batch, topk, splits):
+    """Parts of a token, and whole tokens of algo 0, take the true maximum tile by tile, in as many parts as the one-CTA kernel (algo 1) makes:
+    the same weights in bf16.  Only the fp32 sums of the weights are added in another order (64 additions a tile, 2^-24 each, and as many tiles), which
+    moves a result across a rounding boundary of bf16 in far less than one element of a hundred, and then to its neighbour (where the parts cancel:
+    by their weights' 4e-6 of what they add up)."""
+    c = W.mla_cfg3(batch=batch, n_q=1, h=h, topk=topk, len_lo=600, len_hi=4000)
+    args = [t.to(DEV) for t in (c.q, c.kv_cache, c.kv_scale, c.block_table, c.context_lens, c.indices)]
+    out, lse = _paged_algo(args, c.sm_scale, c.page_size, 0, splits)
+    ref_out, ref_lse = _paged_algo(args, c.sm_scale, c.page_size, 1, splits)
+    o, r = out.float(), ref_out.float()
+    assert ((o - r).abs() <= 2 ** -7 * r.abs() + 2e-5 * r.abs().max()).all()
+    assert (o != r).float().mean().item() < 0.01
+    assert ((lse - ref_lse).abs() <= 2e-6 * ref_lse.abs().clamp(min=1)).all()

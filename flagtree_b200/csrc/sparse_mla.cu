@@ -89,11 +89,11 @@ __device__ __forceinline__ int resolve_row(const MlaParams& p, int token, int lo
   const int slot = logical / p.page_size;
   if (slot >= p.bt_stride) { bad = true; return 0; }      // a context length longer than the table's row
   const int page = p.block_table[seq * p.bt_stride + slot];
-  const int row = page * p.page_size + logical % p.page_size;
-  ok = page >= 0 && row >= 0 && row < p.s_kv;
+  const long long row = static_cast<long long>(page) * p.page_size + logical % p.page_size;   // (in 32 bits a corrupt entry may wrap to a valid row)
+  ok = page >= 0 && row < p.s_kv;
   bad = !ok;
   if (ok && p.kv_scale != nullptr) scale = p.kv_scale[page];
-  return ok ? row : 0;
+  return ok ? static_cast<int>(row) : 0;
 }
 
 // Paged FP8 form, first pass of the two-pass path: one warp per selected row.  The row is resolved through

@@ -693,11 +693,11 @@ sparse_mla_few_heads_kernel(const __grid_constant__ CUtensorMap tm_q, const Para
       }
     };
     auto next_rows = [&]() {
-      const int row = page * p.page_size + in_page;
-      ok = in_page >= 0 && page >= 0 && row >= 0 && row < p.s_kv;
+      const long long row = static_cast<long long>(page) * p.page_size + in_page;   // (in 32 bits a corrupt entry may wrap to a valid row)
+      ok = in_page >= 0 && page >= 0 && row < p.s_kv;
       if (in_page == -2 || (in_page >= 0 && !ok)) misc->bad_index = 1;      // reported, never read
       scale = ok ? p.kv_scale[page] : 0.0f;
-      const uint4* src = reinterpret_cast<const uint4*>(cache + static_cast<long long>(ok ? row : 0) * p.kv_sr);
+      const uint4* src = reinterpret_cast<const uint4*>(cache + (ok ? row : 0) * p.kv_sr);
 #pragma unroll
       for (int k = 0; k < 9; ++k) raw[k] = ok ? src[4 * k] : make_uint4(0u, 0u, 0u, 0u);
     };

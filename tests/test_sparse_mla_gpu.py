@@ -408,6 +408,18 @@ def test_paged_context_longer_than_block_table_is_reported():
             sparse_mla_fwd_paged(*args, c.sm_scale, page_size=c.page_size, check=True, num_splits=1, two_pass=two_pass)
 
 
+@pytest.mark.parametrize("entry", [-1, "num_pages", 1 << 26, (1 << 31) - 1], ids=["negative", "past_the_cache", "wraps_to_row_0", "largest"])
+def test_paged_table_entry_without_meaning_is_reported_and_never_read(entry):
+    """1 << 26 pages of 64 rows are 1 << 32: in 32 bits the entry would name a row of page 0, and its scale would be read far past the array."""
+    c = W.mla_cfg3(batch=2, n_q=1, h=16, topk=200, len_lo=300, len_hi=400)
+    c.block_table[1, 2] = c.kv_cache.shape[0] if entry == "num_pages" else entry
+    c.indices[1, 0, 5] = 2 * c.page_size + 1
+    args = [t.to(DEV) for t in (c.q, c.kv_cache, c.kv_scale, c.block_table, c.context_lens, c.indices)]
+    for kw in (dict(num_splits=1), dict(num_splits=1, two_pass=True), dict(num_splits=4), dict()):
+        with pytest.raises(RuntimeError, match="BAD_INDEX"):
+            sparse_mla_fwd_paged(*args, c.sm_scale, page_size=c.page_size, check=True, **kw)
+
+
 @pytest.mark.parametrize("s_q,h,topk,splits", [(1, 128, 2048, None), (1, 16, 130, None), (3, 128, 1000, 16), (40, 64, 300, 3),
                                                (75, 128, 257, 2), (30, 8, 640, 64)])
 def test_parts_of_a_token_on_the_persistent_pairs(s_q, h, topk, splits):

@@ -756,9 +756,10 @@ extern "C" FTB_API int ftb_sparse_mla_fwd(const ftb_sparse_mla_args* a, void* st
   // 167 / 142; 16 heads, 148 tokens of topk 512 in two parts 88 / 44.
   const bool pairs = a->algo_id == 5 || (a->algo_id == 0 && (a->topk > 512 || (n_splits * 128 <= a->topk && (a->h <= 32 || (a->topk > 256 && a->s_q >= 64)))));
   if (a->kv_is_fp8 && a->dbg_scores == nullptr && a->algo_id != 1 && n_splits <= 64) {
+    const float max_slack = a->algo_id == 5 && n_splits == 1 ? 8.0f : 0.0f;
     n_splits = parts_of(64);
     if (n_splits > 1) p.part_lse = p.part_out + static_cast<size_t>(a->s_q) * n_splits * a->h * 512;
-    const int rc0 = launch_sparse_mla_few(a, n_splits, p.part_out, p.part_lse, a->algo_id == 5 ? 8.0f : 0.0f, st);
+    const int rc0 = launch_sparse_mla_few(a, n_splits, p.part_out, p.part_lse, max_slack, st);
     return rc0 != FTB_OK || n_splits == 1 ? rc0 : merge();
   }
   if (n_splits > 1 && n_splits <= 64 && !a->kv_is_fp8 && a->dbg_scores == nullptr && pairs) {

@@ -182,3 +182,14 @@ def test_paged_parts_have_the_weights_of_the_one_cta_kernel(h, batch, topk, spli
     assert ((o - r).abs() <= 2 ** -7 * r.abs() + 2e-5 * r.abs().max()).all()
     assert (o != r).float().mean().item() < 0.01
     assert ((lse - ref_lse).abs() <= 2e-6 * ref_lse.abs().clamp(min=1)).all()
+
+
+@pytest.mark.parametrize("h,topk,splits", [(16, 700, 4), (128, 300, 2), (64, 60, 3)])
+def test_paged_parts_of_algo_5_take_the_true_maximum_too(h, topk, splits):
+    """The lazy maximum is for whole tokens: scores that grow along the list, by less than its slack of 2^8 a tile, would show it in parts."""
+    c = W.mla_cfg3(batch=3, n_q=1, h=h, topk=topk, len_lo=800, len_hi=2000)
+    c.kv_scale.mul_(torch.linspace(0.5, 4.0, c.kv_scale.numel()))
+    args = [t.to(DEV) for t in (c.q, c.kv_cache, c.kv_scale, c.block_table, c.context_lens, c.indices.sort(dim=2).values)]
+    ref = _paged_algo(args, c.sm_scale, c.page_size, 0, splits)
+    got = _paged_algo(args, c.sm_scale, c.page_size, 5, splits)
+    assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])

@@ -441,9 +441,12 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
             }
             // Lazy maximum: with a slack of 8 the reference only moves when it grows by more than 2^8, so that the
             // accumulator in the other CTA is rarely rescaled (P stays below 256).  Without slack it follows the true
-            // maximum: the largest weight is then 1, which bf16 holds exactly.  The first tile sets it as a whole; later the two
-            // halves of a tile (64 rows: the tile of the kernel for few heads) move it one after the other, and the sums below add in
-            // that kernel's order: the bits of a head do not depend on how many heads the call has.
+            // maximum, and every tile sets it as a whole: the largest weight is then 1, which bf16 holds exactly.  (The half-way stop below for a maximum
+            // that moves in both halves would come with most tiles: 100 tokens of 128 heads, topk 2048 in two parts, 133 us instead of 98.)
+            // With slack the first tile sets it as a whole; later the two halves of a tile (64 rows: the tile of the kernel for few heads) move
+            // it one after the other, and the sums below add in that kernel's order: the bits of a whole token's head do not depend on
+            // how many heads the call has.
+            const bool as_a_whole = i == 0 || p.max_slack == 0.0f;
             auto move_to = [&](float top) {
               const float m_cand = fmaxf(m_run, top * p.scale_log2);
               float a = 1.0f;
@@ -460,9 +463,9 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
               m0->xchg[b][tid] = mx;
               named_bar_sync(2 + (warp & 3), 64);
               const float other = m0->xchg[b][tid ^ 128];
-              alpha_a = move_to(i == 0 ? fmaxf(mx, other) : ch == 0 ? mx : other);
+              alpha_a = move_to(as_a_whole ? fmaxf(mx, other) : ch == 0 ? mx : other);
               m_mine = m_run;
-              if (i != 0) alpha_b = move_to(ch == 0 ? other : mx);
+              if (!as_a_whole) alpha_b = move_to(ch == 0 ? other : mx);
               if (ch != 0) m_mine = m_run;
               l01 = fmul2(l01, alpha_a);
               l23 = fmul2(l23, alpha_a);

@@ -408,6 +408,22 @@ def test_paged_context_longer_than_block_table_is_reported():
             sparse_mla_fwd_paged(*args, c.sm_scale, page_size=c.page_size, check=True, num_splits=1, two_pass=two_pass)
 
 
+@pytest.mark.parametrize("s_q,topk,splits", [(100, 1024, 2), (160, 2048, 2)])
+def test_parts_on_the_pairs_take_the_true_maximum_of_a_tile(s_q, topk, splits):
+    """Parts that a caller asks for, on the pairs: the reference of the weights is the largest score of all 128 rows of a tile and the tiles before it.  With the
+    halves of every tile exchanged the weights are the same in bf16, and only fp32 sums come in another order: far less than one element of a hundred
+    crosses a rounding boundary of bf16.  A reference that moves half-way through a tile changes the weights."""
+    g = torch.Generator().manual_seed(topk)
+    q = torch.randn(s_q, 128, 576, generator=g).bfloat16().to(DEV)
+    kv = torch.randn(4000, 576, generator=g).bfloat16().to(DEV)
+    idx = torch.stack([torch.randperm(4000, generator=g)[:topk] for _ in range(s_q)]).int()
+    swapped = idx.view(s_q, topk // 128, 2, 64).flip(2).reshape(s_q, topk).contiguous()
+    out, lse = sparse_mla_fwd(q, kv, idx.to(DEV), 0.06, check=True, num_splits=splits)
+    out2, lse2 = sparse_mla_fwd(q, kv, swapped.to(DEV), 0.06, check=True, num_splits=splits)
+    assert (out != out2).float().mean().item() < 0.01
+    assert ((lse - lse2).abs() <= 2e-6 * lse.abs().clamp(min=1)).all()
+
+
 @pytest.mark.parametrize("entry", [-1, "num_pages", 1 << 26, (1 << 31) - 1], ids=["negative", "past_the_cache", "wraps_to_row_0", "largest"])
 def test_paged_table_entry_without_meaning_is_reported_and_never_read(entry):
     """1 << 26 pages of 64 rows are 1 << 32: in 32 bits the entry would name a row of page 0, and its scale would be read far past the array."""

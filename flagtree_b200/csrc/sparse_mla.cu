@@ -596,16 +596,32 @@ int check_cuda(cudaError_t e, const char* what);
 int launch_sparse_mla_ring(const ftb_sparse_mla_args* a, int n_splits, float* part_out, float* part_lse, float max_slack, cudaStream_t st);
 int launch_sparse_mla_few(const ftb_sparse_mla_args* a, int n_splits, float* part_out, float* part_lse, float max_slack, cudaStream_t st);
 
-// The persistent kernels: up to 64 heads on the columns of the MMA, one CTA per item; more on its rows, a pair of CTAs per item.
-// The two add in the same order, so that the choice is not to be seen in the bits.  More than 64 heads in groups of 64, an item
-// each, are the faster form while a CTA has one item of at most 16 tiles (us, pairs / groups, 128 heads, topk 2048: 1 token 21.2 / 14.7,
-// 8 tokens 27.3 / 18.8, 32 tokens 48 / 39; 74 tokens of topk 512 24.7 / 22.3, of topk 2048 51 / 58).
+// The two persistent kernels: the one for few heads has a CTA per item of up to 64 heads (more are several items), the other a pair of CTAs per item of up
+// to 128.  With the lazy maximum they add in the same order, so that the choice is not to be seen in the bits.  With the true maximum (parts that a
+// caller asked for) each takes it over its own tile, 64 or 128 rows.
+// A call goes to the one that this model says is through first: launch + waves x (start of an item + time per tile) + rows of partial results, in us, fitted
+// to 400 whole calls and 960 in parts (1 to 300 tokens, 1 to 128 heads, topk 300 to 4096, 1 to 8 parts; within 3 % of the faster one for
+// all whole calls, 9 % for all parts).  Few heads / pairs, whole, topk 2048: 5 tokens of 64 heads 56 / 41, of 16 heads 41 / 37, 100 tokens of 64 heads
+// 58 / 67, 1 token of 128 heads 59 / 44; topk 300: 100 tokens of 16 heads 12.6 / 25.  In two parts, topk 2048: 5 tokens of 64 heads 47 / 35, of 16 heads 30 / 31.
+static bool few_heads_kernel_is_faster(int s_q, int h, int topk, int n_splits, bool lazy, int sms) {
+  const int c = h <= 16 ? 0 : h <= 32 ? 1 : h <= 64 ? 2 : 3;
+  constexpr float few_start[4] = {1.5f, 2.8f, 3.8f, 4.0f}, few_tile[2][4] = {{1.37f, 1.63f, 2.37f, 2.36f}, {1.08f, 1.13f, 1.50f, 1.51f}};
+  constexpr float few_rows[4] = {0.38f, 0.69f, 0.51f, 0.58f}, pair_rows[4] = {0.59f, 0.97f, 0.74f, 0.67f};
+  constexpr float pair_tile[2][4] = {{2.50f, 2.43f, 2.54f, 2.61f}, {1.56f, 1.55f, 1.87f, 2.01f}};
+  constexpr float few_launch[2][4] = {{6.8f, 7.9f, 7.9f, 8.4f}, {4.8f, 4.8f, 4.8f, 5.1f}}, pair_launch[2][4] = {{10.0f, 11.3f, 12.5f, 14.6f}, {7.7f, 8.4f, 9.0f, 10.7f}};
+  const long long items = static_cast<long long>(s_q) * n_splits, groups = (h + 63) / 64, pairs = sms > 1 ? sms / 2 : 1;
+  const int few_tiles = ((topk + 63) / 64 + n_splits - 1) / n_splits, pair_tiles = ((topk + 127) / 128 + n_splits - 1) / n_splits;
+  const float few_waves = static_cast<float>((items * groups + sms - 1) / sms), pair_waves = static_cast<float>((items + pairs - 1) / pairs);
+  const float rows = n_splits > 1 ? static_cast<float>(items) * static_cast<float>(h) * 1e-3f : 0.0f;
+  const float few = few_launch[lazy][c] + few_waves * ((lazy ? few_start[c] : 0.7f) + few_tile[lazy][c] * static_cast<float>(few_tiles)) + few_rows[c] * rows;
+  const float pair = pair_launch[lazy][c] + pair_waves * ((lazy ? 3.5f : 1.5f) + pair_tile[lazy][c] * static_cast<float>(pair_tiles)) + pair_rows[c] * rows;
+  return few <= pair;
+}
 static int launch_persistent(const ftb_sparse_mla_args* a, int n_splits, float* part_out, float* part_lse, float max_slack, cudaStream_t st) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long groups = (a->h + 63) / 64, tiles = (a->topk + 63) / 64;
-  const bool few = a->h <= 64 || (a->s_q * groups * n_splits <= sms && tiles <= 16LL * n_splits);
+  const bool few = few_heads_kernel_is_faster(a->s_q, a->h, a->topk, n_splits, max_slack > 0.0f, sms);
   return (few ? launch_sparse_mla_few : launch_sparse_mla_ring)(a, n_splits, part_out, part_lse, max_slack, st);
 }
 }  // namespace ftb

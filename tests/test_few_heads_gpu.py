@@ -98,7 +98,8 @@ def test_more_than_32_heads_are_refused():
         sparse_mla_fwd(q, kv, idx, 0.1, algo=2)
 
 
-@pytest.mark.parametrize("h,s_q,topk", [(16, 160, 200), (32, 40, 1000), (64, 9, 64), (100, 5, 700), (128, 60, 130)])
+@pytest.mark.parametrize("h,s_q,topk", [(16, 160, 200), (32, 40, 1000), (64, 9, 64), (100, 5, 700), (128, 60, 130), (32, 40, 600), (64, 160, 100), (16, 5, 2000),
+                                         (64, 20, 1500)])
 @pytest.mark.parametrize("steps", [False, True])
 def test_bits_of_a_head_do_not_depend_on_the_heads_of_the_call(h, s_q, topk, steps):
     """The kernel for few heads, its groups of 64 and the pairs for many add in the same order: equal bits, also where maxima move in either

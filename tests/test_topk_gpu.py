@@ -165,6 +165,15 @@ def test_whole_rows_and_long_lists(rows, s_kv, topk, values):
     assert torch.equal(topk_indices(sc.to(DEV), topk).cpu(), topk_indices_ref(sc, topk))
 
 
+@pytest.mark.parametrize("rows,s_kv,topk", [(3, 1000, 333), (150, 1000, 100), (150, 4096, 1300), (150, 4097, 1300), (150, 2048, 682), (1, 4096, 50)])
+@pytest.mark.parametrize("values", [1, 2, 10])
+def test_short_rows_of_few_values(rows, s_kv, topk, values):
+    """Rows whose k-th largest key is one of many equal ones, whole and swept, either side of the length up to which the radix select finishes them."""
+    g = torch.Generator().manual_seed(rows + s_kv + topk + values)
+    sc = torch.randint(0, values, (rows, s_kv), generator=g).float() - 0.3 * (values // 2)
+    assert torch.equal(topk_indices(sc.to(DEV), topk).cpu(), topk_indices_ref(sc, topk))
+
+
 @pytest.mark.parametrize("top", [0.0, 1e6, -1e6])
 def test_sample_that_misleads(top):
     """The sampled positions hold values unlike the rest: a bound that is too high, or a list that overflows, sends the row to the radix select."""

@@ -110,6 +110,16 @@ def _plan_paged(s_q: int, h: int, topk: int, pairs: int) -> Tuple[int, bool]:
     return max(_plan_splits(s_q, h, topk, pairs), min(parts, max(1, (topk + 127) // 128))), True
 
 
+def _table_is_faster(s_q: int, h: int, topk: int) -> bool:
+    """Whole tokens of the paged form: a table of converted rows first?
+
+    A few tokens with long lists leave most SMs idle, and a tile takes the kernel that converts while it gathers longer than the pairs of CTAs on a table
+    take for theirs; the table costs time with every row, though.  Gather / table, device us: 1 token of topk 2048, 16 / 32 / 64 / 128 heads 49 / 39,
+    56 / 39, 70 / 44, 70 / 50; 10 tokens 50 / 48, 56 / 48, 70 / 52, 70 / 59; 20 tokens 50 / 58, 56 / 59, 70 / 61, 70 / 70; 10 tokens of topk 1024
+    28 / 32, 32 / 31, 40 / 33, 40 / 38."""
+    return s_q <= (20 if 32 < h <= 64 else 10) and topk >= (2048 if h <= 16 else 1024) and s_q * topk <= 1 << 20
+
+
 def _split_workspace(a, s_q: int, h: int, n_splits: int, device):
     """Fills the split fields of the argument struct; returns the scratch tensor (kept alive by the caller)."""
     a.n_splits = n_splits
@@ -287,7 +297,8 @@ def sparse_mla_fwd_paged(q: torch.Tensor, kv_cache: torch.Tensor, kv_scale: torc
     test_accuracy_musa_vllm_mla.py:278-283.  Returns (out [B,n_q,h,512] bf16, lse [B,n_q,h] fp32).
 
     The rows are converted while they are gathered.  `two_pass`: convert the selected rows to a compact bf16 table first and run the
-    persistent bf16 kernels on it (needs 1156 bytes of scratch per selected row; a whole token then has the same bits).  With parts of a
+    persistent bf16 kernels on it (needs 1156 bytes of scratch per selected row; a whole token then has the same bits); None with
+    `num_splits=1`: where that is the faster form, for a few tokens with long lists.  With parts of a
     token, and with `two_pass` False, the weights follow the true maximum, otherwise a lazy one.
     """
     _require_cuda(q, kv_cache, kv_scale, block_table, context_lens, indices)
@@ -331,10 +342,12 @@ def sparse_mla_fwd_paged(q: torch.Tensor, kv_cache: torch.Tensor, kv_scale: torc
         block_table.data_ptr(), context_lens.data_ptr(), page_size, n_q, bt_stride)
     lib = _lib.load()
     if num_splits is None:
-        n_splits, rows_first = _plan_paged(s_q, h, topk, _pairs_of(device.index))
+        n_splits, lazy = _plan_paged(s_q, h, topk, _pairs_of(device.index))
     else:
         n_splits = max(1, int(num_splits))
-        rows_first = n_splits == 1
+        lazy = n_splits == 1
+        if two_pass is None and lazy:
+            two_pass = _table_is_faster(s_q, h, topk) or None
     rows_bytes = int(lib.ftb_sparse_mla_dequant_workspace_bytes(s_q, topk)) if two_pass else 0
     if rows_bytes > 0:
         # the dequantised rows, then (from a 16-byte boundary) the partial results of a split
@@ -344,7 +357,7 @@ def sparse_mla_fwd_paged(q: torch.Tensor, kv_cache: torch.Tensor, kv_scale: torc
         _ws = torch.empty(need, dtype=torch.uint8, device=device)
         a.n_splits, a.workspace, a.workspace_bytes, a.algo_id = n_splits, _ws.data_ptr(), need, 6
     else:
-        if two_pass is None and rows_first and n_splits == 1:
+        if two_pass is None and lazy and n_splits == 1:
             a.algo_id = 5                                    # many tokens, or told to keep them whole: the lazy maximum
         _ws = _split_workspace(a, s_q, h, n_splits, device)
     _launch(lib.ftb_sparse_mla_fwd, a, device, "sparse_mla_fwd_paged")

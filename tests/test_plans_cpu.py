@@ -70,3 +70,10 @@ def test_misaligned_split_workspace_is_refused(fp8):
     a.workspace, a.workspace_bytes = 4096 + 8, lib.ftb_sparse_mla_workspace_bytes(4, 16, 4)
     assert lib.ftb_sparse_mla_fwd(C.byref(a), None) == _lib.FTB_ERR_INVALID
     assert "aligned" in _lib.last_error()
+
+
+def test_whole_paged_tokens_take_a_table_where_it_is_the_faster_form():
+    assert ops._table_is_faster(1, 128, 2048) and ops._table_is_faster(20, 64, 1024) and ops._table_is_faster(10, 16, 2048)
+    assert not ops._table_is_faster(21, 64, 2048) and not ops._table_is_faster(11, 128, 2048) and not ops._table_is_faster(1, 128, 1023)
+    assert not ops._table_is_faster(1, 16, 1024) and not ops._table_is_faster(0, 128, 0)
+    assert not ops._table_is_faster(10, 128, 1 << 20)                     # 11 GB of scratch

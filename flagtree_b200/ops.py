@@ -120,13 +120,21 @@ def _table_is_faster(s_q: int, h: int, topk: int) -> bool:
     return s_q <= (20 if 32 < h <= 64 else 10) and topk >= (2048 if h <= 16 else 1024) and s_q * topk <= 1 << 20
 
 
+def _parts_bytes(s_q: int, h: int, n_splits: int) -> int:
+    return s_q * n_splits * h * (D_V + 1) * 4                # ftb_sparse_mla_workspace_bytes() of more than one part
+
+
+def _cand_bytes(num_pages: int) -> int:
+    return 4 * num_pages                                     # ftb_kv_cache_write_workspace_bytes()
+
+
 def _split_workspace(a, s_q: int, h: int, n_splits: int, device):
     """Fills the split fields of the argument struct; returns the scratch tensor (kept alive by the caller)."""
     a.n_splits = n_splits
     if n_splits <= 1:
         a.workspace, a.workspace_bytes = None, 0
         return None
-    nbytes = s_q * n_splits * h * (D_V + 1) * 4              # ftb_sparse_mla_workspace_bytes()
+    nbytes = _parts_bytes(s_q, h, n_splits)
     ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
     a.workspace, a.workspace_bytes = ws.data_ptr(), nbytes
     return ws
@@ -477,7 +485,7 @@ def kv_cache_write_fp8(rows: torch.Tensor, slot_mapping: torch.Tensor, kv_cache:
     assert kv_cache.dtype in (torch.uint8, torch.float8_e4m3fn) and kv_cache.is_contiguous()
     assert rows_per_page == page_size and d == D_QK
     assert kv_scale.dtype == torch.float32 and kv_scale.shape == (num_pages,) and kv_scale.is_contiguous()
-    ws_bytes = 4 * num_pages                                 # ftb_kv_cache_write_workspace_bytes()
+    ws_bytes = _cand_bytes(num_pages)
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=device)
     status = torch.zeros(1, dtype=torch.int32, device=device) if check else None
     a = _lib.KvCacheWriteArgs(rows.data_ptr(), slot_mapping.data_ptr(), kv_cache.data_ptr(), kv_scale.data_ptr(), n,

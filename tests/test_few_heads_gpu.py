@@ -5,6 +5,8 @@ kernel for many heads on the same inputs."""
 import pytest
 import torch
 
+from conftest import paged_algo
+
 pytestmark = pytest.mark.gpu
 
 if torch.cuda.is_available():
@@ -146,28 +148,6 @@ def test_paged_rows_converted_in_the_gather(h, batch, n_q, topk, page):
         assert ((l[fin] - ref_lse[fin]).abs() <= 1e-5 * ref_lse[fin].abs().clamp(min=1)).all()
 
 
-def _paged_algo(args, sm_scale, page_size, algo, splits):
-    """The paged form through the C ABI, with a kernel and a number of parts of the caller's choice."""
-    import ctypes as C
-    from flagtree_b200 import _lib
-    q, cache, scale, table, lens, idx = args
-    b, n_q, h, _ = q.shape
-    topk = idx.shape[2]
-    lib = _lib.load()
-    out = torch.empty(b, n_q, h, 512, dtype=torch.bfloat16, device=DEV)
-    lse = torch.empty(b, n_q, h, dtype=torch.float32, device=DEV)
-    status = torch.zeros(1, dtype=torch.int32, device=DEV)
-    a = _lib.SparseMlaArgs(q.data_ptr(), cache.data_ptr(), idx.data_ptr(), out.data_ptr(), lse.data_ptr(), b * n_q, h, cache.shape[0] * page_size,
-                           topk, h * 576, 576, 576, topk, h * 512, 512, h, sm_scale, 0, algo, status.data_ptr(), 1, scale.data_ptr(),
-                           table.data_ptr(), lens.data_ptr(), page_size, n_q, table.stride(0))
-    ws = torch.empty(max(1, lib.ftb_sparse_mla_workspace_bytes(b * n_q, h, splits)), dtype=torch.uint8, device=DEV)
-    a.n_splits, a.workspace, a.workspace_bytes = splits, ws.data_ptr(), ws.numel()
-    assert lib.ftb_sparse_mla_fwd(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0, _lib.last_error()
-    torch.cuda.synchronize()
-    assert status.item() == 0
-    return out, lse
-
-
 @pytest.mark.parametrize("h", [16, 64, 128])
 @pytest.mark.parametrize("batch,topk,splits", [(3, 2048, 16), (2, 512, 8), (5, 300, 3), (4, 130, 1), (1, 1000, 40)])
 def test_paged_parts_have_the_weights_of_the_one_cta_kernel(h, batch, topk, splits):
@@ -177,8 +157,8 @@ def test_paged_parts_have_the_weights_of_the_one_cta_kernel(h, batch, topk, spli
     by their weights' 4e-6 of what they add up)."""
     c = W.mla_cfg3(batch=batch, n_q=1, h=h, topk=topk, len_lo=600, len_hi=4000)
     args = [t.to(DEV) for t in (c.q, c.kv_cache, c.kv_scale, c.block_table, c.context_lens, c.indices)]
-    out, lse = _paged_algo(args, c.sm_scale, c.page_size, 0, splits)
-    ref_out, ref_lse = _paged_algo(args, c.sm_scale, c.page_size, 1, splits)
+    out, lse = paged_algo(args, c.sm_scale, c.page_size, 0, splits)
+    ref_out, ref_lse = paged_algo(args, c.sm_scale, c.page_size, 1, splits)
     o, r = out.float(), ref_out.float()
     assert ((o - r).abs() <= 2 ** -7 * r.abs() + 2e-5 * r.abs().max()).all()
     assert (o != r).float().mean().item() < 0.01
@@ -191,6 +171,6 @@ def test_paged_parts_of_algo_5_take_the_true_maximum_too(h, topk, splits):
     c = W.mla_cfg3(batch=3, n_q=1, h=h, topk=topk, len_lo=800, len_hi=2000)
     c.kv_scale.mul_(torch.linspace(0.5, 4.0, c.kv_scale.numel()))
     args = [t.to(DEV) for t in (c.q, c.kv_cache, c.kv_scale, c.block_table, c.context_lens, c.indices.sort(dim=2).values)]
-    ref = _paged_algo(args, c.sm_scale, c.page_size, 0, splits)
-    got = _paged_algo(args, c.sm_scale, c.page_size, 5, splits)
+    ref = paged_algo(args, c.sm_scale, c.page_size, 0, splits)
+    got = paged_algo(args, c.sm_scale, c.page_size, 5, splits)
     assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])

@@ -81,11 +81,12 @@ def _check_fp8(m, n, k, nk):
 
 
 # One shape or two per route of the dispatch on 148 SMs: (columns of a tile, CTAs that share it, parts of K).
-ROUTES = {(128, 1, 1): [(60, 2048, 1024), (130, 512, 1024)], (128, 1, 2): [(40, 8192, 7168)], (128, 1, 4): [(33, 3968, 4096)], (128, 1, 8): [(64, 1024, 7168)],
+ROUTES = {(64, 1, 1): [(60, 2048, 1024), (130, 512, 1024)], (64, 1, 4): [(64, 2048, 7168)], (128, 1, 1): [(128, 9600, 384)], (128, 1, 2): [(40, 8192, 7168)],
+          (128, 1, 4): [(33, 3968, 4096)], (128, 1, 8): [(64, 1024, 7168)],
           (256, 2, 1): [(1025, 2176, 384), (1030, 3200, 1664)], (256, 2, 2): [(142, 4608, 13824), (162, 4224, 10240), (395, 2304, 15616)]}
 
 
-# The same after few single tiles have been halved to 64 columns: both sides of that line, some with an odd count of K blocks.
+# Where few single tiles are halved to 64 columns: both sides of that line, some with an odd count of K blocks.
 ROUTES_HALVED = {(64, 1, 1): [(60, 2048, 1024), (1, 128, 384), (128, 9472, 384), (257, 3072, 640)], (64, 1, 4): [(64, 2048, 7168), (100, 1920, 3456)],
                  (128, 1, 1): [(128, 9600, 384)], (128, 1, 4): [(33, 3968, 4096)], (128, 1, 8): [(64, 1920, 7168)]}
 

@@ -15,7 +15,7 @@ def _plan(fp8, m, n, k, sms=148):
     return tuple(plan)
 
 
-@pytest.mark.parametrize("fp8,routes", [(0, test_gemm_gpu.ROUTES), (1, test_gemm_fp8_gpu.ROUTES)])
+@pytest.mark.parametrize("fp8,routes", [(0, test_gemm_gpu.ROUTES), (2, test_gemm_fp8_gpu.ROUTES)])
 def test_gpu_tests_reach_every_route(fp8, routes):
     for route, shapes in routes.items():
         for m, n, k in shapes:
@@ -77,3 +77,12 @@ def test_whole_paged_tokens_take_a_table_where_it_is_the_faster_form():
     assert not ops._table_is_faster(21, 64, 2048) and not ops._table_is_faster(11, 128, 2048) and not ops._table_is_faster(1, 128, 1023)
     assert not ops._table_is_faster(1, 16, 1024) and not ops._table_is_faster(0, 128, 0)
     assert not ops._table_is_faster(10, 128, 1 << 20)                     # 11 GB of scratch
+
+
+def test_scratch_that_the_entry_points_allocate_is_what_the_library_asks_for():
+    """The entry points work the sizes out themselves; the library refuses less."""
+    lib = _lib.load()
+    for s_q, h, n in ((1, 1, 2), (3, 128, 16), (300, 64, 2), (7, 17, 64)):
+        assert ops._parts_bytes(s_q, h, n) == lib.ftb_sparse_mla_workspace_bytes(s_q, h, n)
+    for pages in (1, 37, 4096):
+        assert ops._cand_bytes(pages) == lib.ftb_kv_cache_write_workspace_bytes(pages)

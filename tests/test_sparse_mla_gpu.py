@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 import torch
 
-from conftest import GOLDEN_DIR, LSE_RTOL, OUT_ATOL
+from conftest import GOLDEN_DIR, LSE_RTOL, OUT_ATOL, paged_algo
 
 pytestmark = pytest.mark.gpu
 
@@ -236,17 +236,16 @@ def test_full_size_prefill_sampled_tokens():
 
 def test_full_size_decode_fp8_sampled_sequences():
     """cfg3 at full size (64 sequences x 2 query tokens, h = 128, topk = 2048, paged FP8 cache with contexts of
-    8192..65536 tokens): every output is produced on the GPU by the default path (selected rows dequantised
-    once, then the persistent kernel); three sequences are cut out with their own pages and compared with
-    the CPU oracle; the one-pass kernel must agree on all of them."""
+    8192..65536 tokens): every output is produced on the GPU by the default path (rows converted while they are gathered);
+    three sequences are cut out with their own pages and compared with the CPU oracle; the one-CTA kernel, which shares no code with it,
+    and the form that converts the selected rows to a table first must agree on all of them."""
     c = W.mla_cfg3(device=DEV)
     args = (c.q, c.kv_cache, c.kv_scale, c.block_table, c.context_lens, c.indices, c.sm_scale)
-    out, lse = sparse_mla_fwd_paged(*args, page_size=c.page_size, check=True)                 # two passes
-    out1, lse1 = sparse_mla_fwd_paged(*args, page_size=c.page_size, check=True, num_splits=1, two_pass=False)
-    torch.cuda.synchronize()
+    out, lse = sparse_mla_fwd_paged(*args, page_size=c.page_size, check=True)
     assert torch.isfinite(out.float()).all() and torch.isfinite(lse).all()
-    assert (out.float() - out1.float()).abs().max().item() <= OUT_ATOL
-    assert ((lse - lse1).abs() / lse1.abs().clamp(min=1)).max().item() <= LSE_RTOL
+    for out1, lse1 in (paged_algo(args[:6], c.sm_scale, c.page_size, 1, 1), sparse_mla_fwd_paged(*args, page_size=c.page_size, check=True, two_pass=True)):
+        assert (out.float() - out1.float()).abs().max().item() <= OUT_ATOL
+        assert ((lse - lse1).abs() / lse1.abs().clamp(min=1)).max().item() <= LSE_RTOL
     for b in (0, 17, 63):
         n_pages = (int(c.context_lens[b]) + c.page_size - 1) // c.page_size
         pages = c.block_table[b, :n_pages].long()
@@ -317,12 +316,18 @@ def test_decode_attention_fwd_shim_matches_reference_signature():
     assert (o.float().cpu() - torch.from_numpy(d["out"]).float()).abs().max().item() <= OUT_ATOL
 
 
-@pytest.mark.parametrize("two_pass", [False, True], ids=["one_pass", "dequant_then_persistent"])
-def test_paged_fp8_decode_scaled_down(two_pass):
+def _paged_form(c, form):
+    """A whole-token result of the kernel that converts while it gathers, of the persistent kernels on a converted table, or of the one-CTA kernel."""
+    args = [t.to(DEV) for t in (c.q, c.kv_cache, c.kv_scale, c.block_table, c.context_lens, c.indices)]
+    if form == "one_cta":
+        return paged_algo(args, c.sm_scale, c.page_size, 1, 1)
+    return sparse_mla_fwd_paged(*args, c.sm_scale, page_size=c.page_size, check=True, num_splits=1, two_pass=form == "table")
+
+
+@pytest.mark.parametrize("form", ["gather", "table", "one_cta"])
+def test_paged_fp8_decode_scaled_down(form):
     c = W.mla_cfg3(batch=4, n_q=2, h=128, topk=256, len_lo=300, len_hi=1500)
-    out, lse = sparse_mla_fwd_paged(c.q.to(DEV), c.kv_cache.to(DEV), c.kv_scale.to(DEV), c.block_table.to(DEV),
-                                    c.context_lens.to(DEV), c.indices.to(DEV), c.sm_scale, page_size=c.page_size,
-                                    check=True, num_splits=1, two_pass=two_pass)
+    out, lse = _paged_form(c, form)
     ref_out, ref_lse = sparse_mla_fwd_paged_ref(c.q, c.kv_cache, c.kv_scale, c.block_table, c.context_lens,
                                                 c.indices, c.sm_scale, page_size=c.page_size)
     e_out, e_lse = _errors(out, lse, ref_out, ref_lse)
@@ -330,12 +335,10 @@ def test_paged_fp8_decode_scaled_down(two_pass):
     assert e_out <= OUT_ATOL and e_lse <= LSE_RTOL
 
 
-@pytest.mark.parametrize("two_pass", [False, True], ids=["one_pass", "dequant_then_persistent"])
-def test_paged_fp8_short_context_and_padding(two_pass):
+@pytest.mark.parametrize("form", ["gather", "table", "one_cta"])
+def test_paged_fp8_short_context_and_padding(form):
     c = W.mla_cfg3(batch=3, n_q=2, h=16, topk=128, len_lo=20, len_hi=100)   # topk > context: -1 padded
-    out, lse = sparse_mla_fwd_paged(c.q.to(DEV), c.kv_cache.to(DEV), c.kv_scale.to(DEV), c.block_table.to(DEV),
-                                    c.context_lens.to(DEV), c.indices.to(DEV), c.sm_scale, page_size=c.page_size,
-                                    check=True, num_splits=1, two_pass=two_pass)
+    out, lse = _paged_form(c, form)
     ref_out, ref_lse = sparse_mla_fwd_paged_ref(c.q, c.kv_cache, c.kv_scale, c.block_table, c.context_lens,
                                                 c.indices, c.sm_scale, page_size=c.page_size)
     e_out, e_lse = _errors(out, lse, ref_out, ref_lse)
@@ -458,14 +461,14 @@ def test_parts_of_a_token_on_the_persistent_pairs(s_q, h, topk, splits):
     assert torch.allclose(lse2.cpu() * 0.6931471805599453, lse.cpu(), rtol=1e-5, atol=1e-5)
 
 
-@pytest.mark.parametrize("splits,two_pass", [(1, True), (4, True), (4, False), (None, None)])
+@pytest.mark.parametrize("splits,two_pass", [(1, True), (1, False), (1, None), (4, True), (4, False), (None, None)])
 def test_paged_forms_agree(splits, two_pass):
-    """Two passes and parts of a token against the one-pass kernel on whole tokens; short contexts leave parts empty.  All forms
+    """Whole tokens and parts of them, with and without a table of converted rows, against the one-CTA kernel on whole tokens; short contexts leave parts empty.  All forms
     multiply the same rows rounded to bf16, with fp32 sums in another order: the LSE agrees to some 1e-5, the output to
     roundings of P and of the result (2^-9 each, of values up to 1)."""
     c = W.mla_cfg3(batch=3, n_q=2, h=64, topk=300, len_lo=40, len_hi=900)
     args = (c.q.to(DEV), c.kv_cache.to(DEV), c.kv_scale.to(DEV), c.block_table.to(DEV), c.context_lens.to(DEV), c.indices.to(DEV), c.sm_scale)
-    ref_out, ref_lse = sparse_mla_fwd_paged(*args, page_size=c.page_size, check=True, num_splits=1, two_pass=False)
+    ref_out, ref_lse = paged_algo(args[:6], c.sm_scale, c.page_size, 1, 1)
     out, lse = sparse_mla_fwd_paged(*args, page_size=c.page_size, check=True, num_splits=splits, two_pass=two_pass)
     assert (out.float() - ref_out.float()).abs().max().item() <= 1e-2
     assert ((lse - ref_lse).abs() / ref_lse.abs().clamp(min=1)).max().item() <= 1e-4

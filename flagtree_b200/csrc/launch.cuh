@@ -4,10 +4,11 @@
 // griddep_wait() in all of its threads before its first access to global memory, which returns when the kernels
 // before it have completed and their writes are visible.  Back to back (us, before / now): 50 x 7168 x 2304 bf16
 // 12.3 / 10.1, 64 x 8192 x 3584 e4m3 14.6 / 13.1, one token of 128 heads in parts (two launches) 18.5 / 16.9, a decode step of three
-// sequences (four launches) 45.1 / 40.2, 262 144 cache rows (five launches) 120.4 / 116.7.
+// sequences (four launches) 45.1 / 40.2, 262 144 cache rows (five launches) 116.7 / 113.3.
 // Where griddep_launch() stands: first, unless the CTAs of a kernel have several items of work and end at different times; those execute
 // it last.  The next kernel's CTAs would otherwise crowd on the SMs that are through first and stay there: with a persistent kernel that let
-// the next step's top-k kernel in early, a decode step of 128 tokens took 186 us, without any overlap 179, now 178.  For the same reason a
+// the next step's top-k kernel in early, a decode step of 128 tokens took 186 us, without any overlap 179, now 178.  For the same reason the cache
+// writer's run kernel lets its successor in late where that one has much to do (kv_cache.cu), the bf16 GEMM leaves few rows on few SMs out (gemm.cu), and a
 // kernel of few large CTAs asks for more than half of an SM's shared memory.
 #pragma once
 #include <cuda_runtime.h>

@@ -290,6 +290,32 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// the same value in every lane, made visible to the compiler: loop counts and role state then stay in uniform registers
+__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+// does the predicate hold for any of the threads of the barrier?
+__device__ __forceinline__ bool named_bar_any(int id, int nthreads, bool pred) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %3, 0;\n\t"
+      "bar.red.or.pred q, %1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r) : "r"(id), "r"(nthreads), "r"(pred ? 1u : 0u) : "memory");
+  return r != 0u;
+}
+// two fp32 lanes per instruction
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
+      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+
 // A warp writes 32 rows of 8 P columns of a row-major bf16 matrix, of which lane l has row l in registers: `piece(ch)` gives columns 8 ch .. of it.
 // They turn round in `box` (512 P bytes of shared memory, the warp's own), so that P lanes write 16 P bytes of a row: stored straight
 // from the registers every 16-byte piece is a line of its own.  (row0, col0): the first element; rows and columns from

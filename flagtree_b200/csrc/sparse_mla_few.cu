@@ -1,4 +1,4 @@
-// Sparse MLA forward for few heads (and for few tokens of many heads, 64 at a time), sm_100a: persistent CTAs, the products taken
+// Sparse MLA forward for few heads (and for few tokens or short lists of many heads, 64 at a time), sm_100a: persistent CTAs, the products taken
 // the other way round.
 //
 // The CTA pairs of sparse_mla_ring.cu put the heads on the 128 rows of the MMA, so with 16 heads seven eighths of every
@@ -24,7 +24,7 @@
 // P^T [64 keys x NH] is written over the rope block of the tile, which the second
 // product does not read.
 //
-// The steps (1999 tokens of 16 / 64 heads, topk 2048, us; the pairs take 846 / 958): one issuer that polls for both products 620 / 813, with
+// The steps (1999 tokens of 16 / 64 heads, topk 2048, us; the pairs take 970 / 958, with the softmax of later steps 846 with 16 heads): one issuer that polls for both products 620 / 813, with
 // tiles in thirds and 16 rows freed at a time 780 / 974 (each turn of the issuer cost 330 cycles, most of it the proxy fence), the fence
 // moved to the gather warps 741 / 920, two issuers 512 / 719, the first reference from two tiles 525 / 759.  Device time of few tokens in parts,
 // pairs / here: 1 token of 16 heads 17.0 / 11.3, 74 tokens of 64 heads 45.6 / 40.0, 1 token of 128 heads 21.2 / 14.7, 16 of them 29.9 / 25.5.
@@ -131,36 +131,12 @@ struct Misc {
   float part[8][32], part_odd[8][32];  // per softmax warp and head: maxima, then sums of the even and the odd tiles
 };
 
-__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
-__device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-// does the predicate hold for any of the threads of the barrier?
-__device__ __forceinline__ bool named_bar_any(int id, int nthreads, bool pred) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %3, 0;\n\t"
-      "bar.red.or.pred q, %1, %2, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(r) : "r"(id), "r"(nthreads), "r"(pred ? 1u : 0u) : "memory");
-  return r != 0u;
-}
 // floats <-> integers whose signed order is the order of the floats
 __device__ __forceinline__ int to_ordered(float x) {
   const int i = __float_as_int(x);
   return i >= 0 ? i : i ^ 0x7fffffff;
 }
 __device__ __forceinline__ float from_ordered(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
-// two fp32 lanes per instruction
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
-  float2 r;
-  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
-      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
-      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return r;
-}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "

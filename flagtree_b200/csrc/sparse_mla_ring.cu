@@ -144,22 +144,6 @@ static_assert(sizeof(Misc0) <= 4096 && sizeof(Misc1) <= 4096, "misc area");
 static_assert(kOff0Misc + 4096 + 1024 <= kSmemBytes, "CTA 0 layout fits");
 static_assert(kNV == kNT / kVSlabRows, "V ring slot index = slab index");
 
-// the same value in every lane, made visible to the compiler: loop counts and role state then stay in uniform registers
-__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
-__device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-// does the predicate hold for any of the threads of the barrier?
-__device__ __forceinline__ bool named_bar_any(int id, int nthreads, bool pred) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %3, 0;\n\t"
-      "bar.red.or.pred q, %1, %2, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(r) : "r"(id), "r"(nthreads), "r"(pred ? 1u : 0u) : "memory");
-  return r != 0u;
-}
 __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
@@ -183,15 +167,7 @@ __device__ __forceinline__ void tmem_cp_128x256b(uint32_t taddr, uint32_t desc_l
       ::"r"(taddr), "r"(desc_lo), "r"(desc_hi)
       : "memory");
 }
-// two fp32 lanes per instruction
-__device__ __forceinline__ float2 ffma2(float a0, float a1, float2 b, float2 c) {
-  float2 r;
-  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
-      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
-      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-      : "=f"(r.x), "=f"(r.y) : "f"(a0), "f"(a1), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return r;
-}
+// two fp32 lanes per instruction (ffma2: sm100.cuh)
 __device__ __forceinline__ float2 fmul2(float2 a, float b) {
   float2 r;
   asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
@@ -485,7 +461,7 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
                 float2 e[8];
 #pragma unroll
                 for (int j = 0; j < 16; j += 2) {
-                  const float2 x = ffma2(__uint_as_float(sr[q][16 * g + j]), __uint_as_float(sr[q][16 * g + j + 1]), scale2, neg_m2);
+                  const float2 x = ffma2(make_float2(__uint_as_float(sr[q][16 * g + j]), __uint_as_float(sr[q][16 * g + j + 1])), scale2, neg_m2);
                   e[j >> 1] = make_float2(fast_exp2(x.x), fast_exp2(x.y));
                   pk[q][8 * g + (j >> 1)] = pack_bf16x2(e[j >> 1].x, e[j >> 1].y);
                 }

@@ -198,7 +198,8 @@ __global__ void __launch_bounds__(kThreads) topk_select_kernel(const Params p) {
 // Against persistent CTAs that hold a row in registers and histogram it (us, before / now): 4096 x 32 768 causal 334 / 205, 4096 x 20 001
 // topk 1024 426 / 120, 4096 x 6000 277 / 98, 4096 x 4000 topk 512 189 / 65, 4096 x 1000 topk 512 83 / 51, 592 rows of 33 000 82 / 36,
 // 592 rows of 32 768 equal scores 52 / 40, 128 rows of up to 65 536 30 / 17, 300 short rows of a matrix of 65 536 columns 44 / 16, one row of
-// 32 768 13.1 / 11.5, of 4000 11.2 / 7.8; level or up to 8 % slower: rows of 32 768 with topk 4096 and more (148: 14.9 / 15.5, 4096 with 16 384: 588 / 648).
+// 32 768 13.1 / 11.5, of 4000 11.2 / 7.8; level or up to 10 % slower: rows of 32 768 with topk 4096 and more (148: 14.9 / 15.5, 4096
+// with 16 384: 588 / 648), 30 % short rows of some ten values (1024 rows of 1000, topk 333: 27 / 35).
 // ---------------------------------------------------------------------------------------------------------------
 namespace listed {
 

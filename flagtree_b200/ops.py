@@ -64,7 +64,8 @@ def _plan_splits(s_q: int, h: int, topk: int, pairs: int) -> int:
         waves = -(-s_q * n // pairs)
         return 12.0 + waves * (2.0 + 2.2 * -(-tiles // n)) + (5.4 + 0.2 * s_q * n * h / 128 if n > 1 else 0.0)
 
-    # one CTA per item of up to 64 heads: the library takes that kernel for more heads while every CTA has one item of at most 16 tiles
+    # one CTA per item of up to 64 heads, more in groups of 64 while every CTA has one item of at most 16 tiles (an estimate: the library then takes
+    # the kernel that its own, finer model says is the faster one)
     groups, rows64 = -(-h // 64), max(1, (topk + 63) // 64)
     start, per_tile = (6.0, 1.03) if h <= 16 else (8.0, 1.13) if h <= 32 else (8.6, 1.4)
 

@@ -67,9 +67,9 @@ typedef struct ftb_sparse_mla_args {
   int32_t lse_base2;        /* 0: lse = log sum exp(s);  1: log2 sum 2^(s*log2 e)            */
   int32_t algo_id;          /* 0 = default; 1 = one CTA per (token, output half); 2 = the kernel for few
                                heads with the true maximum (h <= 32, bf16 form without splits); 5 = the
-                               persistent kernels with the lazy maximum: up to 64 heads, and few tokens of
-                               more, on single CTAs, else on CTA pairs (0 = 5 for whole tokens of the bf16
-                               form); 6 = paged FP8 form only: convert the selected rows to a table, then the
+                               persistent kernels with the lazy maximum, on single CTAs of up to 64 heads
+                               or on CTA pairs, whichever a model of their times says (0 = 5 for whole
+                               tokens of the bf16 form); 6 = paged FP8 form only: convert the selected rows to a table, then the
                                persistent kernels                                                */
   int32_t* status;          /* optional device int32: kernels OR-in a non-zero FTB_ERR_* code */
   /* Paged FP8 form (kv_is_fp8 != 0): physical row = block_table[seq, p / page] * page + p % page,

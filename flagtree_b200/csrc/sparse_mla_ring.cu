@@ -422,7 +422,6 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
             // With slack the first tile sets it as a whole; later the two halves of a tile (64 rows: the tile of the kernel for few heads) move
             // it one after the other, and the sums below add in that kernel's order: the bits of a whole token's head do not depend on
             // how many heads the call has.
-            const bool as_a_whole = i == 0 || p.max_slack == 0.0f;
             auto move_to = [&](float top) {
               const float m_cand = fmaxf(m_run, top * p.scale_log2);
               float a = 1.0f;
@@ -439,9 +438,10 @@ sparse_mla_ring_kernel(const __grid_constant__ CUtensorMap tm_q,
               m0->xchg[b][tid] = mx;
               named_bar_sync(2 + (warp & 3), 64);
               const float other = m0->xchg[b][tid ^ 128];
-              alpha_a = move_to(as_a_whole ? fmaxf(mx, other) : ch == 0 ? mx : other);
+              if (p.max_slack == 0.0f) mx = fmaxf(mx, other);
+              alpha_a = move_to(i == 0 ? fmaxf(mx, other) : p.max_slack == 0.0f || ch == 0 ? mx : other);
               m_mine = m_run;
-              if (!as_a_whole) alpha_b = move_to(ch == 0 ? other : mx);
+              if (i != 0 && p.max_slack != 0.0f) alpha_b = move_to(ch == 0 ? other : mx);
               if (ch != 0) m_mine = m_run;
               l01 = fmul2(l01, alpha_a);
               l23 = fmul2(l23, alpha_a);

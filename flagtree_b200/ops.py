@@ -77,9 +77,10 @@ def _plan_splits(s_q: int, h: int, topk: int, pairs: int) -> int:
 
     def cost(n):
         device = pairs_cost(n) if h > 64 and ctas_cost(n) == math.inf else ctas_cost(n)
-        return max(device, 21.5 if n > 1 else 16.0), device      # calls in a row take at least what the host needs: one launch, or two and a workspace
+        # calls in a row take at least what the host needs: two launches and a workspace, or one launch (not counted for few tokens: see below)
+        return max(device, 16.5 if n > 1 or s_q <= 15 else 12.0), device
 
-    return min(range(1, min(16, tiles) + 1), key=cost)
+    return min(range(1, (min(16, tiles) if tiles > 3 else 1) + 1), key=cost)
 
 
 def _auto_splits(s_q: int, h: int, topk: int, device) -> int:
@@ -89,8 +90,10 @@ def _auto_splits(s_q: int, h: int, topk: int, device) -> int:
     there are SMs for it as an item per 64 heads.  Measured on a B200 (device us, in a captured graph).  An SM: 7 per launch, 1 per item
     and 1.03 per tile of 64 rows in it with 16 heads (9 and 1.4 with 64), with parts 1 for the merge and 0.35 per 1000 fp32 rows of 512; topk 2048,
     16 heads, whole / in parts: 1 token 40 / 10.6 (16 parts), 16 tokens 40.5 / 13.3 (8), 74 tokens 41 / 26 (2), 148 tokens 42 / 45.  A pair: 12 per
-    launch, 2 per item, 2.2 per tile of 128 rows; with parts 5.4 and 0.2 per item.  The host takes 16 for a call with one launch and
-    21.5 for one in parts, so that lists which an SM is through with by then stay whole (1 token of topk 256: 16 against 22)."""
+    launch, 2 per item, 2.2 per tile of 128 rows; with parts 5.4 and 0.2 per item.  The host takes 16.5 for a call in parts
+    (12 for one launch), so that lists of up to three tiles of 128, which an SM is through with by then, stay whole (1 token of topk 256: 12 against 16.5).  Longer
+    ones of up to fifteen tokens do not, although 512 entries of 16 heads would be 1.5 faster whole: the largest weight of every part is exactly 1 in bf16, and 1 token of topk 512 is
+    1.75e-3 from the 64-bit result in four parts, 2.1e-3 whole."""
     return _plan_splits(s_q, h, topk, _pairs_of(device.index))
 
 

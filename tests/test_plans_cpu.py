@@ -72,6 +72,17 @@ def test_misaligned_split_workspace_is_refused(fp8):
     assert "aligned" in _lib.last_error()
 
 
+def test_few_tokens_with_lists_of_more_than_three_tiles_are_cut_in_parts():
+    """The parts are not for speed alone: every one has a weight of exactly 1."""
+    for h in (16, 32, 64, 128):
+        for s_q in (1, 2, 5, 8):
+            assert [ops._plan_splits(s_q, h, topk, 74) for topk in (1, 128, 384)] == [1, 1, 1]
+            for topk in (385, 512, 640, 768):
+                assert ops._plan_splits(s_q, h, topk, 74) == -(-topk // 128)
+        assert ops._plan_splits(16, h, 768, 74) >= 3
+    assert ops._plan_splits(0, 128, 2048, 74) >= 1                        # no token: nothing to divide by
+
+
 def test_whole_paged_tokens_take_a_table_where_it_is_the_faster_form():
     assert ops._table_is_faster(1, 128, 2048) and ops._table_is_faster(20, 64, 1024) and ops._table_is_faster(10, 16, 2048)
     assert not ops._table_is_faster(21, 64, 2048) and not ops._table_is_faster(11, 128, 2048) and not ops._table_is_faster(1, 128, 1023)
